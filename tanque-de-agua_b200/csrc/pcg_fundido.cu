@@ -51,8 +51,14 @@ constexpr size_t SMEM_CTA_MAX = 227 * 1024 - 2048;  // dynamic shared memory cap
 // grid-wide matrix-vector product per V-cycle, instead of CTA 0 running the section alone.
 constexpr int SECAO_DENSA_MAX = 2048;
 constexpr int SECAO_DENSA_MIN_ITERS = 30;
-// The coarsest level's sweeps run on one warp up to this many cells, on every warp of CTA 0 above.
-constexpr int GROSSO_UM_WARP = 1024;
+// The build runs up to SECAO_EQUIPES teams of warps a CTA, a column each, and takes from a column's top
+// level only the blocks its unit vector reaches (secaoGrossa): 370 -> 215 us a solve on the 480x270
+// scene, 205 -> 145 us on the 840x536 scene, 15.8 -> 2.7 ms on a 256x92 tank atlas with 4 CTAs.
+constexpr int SECAO_EQUIPES = 3;
+// A section has at most 5 levels: they halve while both sides exceed 12, from SECAO_MAX_CELULAS cells.
+constexpr int SECAO_NIVEIS = 6;
+// The coarsest level's sweeps hold their cells in registers, up to GROSSO_REG a colour and thread.
+constexpr int GROSSO_REG = 4;
 constexpr int NPARC = 4;                           // partial slots per CTA
 // Tolerance mode replaces the recursive FP32 residual by the true one (FP64) each time the
 // recursive one has fallen by this factor since the last replacement: the rounding it gathers,
@@ -101,9 +107,10 @@ struct Fundido {
   float *xc = nullptr, *bc = nullptr;
   int offDenso = -1;  // byte offset of the coarsest level's matrix in CTA 0's shared memory
   bool secaoDensa = false;  // the section's matrix can be built (buffers below allocated)
+  int equipes = 1, bytesSecao = 0;  // Args::equipes, Args::bytesSecao
   float* mSecao = nullptr;   // nW x nW, row i = water cell i of level Lc
   int *wSecao = nullptr, *wInv = nullptr, *nW = nullptr;  // water cells of level Lc, cell -> row, count
-  unsigned* densoG = nullptr;  // the coarsest level's matrix block, copied from CTA 0 to every CTA
+  unsigned* densoG = nullptr;  // the coarsest level's matrix, list and header, copied to the CTAs that use it
   uint16_t* op = nullptr;
   unsigned long long* rotB = nullptr;
   void* kern = nullptr;
@@ -143,6 +150,7 @@ struct Args {
   float *xc, *bc;
   int offDenso;  // coarsest-level matrix in CTA 0's dynamic shared memory (-1: sweeps)
   int secaoDensa;  // 1: the section may be replaced by its matrix
+  int equipes, bytesSecao;  // teams of a CTA that build its columns, and the shared bytes of each
   float* mSecao;
   int *wSecao, *wInv, *nWp;
   unsigned* densoG;
@@ -966,16 +974,29 @@ struct NivelS {
   int v;          // byte offset
 };
 
-// One smoother pass over a level held in shared memory: the level's 16x16 blocks are taken in
-// turn by the CTA's warps, each sweeping its block in registers (varrerReg) from the snapshot
-// `src` and writing `dst`.
+// The threads that run a coarse section together: the CTA, or one of a.equipes teams of whole
+// warps (named barrier 1 + id), thread ti of nt.
+struct Equipe {
+  int ti, nt, id;
+};
+__device__ __forceinline__ void sincEquipe(const Equipe& q) {
+  if (q.nt == TF) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"r"(q.id + 1), "r"(q.nt) : "memory");
+}
+
+// One smoother pass over a level held in shared memory: the level's 16x16 blocks (those of the
+// rectangle r of block coordinates) are taken in turn by the team's warps, each sweeping its
+// block in registers (varrerReg) from the snapshot `src` and writing `dst`.
+struct Ret {
+  int x0, y0, x1, y1;  // inclusive
+};
 __device__ void passoS(float* F, const uint8_t* U, const NivelS n, int desl, int ordem, int src, int dst, bool masc,
-                       int nVarr) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gl = lane >> 3, k = lane & 7;
+                       int nVarr, const Equipe& eq, const Ret& r) {
+  const int lane = threadIdx.x & 31, w = eq.ti >> 5, gl = lane >> 3, k = lane & 7;
   const int nx = n.nx, ny = n.ny;
-  const int nbx = (nx + desl + 15) >> 4, nby = (ny + desl + 15) >> 4;
-  for (int blk = w; blk < nbx * nby; blk += WARPS) {
-    const int ox = (blk % nbx) * 16 - desl, oy = (blk / nbx) * 16 - desl;
+  const int nbr = r.x1 - r.x0 + 1;
+  for (int b = w; b < nbr * (r.y1 - r.y0 + 1); b += eq.nt >> 5) {
+    const int ox = (r.x0 + b % nbr) * 16 - desl, oy = (r.y0 + b / nbr) * 16 - desl;
     float x[2][4], bq[2][4];  // [colour][m], see meiaReg
     int v[2][4], cel[2][4];
     Moldura f;
@@ -1014,15 +1035,14 @@ __device__ void passoS(float* F, const uint8_t* U, const NivelS n, int desl, int
       for (int m = 0; m < 4; m++)
         if (cel[cr][m] >= 0) F[dst + cel[cr][m]] = (v[cr][m] & 16) ? x[cr][m] : 0.0f;
   }
-  __syncthreads();
+  sincEquipe(eq);
 }
 
 // The coarsest solve (resolverGrosso, js/pressao-cpu.js:217-238) is VARREDURAS_GROSSO
 // red-black sweeps from x = 0: a linear map of the right side, fixed for the whole PCG solve
-// because the cell types are.  CTA 0 builds that map once per solve: column j is the sweeps
-// applied to b = e_j, every thread of the first nL sweeping its own column (stored at
-// M[i * nL + j], so a warp touches consecutive words).  Each V-cycle then applies it as a
-// matrix-vector product.  Leaves the header count > DENSO_MAX when the level has more changing
+// because the cell types are.  The grid builds that map once per solve: column j is the sweeps
+// applied to b = e_j (stored at M[i * nL + j], so a warp applying a row touches consecutive
+// words).  Each V-cycle then applies it as a matrix-vector product.  Leaves the header count > DENSO_MAX when the level has more changing
 // cells, and the section keeps the sweeps.
 struct Denso {
   float* M;
@@ -1041,6 +1061,16 @@ __device__ __forceinline__ Denso denso(unsigned char* dyn, int off) {
   return z;
 }
 
+// The half-sweeps of resolverGrosso as (colour) steps: sweep k takes colour 0 then 1 when k is even
+// and 1 then 0 when k is odd, and a half-sweep of one colour reads the other colour alone, so the
+// first half of each sweep after the first repeats the half-sweep before it and changes nothing.
+// Left out are only those repeats: 65 alternating half-sweeps give the bits of all 128.
+constexpr int MEIAS_GROSSO = VARREDURAS_GROSSO + 1;
+
+// Every CTA lists the cells and neighbours; column j is swept by one warp of the grid (CTA
+// j % gridDim.x), lanes over the rows, in its own shared column, and goes to the global copy
+// a.densoG, which the CTAs that apply the matrix load after the next grid barrier.  One thread a
+// column on CTA 0 alone took 231-299 us of every solve while the other CTAs waited.
 __device__ __noinline__ void montarDenso(const Args& a, unsigned char* dyn) {
   const Denso z = denso(dyn, a.offDenso);
   const NivelF n = s_niv[a.L - 1];
@@ -1070,44 +1100,63 @@ __device__ __noinline__ void montarDenso(const Args& a, unsigned char* dyn) {
   }
   __syncthreads();
   const int nL = z.cab[0];
-  if (nL > DENSO_MAX) return;
-  for (int i = threadIdx.x; i < nL; i += TF) {
-    const int e = z.celula[i], c = e & 0xffffff, mk = e >> 24;
-    z.viz4[4 * i + 0] = (mk & 1) ? mapa[c - 1] : -1;
-    z.viz4[4 * i + 1] = (mk & 2) ? mapa[c + 1] : -1;
-    z.viz4[4 * i + 2] = (mk & 4) ? mapa[c - nx] : -1;
-    z.viz4[4 * i + 3] = (mk & 8) ? mapa[c + nx] : -1;
-    z.inv[i] = inversoVizinhos(__popc(mk));
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < nL * nL; k += TF) z.M[k] = 0.0f;
-  __syncthreads();
-  const int j = threadIdx.x;
-  if (j < nL) {
+  if (nL <= DENSO_MAX) {
+    for (int i = threadIdx.x; i < nL; i += TF) {
+      const int e = z.celula[i], c = e & 0xffffff, mk = e >> 24;
+      z.viz4[4 * i + 0] = (mk & 1) ? mapa[c - 1] : -1;
+      z.viz4[4 * i + 1] = (mk & 2) ? mapa[c + 1] : -1;
+      z.viz4[4 * i + 2] = (mk & 4) ? mapa[c - nx] : -1;
+      z.viz4[4 * i + 3] = (mk & 8) ? mapa[c + nx] : -1;
+      z.inv[i] = inversoVizinhos(__popc(mk));
+    }
+    __syncthreads();
     const int n0 = z.cab[1];
-    for (int k = 0; k < VARREDURAS_GROSSO; k++)
-      for (int o = 0; o < 2; o++) {
-        const int cor = (k & 1) ? 1 - o : o;
-        const int i0 = cor ? n0 : 0, i1 = cor ? nL : n0;
-        for (int i = i0; i < i1; i++) {
+    float* col = z.M + w * (DENSO_MAX + 32);  // the warp's column; entry nL stays 0 (a closed neighbour)
+    for (int j = w * gridDim.x + blockIdx.x; j < nL; j += WARPS * gridDim.x) {
+      for (int i = lane; i <= nL; i += 32) col[i] = 0.0f;
+      __syncwarp();
+      for (int h = 0; h < MEIAS_GROSSO; h++) {
+        const int i0 = (h & 1) ? n0 : 0, i1 = (h & 1) ? nL : n0;
+        for (int i = i0 + lane; i < i1; i += 32) {
           float t = 0.0f;
 #pragma unroll
           for (int q = 0; q < 4; q++) {
             const int v = z.viz4[4 * i + q];
-            t += v >= 0 ? z.M[v * nL + j] : 0.0f;
+            t += col[v >= 0 ? v : nL];
           }
-          z.M[i * nL + j] = (t + (i == j ? 1.0f : 0.0f)) * z.inv[i];
+          col[i] = (t + (i == j ? 1.0f : 0.0f)) * z.inv[i];
         }
+        __syncwarp();
       }
+      for (int i = lane; i < nL; i += 32) a.densoG[i * nL + j] = __float_as_uint(col[i]);
+      __syncwarp();
+    }
+  }
+  if (blockIdx.x == 0) {  // the list and the header after the matrix
+    __syncthreads();
+    const unsigned* src = (const unsigned*)z.celula;
+    constexpr int M = DENSO_MAX * DENSO_MAX;
+    for (int k = threadIdx.x; k < (int)(DENSO_BYTES / 4) - M; k += TF) a.densoG[M + k] = src[k];
   }
   __syncthreads();
 }
 
+// The matrix (its used part), list and header from the global copy into this CTA's shared memory.
+__device__ void carregarDenso(const Args& a, unsigned char* dyn) {
+  unsigned* dst = (unsigned*)(dyn + a.offDenso);
+  constexpr int M = DENSO_MAX * DENSO_MAX, R = (int)(DENSO_BYTES / 4) - M;
+  const int nL = (int)__ldcg(a.densoG + M + R - 4);
+  const int usado = nL <= DENSO_MAX ? nL * nL : 0;
+  for (int k = threadIdx.x; k < usado; k += TF) dst[k] = __ldcg(a.densoG + k);
+  for (int k = threadIdx.x; k < R; k += TF) dst[M + k] = __ldcg(a.densoG + M + k);
+  __syncthreads();
+}
+
 // x = M b on the coarsest level (one warp per row, lanes over the row, fixed-order warp sum).
-__device__ void aplicarDenso(const Denso& z, float* F, int xa, int b) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ void aplicarDenso(const Denso& z, float* F, int xa, int b, const Equipe& eq) {
+  const int lane = threadIdx.x & 31, w = eq.ti >> 5;
   const int nL = z.cab[0];
-  for (int i = w; i < nL; i += WARPS) {
+  for (int i = w; i < nL; i += eq.nt >> 5) {
     float s = 0.0f;
     for (int j = lane; j < nL; j += 32) s += z.M[i * nL + j] * F[b + (z.celula[j] & 0xffffff)];
 #pragma unroll
@@ -1127,16 +1176,22 @@ __device__ __forceinline__ void marcaSecao(const Args& a, bool marcar = true) {
   }
 }
 
-// Levels Lc..L-1 of the V-cycle inside CTA 0: loads b of level Lc (a.bc), runs the down
-// passes and restrictions, the coarsest red-black solve (one warp), the prolongations and up
-// passes, and stores x of level Lc (a.xc).
-__device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, NivelS* s, int* tileOff, int coluna) {
+// Levels Lc..L-1 of the V-cycle inside a CTA: loads b of level Lc (a.bc), runs the down
+// passes and restrictions, the coarsest red-black solve, the prolongations and up passes, and
+// stores x of level Lc (a.xc).  With coluna >= 0, the same for b = the unit vector of the section's
+// water cell `coluna`, by one team, into that column of the section's matrix.  From a unit vector
+// the top level's down passes and restriction change the blocks around the cell alone (every
+// other block sweeps zeros into zeros), so a column takes only those; its later levels are whole.
+// smem holds the team's level arrays, dyn the CTA's (the coarsest level's matrix at a.offDenso).
+__device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, unsigned char* dyn, NivelS* tab, int coluna,
+                                         const Equipe eq, bool primeira) {
   const bool marcar = coluna < 0 && blockIdx.x == 0;
+  NivelS* s = tab - a.Lc;  // level l at s[l]
   float* F = (float*)smem;
   uint8_t* U = smem;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = eq.ti >> 5, nw = eq.nt >> 5;
   marcaSecao(a, marcar);
-  if (threadIdx.x == 0) {
+  if (eq.ti == 0) {
     int off = 0;  // bytes
     for (int l = a.Lc; l < a.L; l++) {
       const NivelF n = s_niv[l];
@@ -1153,66 +1208,89 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
       t.v = off;
       off += (N + 15) & ~15;
     }
-    *tileOff = off;
   }
-  __syncthreads();
+  sincEquipe(eq);
   const int celJ = coluna >= 0 ? __ldcg(a.wSecao + coluna) : -1;  // column build: b = unit vector
   for (int l = a.Lc; l < a.L; l++) {
     const NivelS t = s[l];
     const uint8_t* viz = s_niv[l].viz;
     const int N = t.nx * t.ny;
-    for (int c0 = 0; c0 < N; c0 += 4 * TF) {  // loads in batches of 4 per thread
+    if (coluna >= 0)
+      for (int c = eq.ti; c < N; c += eq.nt) {
+        F[t.xa + c] = F[t.xb + c] = 0.0f;
+        F[t.b + c] = l == a.Lc && c == celJ ? 1.0f : 0.0f;
+      }
+    if (!primeira) continue;
+    for (int c0 = 0; c0 < N; c0 += 4 * eq.nt) {  // loads in batches of 4 per thread
       int vv[4];
       float bb[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const int c = c0 + threadIdx.x + k * TF;
+        const int c = c0 + eq.ti + k * eq.nt;
         vv[k] = c < N ? ldcg8(viz + c) : 0;
-        bb[k] = (c < N && l == a.Lc) ? (coluna < 0 ? __ldcg(a.bc + c) : (c == celJ ? 1.0f : 0.0f)) : 0.0f;
+        bb[k] = (c < N && l == a.Lc && coluna < 0) ? __ldcg(a.bc + c) : 0.0f;
       }
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const int c = c0 + threadIdx.x + k * TF;
+        const int c = c0 + eq.ti + k * eq.nt;
         if (c < N) {
           U[t.v + c] = (uint8_t)vv[k];
+          if (coluna >= 0) continue;
           F[t.xa + c] = 0.0f;
           if (l == a.Lc) F[t.b + c] = bb[k];
         }
       }
     }
   }
-  __syncthreads();
+  sincEquipe(eq);
   marcaSecao(a, marcar);
   const float pes[4] = {0.25f, 0.75f, 0.75f, 0.25f};
   // the block preconditioner's single pass (see cicloV) ends in xb: the level's two buffers swap
   // roles in this CTA's table (rebuilt at each call)
+  auto todos = [](const NivelS& n, int desl) {
+    return Ret{0, 0, ((n.nx + desl + 15) >> 4) - 1, ((n.ny + desl + 15) >> 4) - 1};
+  };
   auto trocarS = [&](int l) {
-    if (threadIdx.x == 0) {
+    if (eq.ti == 0) {
       const int t = s[l].xa;
       s[l].xa = s[l].xb;
       s[l].xb = t;
     }
-    __syncthreads();
+    sincEquipe(eq);
   };
   for (int l = a.Lc; l < a.L - 1; l++) {
     NivelS f = s[l];
     const NivelS g = s[l + 1];
+    // the blocks and (for the restriction) cells that can hold anything but 0: all, or around celJ
+    Ret r0 = todos(f, 0), r8 = todos(f, 8), rc{0, 0, f.nx - 1, f.ny - 1}, rg{0, 0, g.nx - 1, g.ny - 1};
+    if (coluna >= 0 && l == a.Lc) {
+      const int i = celJ % f.nx, j = celJ / f.nx;
+      r0 = {i >> 4, j >> 4, i >> 4, j >> 4};
+      // shift 8: the cell's block, or (after the pass of shift 0) the four over its shift-0 block
+      if (a.umaPassada) r8 = {(i + 8) >> 4, (j + 8) >> 4, (i + 8) >> 4, (j + 8) >> 4};
+      else r8 = {r0.x0, r0.y0, min(r0.x0 + 1, r8.x1), min(r0.y0 + 1, r8.y1)};
+      // the cells of those blocks and their neighbours, and the coarse cells whose windows meet them
+      rc = {max(16 * r8.x0 - 9, 0), max(16 * r8.y0 - 9, 0), min(16 * r8.x1 + 8, f.nx - 1), min(16 * r8.y1 + 8, f.ny - 1)};
+      rg = {max((rc.x0 - 2) >> 1, 0), max((rc.y0 - 2) >> 1, 0), min((rc.x1 + 2) >> 1, g.nx - 1),
+            min((rc.y1 + 2) >> 1, g.ny - 1)};
+    }
     if (a.umaPassada) {
-      passoS(F, U, f, 8, 0, f.xa, f.xb, a.bloco != 0, a.varreduras);
+      passoS(F, U, f, 8, 0, f.xa, f.xb, a.bloco != 0, a.varreduras, eq, r8);
       trocarS(l);
       f = s[l];
     } else {
-      passoS(F, U, f, 0, 0, f.xa, f.xb, a.bloco != 0, a.varreduras);
+      passoS(F, U, f, 0, 0, f.xa, f.xb, a.bloco != 0, a.varreduras, eq, r0);
       marcaSecao(a, marcar);
-      passoS(F, U, f, 8, 0, f.xb, f.xa, a.bloco != 0, a.varreduras);
+      passoS(F, U, f, 8, 0, f.xb, f.xa, a.bloco != 0, a.varreduras, eq, r8);
     }
     marcaSecao(a, marcar);
     // restringir: residuals of the fine level into its free x buffer, then the 4x4 gathers.
     // Out-of-range and dry neighbours enter with weight or value 0, which adds +0 to a sum.
     {
-      const int Nf = f.nx * f.ny;
+      const int wf = rc.x1 - rc.x0 + 1, Nf = wf * (rc.y1 - rc.y0 + 1);
       const float* x = F + f.xa;
-      for (int c = threadIdx.x; c < Nf; c += TF) {
+      for (int k = eq.ti; k < Nf; k += eq.nt) {
+        const int c = rc.x0 + k % wf + (rc.y0 + k / wf) * f.nx;
         const int vz = U[f.v + c];
         const float a0 = x[(vz & 1) ? c - 1 : c], a1 = x[(vz & 2) ? c + 1 : c];
         const float a2 = x[(vz & 4) ? c - f.nx : c], a3 = x[(vz & 8) ? c + f.nx : c];
@@ -1224,10 +1302,11 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
         t += (vz & 8) ? a3 : 0.0f;
         F[f.xb + c] = (vz & 16) ? bc - ((float)__popc(vz & 15) * xc - t) : 0.0f;
       }
-      __syncthreads();
+      sincEquipe(eq);
       const float* r = F + f.xb;
-      for (int C = threadIdx.x; C < g.nx * g.ny; C += TF) {
-        const int I = C % g.nx, J = C / g.nx;
+      const int wg = rg.x1 - rg.x0 + 1, Ng = wg * (rg.y1 - rg.y0 + 1);
+      for (int k = eq.ti; k < Ng; k += eq.nt) {
+        const int I = rg.x0 + k % wg, J = rg.y0 + k / wg, C = I + J * g.nx;
         float rv[16];
 #pragma unroll
         for (int bb = 0; bb < 4; bb++) {
@@ -1250,22 +1329,15 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
         F[g.xa + C] = 0.0f;
       }
     }
-    __syncthreads();
+    sincEquipe(eq);
     marcaSecao(a, marcar);
   }
-  const bool comDenso = a.offDenso >= 0 && denso(smem, a.offDenso).cab[0] <= DENSO_MAX;
+  const bool comDenso = a.offDenso >= 0 && denso(dyn, a.offDenso).cab[0] <= DENSO_MAX;
   if (comDenso) {
     const NivelS n = s[a.L - 1];
-    aplicarDenso(denso(smem, a.offDenso), F, n.xa, n.b);
-  } else if (s[a.L - 1].nx * s[a.L - 1].ny > GROSSO_UM_WARP || w == 0) {
-    // resolverGrosso (js/pressao-cpu.js:217-238): one warp on a small level, every warp of the
-    // CTA on a large one (a wide, flat coarsest level of a tank atlas)
-    const bool todos = s[a.L - 1].nx * s[a.L - 1].ny > GROSSO_UM_WARP;
-    const int P = todos ? WARPS : 1;
-    auto sincronizar = [&]() {
-      if (todos) __syncthreads();
-      else __syncwarp();
-    };
+    aplicarDenso(denso(dyn, a.offDenso), F, n.xa, n.b, eq);
+  } else {
+    // resolverGrosso (js/pressao-cpu.js:217-238) on every warp of the team
     const NivelS n = s[a.L - 1];
     const int nx = n.nx, N = n.nx * n.ny;
     float* x = F + n.xa;
@@ -1273,8 +1345,9 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
     // buffer as cell | mask << 24, colour 0 first, in cell order: each warp lists a slice of
     // the cells (a multiple of 32) at the offset of the slices before it.
     int* lista = (int*)(F + n.xb);
-    __shared__ int contW[2][WARPS];
-    const int fatia = ((N + P * 32 - 1) / (P * 32)) * 32;
+    __shared__ unsigned short contWs[SECAO_EQUIPES][2][WARPS];
+    auto& contW = contWs[eq.id];
+    const int fatia = ((N + eq.nt - 1) / eq.nt) * 32;
     const int lo = min(w * fatia, N), hi = min(lo + fatia, N);
     auto muda = [&](int c, int cor) {
       const int vz = c < hi ? U[n.v + c] : 0;
@@ -1285,11 +1358,11 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
     for (int cor = 0; cor < 2; cor++) {
       int k = 0;
       for (int c0 = lo; c0 < hi; c0 += 32) k += __popc(__ballot_sync(0xffffffffu, muda(c0 + lane, cor) >= 0));
-      if (lane == 0) contW[cor][w] = k;
+      if (lane == 0) contW[cor][w] = (unsigned short)k;
     }
-    sincronizar();
+    sincEquipe(eq);
     int cont[2] = {0, 0}, base[2] = {0, 0};
-    for (int q = 0; q < P; q++)
+    for (int q = 0; q < nw; q++)
 #pragma unroll
       for (int cor = 0; cor < 2; cor++) {
         if (q == w) base[cor] = cont[cor];
@@ -1306,14 +1379,58 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
         b += __popc(m);
       }
     }
-    sincronizar();
-    const int t0 = todos ? threadIdx.x : lane, nt = P * 32;
-    for (int k = 0; k < VARREDURAS_GROSSO; k++)
-      for (int o = 0; o < 2; o++) {
-        const int cor = (k & 1) ? 1 - o : o;
+    sincEquipe(eq);
+    if (cont[0] <= GROSSO_REG * eq.nt && cont[1] <= GROSSO_REG * eq.nt) {
+      const int ne = ((cont[0] > cont[1] ? cont[0] : cont[1]) + eq.nt - 1) / eq.nt;  // uniform
+      // Up to GROSSO_REG cells a colour and thread: index, neighbours, right side and 1/k stay in
+      // registers, so a half-sweep is four shared loads, the sum and a store.  (One warp walking
+      // the list took 98-150 us a V-cycle on 930 to 1,000-cell levels.)  A closed neighbour
+      // reads the list's first word, 0 once every thread has its cells.
+      int cel[2][GROSSO_REG], vz[2][GROSSO_REG][4];
+      float bq[2][GROSSO_REG], iq[2][GROSSO_REG];
+      const int zero = n.xb - n.xa;
+#pragma unroll
+      for (int cor = 0; cor < 2; cor++)
+#pragma unroll
+        for (int e = 0; e < GROSSO_REG; e++) {
+          const int k = eq.ti + e * eq.nt;
+          const int E = k < cont[cor] ? lista[(cor ? cont[0] : 0) + k] : -1;
+          const int c = E < 0 ? 0 : E & 0xffffff, mk = E < 0 ? 0 : E >> 24;
+          cel[cor][e] = E < 0 ? -1 : c;
+          vz[cor][e][0] = (mk & 1) ? c - 1 : zero;
+          vz[cor][e][1] = (mk & 2) ? c + 1 : zero;
+          vz[cor][e][2] = (mk & 4) ? c - nx : zero;
+          vz[cor][e][3] = (mk & 8) ? c + nx : zero;
+          bq[cor][e] = E < 0 ? 0.0f : F[n.b + c];
+          iq[cor][e] = inversoVizinhos(__popc(mk));
+        }
+      sincEquipe(eq);
+      if (eq.ti == 0) F[n.xb] = 0.0f;
+      sincEquipe(eq);
+      auto meia = [&](auto COR) {
+        constexpr int cor = decltype(COR)::value;
+#pragma unroll
+        for (int e = 0; e < GROSSO_REG; e++)
+          if (e < ne && cel[cor][e] >= 0) {
+            float t = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; q++) t += x[vz[cor][e][q]];
+            x[cel[cor][e]] = (t + bq[cor][e]) * iq[cor][e];
+          }
+        sincEquipe(eq);
+      };
+#pragma unroll 1
+      for (int h = 0; h < MEIAS_GROSSO; h++) {
+        if (h & 1) meia(std::integral_constant<int, 1>{});
+        else meia(std::integral_constant<int, 0>{});
+      }
+    } else {
+#pragma unroll 1
+      for (int h = 0; h < MEIAS_GROSSO; h++) {
+        const int cor = h & 1;
         const int ini = cor ? cont[0] : 0, n_ = cont[cor];
-        for (int e0 = t0; e0 < n_; e0 += 2 * nt) {
-          const int eA = e0, eB = e0 + nt;
+        for (int e0 = eq.ti; e0 < n_; e0 += 2 * eq.nt) {
+          const int eA = e0, eB = e0 + eq.nt;
           const int EA = lista[ini + eA], EB = eB < n_ ? lista[ini + eB] : -1;
           float va[5], vb[5];
           {
@@ -1351,16 +1468,17 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
             x[EB & 0xffffff] = (t + vb[4]) * inversoVizinhos(__popc(mk));
           }
         }
-        sincronizar();
+        sincEquipe(eq);
       }
+    }
   }
-  __syncthreads();
+  sincEquipe(eq);
   marcaSecao(a, marcar);
   for (int l = a.L - 2; l >= a.Lc; l--) {
     const NivelS g = s[l + 1];
     const NivelS f = s[l];
     // prolongar: coarse x is 0 on every dry coarse cell, out-of-range corners get weight 0
-    for (int c = threadIdx.x; c < f.nx * f.ny; c += TF) {
+    for (int c = eq.ti; c < f.nx * f.ny; c += eq.nt) {
       const int i = c % f.nx, j = c / f.nx;
       const int I0 = grossoBaseF(i), J0 = grossoBaseF(j);
       const float wx0 = pesoBaseF(i), wy0 = pesoBaseF(j);
@@ -1386,28 +1504,28 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, Niv
       }
       if (U[f.v + c] & 16) F[f.xa + c] = xf + e;
     }
-    __syncthreads();
+    sincEquipe(eq);
     marcaSecao(a, marcar);
-    passoS(F, U, f, 8, 1, f.xa, f.xb, a.bloco != 0, a.varreduras);
+    passoS(F, U, f, 8, 1, f.xa, f.xb, a.bloco != 0, a.varreduras, eq, todos(f, 8));
     if (a.umaPassada) {
       trocarS(l);
     } else {
       marcaSecao(a, marcar);
-      passoS(F, U, f, 0, 1, f.xb, f.xa, a.bloco != 0, a.varreduras);
+      passoS(F, U, f, 0, 1, f.xb, f.xa, a.bloco != 0, a.varreduras, eq, todos(f, 0));
     }
     marcaSecao(a, marcar);
   }
   const NivelS t = s[a.Lc];
   const int Nc = t.nx * t.ny;
   if (coluna < 0) {
-    for (int c = threadIdx.x; c < Nc; c += TF) a.xc[c] = F[t.xa + c];
+    for (int c = eq.ti; c < Nc; c += eq.nt) a.xc[c] = F[t.xa + c];
   } else {  // column `coluna` of the section's matrix, rows = water cells of level Lc
     const int nW = __ldcg(a.nWp);
-    for (int c = threadIdx.x; c < Nc; c += TF) {
+    for (int c = eq.ti; c < Nc; c += eq.nt) {
       const int r = __ldcg(a.wInv + c);
       if (r >= 0) a.mSecao[(size_t)r * nW + coluna] = F[t.xa + c];
     }
-  }
+  }  sincEquipe(eq);  // the next column rewrites the table and the arrays
 }
 
 // x of level Lc = M b over its water cells, every CTA staging b in shared memory and each warp
@@ -1447,7 +1565,7 @@ __device__ __forceinline__ void trocarXTmp(int l) {
 // TQ_PRECOND_BLOCK_1 the grid levels above 0 take one smoother pass a leg (shift 8, red-black
 // down and black-red up, so the cycle stays symmetric): 3 Lc + 3 phases.
 template <class T>
-__device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char* smem, NivelS* tabS, int* tileOff,
+__device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char* smem, NivelS* tabS,
                        const Reuniao& ru, double* sh, bool secaoDensa) {
   for (int l = 0; l < a.Lc; l++) {
     const int meia = s_niv[l].meia;
@@ -1465,7 +1583,7 @@ __device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char*
     if (!barreira(a, ep)) return false;
   }
   if (secaoDensa) aplicarSecaoDensa(a, smem);
-  else if (blockIdx.x == 0) secaoGrossa(a, smem, tabS, tileOff, -1);
+  else if (blockIdx.x == 0) secaoGrossa(a, smem, smem, tabS, -1, Equipe{(int)threadIdx.x, TF, 0}, true);
   if (!barreira(a, ep)) return false;
   for (int l = a.Lc - 1; l >= 0; l--) {
     const int meia = s_niv[l].meia;
@@ -1742,8 +1860,7 @@ template <class T>
 __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ double sh[32];
-  __shared__ NivelS tabS[MAX_NIVEIS];
-  __shared__ int tileOff;
+  __shared__ NivelS tabS[SECAO_EQUIPES][SECAO_NIVEIS];
   float* areas = (float*)dyn;
   const Dev& d = a.d;
   const int N = d.N, nx = d.nx, ny = d.ny;
@@ -1929,13 +2046,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     }
   }
   // the coarsest level's matrix (its neighbour masks are complete since the last barrier)
-  if (blockIdx.x == 0 && a.offDenso >= 0) {
-    montarDenso(a, dyn);
-    if (a.secaoDensa) {  // every CTA will need it to build the section's columns
-      const unsigned* src = (const unsigned*)(dyn + a.offDenso);
-      for (int k = threadIdx.x; k < (int)(DENSO_BYTES / 4); k += TF) a.densoG[k] = src[k];
-    }
-  }
+  if (a.offDenso >= 0) montarDenso(a, dyn);
   if (a.secaoDensa && blockIdx.x == (gridDim.x > 1 ? 1 : 0) && threadIdx.x < 32) {
     // the water cells of level Lc, in cell order (one warp, ballot-compacted)
     const NivelF n = s_niv[a.Lc];
@@ -1981,13 +2092,16 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
   if (!barreira(a, ep)) return;  // rb visible before spreading
   // ---- the section's matrix: every CTA builds its share of the columns with its own copy of
   // the coarsest level's matrix
+  const int nW = a.secaoDensa ? __ldcg(a.nWp) : 0;
   const bool secaoDensa = a.secaoDensa && a.iteracoes >= SECAO_DENSA_MIN_ITERS;
+  if (a.offDenso >= 0 && (secaoDensa || blockIdx.x == 0)) carregarDenso(a, dyn);
   if (secaoDensa) {
-    unsigned* blocoDenso = (unsigned*)(dyn + a.offDenso);
-    for (int k = threadIdx.x; k < (int)(DENSO_BYTES / 4); k += TF) blocoDenso[k] = __ldcg(a.densoG + k);
+    const int nt = TF / a.equipes, g = threadIdx.x / nt;
+    const Equipe eq{(int)threadIdx.x - g * nt, nt, g};
+    bool primeira = true;  // a team's masks stay in its area from its first column on
+    for (int col = g * gridDim.x + blockIdx.x; col < nW; col += a.equipes * gridDim.x, primeira = false)
+      secaoGrossa(a, dyn + (size_t)g * a.bytesSecao, dyn, tabS[g], col, eq, primeira);
     __syncthreads();
-    const int nW = __ldcg(a.nWp);
-    for (int col = blockIdx.x; col < nW; col += gridDim.x) secaoGrossa(a, dyn, tabS, &tileOff, col);
     const NivelF nc = s_niv[a.Lc];
     for (int c = gt0; c < nc.nx * nc.ny; c += GT) a.xc[c] = 0.0f;  // off water, x of level Lc stays 0
     if (!barreira(a, ep)) return;
@@ -1998,7 +2112,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
       a.accZ[b] = 0;
       d.accB[b] = 0;
     }
-  if (!cicloV<T>(a, ep, areas, dyn, tabS, &tileOff, Reuniao{escala, d.z, nullptr}, sh, secaoDensa)) return;
+  if (!cicloV<T>(a, ep, areas, dyn, tabS[0], Reuniao{escala, d.z, nullptr}, sh, secaoDensa)) return;
   int cz = 0, cp = 0;  // which of the two z / p buffers holds the latest values
   auto zbAtual = [&](int b) { return zbDe(a, b); };
   somasGlobais(a, nAt, [&](int b) { return __ldcg(&d.rb[b]) * zbAtual(b); }, [](int) { return 0.0; }, sh, somas);
@@ -2140,7 +2254,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     escala = (a.escalar && norma > 0) ? (float)(1.0 / norma) : 1.0f;
     if (blockIdx.x == 0)
       for (int b = threadIdx.x; b < MAX_BOLHAS; b += TF) d.accB[b] = 0;
-    if (!cicloV<T>(a, ep, areas, dyn, tabS, &tileOff, Reuniao{escala, zo, zc}, sh, secaoDensa)) return;
+    if (!cicloV<T>(a, ep, areas, dyn, tabS[0], Reuniao{escala, zo, zc}, sh, secaoDensa)) return;
     cz ^= 1;
     cp ^= 1;
     primeira = false;
@@ -2189,7 +2303,7 @@ Fundido* criarFundido(Pcg* p) {
     bytes += b;
     Lc = l;
   }
-  if (Lc >= p->L) {  // even the coarsest level does not fit
+  if (Lc >= p->L || p->L - Lc > SECAO_NIVEIS) {  // even the coarsest level does not fit
     delete f;
     return nullptr;
   }
@@ -2202,6 +2316,15 @@ Fundido* criarFundido(Pcg* p) {
   size_t porWarp = (size_t)(SUAV_W > REST_W ? SUAV_W : REST_W) * 4;
   size_t areas = (size_t)WARPS * porWarp;
   f->smem = bytes > areas ? bytes : areas;
+  f->bytesSecao = (int)bytes;
+  // teams that build the section's matrix side by side, where their areas and the coarsest
+  // level's matrix fit in a CTA's shared memory
+  for (int q = SECAO_EQUIPES; q > 1; q--)
+    if (TF % (32 * q) == 0 && q * bytes + DENSO_BYTES + 16 <= SMEM_CTA_MAX) {
+      f->equipes = q;
+      if (q * bytes > f->smem) f->smem = q * bytes;
+      break;
+    }
   {  // the coarsest level's matrix after everything else, when the level is small enough
     const size_t nGrosso = (size_t)p->nxL[p->L - 1] * p->nyL[p->L - 1];
     const size_t off = (f->smem + 15) & ~(size_t)15;
@@ -2265,8 +2388,8 @@ Fundido* criarFundido(Pcg* p) {
     ok = ok && (nFlags == 0 || cudaMalloc(&f->solidos, nFlags) == cudaSuccess);
     if (ok && f->secaoDensa)
       ok = cudaMalloc(&f->mSecao, nLc * nLc * 4) == cudaSuccess && cudaMalloc(&f->wSecao, nLc * 4) == cudaSuccess &&
-           cudaMalloc(&f->wInv, nLc * 4) == cudaSuccess && cudaMalloc(&f->nW, 4) == cudaSuccess &&
-           cudaMalloc(&f->densoG, DENSO_BYTES) == cudaSuccess;
+           cudaMalloc(&f->wInv, nLc * 4) == cudaSuccess && cudaMalloc(&f->nW, 4) == cudaSuccess;
+    if (ok && f->offDenso >= 0) ok = cudaMalloc(&f->densoG, DENSO_BYTES) == cudaSuccess;
   }
   if (ok) {
     NivelF tab[MAX_NIVEIS] = {};
@@ -2349,6 +2472,8 @@ int resolverPressaoFundido(Pcg* p, const Dev& d, int iteracoes, double tol, bool
   a.bc = f->bc;
   a.offDenso = f->offDenso;
   a.secaoDensa = f->secaoDensa ? 1 : 0;
+  a.equipes = f->equipes;
+  a.bytesSecao = f->bytesSecao;
   a.mSecao = f->mSecao;
   a.wSecao = f->wSecao;
   a.wInv = f->wInv;
