@@ -2,8 +2,8 @@
 // enclosed air pocket one extra unknown ("supercell").  Restates js/pressao-cpu.js
 // (resolverPCG :296-402, cicloV :241-255 and its parts) on the device.
 //
-// This file is the PLAIN engine: one launch per step of the algorithm, the iteration loop on
-// the host.  The V-cycle vectors (b, x, tmp of every level) are stored as T = float, __half or
+// This file is the PLAIN engine: separate launches, the iteration loop on the host.  A V-cycle takes
+// one launch a leg of each level (suavizador.cuh) and one for its coarse levels.  The V-cycle vectors (b, x, tmp of every level) are stored as T = float, __half or
 // __nv_bfloat16 (levels below 16k cells stay float); arithmetic is FP32; dot products and
 // norms are FP64 with a fixed reduction order (bitwise reproducible); per-bubble sums are
 // 64-bit fixed point.
@@ -13,235 +13,418 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "pcg_interno.cuh"
+#include "suavizador.cuh"
 #include <type_traits>
 
 namespace tq {
 
+// Level 0's masks also carry, during a solve, whether the cell is air of an active bubble that the
+// V-cycle sees as water (it takes its bubble's mean residual and gives its share of z back) and
+// whether it is water to the operator.
+constexpr int V0_BOLHA = 32, V0_AGUA = 64;
+
 // ---------------------------------------------------------------- types and neighbours
-// The preconditioner's level-0 types: bubble air counts as water (js/pressao-cpu.js:305-308);
-// with TQ_PRECOND_BLOCK (bloco) it stays air.
-__global__ void k_mg_tipo0(const uint8_t* tipo, const uint32_t* rot, uint8_t* t0, int N, int bolhas, int bloco) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  uint8_t t = tipo[c];
-  if (bolhas && !bloco && t == AR && rot[c] >= 2) t = AGUA;
-  t0[c] = t;
-}
-
-// tiposGrossos (js/pressao-cpu.js:63-81): air if any child is air, else water if any is water.
-__global__ void k_mg_tipo_grosso(const uint8_t* tf, int fnx, int fny, uint8_t* tg, int gnx, int gny) {
-  int C = blockIdx.x * blockDim.x + threadIdx.x;
-  if (C >= gnx * gny) return;
-  int I = C % gnx, J = C / gnx;
-  bool ar = false, agua = false;
-  for (int b = 0; b < 2; b++)
-    for (int a = 0; a < 2; a++) {
-      int i = 2 * I + a, j = 2 * J + b;
-      if (i >= fnx || j >= fny) continue;
-      uint8_t t = tf[i + j * fnx];
-      if (t == AR) ar = true;
-      else if (t == AGUA) agua = true;
-    }
-  tg[C] = ar ? AR : agua ? AGUA : SOLIDO;
-}
-
-// prepararVizinhos (js/pressao-cpu.js:44-60) packed in one byte: bits 0-3 = free (non-wall)
-// left/right/down/up neighbours, bit 4 = the cell itself is water.
-__global__ void k_viz(const uint8_t* tipo, int nx, int ny, uint8_t* viz) {
+// The preconditioner's level-0 types: bubble air counts as water (js/pressao-cpu.js:305-308); with
+// TQ_PRECOND_BLOCK (bloco) it stays air.  And the operator's free neighbours (bits 0-3) of every
+// cell, from the true types.
+__global__ void k_mg_tipo0(const uint8_t* tipo, const uint32_t* rot, uint8_t* t0, uint8_t* vizOp, int nx, int ny,
+                           int bolhas, int bloco) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nx * ny) return;
-  int i = c % nx, j = c / nx;
+  const int i = c % nx, j = c / nx;
+  uint8_t t = tipo[c];
   int m = 0;
   if (i > 0 && tipo[c - 1] != SOLIDO) m |= 1;
   if (i < nx - 1 && tipo[c + 1] != SOLIDO) m |= 2;
   if (j > 0 && tipo[c - nx] != SOLIDO) m |= 4;
   if (j < ny - 1 && tipo[c + nx] != SOLIDO) m |= 8;
-  if (tipo[c] == AGUA) m |= 16;
+  vizOp[c] = (uint8_t)m;
+  if (bolhas && !bloco && t == AR && rot[c] >= 2) t = AGUA;
+  t0[c] = t;
+}
+
+// The levels' sizes and arrays for the two kernels that prepare them.
+struct Niveis {
+  int L;
+  int nx[MAX_NIVEIS], ny[MAX_NIVEIS];
+  int ini[MAX_NIVEIS + 1];  // k_niveis_viz: first thread of each level
+  uint8_t *tipo[MAX_NIVEIS], *viz[MAX_NIVEIS];
+};
+
+// tiposGrossos (js/pressao-cpu.js:63-81) of levels l0 + 1 .. l0 + 6: air if any child is air, else
+// water if any is water.  A CTA takes 64x64 cells of level l0 and halves them in shared memory (a
+// launch a level took 2.4-3.6 us each).
+constexpr int NIVEIS_POR_VEZ = 6;
+__global__ void __launch_bounds__(256) k_niveis_tipos(Niveis n, int l0) {
+  __shared__ uint8_t t[2][32 * 32];
+  auto mais = [](int a, int b) { return a == AR || b == AR ? (int)AR : a == AGUA || b == AGUA ? (int)AGUA : (int)SOLIDO; };
+  const int L = min(n.L - 1, l0 + NIVEIS_POR_VEZ);
+  for (int l = l0 + 1; l <= L; l++) {
+    const int w = 64 >> (l - l0);  // the CTA's side on level l
+    const uint8_t* f = t[(l - l0 - 1) & 1];
+    for (int c = threadIdx.x; c < w * w; c += 256) {
+      const int i = c % w, j = c / w, I = blockIdx.x * w + i, J = blockIdx.y * w + j;
+      int r = SOLIDO;
+      if (l == l0 + 1) {
+        const int fx = n.nx[l0], fy = n.ny[l0];
+        const uint8_t* src = n.tipo[l0];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int x = 2 * I + (q & 1), y = 2 * J + (q >> 1);
+          if (x < fx && y < fy) r = mais(r, src[x + (size_t)y * fx]);
+        }
+      } else {
+        const uint8_t* o = f + 2 * j * 2 * w + 2 * i;
+        r = mais(mais(o[0], o[1]), mais(o[2 * w], o[2 * w + 1]));
+      }
+      t[(l - l0) & 1][c] = (uint8_t)r;
+      if (I < n.nx[l] && J < n.ny[l]) n.tipo[l][I + (size_t)J * n.nx[l]] = (uint8_t)r;
+    }
+    __syncthreads();
+  }
+}
+
+// Level 0's masks in a solve: k_niveis_viz's bits and V0_AGUA; V0_BOLHA where `bolhas` (celsB counted).
+__global__ void k_viz0(Dev d, const uint8_t* tipo0, uint8_t* viz, int bolhas) {
+  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= d.N) return;
+  int i = c % d.nx, j = c / d.nx;
+  int m = 0;
+  if (i > 0 && tipo0[c - 1] != SOLIDO) m |= 1;
+  if (i < d.nx - 1 && tipo0[c + 1] != SOLIDO) m |= 2;
+  if (j > 0 && tipo0[c - d.nx] != SOLIDO) m |= 4;
+  if (j < d.ny - 1 && tipo0[c + d.nx] != SOLIDO) m |= 8;
+  if (tipo0[c] == AGUA) m |= 16;
+  const int t = d.tipo[c];
+  if (t == AGUA) m |= V0_AGUA;
+  else if (bolhas && t == AR) {
+    const uint32_t b = d.rotulo[c];
+    if (b >= 2 && b < (uint32_t)MAX_BOLHAS && d.celsB[b] > 0) m |= V0_BOLHA;
+  }
   viz[c] = (uint8_t)m;
 }
 
-// TQ_PRECOND_BLOCK's coarse masks: bits 0-3 open where a fine face across the coarse face joins
-// two non-wall fine cells (both coarse cells not wall), bit 4 water.
-__global__ void k_viz_faces(const uint8_t* tf, int fnx, int fny, const uint8_t* tg, int gnx, int gny, uint8_t* viz) {
-  int C = blockIdx.x * blockDim.x + threadIdx.x;
-  if (C >= gnx * gny) return;
-  const int I = C % gnx, J = C / gnx;
+// prepararVizinhos (js/pressao-cpu.js:44-60) of every level from l0 on in one launch, packed in one byte:
+// bits 0-3 = free (non-wall) left/right/down/up neighbours, bit 4 = the cell itself is water.  With
+// `bloco` (TQ_PRECOND_BLOCK) the coarse levels' bits 0-3 are open where a fine face across the coarse
+// face joins two non-wall fine cells (both coarse cells not wall).
+__global__ void k_niveis_viz(Niveis n, int l0, int bloco) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  int l = l0;
+  while (l < n.L && g >= n.ini[l + 1]) l++;
+  if (l >= n.L) return;
+  const int c = g - n.ini[l], nx = n.nx[l], ny = n.ny[l], i = c % nx, j = c / nx;
+  const uint8_t* tipo = n.tipo[l];
   int m = 0;
-  if (tg[C] != SOLIDO) {
-    auto livre = [&](int i, int j) { return i >= 0 && j >= 0 && i < fnx && j < fny && tf[i + j * fnx] != SOLIDO; };
-    auto horiz = [&](int i0, int i1) {
-      return (livre(i0, 2 * J) && livre(i1, 2 * J)) || (livre(i0, 2 * J + 1) && livre(i1, 2 * J + 1));
-    };
-    auto vert = [&](int j0, int j1) {
-      return (livre(2 * I, j0) && livre(2 * I, j1)) || (livre(2 * I + 1, j0) && livre(2 * I + 1, j1));
-    };
-    if (I > 0 && tg[C - 1] != SOLIDO && horiz(2 * I - 1, 2 * I)) m |= 1;
-    if (I < gnx - 1 && tg[C + 1] != SOLIDO && horiz(2 * I + 1, 2 * I + 2)) m |= 2;
-    if (J > 0 && tg[C - gnx] != SOLIDO && vert(2 * J - 1, 2 * J)) m |= 4;
-    if (J < gny - 1 && tg[C + gnx] != SOLIDO && vert(2 * J + 1, 2 * J + 2)) m |= 8;
-    if (tg[C] == AGUA) m |= 16;
+  if (bloco && l >= 1) {
+    if (tipo[c] != SOLIDO) {
+      const uint8_t* tf = n.tipo[l - 1];
+      const int fnx = n.nx[l - 1], fny = n.ny[l - 1];
+      auto livre = [&](int x, int y) { return x >= 0 && y >= 0 && x < fnx && y < fny && tf[x + y * fnx] != SOLIDO; };
+      auto horiz = [&](int i0, int i1) {
+        return (livre(i0, 2 * j) && livre(i1, 2 * j)) || (livre(i0, 2 * j + 1) && livre(i1, 2 * j + 1));
+      };
+      auto vert = [&](int j0, int j1) {
+        return (livre(2 * i, j0) && livre(2 * i, j1)) || (livre(2 * i + 1, j0) && livre(2 * i + 1, j1));
+      };
+      if (i > 0 && tipo[c - 1] != SOLIDO && horiz(2 * i - 1, 2 * i)) m |= 1;
+      if (i < nx - 1 && tipo[c + 1] != SOLIDO && horiz(2 * i + 1, 2 * i + 2)) m |= 2;
+      if (j > 0 && tipo[c - nx] != SOLIDO && vert(2 * j - 1, 2 * j)) m |= 4;
+      if (j < ny - 1 && tipo[c + nx] != SOLIDO && vert(2 * j + 1, 2 * j + 2)) m |= 8;
+    }
+  } else {
+    if (i > 0 && tipo[c - 1] != SOLIDO) m |= 1;
+    if (i < nx - 1 && tipo[c + 1] != SOLIDO) m |= 2;
+    if (j > 0 && tipo[c - nx] != SOLIDO) m |= 4;
+    if (j < ny - 1 && tipo[c + nx] != SOLIDO) m |= 8;
   }
-  viz[C] = (uint8_t)m;
+  if (tipo[c] == AGUA) m |= 16;
+  n.viz[l][c] = (uint8_t)m;
 }
 
 // ---------------------------------------------------------------- V-cycle kernels
-// suavizar (js/pressao-cpu.js:99-150): each 16x16 block reads the snapshot `src` (18x18 with
-// its one-cell border, zero outside the grid), runs VARREDURAS red-black sweeps inside the
-// block, and writes water cells to `dst` (other cells 0).  desl = 0 or 8 shifts the block
-// lattice; ordem = 0 sweeps red then black, 1 black then red.
-template <class T>
-__global__ void __launch_bounds__(256) k_suavizar(NivelDev<T> n, int desl, int ordem, const T* __restrict__ src,
-                                                  T* __restrict__ dst, const T* __restrict__ b) {
-  __shared__ float qs[18 * 18];
+// What level 0's right side is made from: v, scaled by *escala (null: 1), cells of active bubbles
+// their bubble's mean residual (precondicionar, js/pressao-cpu.js:353-355).
+struct Fonte {
+  const float* v;
+  const double* escala = nullptr;
+  const uint32_t* rotulo = nullptr;
+  const double* rb = nullptr;
+  const uint32_t* celsB = nullptr;
+};
+
+constexpr int T_LADRILHO = 512;
+
+// The way down a level on one tile a CTA (descerLadrilho): both passes and the restriction.
+template <class T, class TG, bool NIVEL0>
+__global__ void __launch_bounds__(T_LADRILHO) k_descer(NivelDev<T> n, NivelDev<TG> g, int kx, int ky, int uma, int masc,
+                                                       Fonte F) {
+  extern __shared__ __align__(16) float mem[];
   if (n.parar && *n.parar) return;  // uniform over the CTA
-  const int nx = n.nx, ny = n.ny;
-  const int ox = (int)blockIdx.x * 16 - desl, oy = (int)blockIdx.y * 16 - desl;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int s = threadIdx.x; s < 324; s += 256) {
-    int sx = s % 18 - 1 + ox, sy = s / 18 - 1 + oy;
-    qs[s] = (sx >= 0 && sy >= 0 && sx < nx && sy < ny) ? carregar(src[sx + sy * nx]) : 0.0f;
+  const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
+  const float e = NIVEL0 && F.escala ? (float)*F.escala : 1.0f;
+  descerLadrilho<T>(
+      L, g.nx, g.ny, g.viz, uma != 0, masc != 0, VARREDURAS, mem,
+      [&](int c) { return NIVEL0 ? __ldca(F.v + c) : carregar(n.b[c]); },
+      [&](int c, int v, float bv, bool meu) {
+        if (!NIVEL0) return bv;
+        if (v & V0_BOLHA) {
+          const uint32_t r = F.rotulo[c];
+          bv = (float)(F.rb[r] / F.celsB[r]);
+        }
+        const T bt = guardar<T>(bv * e);
+        if (meu) n.b[c] = bt;
+        return carregar(bt);
+      },
+      [&](int c, float x) { n.x[c] = guardar<T>(x); }, [&](int C, float v) { g.b[C] = guardar<TG>(v); });
+}
+
+// The way up a level: x + the coarse correction and both passes, the level's result in n.tmp, or
+// (saida not null) as floats in saida.
+template <class T, class TG>
+__global__ void __launch_bounds__(T_LADRILHO) k_subir(NivelDev<T> n, NivelDev<TG> g, const TG* xg, int kx, int ky,
+                                                      int uma, int masc, float* saida) {
+  extern __shared__ __align__(16) float mem[];
+  if (n.parar && *n.parar) return;
+  const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
+  subirLadrilho<T>(
+      L, g.nx, g.ny, uma != 0, masc != 0, VARREDURAS, mem, [&](int c) { return carregar(n.x[c]); },
+      [&](int C) { return carregar(xg[C]); }, [&](int c) { return carregar(n.b[c]); },
+      [&](const int (&cel)[2][4], const int (&v)[2][4], const float (&x)[2][4]) {
+#pragma unroll
+        for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+          for (int m = 0; m < 4; m++)
+            if (cel[cr][m] >= 0) {
+              if (saida) saida[cel[cr][m]] = arredondar<T>(x[cr][m]);
+              else n.tmp[cel[cr][m]] = guardar<T>(x[cr][m]);
+            }
+      });
+}
+
+// The coarse levels of at most SECAO_PLANA cells in one CTA, in shared memory: x as swept, its snapshot
+// before the pass (what a block's outer neighbours hold), the right side.  A thread takes two cells
+// side by side, one of each colour, so every thread works in every half-sweep and half the warps
+// meet at its barrier: four shared loads, the sum, a store.  The coarsest level's half-sweeps that
+// repeat the one before (the last colour of a sweep is the first of the next, and a colour reads
+// only the other) are left out, 65 of 128.  8 us with a coarsest level of
+// 49 cells alone, 17 us for three levels from 943 cells, where six launches a level and the 42-46 us of
+// one CTA's 128 half-sweeps were.
+constexpr int SECAO_PLANA = 1024, SECAO_PLANA_NIVEIS = 6, SECAO_PLANA_TOTAL = 1536, T_SECAO = 576;
+struct SecaoPlana {
+  int L, uma;
+  int off[SECAO_PLANA_NIVEIS];
+  NivelDev<float> n[SECAO_PLANA_NIVEIS];
+  float* saida;
+};
+// t / k correctly rounded, as resolverGrosso's division, from i = 1/k rounded: t i is exact for 1, 2 and
+// 4, and for 3 one correction by the residual t - 3 q rounds right (Markstein's theorem on the final
+// step of a division; checked against t / 3.0f for all 2^23 significands).  An infinite quotient
+// stays as it is.  No branch on k: one in the half-sweeps' loop took 137 of its 200 cycles.
+__device__ __forceinline__ float dividirViz(float t, float k, float i) {
+  const float q = t * i, r = fmaf(fmaf(-k, q, t), i, q);
+  return fabsf(q) < INFINITY ? r : q;
+}
+__global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
+  // one array, addressed by offsets: x, the snapshots, the right sides, and a 0 for closed neighbours
+  constexpr int S = SECAO_PLANA_TOTAL, B = 2 * SECAO_PLANA_TOTAL, ZERO = 3 * SECAO_PLANA_TOTAL;
+  __shared__ float X[ZERO + 1];
+  __shared__ uint8_t V[SECAO_PLANA_TOTAL];
+  if (s.n[0].parar && *s.n[0].parar) return;
+  const int t = threadIdx.x, nt = blockDim.x;
+  for (int l = 0; l < s.L; l++) {
+    const int N = s.n[l].nx * s.n[l].ny, o = s.off[l];
+    for (int c = t; c < N; c += nt) {
+      V[o + c] = s.n[l].viz[c];
+      X[o + c] = X[S + o + c] = 0.0f;  // a pass takes the snapshots of the cells that change alone
+      if (l == 0) X[B + o + c] = s.n[0].b[c];
+    }
   }
-  const int gx = ox + tx, gy = oy + ty;
-  const bool dentro = gx >= 0 && gy >= 0 && gx < nx && gy < ny;
-  const int c = gx + gy * nx;
-  int vz = dentro ? n.viz[c] : 0;
-  float bv = dentro ? carregar(b[c]) : 0.0f;
-  const int li = (ty + 1) * 18 + tx + 1;
-  const int m = vz & 15;
-  const int k = __popc(m);
-  const bool ativo = (vz & 16) && k > 0;
-  const float invk = ativo ? 1.0f / (float)k : 0.0f;
-  const int minhaCor = (gx + gy + 1) & 1;
+  if (t == 0) X[ZERO] = 0.0f;
   __syncthreads();
+  const float pes[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+  // The thread's two cells of a level (cells 2s and 2s + 1 of a row, colour e ^ ordem at [e]): index
+  // (-1: none that changes), neighbours, free neighbours, right side.
+  struct Par {
+    int c[2], v[2][4], k[2];
+    float b[2];
+  };
+  auto threads = [&](int l) { return (((s.n[l].nx + 1) >> 1) * s.n[l].ny + 31) & ~31; };
+  auto par = [&](int l, int ordem, int desl, bool blocos) {  // desl: the blocks' shift; blocos: snapshots
+    Par p;
+    const int nx = s.n[l].nx, ny = s.n[l].ny, hw = (nx + 1) >> 1, o = s.off[l], j = t / hw;
 #pragma unroll
-  for (int it = 0; it < VARREDURAS; it++) {
+    for (int e = 0; e < 2; e++) {
+      const int i = 2 * (t % hw) + (((e ^ ordem) + 1 + j) & 1);
+      const bool dentro = j < ny && i < nx;
+      const int c = dentro ? o + i + j * nx : o, vz = dentro ? V[c] : 0, mk = vz & 15;
+      const int bi = (i + desl) & 15, bj = (j + desl) & 15;
+      // a neighbour of the cell's block is read as swept, one outside it from the snapshot
+      p.c[e] = (vz & 16) && mk ? c : -1;
+      p.v[e][0] = !(mk & 1) ? ZERO : (blocos && bi == 0 ? S : 0) + c - 1;
+      p.v[e][1] = !(mk & 2) ? ZERO : (blocos && bi == 15 ? S : 0) + c + 1;
+      p.v[e][2] = !(mk & 4) ? ZERO : (blocos && bj == 0 ? S : 0) + c - nx;
+      p.v[e][3] = !(mk & 8) ? ZERO : (blocos && bj == 15 ? S : 0) + c + nx;
+      p.k[e] = __popc(mk);
+      p.b[e] = X[B + c];
+    }
+    return p;
+  };
+  auto sinc = [&](int n) {
+    if (n == 32) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+  };
+  // one pass over level l by its first threads (whole warps over its cells)
+  auto passo = [&](int l, int desl, int ordem) {
+    const int n = threads(l);
+    if (t >= n) return;
+    const Par p = par(l, ordem, desl, true);
+    float q[2], iq[2];
 #pragma unroll
-    for (int o = 0; o < 2; o++) {
-      int cor = o ^ ordem;
-      if (ativo && minhaCor == cor) {
-        float s = 0.0f;
-        if (m & 1) s += qs[li - 1];
-        if (m & 2) s += qs[li + 1];
-        if (m & 4) s += qs[li - 18];
-        if (m & 8) s += qs[li + 18];
-        float q = qs[li];
-        qs[li] = q + ((s + bv) * invk - q);
+    for (int e = 0; e < 2; e++) {
+      q[e] = p.c[e] >= 0 ? X[p.c[e]] : 0.0f;
+      iq[e] = inversoVizinhos(p.k[e]);
+      if (p.c[e] >= 0) X[S + p.c[e]] = q[e];
+    }
+    sinc(n);
+#pragma unroll 1
+    for (int h = 0; h < VARREDURAS; h++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const float sm = ((X[p.v[e][0]] + X[p.v[e][1]]) + X[p.v[e][2]]) + X[p.v[e][3]];
+        q[e] = q[e] + fmaf(sm + p.b[e], iq[e], -q[e]);
+        if (p.c[e] >= 0) X[p.c[e]] = q[e];
+        sinc(n);
       }
+  };
+  for (int l = 0; l < s.L - 1; l++) {
+    if (!s.uma) {
+      passo(l, 0, 0);
+      __syncthreads();
+    }
+    passo(l, 8, 0);
+    const int nx = s.n[l].nx, ny = s.n[l].ny, N = nx * ny, o = s.off[l];
+    __syncthreads();
+    for (int k = t; k < N; k += nt) {  // residuals into the snapshot array
+      const int c = o + k, vz = V[c];
+      float sm = 0.0f;
+      sm += (vz & 1) ? X[c - 1] : 0.0f;
+      sm += (vz & 2) ? X[c + 1] : 0.0f;
+      sm += (vz & 4) ? X[c - nx] : 0.0f;
+      sm += (vz & 8) ? X[c + nx] : 0.0f;
+      X[S + c] = (vz & 16) ? X[B + c] - fmaf((float)__popc(vz & 15), X[c], -sm) : 0.0f;
+    }
+    __syncthreads();
+    const int gx = s.n[l + 1].nx, G = gx * s.n[l + 1].ny, og = s.off[l + 1];
+    for (int C = t; C < G; C += nt) {
+      const int I = C % gx, J = C / gx;
+      float sm = 0.0f;
+      if (V[og + C] & 16)
+#pragma unroll
+        for (int bb = 0; bb < 4; bb++)
+#pragma unroll
+          for (int aa = 0; aa < 4; aa++) {
+            const int i = 2 * I - 1 + aa, j = 2 * J - 1 + bb;
+            if (i >= 0 && j >= 0 && i < nx && j < ny)
+              sm = __fadd_rn(sm, __fmul_rn(X[S + o + i + j * nx], pes[aa] * pes[bb]));
+          }
+      X[B + og + C] = sm;
+    }
+    __syncthreads();
+  }
+  {  // resolverGrosso (js/pressao-cpu.js:217-238)
+    const int n = threads(s.L - 1);
+    if (t < n) {
+      const Par p = par(s.L - 1, 0, 0, false);
+      const float kf[2] = {(float)p.k[0], (float)p.k[1]};
+      const float iq[2] = {inversoVizinhos(p.k[0]), inversoVizinhos(p.k[1])};
+      auto meia = [&](auto E) {
+        constexpr int e = decltype(E)::value;
+        const float sm = ((X[p.v[e][0]] + X[p.v[e][1]]) + X[p.v[e][2]]) + X[p.v[e][3]];
+        if (p.c[e] >= 0) X[p.c[e]] = dividirViz(sm + p.b[e], kf[e], iq[e]);
+        sinc(n);
+      };
+#pragma unroll 1
+      for (int h = 0; h < VARREDURAS_GROSSO / 2; h++) {
+        meia(std::integral_constant<int, 0>{});
+        meia(std::integral_constant<int, 1>{});
+      }
+      meia(std::integral_constant<int, 0>{});
+    }
+    __syncthreads();
+  }
+  for (int l = s.L - 2; l >= 0; l--) {
+    const int nx = s.n[l].nx, N = nx * s.n[l].ny, o = s.off[l];
+    const int gx = s.n[l + 1].nx, gy = s.n[l + 1].ny, og = s.off[l + 1];
+    for (int k = t; k < N; k += nt) {
+      if (!(V[o + k] & 16)) continue;
+      const int i = k % nx, j = k / nx, I0 = grossoBaseF(i), J0 = grossoBaseF(j);
+      const float wx0 = pesoBaseF(i), wy0 = pesoBaseF(j);
+      float e = 0.0f;
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+          const int I = I0 + a, J = J0 + b;
+          if (I >= 0 && J >= 0 && I < gx && J < gy)
+            e = fmaf(X[og + I + J * gx], (a ? 1.0f - wx0 : wx0) * (b ? 1.0f - wy0 : wy0), e);
+        }
+      X[o + k] = X[o + k] + e;
+    }
+    __syncthreads();
+    passo(l, 8, 1);
+    __syncthreads();
+    if (!s.uma) {
+      passo(l, 0, 1);
       __syncthreads();
     }
   }
-  if (dentro) dst[c] = guardar<T>((vz & 16) ? qs[li] : 0.0f);
-}
-
-// restringir (js/pressao-cpu.js:159-188) as a gather: coarse b = P^T (b - A x) over the 4x4
-// fine window (weights 1/4, 3/4, 3/4, 1/4), only on coarse water cells; coarse x = 0.
-template <class TF>
-__device__ inline float residuoFino(const NivelDev<TF>& f, const TF* __restrict__ x, const TF* __restrict__ b, int i, int j) {
-  if (i < 0 || j < 0 || i >= f.nx || j >= f.ny) return 0.0f;
-  int c = i + j * f.nx;
-  int vz = f.viz[c];
-  if (!(vz & 16)) return 0.0f;
-  float s = 0.0f;
-  if (vz & 1) s += carregar(x[c - 1]);
-  if (vz & 2) s += carregar(x[c + 1]);
-  if (vz & 4) s += carregar(x[c - f.nx]);
-  if (vz & 8) s += carregar(x[c + f.nx]);
-  return carregar(b[c]) - ((float)__popc(vz & 15) * carregar(x[c]) - s);
-}
-
-template <class TF, class TG>
-__global__ void k_restringir(NivelDev<TF> f, const TF* __restrict__ xf, const TF* __restrict__ bf, NivelDev<TG> g) {
-  int C = blockIdx.x * blockDim.x + threadIdx.x;
-  if (C >= g.nx * g.ny || (f.parar && *f.parar)) return;
-  g.x[C] = guardar<TG>(0.0f);
-  if (!(g.viz[C] & 16)) {
-    g.b[C] = guardar<TG>(0.0f);
-    return;
-  }
-  int I = C % g.nx, J = C / g.nx;
-  const float w[4] = {0.25f, 0.75f, 0.75f, 0.25f};
-  float s = 0.0f;
-  for (int bb = 0; bb < 4; bb++) {
-    int j = 2 * J - 1 + bb;
-    for (int a = 0; a < 4; a++) {
-      int i = 2 * I - 1 + a;
-      s += residuoFino(f, xf, bf, i, j) * (w[a] * w[bb]);
-    }
-  }
-  g.b[C] = guardar<TG>(s);
-}
-
-// prolongar (js/pressao-cpu.js:191-214): fine x += bilinear interpolation of the coarse
-// correction, coarse water cells only.
-__device__ inline int grossoBase(int i) { return (i & 1) == 0 ? (i >> 1) - 1 : (i - 1) >> 1; }
-__device__ inline float pesoBase(int i) { return (i & 1) == 0 ? 0.25f : 0.75f; }
-
-template <class TG, class TF>
-__global__ void k_prolongar(NivelDev<TG> g, NivelDev<TF> f, TF* __restrict__ xf) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= f.nx * f.ny || (f.parar && *f.parar)) return;
-  if (!(f.viz[c] & 16)) return;
-  int i = c % f.nx, j = c / f.nx;
-  int I0 = grossoBase(i), J0 = grossoBase(j);
-  float wx0 = pesoBase(i), wy0 = pesoBase(j);
-  float e = 0.0f;
-  for (int b = 0; b < 2; b++) {
-    int J = J0 + b;
-    if (J < 0 || J >= g.ny) continue;
-    float wy = b ? 1.0f - wy0 : wy0;
-    for (int a = 0; a < 2; a++) {
-      int I = I0 + a;
-      if (I < 0 || I >= g.nx) continue;
-      int C = I + J * g.nx;
-      if (g.viz[C] & 16) e += carregar(g.x[C]) * ((a ? 1.0f - wx0 : wx0) * wy);
-    }
-  }
-  xf[c] = guardar<TF>(carregar(xf[c]) + e);
+  for (int c = t; c < s.n[0].nx * s.n[0].ny; c += nt) s.saida[c] = X[c];
 }
 
 // resolverGrosso (js/pressao-cpu.js:217-238): VARREDURAS_GROSSO alternating red-black sweeps
-// in place on the coarsest level, one CTA; the level lives in shared memory when it fits.
-__global__ void __launch_bounds__(1024) k_grosso(NivelDev<float> n, int emShared) {
+// in place on a coarsest level of more than SECAO_PLANA cells, from x = 0, one CTA; the level lives
+// in shared memory when it fits.  65 half-sweeps as in k_secao.
+template <class T>
+__global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
   extern __shared__ unsigned char dyn[];
   if (n.parar && *n.parar) return;  // uniform over the CTA
   const int N = n.nx * n.ny, nx = n.nx;
-  float* x = n.x;
-  const float* b = n.b;
+  float* xs = (float*)dyn;
+  float* bs = xs + N;
+  uint8_t* vs = (uint8_t*)(bs + N);
   const uint8_t* viz = n.viz;
-  if (emShared) {
-    float* xs = (float*)dyn;
-    float* bs = xs + N;
-    uint8_t* vs = (uint8_t*)(bs + N);
+  if (emShared)
     for (int c = threadIdx.x; c < N; c += blockDim.x) {
-      xs[c] = x[c];
-      bs[c] = b[c];
+      xs[c] = 0.0f;
+      bs[c] = carregar(n.b[c]);
       vs[c] = viz[c];
     }
-    x = xs;
-    b = bs;
-    viz = vs;
+  else
+    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = guardar<T>(0.0f);
+  __syncthreads();
+  for (int h = 0; h <= VARREDURAS_GROSSO; h++) {
+    const int cor = h & 1;
+    for (int c = threadIdx.x; c < N; c += blockDim.x) {
+      int i = c % nx, j = c / nx;
+      int vz = emShared ? vs[c] : viz[c];
+      if (!(vz & 16) || ((i + j + 1) & 1) != cor) continue;
+      int q = __popc(vz & 15);
+      if (!q) continue;
+      auto x = [&](int k) { return emShared ? xs[k] : carregar(n.x[k]); };
+      float s = 0.0f;
+      if (vz & 1) s += x(c - 1);
+      if (vz & 2) s += x(c + 1);
+      if (vz & 4) s += x(c - nx);
+      if (vz & 8) s += x(c + nx);
+      const float r = dividirViz(s + (emShared ? bs[c] : carregar(n.b[c])), (float)q, inversoVizinhos(q));
+      if (emShared) xs[c] = r;
+      else n.x[c] = guardar<T>(r);
+    }
     __syncthreads();
   }
-  for (int k = 0; k < VARREDURAS_GROSSO; k++)
-    for (int o = 0; o < 2; o++) {
-      int cor = (k & 1) ? 1 - o : o;
-      for (int c = threadIdx.x; c < N; c += blockDim.x) {
-        int i = c % nx, j = c / nx;
-        int vz = viz[c];
-        if (!(vz & 16) || ((i + j + 1) & 1) != cor) continue;
-        int q = __popc(vz & 15);
-        if (!q) continue;
-        float s = 0.0f;
-        if (vz & 1) s += x[c - 1];
-        if (vz & 2) s += x[c + 1];
-        if (vz & 4) s += x[c - nx];
-        if (vz & 8) s += x[c + nx];
-        x[c] = (s + b[c]) / (float)q;
-      }
-      __syncthreads();
-    }
   if (emShared)
-    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = x[c];
+    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = guardar<T>(xs[c]);
 }
 
 // ---------------------------------------------------------------- PCG kernels
@@ -341,37 +524,29 @@ __global__ void k_bolhas_linhas(Dev d, int modo) {
   else d.apb[b] = d.facesB[b] * d.pb[b] - soma;
 }
 
-// precondicionar, js/pressao-cpu.js:352-361 — before the V-cycle: level-0 b = r, each active
-// bubble's residual spread evenly over its cells; x = 0.  `escala` normalises the right-hand
-// side for half-precision storage (the V-cycle is linear).
+// Level 0's right side made from F on a grid of one level (k_descer makes it elsewhere).
 template <class T>
-__global__ void k_pre_espalhar(Dev d, NivelDev<T> n0, int bolhas) {
+__global__ void k_fonte(NivelDev<T> n0, Fonte F) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N || d.esc->pronto) return;
-  float e = (float)d.esc->escalaMG;
-  float v = d.r[c];
-  if (bolhas && d.tipo[c] == AR) {
-    uint32_t b = d.rotulo[c];
-    if (b >= 2 && b < (uint32_t)MAX_BOLHAS && d.celsB[b] > 0) v = (float)(d.rb[b] / d.celsB[b]);
-  }
-  n0.b[c] = guardar<T>(v * e);
-  n0.x[c] = guardar<T>(0.0f);
+  if (c >= n0.nx * n0.ny || (n0.parar && *n0.parar)) return;
+  float v = F.v[c];
+  if (n0.viz[c] & V0_BOLHA) v = (float)(F.rb[F.rotulo[c]] / F.celsB[F.rotulo[c]]);
+  n0.b[c] = guardar<T>(v * (F.escala ? (float)*F.escala : 1.0f));
 }
-// After the V-cycle: z = x, except active bubble cells, whose mean correction becomes the
-// bubble's z (the transpose of spreading) and whose grid value is zeroed.
+// After the V-cycle (precondicionar, js/pressao-cpu.js:357-361): z = x, except active bubble
+// cells, whose mean correction becomes the bubble's z (the transpose of spreading) and whose grid
+// value is zeroed.
 template <class T>
-__global__ void k_pre_juntar(Dev d, NivelDev<T> n0, int bolhas) {
+__global__ void k_pre_juntar(Dev d, const uint8_t* viz0, const T* x0) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N || d.esc->pronto) return;
   float inv = (float)(1.0 / d.esc->escalaMG);
-  float x = carregar(n0.x[c]) * inv;
-  if (bolhas && d.tipo[c] == AR) {
-    uint32_t b = d.rotulo[c];
-    if (b >= 2 && b < (uint32_t)MAX_BOLHAS && d.celsB[b] > 0) {
-      somaFixa(&d.accB[b], (double)x / d.celsB[b], ESCALA_PCG);
-      d.z[c] = 0.0f;
-      return;
-    }
+  float x = carregar(x0[c]) * inv;
+  if (viz0[c] & V0_BOLHA) {
+    const uint32_t b = d.rotulo[c];
+    somaFixa(&d.accB[b], (double)x / d.celsB[b], ESCALA_PCG);
+    d.z[c] = 0.0f;
+    return;
   }
   d.z[c] = x;
 }
@@ -718,8 +893,10 @@ Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
     // The attribute is per kernel, shared by every solver in the process: it is always raised
     // to the 200 KB cap, never set to this grid's size, which would fail the launches of a
     // solver on a grid with a larger coarsest level.
-    if (cudaFuncSetAttribute(k_grosso, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-      p->smemGrosso = 0;
+    auto subir = [](auto* k) {
+      return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess;
+    };
+    if (!subir(k_grosso<float>) || !subir(k_grosso<__half>) || !subir(k_grosso<__nv_bfloat16>)) p->smemGrosso = 0;
   }
   if (ok && motor == TQ_ENGINE_FUSED) {
     // Grids with a single level (min(nx, ny) <= 12) have nothing to hand to the coarse
@@ -776,101 +953,151 @@ static void comTipo(Pcg* p, int l, F f) {
   else f((__nv_bfloat16*)nullptr);
 }
 
-static void suavizarNivel(Pcg* p, int l, int desl, int ordem, bool paraTmp, cudaStream_t s) {
-  comTipo(p, l, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    NivelDev<T> n = nivel<T>(p, l);
-    dim3 g((n.nx + desl + 15) / 16, (n.ny + desl + 15) / 16);
-    if (paraTmp) lanca(k_suavizar<T>, g, 256, 0, s, n, desl, ordem, n.x, n.tmp, n.b);
-    else lanca(k_suavizar<T>, g, 256, 0, s, n, desl, ordem, n.tmp, n.x, n.b);
-  });
-}
-
-static void restringirNivel(Pcg* p, int l, cudaStream_t s) {
+// Dispatch on the storage types of levels l and l + 1 (16-bit down to some level, FP32 below it).
+template <class F>
+static void comTipos(Pcg* p, int l, F f) {
   comTipo(p, l, [&](auto* tf) {
+    if (p->meia[l] && p->meia[l + 1]) f(tf, tf);
+    else f(tf, (float*)nullptr);
+  });
+}
+
+// The tile of a leg: by blocks a side, the launch's length in rounds of block sweeps, a CTA an SM
+// (two of the smallest tile's) with 16 warps, is waves x rounds; the shortest wins, the smaller tile
+// of equals (a smaller tile sweeps more blocks around it, a larger one leaves SMs without a tile).
+static int escolherLadrilho(int nx, int ny, bool subir, bool uma) {
+  constexpr int SMS = 148;
+  int melhor = 1;
+  long custo = -1;
+  for (int k = 1; k <= 4; k++) {
+    const long n = (long)blocos(nx, 16 * k) * blocos(ny, 16 * k);
+    const long ondas = (n + SMS * (k == 1 ? 2 : 1) - 1) / (SMS * (k == 1 ? 2 : 1));
+    auto voltas = [&](int b) { return (b * b + (k == 1 ? 8 : 15)) / (k == 1 ? 9 : 16); };
+    const int r = uma ? voltas(subir ? k : k + 1) : subir ? voltas(k + 1) + voltas(k) : voltas(k + 2) + voltas(k + 1);
+    const long c = ondas * (r + 2);
+    if (custo < 0 || c < custo) {
+      custo = c;
+      melhor = k;
+    }
+  }
+  return melhor;
+}
+
+template <class K>
+static size_t prepararLadrilho(K kern, int k) {
+  const size_t b = bytesLadrilho(k, k);
+  if (b > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytesLadrilho(4, 4));
+  return b;
+}
+static int threadsLadrilho(int k) { return k == 1 ? 288 : T_LADRILHO; }
+
+// masc: the coarse levels of TQ_PRECOND_BLOCK, whose masks close faces between water cells
+static void descerNivel(Pcg* p, int l, bool bloco, bool uma, const Fonte& F, cudaStream_t s) {
+  uma = uma && l >= 1;
+  const int k = escolherLadrilho(p->nxL[l], p->nyL[l], false, uma);
+  const dim3 gr(blocos(p->nxL[l], 16 * k), blocos(p->nyL[l], 16 * k));
+  comTipos(p, l, [&](auto* tf, auto* tg) {
     using TF = std::remove_pointer_t<decltype(tf)>;
-    comTipo(p, l + 1, [&](auto* tg) {
-      using TG = std::remove_pointer_t<decltype(tg)>;
-      NivelDev<TF> f = nivel<TF>(p, l);
-      NivelDev<TG> g = nivel<TG>(p, l + 1);
-      lanca(k_restringir<TF, TG>, blocos((long)g.nx * g.ny, 256), 256, 0, s, f, f.x, f.b, g);
-    });
-  });
-}
-
-static void prolongarNivel(Pcg* p, int l, cudaStream_t s) {
-  comTipo(p, l + 1, [&](auto* tg) {
     using TG = std::remove_pointer_t<decltype(tg)>;
-    comTipo(p, l, [&](auto* tf) {
-      using TF = std::remove_pointer_t<decltype(tf)>;
-      NivelDev<TG> g = nivel<TG>(p, l + 1);
-      NivelDev<TF> f = nivel<TF>(p, l);
-      lanca(k_prolongar<TG, TF>, blocos((long)f.nx * f.ny, 256), 256, 0, s, g, f, f.x);
-    });
+    const NivelDev<TF> f = nivel<TF>(p, l);
+    const NivelDev<TG> g = nivel<TG>(p, l + 1);
+    auto kern = l == 0 ? k_descer<TF, TG, true> : k_descer<TF, TG, false>;
+    const size_t b = prepararLadrilho(kern, k);
+    lanca(kern, gr, threadsLadrilho(k), b, s, f, g, k, k, uma ? 1 : 0, bloco && l >= 1 ? 1 : 0, F);
+  });
+}
+// xg: the coarse level's x (its result)
+static void subirNivel(Pcg* p, int l, const void* xg, bool bloco, bool uma, float* saida, cudaStream_t s) {
+  uma = uma && l >= 1;
+  const int k = escolherLadrilho(p->nxL[l], p->nyL[l], true, uma), d = uma ? 8 : 0;
+  const dim3 gr(blocos(p->nxL[l] + d, 16 * k), blocos(p->nyL[l] + d, 16 * k));
+  comTipos(p, l, [&](auto* tf, auto* tg) {
+    using TF = std::remove_pointer_t<decltype(tf)>;
+    using TG = std::remove_pointer_t<decltype(tg)>;
+    const size_t b = prepararLadrilho(k_subir<TF, TG>, k);
+    lanca(k_subir<TF, TG>, gr, threadsLadrilho(k), b, s, nivel<TF>(p, l), nivel<TG>(p, l + 1), (const TG*)xg, k, k,
+          uma ? 1 : 0, bloco && l >= 1 ? 1 : 0, saida);
   });
 }
 
-// cicloV (js/pressao-cpu.js:241-255); level-0 b and x = 0 already in place.
-// umaPassada (TQ_PRECOND_BLOCK_1): the levels above 0 take one smoother pass a leg (shift 8), whose
-// output (in tmp) becomes the level's x by swapping the two buffers; each level swaps twice a
-// cycle, so the buffers are back in place at its end (and a captured graph repeats itself).
-static void cicloV(Pcg* p, cudaStream_t s, bool umaPassada = false) {
+// cicloV (js/pressao-cpu.js:241-255) on a right side made from F (level 0's b is written); every
+// level's result ends in its tmp, level 0's returned, or as floats in saida when there is one.
+// umaPassada (TQ_PRECOND_BLOCK_1): the levels above 0 take one smoother pass a leg (shift 8).
+static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bool umaPassada, float* saida) {
   const int L = p->L;
-  auto trocar = [&](int l) { std::swap(p->xL[l], p->tmpL[l]); };
-  for (int l = 0; l < L - 1; l++) {
-    if (umaPassada && l >= 1) {
-      suavizarNivel(p, l, 8, 0, true, s);
-      trocar(l);
-    } else {
-      suavizarNivel(p, l, 0, 0, true, s);
-      suavizarNivel(p, l, 8, 0, false, s);
+  // the section: the coarse levels of at most SECAO_PLANA cells (not level 0)
+  int Ls = L, total = 0;
+  while (Ls > 1 && L - Ls < SECAO_PLANA_NIVEIS && p->nxL[Ls - 1] * p->nyL[Ls - 1] <= SECAO_PLANA &&
+         ((p->nxL[Ls - 1] + 1) / 2) * p->nyL[Ls - 1] <= T_SECAO &&
+         total + p->nxL[Ls - 1] * p->nyL[Ls - 1] <= SECAO_PLANA_TOTAL)
+    Ls--, total += p->nxL[Ls] * p->nyL[Ls];
+  const int Lf = Ls < L ? Ls : L - 1;  // the levels with tile legs: 0 .. Lf - 1
+  for (int l = 0; l < Lf; l++) descerNivel(p, l, bloco, umaPassada, F, s);
+  const void* x;
+  if (Ls < L) {
+    SecaoPlana sp{};
+    sp.L = L - Ls;
+    sp.uma = umaPassada ? 1 : 0;
+    int off = 0;
+    for (int l = Ls; l < L; l++) {
+      sp.n[l - Ls] = nivel<float>(p, l);
+      sp.off[l - Ls] = off;
+      off += p->nxL[l] * p->nyL[l];
     }
-    restringirNivel(p, l, s);
+    sp.saida = (float*)p->tmpL[Ls];
+    x = sp.saida;
+    lanca(k_secao, 1, (((p->nxL[Ls] + 1) / 2) * p->nyL[Ls] + 31) & ~31, 0, s, sp);
+  } else {
+    comTipo(p, L - 1, [&](auto* t) {
+      using T = std::remove_pointer_t<decltype(t)>;
+      lanca(k_grosso<T>, 1, 1024, p->smemGrosso, s, nivel<T>(p, L - 1), p->smemGrosso ? 1 : 0);
+    });
+    x = p->xL[L - 1];
   }
-  NivelDev<float> g = nivel<float>(p, L - 1);
-  if (L == 1) cudaMemsetAsync(g.x, 0, sizeof(float) * g.nx * g.ny, s);
-  lanca(k_grosso, 1, 1024, p->smemGrosso, s, g, p->smemGrosso ? 1 : 0);
-  for (int l = L - 2; l >= 0; l--) {
-    prolongarNivel(p, l, s);
-    if (umaPassada && l >= 1) {
-      suavizarNivel(p, l, 8, 1, true, s);
-      trocar(l);
-    } else {
-      suavizarNivel(p, l, 8, 1, true, s);
-      suavizarNivel(p, l, 0, 1, false, s);
-    }
+  for (int l = Lf - 1; l >= 0; l--) {
+    subirNivel(p, l, x, bloco, umaPassada, l == 0 ? saida : nullptr, s);
+    x = p->tmpL[l];
   }
+  return x;
+}
+
+static void fonteNivelUnico(Pcg* p, const Fonte& F, cudaStream_t s) {
+  if (p->L > 1) return;
+  comTipo(p, 0, [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    lanca(k_fonte<T>, blocos(p->N, 256), 256, 0, s, nivel<T>(p, 0), F);
+  });
 }
 
 // Types and neighbour masks of every level for this solve (bloco: TQ_PRECOND_BLOCK's coarse
 // masks from the fine faces).
-static void prepararNiveis(Pcg* p, const uint8_t* tipo0, bool bloco, cudaStream_t s) {
+static void prepararNiveis(Pcg* p, const uint8_t* tipo0, bool bloco, cudaStream_t s, bool comNivel0 = true) {
   if (tipo0 != p->tipoL[0]) cudaMemcpyAsync(p->tipoL[0], tipo0, p->N, cudaMemcpyDeviceToDevice, s);
-  for (int l = 1; l < p->L; l++)
-    lanca(k_mg_tipo_grosso, blocos((long)p->nxL[l] * p->nyL[l], 256), 256, 0, s, p->tipoL[l - 1], p->nxL[l - 1],
-          p->nyL[l - 1], p->tipoL[l], p->nxL[l], p->nyL[l]);
+  Niveis n{};
+  n.L = p->L;
+  const int l0 = comNivel0 ? 0 : 1;
   for (int l = 0; l < p->L; l++) {
-    const int nb = blocos((long)p->nxL[l] * p->nyL[l], 256);
-    if (bloco && l >= 1)
-      lanca(k_viz_faces, nb, 256, 0, s, p->tipoL[l - 1], p->nxL[l - 1], p->nyL[l - 1], p->tipoL[l], p->nxL[l],
-            p->nyL[l], p->vizL[l]);
-    else
-      lanca(k_viz, nb, 256, 0, s, p->tipoL[l], p->nxL[l], p->nyL[l], p->vizL[l]);
+    n.nx[l] = p->nxL[l];
+    n.ny[l] = p->nyL[l];
+    n.tipo[l] = p->tipoL[l];
+    n.viz[l] = p->vizL[l];
+    n.ini[l + 1] = n.ini[l] + (l >= l0 ? n.nx[l] * n.ny[l] : 0);
   }
+  for (int l = 0; l < p->L - 1; l += NIVEIS_POR_VEZ)
+    lanca(k_niveis_tipos, dim3(blocos(n.nx[l], 64), blocos(n.ny[l], 64)), 256, 0, s, n, l);
+  if (n.ini[p->L] > 0) lanca(k_niveis_viz, blocos(n.ini[p->L], 256), 256, 0, s, n, l0, bloco ? 1 : 0);
 }
 
 static void precondicionar(Pcg* p, const Dev& d, bool bolhas, bool bloco, bool umaPassada, cudaStream_t s) {
   int nb = blocos(d.N, 256);
+  Fonte F{d.r, &d.esc->escalaMG, d.rotulo, d.rb, d.celsB};
+  fonteNivelUnico(p, F, s);
+  const void* x = cicloV(p, F, s, bloco, umaPassada, nullptr);
   const bool espalhar = bolhas && !bloco;  // with BLOCK the V-cycle does not see the bubbles
-  comTipo(p, 0, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    lanca(k_pre_espalhar<T>, nb, 256, 0, s, d, nivel<T>(p, 0), espalhar ? 1 : 0);
-  });
-  cicloV(p, s, umaPassada);
   if (espalhar) cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
   comTipo(p, 0, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
-    lanca(k_pre_juntar<T>, nb, 256, 0, s, d, nivel<T>(p, 0), espalhar ? 1 : 0);
+    lanca(k_pre_juntar<T>, nb, 256, 0, s, d, p->vizL[0], (const T*)x);
   });
   if (bolhas) lanca(k_pre_bolhas, blocos(MAX_BOLHAS, 256), 256, 0, s, d, bloco ? 1 : 0);
 }
@@ -907,9 +1134,8 @@ int resolverPressao(Pcg* p, const Dev& d0, int iteracoes, double tol, bool bolha
   const int nb = blocos(d.N, 256);
   const int nbx = blocos(d.N > MAX_BOLHAS ? d.N : MAX_BOLHAS, 256);
   // operator (true types) and preconditioner types
-  lanca(k_viz, nb, 256, 0, s, d.tipo, d.nx, d.ny, p->vizOp);
-  lanca(k_mg_tipo0, nb, 256, 0, s, d.tipo, d.rotulo, p->tipoL[0], d.N, bolhas ? 1 : 0, bloco ? 1 : 0);
-  prepararNiveis(p, p->tipoL[0], bloco, s);
+  lanca(k_mg_tipo0, nb, 256, 0, s, d.tipo, d.rotulo, p->tipoL[0], p->vizOp, d.nx, d.ny, bolhas ? 1 : 0, bloco ? 1 : 0);
+  prepararNiveis(p, p->tipoL[0], bloco, s, false);
   cudaMemsetAsync(d.facesB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
   cudaMemsetAsync(d.celsB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
   // the previous solve left its stop flag set: clear it before the first kernel that tests it
@@ -919,6 +1145,7 @@ int resolverPressao(Pcg* p, const Dev& d0, int iteracoes, double tol, bool bolha
     lanca(k_bolhas_faces, nb, 256, 0, s, d);
     lanca(k_bolhas_celulas, nb, 256, 0, s, d);
   }
+  lanca(k_viz0, nb, 256, 0, s, d, p->tipoL[0], p->vizL[0], bolhas && !bloco ? 1 : 0);
   lanca(k_bolhas_inicio, blocos(MAX_BOLHAS, 256), 256, 0, s, d);
   lanca(k_pcg_inicio, nb, 256, 0, s, d, p->vizOp, bolhas ? 1 : 0, q64);
   if (bolhas) {
@@ -993,32 +1220,22 @@ int lerPerfilPcg(Pcg* p, unsigned long long* out, int cap) { return lerPerfilFun
 
 // One V-cycle on caller-provided device buffers (tq_vcycle).
 template <class T>
-__global__ void k_carregar_b(NivelDev<T> n0, const float* b) {
+__global__ void k_descarregar_x(const T* x0, float* x, int N) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n0.nx * n0.ny) return;
-  n0.b[c] = guardar<T>(b[c]);
-  n0.x[c] = guardar<T>(0.0f);
-}
-template <class T>
-__global__ void k_descarregar_x(NivelDev<T> n0, float* x) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n0.nx * n0.ny) return;
-  x[c] = carregar(n0.x[c]);
+  if (c < N) x[c] = carregar(x0[c]);
 }
 int cicloVDispositivo(Pcg* p, const uint8_t* tipo, const float* b, float* x, cudaStream_t s, bool preparar,
                       const int* parar) {
   if (preparar) prepararNiveis(p, tipo, false, s);
   p->parar = parar;  // the cycle's kernels return at once while *parar != 0
-  int nb = blocos(p->N, 256);
-  comTipo(p, 0, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    lanca(k_carregar_b<T>, nb, 256, 0, s, nivel<T>(p, 0), b);
-  });
-  cicloV(p, s);
-  comTipo(p, 0, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    lanca(k_descarregar_x<T>, nb, 256, 0, s, nivel<T>(p, 0), x);
-  });
+  Fonte F{b};
+  fonteNivelUnico(p, F, s);
+  const void* r = cicloV(p, F, s, false, false, x);
+  if (p->L == 1)
+    comTipo(p, 0, [&](auto* tag) {
+      using T = std::remove_pointer_t<decltype(tag)>;
+      lanca(k_descarregar_x<T>, blocos(p->N, 256), 256, 0, s, (const T*)r, x, p->N);
+    });
   p->parar = nullptr;
   return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_E_CUDA;
 }

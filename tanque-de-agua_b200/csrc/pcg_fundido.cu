@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "pcg_interno.cuh"
+#include "suavizador.cuh"
 
 namespace tq {
 
@@ -425,18 +426,9 @@ constexpr int OP_AGUA = 16, OP_FACE = 32, OP_VIZ_BOLHA = 64, OP_BOLHA = 128;
 // Level 0's neighbour masks also carry, above bits 0-4, the cell's OP_BOLHA and OP_AGUA.
 constexpr int V0_BOLHA = 32, V0_AGUA = 64;
 
-__device__ __forceinline__ int grossoBaseF(int i) { return (i & 1) == 0 ? (i >> 1) - 1 : (i - 1) >> 1; }
-__device__ __forceinline__ float pesoBaseF(int i) { return (i & 1) == 0 ? 0.25f : 0.75f; }
-
-// ---------------------------------------------------------------- block sweeps
-// 1/k for k free neighbours (k = 1..4), the correctly rounded float constants.
-__device__ __forceinline__ float inversoVizinhos(int k) {
-  return k == 1 ? 1.0f : k == 2 ? 0.5f : k == 3 ? (1.0f / 3.0f) : 0.25f;
-}
-
 // ---------------------------------------------------------------- grid-level smoother
 // Modes of a smoother pass over a grid level:
-//   M_NORMAL   snapshot = src, right side = b;
+//   M_NORMAL   snapshot = src, right side = b (on the way down; M_VOLTA, the same on the way up);
 //   M_PROL     snapshot = x + P(x_coarse) (prolongar, js/pressao-cpu.js:191-214), built while
 //              loading: the first pass on the way up;
 //   M_ZERO     snapshot = 0: the first pass on the way down, whose x the restriction (or the
@@ -446,7 +438,9 @@ __device__ __forceinline__ float inversoVizinhos(int k) {
 //   M_JUNTAR   level 0, last pass: instead of storing x, gathers z = x / escala (:357-361),
 //              bubble cells' share into the bubble's fixed-point sum, and the partials of r.z
 //              and r.zOld.
-enum { M_NORMAL = 0, M_PROL = 1, M_ZERO = 2, M_ESPALHAR = 3, M_JUNTAR = 4 };
+enum { M_NORMAL = 0, M_PROL = 1, M_ZERO = 2, M_ESPALHAR = 3, M_JUNTAR = 4, M_VOLTA = 5 };
+// Red-black on the way down, black-red up: each mode belongs to one leg.
+__host__ __device__ constexpr int ordemDe(int modo) { return modo == M_PROL || modo == M_JUNTAR || modo == M_VOLTA; }
 
 // What the spread and the gather need (level 0).
 struct Reuniao {
@@ -454,80 +448,6 @@ struct Reuniao {
   float* zNovo;
   const float* zVelho;   // previous z (r.zOld), or null
 };
-
-// ---------------------------------------------------------------- register-resident block sweep
-// Lane l of the warp that owns a 16x16 block holds, for each colour c and m = 0..3, the cell of
-// colour c in row 4g + m (g = l >> 3) among the columns 2k, 2k + 1 (k = l & 7): its column is
-// (c + 1 + m) & 1, since a cell's colour is (row + column + 1) & 1 (js/pressao-cpu.js:120).  It
-// also holds the block's frame next to its cells: left and right of its rows (k = 0, k = 7),
-// below and above its columns (g = 0, g = 3).  In a half-sweep of colour COR every neighbour of
-// an updated cell has the other colour: the lane's own other cell in the row, the rows m -/+ 1
-// of the lane (same column), the row in lane l -/+ 1, the row below row 0 in lane l - 8 (its
-// m = 3), the row above row 3 in lane l + 8 (its m = 0), or the frame: 6 shuffles a half-sweep,
-// which keeps the shuffle pipe, shared by the SM's warps, half as busy as rows g + 4m would.
-// A half-sweep reads no value that it writes.
-// Every snapshot holds x = 0 on cells that are not water (the passes store 0 there, the frame
-// outside the grid is 0), so a wall neighbour adds +0 and the sum needs no mask; only 1/k and
-// whether the cell changes come from the mask.  The exception is TQ_PRECOND_BLOCK's coarse
-// levels, whose masks close faces between two water cells across a thin wall: with `masc` the
-// neighbours the mask leaves out are dropped from the sum (masc is uniform over the grid).
-struct Moldura {
-  float esq[4], dir[4];  // frame left / right of the lane's rows (k = 0 / k = 7)
-  float bai[2], cim[2];  // frame below / above the lane's columns (g = 0 / g = 3), by column
-};
-
-template <int COR>
-__device__ __forceinline__ void meiaReg(float (&x)[2][4], const float (&bq)[2][4], const float (&iq)[2][4],
-                                        const float (&at)[2][4], const Moldura& f, const int (&v)[2][4], bool masc) {
-  const int lane = threadIdx.x & 31, g = lane >> 3, k = lane & 7;
-  float H[4];
-#pragma unroll
-  for (int m = 0; m < 4; m++)  // row m's neighbour in lane l + 1 (colour COR in the odd column) or l - 1
-    H[m] = __shfl_sync(0xffffffffu, x[1 - COR][m], (((COR + 1 + m) & 1) ? lane + 1 : lane - 1) & 31);
-  const float D = __shfl_sync(0xffffffffu, x[1 - COR][3], (lane - 8) & 31);
-  const float U = __shfl_sync(0xffffffffu, x[1 - COR][0], (lane + 8) & 31);
-#pragma unroll
-  for (int m = 0; m < 4; m++) {
-    const int jc = (COR + 1 + m) & 1;  // the column of colour COR in row m
-    const float y = x[1 - COR][m];
-    float esq = jc ? y : (k == 0 ? f.esq[m] : H[m]);
-    float dir = jc ? (k == 7 ? f.dir[m] : H[m]) : y;
-    float baixo = m >= 1 ? x[1 - COR][m >= 1 ? m - 1 : 0] : (g >= 1 ? D : f.bai[jc]);
-    float cima = m <= 2 ? x[1 - COR][m <= 2 ? m + 1 : 3] : (g <= 2 ? U : f.cim[jc]);
-    if (masc) {
-      const int mk = v[COR][m];
-      esq = (mk & 1) ? esq : 0.0f;
-      dir = (mk & 2) ? dir : 0.0f;
-      baixo = (mk & 4) ? baixo : 0.0f;
-      cima = (mk & 8) ? cima : 0.0f;
-    }
-    const float sm = ((esq + dir) + baixo) + cima;
-    const float q = x[COR][m];
-    const float dlt = (sm + bq[COR][m]) * iq[COR][m] - q;
-    x[COR][m] = fmaf(at[COR][m], dlt, q);  // at = 1 (the cell changes) or 0: exact either way
-  }
-}
-
-// The VARREDURAS red-black sweeps (js/pressao-cpu.js:114-137) of the warp's block in registers;
-// v = neighbour mask | 16 water | 128 in grid, bq = right side; ordem 0 sweeps colour 0 first.
-__device__ __forceinline__ void varrerReg(float (&x)[2][4], const int (&v)[2][4], const float (&bq)[2][4],
-                                         const Moldura& f, int ordem, bool masc, int nVarr) {
-  float iq[2][4], at[2][4];
-#pragma unroll
-  for (int c = 0; c < 2; c++)
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-      const int mk = v[c][m] & 15;
-      iq[c][m] = inversoVizinhos(__popc(mk));
-      at[c][m] = ((v[c][m] & 16) && mk) ? 1.0f : 0.0f;
-    }
-  // rolled loop: the pass code stays small in the instruction cache, which each phase enters cold
-#pragma unroll 1
-  for (int h = 0; h < 2 * nVarr; h++) {
-    if (((h & 1) ^ ordem) == 0) meiaReg<0>(x, bq, iq, at, f, v, masc);
-    else meiaReg<1>(x, bq, iq, at, f, v, masc);
-  }
-}
 
 // Bilinear coarse correction at fine cell (sx, sy) from the 11x11 coarse tile ct whose origin is
 // (cx0, cy0) (prolongar, js/pressao-cpu.js:191-214).
@@ -548,7 +468,7 @@ __device__ __forceinline__ float correcaoGrossa(const float* ct, int cx0, int cy
 // meiaReg).  Every global load of the block (cells, frame, flags, right side; with PROL the
 // coarse tile) goes out in one batch.
 template <class T, int MODO>
-__device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, int blk, int nbx, int desl, int ordem,
+__device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, int blk, int nbx, int desl, bool masc,
                                               const T* src, T* dst, float* area, const NivelF& g,
                                               const float* xcSecao, const Reuniao& ru, double& s0, double& s1) {
   constexpr bool PROL = MODO == M_PROL;
@@ -701,7 +621,9 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
   for (int cr = 0; cr < 2; cr++)
 #pragma unroll
     for (int m = 0; m < 4; m++) mexe |= (v[cr][m] & 16) && (v[cr][m] & 15);
-  if (__any_sync(0xffffffffu, mexe)) varrerReg(x, v, bq, f, ordem, a.bloco != 0, a.varreduras);
+  // (level 0's masks close no face between water cells: x = 0 off water, so it needs no masking)
+  if (__any_sync(0xffffffffu, mexe))
+    varrerReg(x, v, bq, f, ordemDe(MODO), MODO != M_ESPALHAR && MODO != M_JUNTAR && masc, a.varreduras);
   if (MODO == M_JUNTAR) {
     const float inv = 1.0f / ru.escala;
     float rv[2][4], zv[2][4];
@@ -773,7 +695,7 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
 }
 
 template <class T, int MODO>
-__device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, int ordem, bool paraTmp, float* areas,
+__device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, bool paraTmp, float* areas,
                                            const Reuniao& ru, double* sh) {
   const NivelF n = s_niv[l];
   const int nbx = (n.nx + desl + 15) >> 4, nby = (n.ny + desl + 15) >> 4;
@@ -792,22 +714,22 @@ __device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, int o
   const int tot = WARPS * gridDim.x, exc = nb - tot;
   const int tw = w * gridDim.x + blockIdx.x;  // the warp's first block index
   auto blocoDe = [&](int t) { return exc > 0 ? nb - 1 - (t + exc) % nb : t; };
-  if (a.sol[l]) {
-    // Blocks of wall alone are skipped: their cells hold x = 0 in both snapshots (zeroed before
-    // the solve, and a pass writes 0 off water) and b = 0, so a pass would rewrite the same
-    // zeros.  The flags of the warp's first 32 blocks come in one load, lane k's for its k-th.
-    const uint8_t* fl = a.sol[l] + (desl ? blocosNivel(n.nx, n.ny, 0) : 0);
+  // Blocks of wall alone are skipped on the levels that flag them: their cells hold x = 0 in both
+  // snapshots (zeroed before the solve, and a pass writes 0 off water) and b = 0, so a pass would
+  // rewrite the same zeros.  The flags of the warp's first 32 blocks come in one load, lane k's for
+  // its k-th.
+  const uint8_t* fl = a.sol[l] ? a.sol[l] + (desl ? blocosNivel(n.nx, n.ny, 0) : 0) : nullptr;
+  unsigned paredes = 0;
+  if (fl) {
     const int tk = tw + (threadIdx.x & 31) * tot;
-    const unsigned paredes = __ballot_sync(0xffffffffu, tk < nb && ldcg8(fl + blocoDe(tk)) != 0);
-    int k = 0;
-    for (int t = tw; t < nb; t += tot, k++) {
-      const int blk = blocoDe(t);
-      if (k < 32 ? (paredes >> k) & 1u : ldcg8(fl + blk) != 0) continue;
-      suavizarBloco<T, MODO>(a, n, blk, nbx, desl, ordem, src, dst, area, g, xcSecao, ru, s0, s1);
-    }
-  } else {
-    for (int t = tw; t < nb; t += tot)
-      suavizarBloco<T, MODO>(a, n, blocoDe(t), nbx, desl, ordem, src, dst, area, g, xcSecao, ru, s0, s1);
+    paredes = __ballot_sync(0xffffffffu, tk < nb && ldcg8(fl + blocoDe(tk)) != 0);
+  }
+  const bool masc = a.bloco && l >= 1;
+  int k = 0;
+  for (int t = tw; t < nb; t += tot, k++) {
+    const int blk = blocoDe(t);
+    if (fl && (k < 32 ? (paredes >> k) & 1u : ldcg8(fl + blk) != 0)) continue;
+    suavizarBloco<T, MODO>(a, n, blk, nbx, desl, masc, src, dst, area, g, xcSecao, ru, s0, s1);
   }
   if (MODO == M_JUNTAR) {
     const double t0 = somaBloco(s0, sh);
@@ -822,17 +744,15 @@ __device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, int o
 // Every grid level below the coarse section is stored as T (criarFundido), so a 16-bit kernel
 // carries no FP32 copy of the passes: smaller code, which each phase enters cold.
 template <class T>
-__device__ void faseSuavizar(const Args& a, int l, int desl, int ordem, bool paraTmp, int modo, float* areas, int meia,
-                             const Reuniao& ru, double* sh) {
-  (void)meia;
-  {
-    switch (modo) {
-      case M_PROL: faseSuavizarT<T, M_PROL>(a, l, desl, ordem, paraTmp, areas, ru, sh); break;
-      case M_ZERO: faseSuavizarT<T, M_ZERO>(a, l, desl, ordem, paraTmp, areas, ru, sh); break;
-      case M_ESPALHAR: faseSuavizarT<T, M_ESPALHAR>(a, l, desl, ordem, paraTmp, areas, ru, sh); break;
-      case M_JUNTAR: faseSuavizarT<T, M_JUNTAR>(a, l, desl, ordem, paraTmp, areas, ru, sh); break;
-      default: faseSuavizarT<T, M_NORMAL>(a, l, desl, ordem, paraTmp, areas, ru, sh);
-    }
+__device__ void faseSuavizar(const Args& a, int l, int desl, bool paraTmp, int modo, float* areas, const Reuniao& ru,
+                             double* sh) {
+  switch (modo) {
+    case M_PROL: faseSuavizarT<T, M_PROL>(a, l, desl, paraTmp, areas, ru, sh); break;
+    case M_ZERO: faseSuavizarT<T, M_ZERO>(a, l, desl, paraTmp, areas, ru, sh); break;
+    case M_ESPALHAR: faseSuavizarT<T, M_ESPALHAR>(a, l, desl, paraTmp, areas, ru, sh); break;
+    case M_JUNTAR: faseSuavizarT<T, M_JUNTAR>(a, l, desl, paraTmp, areas, ru, sh); break;
+    case M_VOLTA: faseSuavizarT<T, M_VOLTA>(a, l, desl, paraTmp, areas, ru, sh); break;
+    default: faseSuavizarT<T, M_NORMAL>(a, l, desl, paraTmp, areas, ru, sh);
   }
 }
 
@@ -990,7 +910,7 @@ __device__ __forceinline__ void sincEquipe(const Equipe& q) {
 struct Ret {
   int x0, y0, x1, y1;  // inclusive
 };
-__device__ void passoS(float* F, const uint8_t* U, const NivelS n, int desl, int ordem, int src, int dst, bool masc,
+__device__ __noinline__ void passoS(float* F, const uint8_t* U, const NivelS n, int desl, int ordem, int src, int dst, bool masc,
                        int nVarr, const Equipe& eq, const Ret& r) {
   const int lane = threadIdx.x & 31, w = eq.ti >> 5, gl = lane >> 3, k = lane & 7;
   const int nx = n.nx, ny = n.ny;
@@ -1568,15 +1488,14 @@ template <class T>
 __device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char* smem, NivelS* tabS,
                        const Reuniao& ru, double* sh, bool secaoDensa) {
   for (int l = 0; l < a.Lc; l++) {
-    const int meia = s_niv[l].meia;
     if (a.umaPassada && l >= 1) {
-      faseSuavizar<T>(a, l, 8, 0, true, M_ZERO, areas, meia, ru, sh);
+      faseSuavizar<T>(a, l, 8, true, M_ZERO, areas, ru, sh);
       trocarXTmp(l);
       if (!barreira(a, ep)) return false;
     } else {
-      faseSuavizar<T>(a, l, 0, 0, true, l == 0 ? M_ESPALHAR : M_ZERO, areas, meia, ru, sh);
+      faseSuavizar<T>(a, l, 0, true, l == 0 ? M_ESPALHAR : M_ZERO, areas, ru, sh);
       if (!barreira(a, ep)) return false;
-      faseSuavizar<T>(a, l, 8, 0, false, M_NORMAL, areas, meia, ru, sh);
+      faseSuavizar<T>(a, l, 8, false, M_NORMAL, areas, ru, sh);
       if (!barreira(a, ep)) return false;
     }
     faseRestringir<T>(a, l, areas);
@@ -1586,15 +1505,14 @@ __device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char*
   else if (blockIdx.x == 0) secaoGrossa(a, smem, smem, tabS, -1, Equipe{(int)threadIdx.x, TF, 0}, true);
   if (!barreira(a, ep)) return false;
   for (int l = a.Lc - 1; l >= 0; l--) {
-    const int meia = s_niv[l].meia;
-    faseSuavizar<T>(a, l, 8, 1, true, M_PROL, areas, meia, ru, sh);
+    faseSuavizar<T>(a, l, 8, true, M_PROL, areas, ru, sh);
     if (a.umaPassada && l >= 1) {
       trocarXTmp(l);
       if (!barreira(a, ep)) return false;
       continue;
     }
     if (!barreira(a, ep)) return false;
-    faseSuavizar<T>(a, l, 0, 1, false, l == 0 ? M_JUNTAR : M_NORMAL, areas, meia, ru, sh);
+    faseSuavizar<T>(a, l, 0, false, l == 0 ? M_JUNTAR : M_VOLTA, areas, ru, sh);
     if (!barreira(a, ep)) return false;
   }
   return true;
