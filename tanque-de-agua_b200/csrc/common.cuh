@@ -124,8 +124,7 @@ struct Dev {
   uint8_t* vivo;
   uint32_t *volB, *facesB, *celsB;
   long long* accB;  // fixed-point per-bubble sums
-  double *rhsB, *yB, *rb, *zb, *zvb, *pb, *apb;
-  float *ybf, *pbf;  // bubble values as the f32 grid sees them
+  double *rhsB, *yB, *rb, *zb, *pb, *apb;
   // PCG vectors
   float *r, *z, *zOld, *p, *ap;
   // reductions

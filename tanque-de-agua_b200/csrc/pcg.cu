@@ -25,21 +25,30 @@ constexpr int V0_BOLHA = 32, V0_AGUA = 64;
 
 // ---------------------------------------------------------------- types and neighbours
 // The preconditioner's level-0 types: bubble air counts as water (js/pressao-cpu.js:305-308); with
-// TQ_PRECOND_BLOCK (bloco) it stays air.  And the operator's free neighbours (bits 0-3) of every
-// cell, from the true types.
-__global__ void k_mg_tipo0(const uint8_t* tipo, const uint32_t* rot, uint8_t* t0, uint8_t* vizOp, int nx, int ny,
-                           int bolhas, int bloco) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nx * ny) return;
-  const int i = c % nx, j = c / nx;
-  uint8_t t = tipo[c];
+// TQ_PRECOND_BLOCK (bloco) it stays air.  The operator's free neighbours (bits 0-3) of every cell,
+// from the true types.  And the bubbles' faces (montarBolhas, js/pressao-cpu.js:271-288): the (interior
+// bubble cell, water neighbour) pairs of each label; a label with any is an active bubble.
+__global__ void k_plano_tipos(Dev d, uint8_t* t0, uint8_t* vizOp, int bolhas, int bloco) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= d.N) return;
+  const int nx = d.nx, ny = d.ny, i = c % nx, j = c / nx;
+  const int viz[4] = {i > 0 ? d.tipo[c - 1] : SOLIDO, i < nx - 1 ? d.tipo[c + 1] : SOLIDO,
+                      j > 0 ? d.tipo[c - nx] : SOLIDO, j < ny - 1 ? d.tipo[c + nx] : SOLIDO};
+  uint8_t t = d.tipo[c];
   int m = 0;
-  if (i > 0 && tipo[c - 1] != SOLIDO) m |= 1;
-  if (i < nx - 1 && tipo[c + 1] != SOLIDO) m |= 2;
-  if (j > 0 && tipo[c - nx] != SOLIDO) m |= 4;
-  if (j < ny - 1 && tipo[c + nx] != SOLIDO) m |= 8;
+#pragma unroll
+  for (int q = 0; q < 4; q++) m |= (viz[q] != SOLIDO) << q;
   vizOp[c] = (uint8_t)m;
-  if (bolhas && !bloco && t == AR && rot[c] >= 2) t = AGUA;
+  if (bolhas && t == AR) {
+    const uint32_t b = d.rotulo[c];
+    if (b >= 2) {
+      if (!bloco) t = AGUA;
+      if (b < (uint32_t)MAX_BOLHAS && i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1) {
+        const unsigned k = (viz[0] == AGUA) + (viz[1] == AGUA) + (viz[2] == AGUA) + (viz[3] == AGUA);
+        if (k) atomicAdd(&d.facesB[b], k);
+      }
+    }
+  }
   t0[c] = t;
 }
 
@@ -82,26 +91,6 @@ __global__ void __launch_bounds__(256) k_niveis_tipos(Niveis n, int l0) {
     }
     __syncthreads();
   }
-}
-
-// Level 0's masks in a solve: k_niveis_viz's bits and V0_AGUA; V0_BOLHA where `bolhas` (celsB counted).
-__global__ void k_viz0(Dev d, const uint8_t* tipo0, uint8_t* viz, int bolhas) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx, j = c / d.nx;
-  int m = 0;
-  if (i > 0 && tipo0[c - 1] != SOLIDO) m |= 1;
-  if (i < d.nx - 1 && tipo0[c + 1] != SOLIDO) m |= 2;
-  if (j > 0 && tipo0[c - d.nx] != SOLIDO) m |= 4;
-  if (j < d.ny - 1 && tipo0[c + d.nx] != SOLIDO) m |= 8;
-  if (tipo0[c] == AGUA) m |= 16;
-  const int t = d.tipo[c];
-  if (t == AGUA) m |= V0_AGUA;
-  else if (bolhas && t == AR) {
-    const uint32_t b = d.rotulo[c];
-    if (b >= 2 && b < (uint32_t)MAX_BOLHAS && d.celsB[b] > 0) m |= V0_BOLHA;
-  }
-  viz[c] = (uint8_t)m;
 }
 
 // prepararVizinhos (js/pressao-cpu.js:44-60) of every level from l0 on in one launch, packed in one byte:
@@ -179,27 +168,14 @@ __global__ void __launch_bounds__(T_LADRILHO) k_descer(NivelDev<T> n, NivelDev<T
       [&](int c, float x) { n.x[c] = guardar<T>(x); }, [&](int C, float v) { g.b[C] = guardar<TG>(v); });
 }
 
-// The way up a level: x + the coarse correction and both passes, the level's result in n.tmp, or
-// (saida not null) as floats in saida.
-template <class T, class TG>
-__global__ void __launch_bounds__(T_LADRILHO) k_subir(NivelDev<T> n, NivelDev<TG> g, const TG* xg, int kx, int ky,
-                                                      int uma, int masc, float* saida) {
-  extern __shared__ __align__(16) float mem[];
-  if (n.parar && *n.parar) return;
-  const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
-  subirLadrilho<T>(
-      L, g.nx, g.ny, uma != 0, masc != 0, VARREDURAS, mem, [&](int c) { return carregar(n.x[c]); },
-      [&](int C) { return carregar(xg[C]); }, [&](int c) { return carregar(n.b[c]); },
-      [&](const int (&cel)[2][4], const int (&v)[2][4], const float (&x)[2][4]) {
-#pragma unroll
-        for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-          for (int m = 0; m < 4; m++)
-            if (cel[cr][m] >= 0) {
-              if (saida) saida[cel[cr][m]] = arredondar<T>(x[cr][m]);
-              else n.tmp[cel[cr][m]] = guardar<T>(x[cr][m]);
-            }
-      });
+// Level 0's right side made from F on a grid of one level (k_descer makes it elsewhere).
+template <class T>
+__global__ void k_fonte(NivelDev<T> n0, Fonte F) {
+  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n0.nx * n0.ny || (n0.parar && *n0.parar)) return;
+  float v = F.v[c];
+  if (n0.viz[c] & V0_BOLHA) v = (float)(F.rb[F.rotulo[c]] / F.celsB[F.rotulo[c]]);
+  n0.b[c] = guardar<T>(v * (F.escala ? (float)*F.escala : 1.0f));
 }
 
 // The coarse levels of at most SECAO_PLANA cells in one CTA, in shared memory: x as swept, its snapshot
@@ -428,172 +404,415 @@ __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
 }
 
 // ---------------------------------------------------------------- PCG kernels
-// Value a water cell's neighbour contributes to A*v (js/pressao-cpu.js:84-93 after difundir,
-// :318-324): water -> v, air of an active bubble -> that bubble's value (as stored in the
-// f32 grid), anything else -> 0.
-__device__ inline float valorViz(const Dev& d, const float* v, const float* vbf, int n, bool bolhas) {
-  uint8_t t = d.tipo[n];
-  if (t == AGUA) return v[n];
-  if (bolhas && t == AR) {
-    uint32_t r = d.rotulo[n];
-    if (r >= 2 && r < (uint32_t)MAX_BOLHAS && d.facesB[r] > 0) return vbf[r];
-  }
-  return 0.0f;
-}
-__device__ inline float aplicarA(const Dev& d, const uint8_t* vizOp, const float* v, const float* vbf, int c, bool bolhas) {
-  int vz = vizOp[c];
-  float s = 0.0f;
-  if (vz & 1) s += valorViz(d, v, vbf, c - 1, bolhas);
-  if (vz & 2) s += valorViz(d, v, vbf, c + 1, bolhas);
-  if (vz & 4) s += valorViz(d, v, vbf, c - d.nx, bolhas);
-  if (vz & 8) s += valorViz(d, v, vbf, c + d.nx, bolhas);
-  return (float)__popc(vz & 15) * v[c] - s;
-}
-
-// r = -div - A q on water cells (js/pressao-cpu.js:331-338); q = 0 elsewhere.
-__global__ void k_pcg_inicio(Dev d, const uint8_t* vizOp, int bolhas, double* q64) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  if (d.tipo[c] != AGUA) {
-    d.q[c] = 0.0f;
-    d.r[c] = 0.0f;
-    return;
-  }
-  d.r[c] = -d.div[c] - aplicarA(d, vizOp, d.q, d.ybf, c, bolhas != 0);
-  if (q64) q64[c] = (double)d.q[c];  // tolerance mode: the FP64 iterate
-}
-
-// Active bubbles (montarBolhas, js/pressao-cpu.js:271-288): faces = number of (interior bubble
-// cell, water neighbour) pairs; cels = every air cell carrying an active label (:345-351).
-__global__ void k_bolhas_faces(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  const int nx = d.nx;
-  int i = c % nx, j = c / nx;
-  if (i < 1 || j < 1 || i >= nx - 1 || j >= d.ny - 1) return;
-  uint32_t b = d.rotulo[c];
-  if (b < 2 || b >= (uint32_t)MAX_BOLHAS || d.tipo[c] != AR) return;
-  unsigned k = (d.tipo[c - 1] == AGUA) + (d.tipo[c + 1] == AGUA) + (d.tipo[c - nx] == AGUA) + (d.tipo[c + nx] == AGUA);
-  if (k) atomicAdd(&d.facesB[b], k);
-}
-__global__ void k_bolhas_celulas(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  uint32_t b = d.rotulo[c];
-  if (b < 2 || b >= (uint32_t)MAX_BOLHAS || d.tipo[c] != AR || d.facesB[b] == 0) return;
-  atomicAdd(&d.celsB[b], 1u);
-}
-// Initial bubble values: y from the caller (f32), zero for inactive labels.
-__global__ void k_bolhas_inicio(Dev d) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= MAX_BOLHAS) return;
-  bool at = b >= 2 && d.facesB[b] > 0;
-  double y = at ? (double)d.yBolhaF[b] : 0.0;
-  d.yB[b] = y;
-  d.ybf[b] = (float)y;
-  d.rb[b] = d.zb[b] = d.zvb[b] = d.pb[b] = d.apb[b] = 0.0;
-  d.pbf[b] = 0.0f;
-}
-
-// Bubble rows of A*v (aplicarBolhas, js/pressao-cpu.js:325-328): out[b] = faces[b]*vb[b] -
-// sum over the bubble's water faces of v[water cell].  The sum is 64-bit fixed point (2^-40).
-constexpr double ESCALA_PCG = 1099511627776.0;  // 2^40
-__global__ void k_bolhas_somar_v(Dev d, const float* v) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N || d.esc->pronto) return;
-  const int nx = d.nx;
-  int i = c % nx, j = c / nx;
-  if (i < 1 || j < 1 || i >= nx - 1 || j >= d.ny - 1) return;
-  uint32_t b = d.rotulo[c];
-  if (b < 2 || b >= (uint32_t)MAX_BOLHAS || d.tipo[c] != AR) return;
-  double s = 0;
-  if (d.tipo[c - 1] == AGUA) s += (double)v[c - 1];
-  if (d.tipo[c + 1] == AGUA) s += (double)v[c + 1];
-  if (d.tipo[c - nx] == AGUA) s += (double)v[c - nx];
-  if (d.tipo[c + nx] == AGUA) s += (double)v[c + nx];
-  if (s != 0) somaFixa(&d.accB[b], s, ESCALA_PCG);
-}
-// modo 0: rb = rhs - (faces*y - sum)  (initial bubble residual, :339-341)
-// modo 1: apb = faces*pb - sum
-__global__ void k_bolhas_linhas(Dev d, int modo) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= MAX_BOLHAS || d.esc->pronto) return;
-  if (b < 2 || d.facesB[b] == 0) return;
-  double soma = (double)d.accB[b] / ESCALA_PCG;
-  if (modo == 0) d.rb[b] = (double)d.rhsBolhaF[b] - (d.facesB[b] * d.yB[b] - soma);
-  else d.apb[b] = d.facesB[b] * d.pb[b] - soma;
-}
-
-// Level 0's right side made from F on a grid of one level (k_descer makes it elsewhere).
-template <class T>
-__global__ void k_fonte(NivelDev<T> n0, Fonte F) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n0.nx * n0.ny || (n0.parar && *n0.parar)) return;
-  float v = F.v[c];
-  if (n0.viz[c] & V0_BOLHA) v = (float)(F.rb[F.rotulo[c]] / F.celsB[F.rotulo[c]]);
-  n0.b[c] = guardar<T>(v * (F.escala ? (float)*F.escala : 1.0f));
-}
-// After the V-cycle (precondicionar, js/pressao-cpu.js:357-361): z = x, except active bubble
-// cells, whose mean correction becomes the bubble's z (the transpose of spreading) and whose grid
-// value is zeroed.
-template <class T>
-__global__ void k_pre_juntar(Dev d, const uint8_t* viz0, const T* x0) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N || d.esc->pronto) return;
-  float inv = (float)(1.0 / d.esc->escalaMG);
-  float x = carregar(x0[c]) * inv;
-  if (viz0[c] & V0_BOLHA) {
-    const uint32_t b = d.rotulo[c];
-    somaFixa(&d.accB[b], (double)x / d.celsB[b], ESCALA_PCG);
-    d.z[c] = 0.0f;
-    return;
-  }
-  d.z[c] = x;
-}
-// The bubbles' z: the gathered mean correction, or with TQ_PRECOND_BLOCK (bloco) a Jacobi step on
-// the bubble's row, r_b / faces_b.
-__global__ void k_pre_bolhas(Dev d, int bloco) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= MAX_BOLHAS || d.esc->pronto) return;
-  const bool at = b >= 2 && d.facesB[b] > 0;
-  d.zb[b] = !at ? 0.0 : bloco ? d.rb[b] / (double)d.facesB[b] : (double)d.accB[b] / ESCALA_PCG;
-}
-
-// ap = A p on water cells (js/pressao-cpu.js:367-373).
-__global__ void k_aplicar(Dev d, const uint8_t* vizOp, int bolhas) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N || d.esc->pronto) return;
-  d.ap[c] = d.tipo[c] == AGUA ? aplicarA(d, vizOp, d.p, d.pbf, c, bolhas != 0) : 0.0f;
-}
-
-// q += alpha p, r -= alpha Ap on water; bubbles likewise (js/pressao-cpu.js:377-385).
-__global__ void k_atualizar(Dev d, double* q64) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d.esc->pronto) return;
-  double alfa = d.esc->alpha;
-  if (c < MAX_BOLHAS && c >= 2 && d.facesB[c] > 0) {
-    d.yB[c] += alfa * d.pb[c];
-    d.rb[c] -= alfa * d.apb[c];
-    d.ybf[c] = (float)d.yB[c];
-  }
-  if (c >= d.N || d.tipo[c] != AGUA) return;
-  float a = (float)alfa;
-  if (q64) q64[c] += alfa * (double)d.p[c];
-  else d.q[c] = d.q[c] + a * d.p[c];
-  d.r[c] = d.r[c] - a * d.ap[c];
-}
-
-__device__ inline double somaBloco(double v, double* sh);  // block sum (valid in thread 0), below
-
+// One iteration is three kernels and a V-cycle: p = z + beta p with A p and p.Ap (k_plano_da), the
+// q / r / bubble updates with r.r (k_plano_b), and the V-cycle, whose first kernel spreads r and whose
+// last one gathers z with r.z and r.zOld.  Each sums its dot products in blocks, and its last block to
+// finish adds the blocks' partials in block order and the active bubbles' terms in label order, makes
+// the scalar and updates the bubbles: the next kernel finds alpha, the norm or beta ready.  (A launch
+// for every step, with the dot products each a pass over the grid and a walk of the 4,096 labels,
+// took 15 launches of 3-20 us beside the V-cycle.)
+constexpr double ESCALA_PCG = 1099511627776.0;  // 2^40, the bubbles' fixed-point sums
 // Tolerance mode replaces the recursive FP32 residual by the true one each time the recursive one
 // has fallen by this factor since the last replacement (as the fused engine and the oracle do).
 constexpr double FATOR_TROCA = 1e-3;
+constexpr int T_PCG = 256;
+constexpr int BLOCOS_PCG = 1184;  // 8 a SM; with more cells each thread takes several
+static int blocosPcg(int N) { return blocos(N, T_PCG) < BLOCOS_PCG ? blocos(N, T_PCG) : BLOCOS_PCG; }
+
+// What the solve's kernels share beside Dev: the operator's descriptor of every cell, the active
+// bubbles (count first, then labels ascending) and the blocks' partial sums (two a block).
+struct Plano {
+  uint16_t* op;
+  int* ativos;
+  double* parc;
+  int bolhas, bloco, meia;  // air labels in use, TQ_PRECOND_BLOCK, 16-bit V-cycle storage
+};
+// Bits 0-3 the neighbour is water, OP_AGUA water, OP_FACE interior air of an active bubble, OP_VIZ_BOLHA
+// a neighbour is air of an active bubble; bits 8-10 the number of free neighbours.
+constexpr int OP_AGUA = 16, OP_FACE = 32, OP_VIZ_BOLHA = 64;
+
+__device__ inline bool bolhaAtiva(const Dev& d, uint32_t b) {
+  return b >= 2 && b < (uint32_t)MAX_BOLHAS && d.facesB[b] > 0;
+}
+
+// Block sum of a double (valid in thread 0).
+__device__ inline double somaBloco(double v, double* sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) sh[w] = v;
+  __syncthreads();
+  double t = 0;
+  if (w == 0) {
+    t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  }
+  __syncthreads();
+  return t;
+}
+
+// The block's partials of one or two sums; true in every thread of the block that finishes last,
+// whose writes by the other blocks are then visible.
+__device__ inline bool ultimoBloco(const Dev& d, const Plano& P, int bloco, int blocosTot, double s1, double s2,
+                                   bool dois, double* sh) {
+  __shared__ bool ultimo;
+  const double t1 = somaBloco(s1, sh), t2 = dois ? somaBloco(s2, sh) : 0.0;
+  if (threadIdx.x == 0) {
+    P.parc[2 * bloco] = t1;
+    if (dois) P.parc[2 * bloco + 1] = t2;
+    __threadfence();
+    ultimo = atomicAdd(&d.esc->tickets[0], 1u) == (unsigned)blocosTot - 1;
+  }
+  __syncthreads();
+  if (!ultimo) return false;
+  __threadfence();
+  if (threadIdx.x == 0) d.esc->tickets[0] = 0;
+  return true;
+}
+// Sums of the blocks' partials and of a term per active bubble (valid in thread 0): the last block.
+template <class F>
+__device__ inline void somasFinais(const Plano& P, int blocosTot, bool dois, double out[2], double* sh, F termo) {
+  double p1 = 0, p2 = 0;
+  for (int k = threadIdx.x; k < blocosTot; k += blockDim.x) {
+    p1 += __ldcg(&P.parc[2 * k]);
+    if (dois) p2 += __ldcg(&P.parc[2 * k + 1]);
+  }
+  double q1 = 0, q2 = 0;
+  const int nAt = P.bolhas ? P.ativos[0] : 0;
+  for (int k = threadIdx.x; k < nAt; k += blockDim.x) termo(P.ativos[1 + k], q1, q2);
+  out[0] = somaBloco(p1, sh);
+  out[0] += somaBloco(q1, sh);
+  if (dois) {
+    out[1] = somaBloco(p2, sh);
+    out[1] += somaBloco(q2, sh);
+  }
+}
+
+// Level 0's masks and descriptors, the bubbles' cells (every air cell of an active label,
+// js/pressao-cpu.js:345-351), r = -div - A q on water with r.r (:331-338) and the bubbles' sums of q over
+// their water faces; q = 0 off water.  The last block lists the active bubbles and closes their rows,
+// rb = rhs - (faces y - sum) (:339-341), and the initial norm.
+__global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const uint8_t* vizOp, const uint8_t* tipo0,
+                                                        uint8_t* viz0, double* q64) {
+  __shared__ double sh[32];
+  const int nx = d.nx, N = d.N;
+  double s = 0;
+  for (int c = blockIdx.x * T_PCG + threadIdx.x; c < N; c += gridDim.x * T_PCG) {
+    const int nb[4] = {c - 1, c + 1, c - nx, c + nx};
+    const int t = d.tipo[c], livres = vizOp[c];
+    int v0 = tipo0[c] == AGUA ? 16 : 0, op = __popc(livres) << 8;
+    float sv = 0.0f;
+    double face = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (!(livres & (1 << k))) continue;
+      v0 |= 1 << k;  // (the preconditioner's types are wall where the true ones are)
+      const int tn = d.tipo[nb[k]];
+      if (tn == AGUA) {
+        op |= 1 << k;
+        const float qn = d.q[nb[k]];
+        sv += qn;
+        face += (double)qn;
+      } else if (P.bolhas && tn == AR) {
+        const uint32_t r = d.rotulo[nb[k]];
+        if (bolhaAtiva(d, r)) {
+          op |= OP_VIZ_BOLHA;
+          sv += d.yBolhaF[r];
+        }
+      }
+    }
+    uint32_t b = 0;
+    if (t == AGUA) {
+      op |= OP_AGUA;
+      v0 |= V0_AGUA;
+      const float q = d.q[c], r = -d.div[c] - ((float)__popc(livres) * q - sv);
+      d.r[c] = r;
+      if (q64) q64[c] = (double)q;  // tolerance mode: the FP64 iterate
+      s += (double)r * (double)r;
+    } else {
+      d.r[c] = 0.0f;
+      if (P.bolhas && t == AR) {
+        const uint32_t r = d.rotulo[c];
+        if (bolhaAtiva(d, r)) {
+          b = r;
+          if (!P.bloco) v0 |= V0_BOLHA;
+          const int i = c % nx, j = c / nx;
+          if (i >= 1 && j >= 1 && i < nx - 1 && j < d.ny - 1) {
+            op |= OP_FACE;
+            if (face != 0) somaFixa(&d.accB[b], face, ESCALA_PCG);
+          }
+        }
+      }
+    }
+    P.op[c] = (uint16_t)op;
+    viz0[c] = (uint8_t)v0;
+    const unsigned com = __ballot_sync(__activemask(), b != 0);  // cells of one bubble lie together
+    if (b) {
+      const unsigned g = __match_any_sync(com, b);
+      if ((int)(threadIdx.x & 31) == __ffs(g) - 1) atomicAdd(&d.celsB[b], (unsigned)__popc(g));
+    }
+  }
+  if (!ultimoBloco(d, P, blockIdx.x, gridDim.x, s, 0, false, sh)) return;
+  if (P.bolhas) {  // the active labels in ascending order: 16 consecutive ones a thread
+    __shared__ int pref[T_PCG];
+    constexpr int K = MAX_BOLHAS / T_PCG;
+    unsigned m = 0;
+    for (int k = 0; k < K; k++) {
+      const int b = threadIdx.x * K + k;
+      const bool at = b >= 2 && __ldcg(&d.facesB[b]) > 0;
+      if (at) m |= 1u << k;
+      d.pb[b] = d.zb[b] = 0.0;
+      const double y = at ? (double)d.yBolhaF[b] : 0.0;
+      d.yB[b] = y;
+      d.rb[b] = at ? (double)d.rhsBolhaF[b] - (__ldcg(&d.facesB[b]) * y - (double)__ldcg(&d.accB[b]) / ESCALA_PCG) : 0.0;
+      d.accB[b] = 0;
+    }
+    pref[threadIdx.x] = __popc(m);
+    __syncthreads();
+    for (int o = 1; o < T_PCG; o <<= 1) {
+      const int v = threadIdx.x >= (unsigned)o ? pref[threadIdx.x - o] : 0;
+      __syncthreads();
+      pref[threadIdx.x] += v;
+      __syncthreads();
+    }
+    int pos = pref[threadIdx.x] - __popc(m);
+    for (int k = 0; k < K; k++)
+      if (m >> k & 1) P.ativos[1 + pos++] = threadIdx.x * K + k;
+    if (threadIdx.x == T_PCG - 1) P.ativos[0] = pref[T_PCG - 1];
+    __syncthreads();
+  }
+  double x[2];
+  somasFinais(P, gridDim.x, false, x, sh, [&](int b, double& q1, double&) { q1 += d.rb[b] * d.rb[b]; });
+  if (threadIdx.x == 0) {
+    Escalares* e = d.esc;
+    const double nr = sqrt(x[0]);
+    e->norma0 = e->norma = nr;
+    e->normas[0] = nr;
+    e->iters = 0;
+    e->pronto = 0;
+    e->verificar = 0;
+    e->reiniciar = 0;
+    e->trocas = 0;
+    e->convergiu = 0;
+    e->normaVerd = -1.0;
+    e->proxTroca = nr * FATOR_TROCA;
+    e->escalaMG = (P.meia && nr > 0) ? 1.0 / nr : 1.0;
+  }
+}
+
+// p = z + beta p (z on the first iteration), A p and p.Ap (js/pressao-cpu.js:84-93, 363-373, 395-396); air of an
+// active bubble gives a water cell its bubble's p, and takes the sum of p over its water faces.
+// The last block: the bubbles' p and rows, p.Ap and alpha.
+__global__ void __launch_bounds__(T_PCG) k_plano_da(Dev d, Plano P, const float* z, const float* pv, float* pn, int prim) {
+  __shared__ double sh[32];
+  if (d.esc->pronto) return;  // uniform over the grid
+  const int nx = d.nx, N = d.N;
+  const double beta = prim ? 0.0 : d.esc->beta;
+  const float bf = (float)beta;
+  auto pbNovo = [&](int b) { return prim ? d.zb[b] : d.zb[b] + beta * d.pb[b]; };
+  double s = 0;
+  for (int c = blockIdx.x * T_PCG + threadIdx.x; c < N; c += gridDim.x * T_PCG) {
+    const int m = P.op[c];
+    // the five z and p go out with the descriptor (an index past the grid's end reads c itself; the
+    // descriptor picks the neighbours that count)
+    const int nb[5] = {c, c > 0 ? c - 1 : c, c < N - 1 ? c + 1 : c, c >= nx ? c - nx : c, c < N - nx ? c + nx : c};
+    float pq[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) pq[k] = prim ? z[nb[k]] : z[nb[k]] + bf * pv[nb[k]];
+    if (m & OP_AGUA) {
+      float sv = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (m & (1 << k)) sv += pq[k + 1];
+        else if (m & OP_VIZ_BOLHA) {
+          const int i = c % nx, j = c / nx;
+          const bool existe = k == 0 ? i > 0 : k == 1 ? i < nx - 1 : k == 2 ? j > 0 : j < d.ny - 1;
+          if (existe && d.tipo[nb[k + 1]] == AR) {
+            const uint32_t r = d.rotulo[nb[k + 1]];
+            if (bolhaAtiva(d, r)) sv += (float)pbNovo(r);
+          }
+        }
+      }
+      const float ap = (float)(m >> 8) * pq[0] - sv;
+      pn[c] = pq[0];
+      d.ap[c] = ap;
+      s += (double)pq[0] * (double)ap;
+    } else if (m & OP_FACE) {
+      double t = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (m & (1 << k)) t += (double)pq[k + 1];
+      if (t != 0) somaFixa(&d.accB[d.rotulo[c]], t, ESCALA_PCG);
+    }
+  }
+  if (!ultimoBloco(d, P, blockIdx.x, gridDim.x, s, 0, false, sh)) return;
+  double x[2];
+  somasFinais(P, gridDim.x, false, x, sh, [&](int b, double& q1, double&) {
+    const double pb = pbNovo(b), ap = d.facesB[b] * pb - (double)__ldcg(&d.accB[b]) / ESCALA_PCG;
+    d.pb[b] = pb;
+    d.apb[b] = ap;
+    d.accB[b] = 0;
+    q1 += pb * ap;
+  });
+  if (threadIdx.x == 0) {
+    Escalares* e = d.esc;
+    e->pap = x[0];
+    e->alpha = fabs(x[0]) < 1e-30 ? 0.0 : e->rz / x[0];
+  }
+}
+
+// q += alpha p, r -= alpha Ap on water with r.r; the last block the bubbles and the norm
+// (js/pressao-cpu.js:377-386).
+__global__ void __launch_bounds__(T_PCG) k_plano_b(Dev d, Plano P, const float* p, double* q64, int it, double tol, int cap) {
+  __shared__ double sh[32];
+  if (d.esc->pronto) return;
+  const double alfa = d.esc->alpha;
+  const float a = (float)alfa;
+  double s = 0;
+  for (int c = blockIdx.x * T_PCG + threadIdx.x; c < d.N; c += gridDim.x * T_PCG) {
+    const int m = P.op[c];
+    const float pc = p[c], rc = d.r[c], apc = d.ap[c];
+    const double qd = q64 ? q64[c] : 0.0;
+    const float qf = q64 ? 0.0f : d.q[c];
+    if (!(m & OP_AGUA)) continue;
+    if (q64) q64[c] = qd + alfa * (double)pc;
+    else d.q[c] = qf + a * pc;
+    const float r = rc - a * apc;
+    d.r[c] = r;
+    s += (double)r * (double)r;
+  }
+  if (!ultimoBloco(d, P, blockIdx.x, gridDim.x, s, 0, false, sh)) return;
+  double x[2];
+  somasFinais(P, gridDim.x, false, x, sh, [&](int b, double& q1, double&) {
+    d.yB[b] += alfa * d.pb[b];
+    const double rb = d.rb[b] - alfa * d.apb[b];
+    d.rb[b] = rb;
+    q1 += rb * rb;
+  });
+  if (threadIdx.x == 0) {
+    Escalares* e = d.esc;
+    const double nr = sqrt(x[0]);
+    e->norma = nr;
+    if (it + 1 < 1024) e->normas[it + 1] = nr;
+    e->iters = it + 1;
+    // tolerance mode: the recursive residual met the tolerance, or fell by FATOR_TROCA since
+    // the last replacement, or the cap came: the true residual decides (k_verdade, k_verdade_fim)
+    e->verificar = tol > 0 && (nr <= tol * e->norma0 || nr <= e->proxTroca || it + 1 >= cap);
+    e->escalaMG = (P.meia && nr > 0) ? 1.0 / nr : 1.0;
+  }
+}
+
+// The gather of z after the V-cycle (precondicionar, js/pressao-cpu.js:357-361): z = x / escala; cells of an
+// active bubble give their mean correction to the bubble's z (the transpose of spreading) and keep 0.
+struct Juncao {
+  Dev d;
+  Plano P;
+  const float* zVelho;  // null on the first iteration
+  float* zNovo;
+};
+template <class T>
+__device__ __forceinline__ void juntarCelula(const Juncao& J, int c, int v, float x, float inv, float r, float zv,
+                                             double& s1, double& s2) {
+  const float z = arredondar<T>(x) * inv;
+  if (v & V0_BOLHA) {
+    const uint32_t b = J.d.rotulo[c];
+    somaFixa(&J.d.accB[b], (double)z / J.d.celsB[b], ESCALA_PCG);
+    J.zNovo[c] = 0.0f;
+    return;
+  }
+  J.zNovo[c] = z;
+  if (v & V0_AGUA) {
+    s1 += (double)r * (double)z;
+    s2 += (double)r * (double)zv;
+  }
+}
+// After the gather: r.z and r.zOld, and by the last block the bubbles' z (with TQ_PRECOND_BLOCK a Jacobi
+// step on the bubble's row) and beta (js/pressao-cpu.js:388-394).
+__device__ inline void fimJuncao(const Juncao& J, int bloco, int blocosTot, double s1, double s2) {
+  __shared__ double sh[32];
+  const Dev& d = J.d;
+  if (!ultimoBloco(d, J.P, bloco, blocosTot, s1, s2, true, sh)) return;
+  double x[2];
+  somasFinais(J.P, blocosTot, true, x, sh, [&](int b, double& q1, double& q2) {
+    const double zv = d.zb[b];
+    const double zb = J.P.bloco ? d.rb[b] / (double)d.facesB[b] : (double)__ldcg(&d.accB[b]) / ESCALA_PCG;
+    d.zb[b] = zb;
+    d.accB[b] = 0;
+    q1 += d.rb[b] * zb;
+    q2 += d.rb[b] * zv;
+  });
+  if (threadIdx.x == 0) {
+    Escalares* e = d.esc;
+    // (after a residual replacement the direction carries on: no restart)
+    e->beta = !J.zVelho || fabs(e->rz) < 1e-30 ? 0.0 : fmax(0.0, (x[0] - x[1]) / e->rz);
+    e->reiniciar = 0;
+    e->rz = x[0];
+  }
+}
+// The gather on a grid of one level (k_subir's last launch does it elsewhere).
+template <class T>
+__global__ void __launch_bounds__(T_PCG) k_juntar(Juncao J, const uint8_t* viz0, const T* x0) {
+  const Dev& d = J.d;
+  if (d.esc->pronto) return;
+  const float inv = (float)(1.0 / d.esc->escalaMG);
+  double s1 = 0, s2 = 0;
+  for (int c = blockIdx.x * T_PCG + threadIdx.x; c < d.N; c += gridDim.x * T_PCG)
+    juntarCelula<T>(J, c, viz0[c], carregar(x0[c]), inv, d.r[c], J.zVelho ? J.zVelho[c] : 0.0f, s1, s2);
+  fimJuncao(J, blockIdx.x, gridDim.x, s1, s2);
+}
+
+// The way up a level: x + the coarse correction and both passes, the level's result in n.tmp, or
+// (saida not null) as floats in saida, or (JUNTA, level 0 of a solve) gathered into z.
+template <class T, class TG, bool JUNTA>
+__global__ void __launch_bounds__(T_LADRILHO) k_subir(NivelDev<T> n, NivelDev<TG> g, const TG* xg, int kx, int ky,
+                                                      int uma, int masc, float* saida,
+                                                      const __grid_constant__ Juncao J) {
+  extern __shared__ __align__(16) float mem[];
+  if (n.parar && *n.parar) return;
+  const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
+  double s1 = 0, s2 = 0;
+  const float inv = JUNTA ? (float)(1.0 / J.d.esc->escalaMG) : 1.0f;
+  subirLadrilho<T>(
+      L, g.nx, g.ny, uma != 0, masc != 0, VARREDURAS, mem, [&](int c) { return carregar(n.x[c]); },
+      [&](int C) { return carregar(xg[C]); }, [&](int c) { return carregar(n.b[c]); },
+      [&](const int (&cel)[2][4], const int (&v)[2][4], const float (&x)[2][4]) {
+        if constexpr (JUNTA) {
+          float r[2][4], zv[2][4];
+#pragma unroll
+          for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+              const int c = cel[cr][m] < 0 ? 0 : cel[cr][m];
+              r[cr][m] = J.d.r[c];
+              zv[cr][m] = J.zVelho ? J.zVelho[c] : 0.0f;
+            }
+#pragma unroll
+          for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+              if (cel[cr][m] >= 0)
+                juntarCelula<T>(J, cel[cr][m], v[cr][m], x[cr][m], inv, r[cr][m], zv[cr][m], s1, s2);
+        } else {
+#pragma unroll
+          for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+              if (cel[cr][m] >= 0) {
+                if (saida) saida[cel[cr][m]] = arredondar<T>(x[cr][m]);
+                else n.tmp[cel[cr][m]] = guardar<T>(x[cr][m]);
+              }
+        }
+      });
+  if (JUNTA) fimJuncao(J, blockIdx.x + blockIdx.y * gridDim.x, gridDim.x * gridDim.y, s1, s2);
+}
 
 // Tolerance mode, once the recursive residual met the tolerance (Escalares::verificar): the true
 // residual in FP64 from the FP64 iterate and the bubble pressures.  Water cells: rt = -div - A q
 // into d.ap (free until the next A p) and rt^2 into per-CTA partials; interior air of active
 // bubbles: the sum of q over its water faces into the bubble's fixed-point sum (accB, zeroed
 // before).  k_verdade_fim finishes the norm and decides.
+constexpr int BLOCOS_VERDADE = 296;  // 2 a SM
 __global__ void __launch_bounds__(256) k_verdade(Dev d, const uint8_t* vizOp, const double* q64, int bolhas) {
   __shared__ double sh[32];
   if (!d.esc->verificar || d.esc->pronto) return;  // uniform over the grid
@@ -672,9 +891,11 @@ __global__ void __launch_bounds__(256) k_verdade_fim(Dev d, int blocosVerdade, i
     }
   }
   __syncthreads();
-  if (substituir && bolhas)
-    for (int b = threadIdx.x; b < MAX_BOLHAS; b += blockDim.x)
-      if (b >= 2 && d.facesB[b] > 0) d.rb[b] = rbv(b);
+  if (bolhas)
+    for (int b = threadIdx.x; b < MAX_BOLHAS; b += blockDim.x) {
+      if (substituir && b >= 2 && d.facesB[b] > 0) d.rb[b] = rbv(b);
+      d.accB[b] = 0;  // the next iteration's sums start from 0
+    }
 }
 // After a replacement: r = the true residual on water cells.
 __global__ void k_substituir(Dev d) {
@@ -683,35 +904,6 @@ __global__ void k_substituir(Dev d) {
   if (d.tipo[c] == AGUA) d.r[c] = d.ap[c];
 }
 
-// p = z + beta p on water (0 elsewhere); bubbles likewise (js/pressao-cpu.js:395-396).
-__global__ void k_direcao(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d.esc->pronto) return;
-  double beta = d.esc->beta;
-  if (c < MAX_BOLHAS && c >= 2 && d.facesB[c] > 0) {
-    d.pb[c] = d.zb[c] + beta * d.pb[c];
-    d.pbf[c] = (float)d.pb[c];
-  }
-  if (c >= d.N) return;
-  d.p[c] = d.tipo[c] == AGUA ? d.z[c] + (float)beta * d.p[c] : 0.0f;
-}
-// p = z, pb = zb (js/pressao-cpu.js:363-364)
-__global__ void k_copiar_pz(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < MAX_BOLHAS) {
-    d.pb[c] = d.zb[c];
-    d.pbf[c] = (float)d.zb[c];
-    d.zvb[c] = 0.0;
-  }
-  if (c < d.N) d.p[c] = d.z[c];
-}
-// zOld = z, zvb = zb (js/pressao-cpu.js:388-389)
-__global__ void k_guardar_z(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d.esc->pronto) return;
-  if (c < MAX_BOLHAS) d.zvb[c] = d.zb[c];
-  if (c < d.N) d.zOld[c] = d.z[c];
-}
 // End of the solve: non-water q = 0; bubbles hand back their pressure (js/pressao-cpu.js:399-400).
 // Tolerance mode: q = the FP64 iterate rounded; the solve's convergence record (thread 0).
 __global__ void k_pcg_fim(Dev d, int bolhas, const double* q64, double tol) {
@@ -735,122 +927,28 @@ __global__ void k_pcg_fim(Dev d, int bolhas, const double* q64, double tol) {
   }
 }
 
-// ---------------------------------------------------------------- dot products
-// Two FP64 dot products over water cells (a*b1, a*b2) plus the bubble terms, in a fixed
-// reduction order; the last block to finish does the scalar step of the running solve.
-enum ModoProduto { NORMA0 = 0, RZ0 = 1, PAP = 2, NORMA = 3, BETA = 4 };
-
-constexpr int DOT_BLOCOS = 296;
-constexpr int DOT_T = 256;
-
-__device__ inline double somaBloco(double v, double* sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0;
-  if (w == 0) {
-    t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  }
-  __syncthreads();
-  return t;  // valid in thread 0
-}
-
-__global__ void __launch_bounds__(DOT_T) k_produto(Dev d, int modo, const float* a, const float* b1, const float* b2,
-                                                 int it, double tol, int bolhas, int meiaPrecisao, int cap) {
-  __shared__ double sh[32];
-  __shared__ bool ultimo;
-  if (modo != NORMA0 && d.esc->pronto) return;  // uniform over the grid
-  double s1 = 0, s2 = 0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.N; c += gridDim.x * blockDim.x) {
-    if (d.tipo[c] != AGUA) continue;
-    double av = a[c];
-    s1 += av * (double)b1[c];
-    if (b2) s2 += av * (double)b2[c];
-  }
-  double t1 = somaBloco(s1, sh);
-  double t2 = b2 ? somaBloco(s2, sh) : 0.0;
-  if (threadIdx.x == 0) {
-    d.parciais[2 * blockIdx.x] = t1;
-    d.parciais[2 * blockIdx.x + 1] = t2;
-    __threadfence();
-    unsigned v = atomicAdd(&d.esc->tickets[0], 1u);
-    ultimo = v == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!ultimo) return;
-  __threadfence();
-  // the last block: partials in block order, then the bubble terms in label order
-  double p1 = 0, p2 = 0;
-  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-    p1 += __ldcg(&d.parciais[2 * k]);
-    p2 += __ldcg(&d.parciais[2 * k + 1]);
-  }
-  double q1 = 0, q2 = 0;
-  if (bolhas) {
-    for (int b = threadIdx.x; b < MAX_BOLHAS; b += blockDim.x) {
-      if (b < 2 || d.facesB[b] == 0) continue;
-      switch (modo) {
-        case NORMA0:
-        case NORMA: q1 += d.rb[b] * d.rb[b]; break;
-        case RZ0: q1 += d.rb[b] * d.zb[b]; break;
-        case PAP: q1 += d.pb[b] * d.apb[b]; break;
-        case BETA: q1 += d.rb[b] * d.zb[b]; q2 += d.rb[b] * d.zvb[b]; break;
-      }
-    }
-  }
-  double T1 = somaBloco(p1, sh), T2 = somaBloco(p2, sh);
-  double B1 = somaBloco(q1, sh), B2 = somaBloco(q2, sh);
-  if (threadIdx.x == 0) {
-    Escalares* e = d.esc;
-    e->tickets[0] = 0;
-    double x1 = T1 + B1, x2 = T2 + B2;
-    switch (modo) {
-      case NORMA0: {
-        double nr = sqrt(x1);
-        e->norma0 = e->norma = nr;
-        e->normas[0] = nr;
-        e->iters = 0;
-        e->pronto = 0;
-        e->verificar = 0;
-        e->reiniciar = 0;
-        e->trocas = 0;
-        e->convergiu = 0;
-        e->normaVerd = -1.0;
-        e->proxTroca = nr * FATOR_TROCA;
-        e->escalaMG = (meiaPrecisao && nr > 0) ? 1.0 / nr : 1.0;
-        break;
-      }
-      case RZ0: e->rz = x1; break;
-      case PAP: e->pap = x1; e->alpha = fabs(x1) < 1e-30 ? 0.0 : e->rz / x1; break;
-      case NORMA: {
-        double nr = sqrt(x1);
-        e->norma = nr;
-        if (it + 1 < 1024) e->normas[it + 1] = nr;
-        e->iters = it + 1;
-        // tolerance mode: the recursive residual met the tolerance, or fell by FATOR_TROCA since
-        // the last replacement, or the cap came: the true residual decides (k_verdade,
-        // k_verdade_fim)
-        e->verificar = tol > 0 && (nr <= tol * e->norma0 || nr <= e->proxTroca || it + 1 >= cap);
-        e->escalaMG = (meiaPrecisao && nr > 0) ? 1.0 / nr : 1.0;
-        break;
-      }
-      case BETA: {
-        double rzNovo = x1, cruzado = x2;
-        // (after a residual replacement the direction carries on: no restart)
-        e->beta = fabs(e->rz) < 1e-30 ? 0.0 : fmax(0.0, (rzNovo - cruzado) / e->rz);
-        e->reiniciar = 0;
-        e->rz = rzNovo;
-        break;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- the solver object
+// The tile of a leg: by blocks a side, the launch's length in rounds of block sweeps, a CTA an SM
+// (two of the smallest tile's) with 16 warps, is waves x rounds; the shortest wins, the smaller tile
+// of equals (a smaller tile sweeps more blocks around it, a larger one leaves SMs without a tile).
+static int escolherLadrilho(int nx, int ny, bool subir, bool uma) {
+  constexpr int SMS = 148;
+  int melhor = 1;
+  long custo = -1;
+  for (int k = 1; k <= 4; k++) {
+    const long n = (long)blocos(nx, 16 * k) * blocos(ny, 16 * k);
+    const long ondas = (n + SMS * (k == 1 ? 2 : 1) - 1) / (SMS * (k == 1 ? 2 : 1));
+    auto voltas = [&](int b) { return (b * b + (k == 1 ? 8 : 15)) / (k == 1 ? 9 : 16); };
+    const int r = uma ? voltas(subir ? k : k + 1) : subir ? voltas(k + 1) + voltas(k) : voltas(k + 2) + voltas(k + 1);
+    const long c = ondas * (r + 2);
+    if (custo < 0 || c < custo) {
+      custo = c;
+      melhor = k;
+    }
+  }
+  return melhor;
+}
+
 
 
 Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
@@ -907,6 +1005,15 @@ Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
       p->motor = TQ_ENGINE_PLAIN;
     }
   }
+  if (ok && p->motor == TQ_ENGINE_PLAIN) {
+    // the partial sums of k_plano_da / k_plano_b's blocks, or of the gather's tiles if more
+    const int k = escolherLadrilho(nx, ny, true, false);
+    const size_t lad = (size_t)blocos(nx, 16 * k) * blocos(ny, 16 * k);
+    const size_t np = 2 * (lad > (size_t)BLOCOS_PCG ? lad : (size_t)BLOCOS_PCG);
+    ok = cudaMalloc(&p->op, (size_t)p->N * 2) == cudaSuccess && cudaMalloc(&p->p2, (size_t)p->N * 4) == cudaSuccess &&
+         cudaMalloc(&p->parc, np * sizeof(double)) == cudaSuccess &&
+         cudaMalloc(&p->ativos, (MAX_BOLHAS + 1) * sizeof(int)) == cudaSuccess;
+  }
   if (!ok) {
     destruirPcg(p);
     return nullptr;
@@ -925,6 +1032,10 @@ void destruirPcg(Pcg* p) {
     cudaFree(p->tmpL[l]);
   }
   cudaFree(p->vizOp);
+  cudaFree(p->op);
+  cudaFree(p->p2);
+  cudaFree(p->parc);
+  cudaFree(p->ativos);
   if (p->q64) cudaFree(p->q64);
   destruirRegioes(p->regioes);
   delete p;
@@ -962,27 +1073,6 @@ static void comTipos(Pcg* p, int l, F f) {
   });
 }
 
-// The tile of a leg: by blocks a side, the launch's length in rounds of block sweeps, a CTA an SM
-// (two of the smallest tile's) with 16 warps, is waves x rounds; the shortest wins, the smaller tile
-// of equals (a smaller tile sweeps more blocks around it, a larger one leaves SMs without a tile).
-static int escolherLadrilho(int nx, int ny, bool subir, bool uma) {
-  constexpr int SMS = 148;
-  int melhor = 1;
-  long custo = -1;
-  for (int k = 1; k <= 4; k++) {
-    const long n = (long)blocos(nx, 16 * k) * blocos(ny, 16 * k);
-    const long ondas = (n + SMS * (k == 1 ? 2 : 1) - 1) / (SMS * (k == 1 ? 2 : 1));
-    auto voltas = [&](int b) { return (b * b + (k == 1 ? 8 : 15)) / (k == 1 ? 9 : 16); };
-    const int r = uma ? voltas(subir ? k : k + 1) : subir ? voltas(k + 1) + voltas(k) : voltas(k + 2) + voltas(k + 1);
-    const long c = ondas * (r + 2);
-    if (custo < 0 || c < custo) {
-      custo = c;
-      melhor = k;
-    }
-  }
-  return melhor;
-}
-
 template <class K>
 static size_t prepararLadrilho(K kern, int k) {
   const size_t b = bytesLadrilho(k, k);
@@ -1007,23 +1097,28 @@ static void descerNivel(Pcg* p, int l, bool bloco, bool uma, const Fonte& F, cud
   });
 }
 // xg: the coarse level's x (its result)
-static void subirNivel(Pcg* p, int l, const void* xg, bool bloco, bool uma, float* saida, cudaStream_t s) {
+// (saida, J: level 0's alone)
+static void subirNivel(Pcg* p, int l, const void* xg, bool bloco, bool uma, float* saida, const Juncao* J,
+                       cudaStream_t s) {
   uma = uma && l >= 1;
   const int k = escolherLadrilho(p->nxL[l], p->nyL[l], true, uma), d = uma ? 8 : 0;
   const dim3 gr(blocos(p->nxL[l] + d, 16 * k), blocos(p->nyL[l] + d, 16 * k));
   comTipos(p, l, [&](auto* tf, auto* tg) {
     using TF = std::remove_pointer_t<decltype(tf)>;
     using TG = std::remove_pointer_t<decltype(tg)>;
-    const size_t b = prepararLadrilho(k_subir<TF, TG>, k);
-    lanca(k_subir<TF, TG>, gr, threadsLadrilho(k), b, s, nivel<TF>(p, l), nivel<TG>(p, l + 1), (const TG*)xg, k, k,
-          uma ? 1 : 0, bloco && l >= 1 ? 1 : 0, saida);
+    auto kern = J ? k_subir<TF, TG, true> : k_subir<TF, TG, false>;
+    const size_t b = prepararLadrilho(kern, k);
+    lanca(kern, gr, threadsLadrilho(k), b, s, nivel<TF>(p, l), nivel<TG>(p, l + 1), (const TG*)xg, k, k, uma ? 1 : 0,
+          bloco && l >= 1 ? 1 : 0, saida, J ? *J : Juncao{});
   });
 }
 
 // cicloV (js/pressao-cpu.js:241-255) on a right side made from F (level 0's b is written); every
-// level's result ends in its tmp, level 0's returned, or as floats in saida when there is one.
+// level's result ends in its tmp, level 0's returned, or as floats in saida, or gathered by J, when
+// there is one (on more than one level).
 // umaPassada (TQ_PRECOND_BLOCK_1): the levels above 0 take one smoother pass a leg (shift 8).
-static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bool umaPassada, float* saida) {
+static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bool umaPassada, float* saida,
+                          const Juncao* J) {
   const int L = p->L;
   // the section: the coarse levels of at most SECAO_PLANA cells (not level 0)
   int Ls = L, total = 0;
@@ -1055,7 +1150,7 @@ static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bo
     x = p->xL[L - 1];
   }
   for (int l = Lf - 1; l >= 0; l--) {
-    subirNivel(p, l, x, bloco, umaPassada, l == 0 ? saida : nullptr, s);
+    subirNivel(p, l, x, bloco, umaPassada, l == 0 ? saida : nullptr, l == 0 ? J : nullptr, s);
     x = p->tmpL[l];
   }
   return x;
@@ -1088,24 +1183,17 @@ static void prepararNiveis(Pcg* p, const uint8_t* tipo0, bool bloco, cudaStream_
   if (n.ini[p->L] > 0) lanca(k_niveis_viz, blocos(n.ini[p->L], 256), 256, 0, s, n, l0, bloco ? 1 : 0);
 }
 
-static void precondicionar(Pcg* p, const Dev& d, bool bolhas, bool bloco, bool umaPassada, cudaStream_t s) {
-  int nb = blocos(d.N, 256);
+// z = the preconditioned residual (J.zNovo), the bubbles' z, r.z and beta.
+static void precondicionar(Pcg* p, const Juncao& J, bool bloco, bool umaPassada, cudaStream_t s) {
+  const Dev& d = J.d;
   Fonte F{d.r, &d.esc->escalaMG, d.rotulo, d.rb, d.celsB};
   fonteNivelUnico(p, F, s);
-  const void* x = cicloV(p, F, s, bloco, umaPassada, nullptr);
-  const bool espalhar = bolhas && !bloco;  // with BLOCK the V-cycle does not see the bubbles
-  if (espalhar) cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
-  comTipo(p, 0, [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    lanca(k_pre_juntar<T>, nb, 256, 0, s, d, p->vizL[0], (const T*)x);
-  });
-  if (bolhas) lanca(k_pre_bolhas, blocos(MAX_BOLHAS, 256), 256, 0, s, d, bloco ? 1 : 0);
-}
-
-static void produto(Pcg* p, const Dev& d, int modo, const float* a, const float* b1, const float* b2, int it,
-                    double tol, bool bolhas, int cap, cudaStream_t s) {
-  lanca(k_produto, DOT_BLOCOS, DOT_T, 0, s, d, modo, a, b1, b2, it, tol, bolhas ? 1 : 0,
-        p->precisao != TQ_PREC_FP32 ? 1 : 0, cap);
+  const void* x = cicloV(p, F, s, bloco, umaPassada, nullptr, &J);
+  if (p->L == 1)
+    comTipo(p, 0, [&](auto* tag) {
+      using T = std::remove_pointer_t<decltype(tag)>;
+      lanca(k_juntar<T>, blocosPcg(d.N), T_PCG, 0, s, J, p->vizL[0], (const T*)x);
+    });
 }
 
 // Iterations the plain engine queues between two reads of the stop flag.  Every kernel of an
@@ -1131,48 +1219,25 @@ int resolverPressao(Pcg* p, const Dev& d0, int iteracoes, double tol, bool bolha
   if (p->motor == TQ_ENGINE_FUSED) return resolverPressaoFundido(p, d, iteracoes, tol, bolhas, precond, s);
   const bool bloco = precond == TQ_PRECOND_BLOCK || precond == TQ_PRECOND_BLOCK_1;
   const bool umaPassada = precond == TQ_PRECOND_BLOCK_1;
-  const int nb = blocos(d.N, 256);
+  const int nb = blocos(d.N, 256), nbp = blocosPcg(d.N);
   const int nbx = blocos(d.N > MAX_BOLHAS ? d.N : MAX_BOLHAS, 256);
-  // operator (true types) and preconditioner types
-  lanca(k_mg_tipo0, nb, 256, 0, s, d.tipo, d.rotulo, p->tipoL[0], p->vizOp, d.nx, d.ny, bolhas ? 1 : 0, bloco ? 1 : 0);
+  const Plano P{p->op, p->ativos, p->parc, bolhas ? 1 : 0, bloco ? 1 : 0, p->precisao != TQ_PREC_FP32 ? 1 : 0};
+  zerarBolhas(d, s);
+  // operator (true types) and preconditioner types, the levels', level 0's masks with r and its norm
+  lanca(k_plano_tipos, nb, 256, 0, s, d, p->tipoL[0], p->vizOp, bolhas ? 1 : 0, bloco ? 1 : 0);
   prepararNiveis(p, p->tipoL[0], bloco, s, false);
-  cudaMemsetAsync(d.facesB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
-  cudaMemsetAsync(d.celsB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
-  // the previous solve left its stop flag set: clear it before the first kernel that tests it
-  // (the initial bubble sums and rows below; NORMA0 resets the rest of the record)
-  cudaMemsetAsync(&d.esc->pronto, 0, sizeof(int), s);
-  if (bolhas) {
-    lanca(k_bolhas_faces, nb, 256, 0, s, d);
-    lanca(k_bolhas_celulas, nb, 256, 0, s, d);
-  }
-  lanca(k_viz0, nb, 256, 0, s, d, p->tipoL[0], p->vizL[0], bolhas && !bloco ? 1 : 0);
-  lanca(k_bolhas_inicio, blocos(MAX_BOLHAS, 256), 256, 0, s, d);
-  lanca(k_pcg_inicio, nb, 256, 0, s, d, p->vizOp, bolhas ? 1 : 0, q64);
-  if (bolhas) {
-    cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
-    lanca(k_bolhas_somar_v, nb, 256, 0, s, d, d.q);
-    lanca(k_bolhas_linhas, blocos(MAX_BOLHAS, 256), 256, 0, s, d, 0);
-  }
-  produto(p, d, NORMA0, d.r, d.r, nullptr, 0, tol, bolhas, iteracoes, s);
+  lanca(k_plano_inicio, nbp, T_PCG, 0, s, d, P, p->vizOp, p->tipoL[0], p->vizL[0], q64);
   p->parar = &d.esc->pronto;  // the V-cycle kernels return once the solve has stopped
-  precondicionar(p, d, bolhas, bloco, umaPassada, s);
-  lanca(k_copiar_pz, nbx, 256, 0, s, d);
-  produto(p, d, RZ0, d.r, d.z, nullptr, 0, tol, bolhas, iteracoes, s);
+  float *zc = d.z, *zo = d.zOld, *pv = d.p, *pn = p->p2;  // z, p and the previous ones swap buffers
+  precondicionar(p, Juncao{d, P, nullptr, zc}, bloco, umaPassada, s);
   int it = 0;
   for (; it < iteracoes; it++) {
-    lanca(k_aplicar, nb, 256, 0, s, d, p->vizOp, bolhas ? 1 : 0);
-    if (bolhas) {
-      cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
-      lanca(k_bolhas_somar_v, nb, 256, 0, s, d, d.p);
-      lanca(k_bolhas_linhas, blocos(MAX_BOLHAS, 256), 256, 0, s, d, 1);
-    }
-    produto(p, d, PAP, d.p, d.ap, nullptr, it, tol, bolhas, iteracoes, s);
-    lanca(k_atualizar, nbx, 256, 0, s, d, q64);
-    produto(p, d, NORMA, d.r, d.r, nullptr, it, tol, bolhas, iteracoes, s);
-    if (q64) {  // the true residual, when NORMA found the recursive one within the tolerance
-      if (bolhas) cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
-      lanca(k_verdade, DOT_BLOCOS, 256, 0, s, d, p->vizOp, q64, bolhas ? 1 : 0);
-      lanca(k_verdade_fim, 1, 256, 0, s, d, DOT_BLOCOS, iteracoes, tol, bolhas ? 1 : 0,
+    lanca(k_plano_da, nbp, T_PCG, 0, s, d, P, zc, pv, pn, it == 0 ? 1 : 0);
+    std::swap(pv, pn);
+    lanca(k_plano_b, nbp, T_PCG, 0, s, d, P, pv, q64, it, tol, iteracoes);
+    if (q64) {  // the true residual, when the recursive one is within the tolerance
+      lanca(k_verdade, BLOCOS_VERDADE, 256, 0, s, d, p->vizOp, q64, bolhas ? 1 : 0);
+      lanca(k_verdade_fim, 1, 256, 0, s, d, BLOCOS_VERDADE, iteracoes, tol, bolhas ? 1 : 0,
             p->precisao != TQ_PREC_FP32 ? 1 : 0);
       lanca(k_substituir, nb, 256, 0, s, d);
     }
@@ -1186,10 +1251,8 @@ int resolverPressao(Pcg* p, const Dev& d0, int iteracoes, double tol, bool bolha
       }
       if (pronto) break;
     }
-    lanca(k_guardar_z, nbx, 256, 0, s, d);
-    precondicionar(p, d, bolhas, bloco, umaPassada, s);
-    produto(p, d, BETA, d.r, d.z, d.zOld, it, tol, bolhas, iteracoes, s);
-    lanca(k_direcao, nbx, 256, 0, s, d);
+    precondicionar(p, Juncao{d, P, zc, zo}, bloco, umaPassada, s);
+    std::swap(zc, zo);
   }
   p->parar = nullptr;
   lanca(k_pcg_fim, nbx, 256, 0, s, d, bolhas ? 1 : 0, q64, tol);
@@ -1230,7 +1293,7 @@ int cicloVDispositivo(Pcg* p, const uint8_t* tipo, const float* b, float* x, cud
   p->parar = parar;  // the cycle's kernels return at once while *parar != 0
   Fonte F{b};
   fonteNivelUnico(p, F, s);
-  const void* r = cicloV(p, F, s, false, false, x);
+  const void* r = cicloV(p, F, s, false, false, x, nullptr);
   if (p->L == 1)
     comTipo(p, 0, [&](auto* tag) {
       using T = std::remove_pointer_t<decltype(tag)>;

@@ -2404,9 +2404,7 @@ int resolverPressaoFundido(Pcg* p, const Dev& d, int iteracoes, double tol, bool
     cudaMemsetAsync(f->perfil, 0, sizeof(unsigned long long), s);
     cudaMemsetAsync(f->perfil + PERFIL_MAX + 1, 0, sizeof(unsigned long long), s);
   }
-  cudaMemsetAsync(d.facesB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
-  cudaMemsetAsync(d.celsB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
-  cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
+  zerarBolhas(d, s);
   if (d.nTanques && tol > 0) cudaMemsetAsync(d.r0T, 0, (size_t)d.nTanques * sizeof(double), s);
   cudaMemsetAsync(f->bar, 0, 2 * sizeof(unsigned), s);
   // f->erro is not cleared here: a solve that gave up keeps it set until erroFundido reads it,

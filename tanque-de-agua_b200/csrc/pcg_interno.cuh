@@ -24,11 +24,21 @@ struct Pcg {
   void *bL[MAX_NIVEIS], *xL[MAX_NIVEIS], *tmpL[MAX_NIVEIS];  // 4 bytes per element allocated
   uint8_t* vizOp;
   double* q64 = nullptr;  // the plain engine's FP64 iterate (tolerance mode), allocated on first use
+  // the plain engine's operator descriptors, second p, partial sums and active bubbles (pcg.cu, Plano)
+  uint16_t* op = nullptr;
+  float* p2 = nullptr;
+  double* parc = nullptr;
+  int* ativos = nullptr;
   const int* parar = nullptr;  // the running plain solve's stop flag (NivelDev::parar)
   size_t smemGrosso = 0;
   Fundido* fundido = nullptr;
   Regioes* regioes = nullptr;  // tolerance mode's closed-region projection, allocated on first use
 };
+
+// The bubbles' face and cell counts and fixed-point sums to 0: one block of memory (Dev::accB, facesB, celsB).
+inline void zerarBolhas(const Dev& d, cudaStream_t s) {
+  cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * (sizeof(long long) + 2 * sizeof(uint32_t)), s);
+}
 
 // pcg_fundido.cu
 Fundido* criarFundido(Pcg* p);

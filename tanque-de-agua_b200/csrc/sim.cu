@@ -340,12 +340,13 @@ int tq_create(const tq_options* o, tq_sim** out) {
        aloca(s, &d.pressaoBolha, MAX_BOLHAS) && aloca(s, &d.volumeAlvo, MAX_BOLHAS) &&
        aloca(s, &d.volumeBolhaF, MAX_BOLHAS) && aloca(s, &d.rhsBolhaF, MAX_BOLHAS) &&
        aloca(s, &d.yBolhaF, MAX_BOLHAS) && aloca(s, &d.vivo, MAX_BOLHAS) && aloca(s, &d.volB, MAX_BOLHAS) &&
-       aloca(s, &d.facesB, MAX_BOLHAS) && aloca(s, &d.celsB, MAX_BOLHAS) && aloca(s, &d.accB, MAX_BOLHAS) &&
+       aloca(s, &d.accB, 2 * MAX_BOLHAS) &&  // with facesB and celsB behind it (zerarBolhas)
        aloca(s, &d.rhsB, MAX_BOLHAS) && aloca(s, &d.yB, MAX_BOLHAS) && aloca(s, &d.rb, MAX_BOLHAS) &&
-       aloca(s, &d.zb, MAX_BOLHAS) && aloca(s, &d.zvb, MAX_BOLHAS) && aloca(s, &d.pb, MAX_BOLHAS) &&
-       aloca(s, &d.apb, MAX_BOLHAS) && aloca(s, &d.ybf, MAX_BOLHAS) && aloca(s, &d.pbf, MAX_BOLHAS) &&
+       aloca(s, &d.zb, MAX_BOLHAS) && aloca(s, &d.pb, MAX_BOLHAS) && aloca(s, &d.apb, MAX_BOLHAS) &&
        aloca(s, &d.r, N) && aloca(s, &d.z, N) && aloca(s, &d.zOld, N) && aloca(s, &d.p, N) &&
        aloca(s, &d.ap, N) && aloca(s, &d.parciais, 4096) && aloca(s, &d.esc, 1);
+  d.facesB = (uint32_t*)(d.accB + MAX_BOLHAS);
+  d.celsB = d.facesB + MAX_BOLHAS;
   int nbMax = blocos(cap > (int)N ? cap : (int)N, 1024) + 1;
   ok = ok && aloca(s, &s->cont, nbMax) && aloca(s, &s->offs, nbMax) && aloca(s, &s->estado, 4);
   if (ok) s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, o->fused_ctas);

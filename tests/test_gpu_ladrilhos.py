@@ -6,7 +6,7 @@ import pytest
 
 from estado import erro_relativo
 from oraculo import carregar_oraculo
-from tanque import ciclo_v
+from tanque import ciclo_v, resolver_pressao
 from tanque.constantes import AGUA, AR, SOLIDO
 
 pytestmark = pytest.mark.gpu
@@ -35,3 +35,31 @@ def test_legs(lib_gpu, nx, ny, fundo):
     x = ciclo_v(tipo, b)
     assert np.all(np.isfinite(x))
     assert erro_relativo(x, ref) < 2e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(40, 9), (13, 13), (33, 47), (257, 65), (700, 520)], ids=str)
+def test_pcg_com_bolhas(lib_gpu, nx, ny):
+    """The plain engine's three kernels an iteration on one level, at block edges and with several cells a
+    thread, bubbles of one cell to many: q to 1e-4, norms and bubble pressures to 1e-3 of the oracle's
+    (the bounds of the fixed-count solves)."""
+    rng = np.random.default_rng(nx + ny)
+    tipo = np.full((ny, nx), AGUA, np.uint8)
+    tipo[int(ny * 0.75):] = AR
+    tipo[0] = tipo[-1] = SOLIDO
+    tipo[:, 0] = tipo[:, -1] = SOLIDO
+    rotulo = np.where(tipo == AR, 1, 0).astype(np.uint32)
+    for b, (i, j, w, h) in enumerate([(2, 2, 1, 1), (nx // 2, ny // 3, 4, 2), (nx // 3, 2, min(40, nx // 4), 2)]):
+        tipo[j:j + h, i:i + w] = AR
+        rotulo[j:j + h, i:i + w] = 2 + 5 * b
+    div = np.where(tipo == AGUA, 0.1 * rng.standard_normal((ny, nx)), 0).astype(np.float32)
+    rhs = (0.05 * rng.standard_normal(4096)).astype(np.float32)
+    saidas = []
+    for lig in (None, carregar_oraculo()):
+        q = np.zeros((ny, nx), np.float32)
+        bolhas = {"rotulo": rotulo, "rhs": rhs, "y": np.zeros(4096, np.float32)}
+        normas = resolver_pressao(tipo, div, q, 3, 0.0, bolhas, ligacao=lig)
+        saidas.append((q, bolhas["y"], normas))
+    (qg, yg, ng), (qo, yo, no) = saidas
+    assert erro_relativo(qg, qo) < 1e-4
+    assert erro_relativo(yg, yo) < 1e-3
+    assert erro_relativo(ng, no) < 1e-3
