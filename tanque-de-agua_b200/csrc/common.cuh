@@ -117,8 +117,7 @@ struct Dev {
   uint32_t* rotulo;
   uint8_t* pend;
   int* lista;
-  float *div, *q, *qAr, *fase, *faseTmp, *nX, *nY, *kap;
-  uint8_t *cheio, *cheioTmp;
+  float *div, *q, *qAr, *fase, *nX, *nY, *kap;
   // bubbles
   float *pressaoBolha, *volumeAlvo, *volumeBolhaF, *rhsBolhaF, *yBolhaF;
   uint8_t* vivo;

@@ -59,17 +59,59 @@ __global__ void k_zerar_mascara(float* sdf, int mw, int mh) {
   sdf[idx] = (float)molduraMascara(idx % mw, idx / mw, mw, mh);
 }
 
-// #tipos (js/fisica-cpu.js:293-299); with `ar`, the first step of #propagarRotulos (:412,
-// non-air cells lose their label) and the initial water fraction of #superficie (:309).
-__global__ void k_tipos(Dev d, int ar, int fase) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  uint8_t t = d.solido[c] ? SOLIDO : d.accCel[c].y > 0 ? AGUA : AR;
-  d.tipo[c] = t;
-  if (ar && t != AR) d.rotulo[c] = 0;
-  if (fase) {
-    double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
-    d.fase[c] = t == SOLIDO ? 0.0f : (float)fmin(1.0, dens / PARTICULAS_POR_CELULA);
+// Adds 1 to *cont for every lane with `sim` and returns the lane's slot: one atomic a warp.
+__device__ __forceinline__ int reservar(int* cont, bool sim) {
+  const unsigned m = __ballot_sync(0xffffffffu, sim);
+  if (!m) return 0;
+  const int lane = threadIdx.x & 31, lider = __ffs(m) - 1;
+  int base = 0;
+  if (lane == lider) base = atomicAdd(cont, __popc(m));
+  return __shfl_sync(0xffffffffu, base, lider) + __popc(m & ((1u << lane) - 1u));
+}
+
+// #tipos (js/fisica-cpu.js:293-299) and, with `faces`, the face velocities: the sums' quotient, gravity
+// where a particle contributed, zero on wall faces (js/fisica-cpu.js:265-266 + :271-291 in the integer form of
+// js/gpu/fisica.js:135-160).  With `ar`, the first step of #propagarRotulos (:412, non-air cells lose
+// their label) and the list of the cells its first pass may label (see k_rotulos_resolver).
+__global__ void __launch_bounds__(256) k_tipos(Dev d, int faces, float gdx, float gdy, int ar) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nx = d.nx, ny = d.ny;
+  if (faces) {
+    if (k < d.nu) {
+      const int i = k % (nx + 1), j = k / (nx + 1);
+      const int2 a = d.accU[k];
+      float val = 0.0f;
+      if (a.y > 0) val = __fadd_rn(__fdiv_rn((float)a.x, (float)a.y), gdx);
+      const bool s = i == 0 || i == nx || d.solido[i - 1 + j * nx] || d.solido[i + j * nx];
+      d.u[k] = s ? 0.0f : val;
+    }
+    if (k < d.nv) {
+      const int i = k % nx, j = k / nx;
+      const int2 a = d.accV[k];
+      float val = 0.0f;
+      if (a.y > 0) val = __fadd_rn(__fdiv_rn((float)a.x, (float)a.y), gdy);
+      const bool s = j == 0 || j == ny || d.solido[i + (j - 1) * nx] || d.solido[i + j * nx];
+      d.v[k] = s ? 0.0f : val;
+    }
+  }
+  bool p = false;
+  if (k < d.N) {
+    const uint8_t t = d.solido[k] ? SOLIDO : d.accCel[k].y > 0 ? AGUA : AR;
+    d.tipo[k] = t;
+    if (!faces) {  // the flags alone: the water fraction too (in a substep k_superficie makes it)
+      const double dens = (float)d.accCel[k].x * (1.0f / 65536.0f);
+      d.fase[k] = t == SOLIDO ? 0.0f : (float)fmin(1.0, dens / PARTICULAS_POR_CELULA);
+    }
+    if (ar) {
+      if (t != AR) d.rotulo[k] = 0;
+      const int i = k % nx, j = k / nx;
+      p = i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1 && t == AR && d.rotulo[k] == 0;
+      d.pend[k] = p ? 1 : 0;
+    }
+  }
+  if (ar) {
+    const int slot = reservar(&d.esc->pendentes, p);
+    if (p) d.lista[slot] = k;
   }
 }
 
@@ -81,297 +123,378 @@ __global__ void k_tipos(Dev d, int ar, int fase) {
 // point only backwards in raster order, so it has exactly one solution, and repeating the
 // update until nothing changes reaches it whatever order the cells are visited in.  Only the
 // cells that were unlabelled air at the start of the pass ("pending") change; for a pending
-// right/upper neighbour the before-the-pass value is 0.
-__global__ void k_rotulos_pendentes(Dev d, int passada) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx, j = c / d.nx;
-  bool interior = i >= 1 && j >= 1 && i < d.nx - 1 && j < d.ny - 1;
-  bool p = interior && d.tipo[c] == AR && d.rotulo[c] == 0;
-  if (passada > 0) p = p && d.pend[c];
-  d.pend[c] = p ? 1 : 0;
-  if (p) {
-    int slot = atomicAdd(&d.esc->pendentes, 1);
-    d.lista[slot] = c;
-  }
-}
-
-__global__ void k_rotulos_resolver(Dev d) {
+// right/upper neighbour the before-the-pass value is 0.  One CTA does both passes: the second's
+// pending cells are those of the first's list that are still unlabelled.
+__global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
   __shared__ int mudou;
   const int n = d.esc->pendentes;
   const int nx = d.nx;
   uint32_t* rot = d.rotulo;
-  const uint8_t* pend = d.pend;
-  // Each sweep fixes at least one more cell of the longest dependency chain; n + 2 sweeps
-  // always suffice.
-  for (int volta = 0; volta < n + 2; volta++) {
-    if (threadIdx.x == 0) mudou = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      int c = d.lista[t];
-      uint32_t r = rot[c - 1];
-      if (!r) r = pend[c + 1] ? 0u : rot[c + 1];
-      if (!r) r = rot[c - nx];
-      if (!r) r = pend[c + nx] ? 0u : rot[c + nx];
-      if (r != rot[c]) {
-        rot[c] = r;
-        mudou = 1;
+  uint8_t* pend = d.pend;
+  for (int passada = 0; passada < 2; passada++) {
+    if (passada == 1) {
+      for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const int c = d.lista[t];
+        if (pend[c] && rot[c] != 0) pend[c] = 0;
       }
+      __syncthreads();
     }
-    __syncthreads();
-    if (!mudou) break;
+    // Each sweep fixes at least one more cell of the longest dependency chain; n + 2 sweeps
+    // always suffice.
+    for (int volta = 0; volta < n + 2; volta++) {
+      if (threadIdx.x == 0) mudou = 0;
+      __syncthreads();
+      for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const int c = d.lista[t];
+        if (!pend[c]) continue;
+        uint32_t r = rot[c - 1];
+        if (!r) r = pend[c + 1] ? 0u : rot[c + 1];
+        if (!r) r = rot[c - nx];
+        if (!r) r = pend[c + nx] ? 0u : rot[c + nx];
+        if (r != rot[c]) {
+          rot[c] = r;
+          mudou = 1;
+        }
+      }
+      __syncthreads();
+      if (!mudou) break;
+      __syncthreads();
+    }
     __syncthreads();
   }
   if (threadIdx.x == 0) d.esc->pendentes = 0;
 }
 
 // ---------------------------------------------------------------- surface
-// #estenderNaParede (js/fisica-cpu.js:353-374): three layers, each a wall cell not yet filled
-// takes the mean of its filled 4-neighbours.  `marca` records the layer a wall cell was
-// filled in (255: not yet); a neighbour counts as filled in layer L if it is not a wall or was
-// filled in an earlier layer, so f can be updated in place.
-__global__ void k_estender(Dev d, int camada) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  uint8_t* marca = d.cheio;
-  if (d.tipo[c] != SOLIDO) return;
-  if (camada > 1 && marca[c] < camada) return;
-  int i = c % d.nx, j = c / d.nx;
-  const int nx = d.nx, ny = d.ny;
-  auto cheio = [&](int n) { return d.tipo[n] != SOLIDO || (camada > 1 && marca[n] < camada); };
-  double s = 0;
-  int k = 0;
-  float* f = d.fase;
-  if (i > 0 && cheio(c - 1)) { s += (double)f[c - 1]; k++; }
-  if (i < nx - 1 && cheio(c + 1)) { s += (double)f[c + 1]; k++; }
-  if (j > 0 && cheio(c - nx)) { s += (double)f[c - nx]; k++; }
-  if (j < ny - 1 && cheio(c + nx)) { s += (double)f[c + nx]; k++; }
-  if (k) {
-    d.faseTmp[c] = (float)(s / k);
-    marca[c] = (uint8_t)camada;
-  } else if (camada == 1) {
-    marca[c] = 255;
-  }
-}
-// The new values of a layer land in faseTmp and are committed here, so no cell of the layer
-// reads a value written in the same layer.
-__global__ void k_estender_gravar(Dev d, int camada) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  if (d.tipo[c] == SOLIDO && d.cheio[c] == camada) d.fase[c] = d.faseTmp[c];
-}
+// #superficie (js/fisica-cpu.js:306-345) on one 32x32 tile a CTA, in shared memory: the water fraction of
+// every cell, three times carried into the walls (#estenderNaParede, :353-374: three layers, each a
+// wall cell taking the mean of its neighbours that are no wall or were filled in an earlier layer) with
+// two separable (1 2 1)/4 blurs in between (:314-328), the normals grad f / |grad f| and the
+// curvature -div n / (2h) on the interior (:330-345; border cells are never written, they stay 0).  A
+// tile also computes the 13 cells around it that its result depends on, each stage needing one or
+// three fewer.  The 24 launches over the grid that this replaces took 105 us a substep on 160x100 cells,
+// where each waited for the one before, and 128 us on 840x536; this one takes 39 and 52 us.
+// The blurs walk a row or column a thread, so each value is converted to double once.
+constexpr int SUP_T = 32, SUP_H = 13, SUP_W = SUP_T + 2 * SUP_H, SUP_P = SUP_W + 1;  // odd pitch: no bank conflicts
+constexpr int SUP_THREADS = 256, SUP_SEG = 15;  // 4 segments of 15 cells a line
+constexpr uint8_t SUP_LIVRE = 0, SUP_FUNDO = 200, SUP_FORA = 255;  // marks: no wall; wall beyond layer 3; off the grid
 
-// The separable (1 2 1)/4 blur of #superficie (js/fisica-cpu.js:314-328).
-__global__ void k_borrar_x(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx;
-  int im = i > 0 ? c - 1 : c, ip = i < d.nx - 1 ? c + 1 : c;
-  const float* f = d.fase;
-  d.faseTmp[c] = (float)(((double)f[im] + 2 * (double)f[c] + (double)f[ip]) * 0.25);
-}
-__global__ void k_borrar_y(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int j = c / d.nx;
-  int jm = j > 0 ? c - d.nx : c, jp = j < d.ny - 1 ? c + d.nx : c;
-  const float* t = d.faseTmp;
-  d.fase[c] = (float)(((double)t[jm] + 2 * (double)t[c] + (double)t[jp]) * 0.25);
-}
-
-// Normal = grad f / |grad f| and curvature = -div n / (2h) on the interior
-// (js/fisica-cpu.js:330-345).  Border cells are never written (they stay 0).
-__global__ void k_normais(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx, j = c / d.nx;
-  if (i < 1 || j < 1 || i >= d.nx - 1 || j >= d.ny - 1) return;
-  const float* f = d.fase;
-  double gx = ((double)f[c + 1] - (double)f[c - 1]) * 0.5, gy = ((double)f[c + d.nx] - (double)f[c - d.nx]) * 0.5;
-  double g = hypot(gx, gy);
-  d.nX[c] = g > 1e-3 ? (float)(gx / g) : 0.0f;
-  d.nY[c] = g > 1e-3 ? (float)(gy / g) : 0.0f;
-}
-__global__ void k_curvatura(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx, j = c / d.nx;
-  if (i < 1 || j < 1 || i >= d.nx - 1 || j >= d.ny - 1) return;
-  double a = ((double)d.nX[c + 1] - (double)d.nX[c - 1]) + ((double)d.nY[c + d.nx] - (double)d.nY[c - d.nx]);
-  d.kap[c] = (float)(-a / (2 * d.h));
-}
-
-// #pressaoDoAr (js/fisica-cpu.js:381-403): surface-tension jump on interior air cells, in
-// units of q = p*dt/(rho*h).
-__global__ void k_pressao_ar(Dev d, double dt, double tensao) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  int i = c % d.nx, j = c / d.nx;
-  const int nx = d.nx;
-  float out = 0.0f;
-  if (i >= 1 && j >= 1 && i < nx - 1 && j < d.ny - 1 && d.tipo[c] == AR) {
-    double pp = 0;
-    if (tensao > 0) {
-      const float* kap = d.kap;
-      double s = kap[c];
-      int k = 1;
-      if (d.tipo[c - 1] == AGUA) { s += (double)kap[c - 1]; k++; }
-      if (d.tipo[c + 1] == AGUA) { s += (double)kap[c + 1]; k++; }
-      if (d.tipo[c - nx] == AGUA) { s += (double)kap[c - nx]; k++; }
-      if (d.tipo[c + nx] == AGUA) { s += (double)kap[c + nx]; k++; }
-      double kMax = 1 / d.h;
-      if (k > 1) pp += tensao * fmax(-kMax, fmin(kMax, s / k));
+__global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
+  __shared__ float f[SUP_W * SUP_P], g[SUP_W * SUP_P];
+  __shared__ uint8_t mk[SUP_W * SUP_P];  // SUP_LIVRE, the layer a wall cell is filled in (1-3), SUP_FUNDO, SUP_FORA
+  const int nx = d.nx, ny = d.ny, x0 = blockIdx.x * SUP_T - SUP_H, y0 = blockIdx.y * SUP_T - SUP_H;
+  for (int t = threadIdx.x; t < SUP_W * SUP_W; t += SUP_THREADS) {
+    const int i = t % SUP_W, j = t / SUP_W, gx = x0 + i, gy = y0 + j, o = j * SUP_P + i;
+    float v = 0.0f;
+    uint8_t m = SUP_FORA;
+    if (gx >= 0 && gy >= 0 && gx < nx && gy < ny) {
+      const int c = gx + gy * nx;
+      m = d.tipo[c] == SOLIDO ? SUP_FUNDO : SUP_LIVRE;
+      // the initial water fraction (:309)
+      const double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
+      if (m == SUP_LIVRE) v = (float)fmin(1.0, dens / PARTICULAS_POR_CELULA);
     }
-    out = (float)(pp * (dt / (DENSIDADE_AGUA * d.h)));
+    f[o] = v;
+    g[o] = 0.0f;
+    mk[o] = m;
   }
-  d.qAr[c] = out;
-}
-
-// #classificar + #miolo (js/fisica-cpu.js:456-494): the right-hand side of the projection,
-// divergence minus the density correction minus the known air pressure of neighbours.
-__global__ void k_classificar(Dev d, double dt, double tau) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  const int nx = d.nx, ny = d.ny;
-  int i = c % nx, j = c / nx;
-  if (d.tipo[c] != AGUA) {
-    d.div[c] = 0.0f;
-    d.q[c] = 0.0f;
-    return;
+  __syncthreads();
+  // the cells at least `b` inside the tile's region, one after the other over the threads
+  auto cada = [&](int b, auto fn) {
+    const int w = SUP_W - 2 * b;
+    for (int t = threadIdx.x; t < w * w; t += SUP_THREADS) fn((b + t / w) * SUP_P + b + t % w);
+  };
+  // the layer each wall cell is filled in follows from the types alone: a wall cell beside a cell of
+  // the layer before
+  for (int L = 1; L <= 3; L++) {
+    cada(L, [&](int o) {
+      if (mk[o] == SUP_FUNDO && (mk[o - 1] == L - 1 || mk[o + 1] == L - 1 || mk[o - SUP_P] == L - 1 || mk[o + SUP_P] == L - 1))
+        mk[o] = (uint8_t)L;
+    });
+    __syncthreads();
   }
-  double alvo = d.h / fmax(tau, dt);
-  double dv = (double)d.u[i + 1 + j * (nx + 1)] - (double)d.u[i + j * (nx + 1)] +
-              (double)d.v[i + (j + 1) * nx] - (double)d.v[i + j * nx];
-  double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
-  double excesso = dens / PARTICULAS_POR_CELULA - 1;
-  if (excesso < 0) {
-    bool miolo = i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1;
-    for (int b = -1; b <= 1 && miolo; b++)
-      for (int a = -1; a <= 1; a++) {
-        int n = i + a + (j + b) * nx;
-        if (d.solido[n] || d.accCel[n].y == 0) { miolo = false; break; }
+  // one extension from the cells `b` inside on: layer L reads the layers before it
+  auto estender = [&](int b) {
+    for (int L = 1; L <= 3; L++) {
+      cada(b + L, [&](int o) {
+        if (mk[o] != L) return;
+        double s = 0;
+        int k = 0;
+        const int nb[4] = {o - 1, o + 1, o - SUP_P, o + SUP_P};
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (mk[nb[q]] < L) {
+            s += (double)f[nb[q]];
+            k++;
+          }
+        f[o] = (float)(s / k);
+      });
+      __syncthreads();
+    }
+  };
+  const int seg = threadIdx.x >> 6, linha = threadIdx.x & 63;
+  // blur of the cells `b` inside: rows into g, then columns back into f (b + 1 inside)
+  auto borrar = [&](int b) {
+    if (linha >= b && linha < SUP_W - b) {
+      const int i0 = max(seg * SUP_SEG, b + 1), i1 = min((seg + 1) * SUP_SEG, SUP_W - b - 1), r = linha * SUP_P;
+      double a = i0 < i1 ? (double)f[r + i0 - 1] : 0.0, c = i0 < i1 ? (double)f[r + i0] : 0.0;
+      for (int i = i0; i < i1; i++) {
+        const double n = (double)f[r + i + 1];
+        const int gx = x0 + i;
+        g[r + i] = (float)(((gx > 0 ? a : c) + 2 * c + (gx < nx - 1 ? n : c)) * 0.25);
+        a = c;
+        c = n;
       }
-    if (!miolo) excesso = 0;
+    }
+    __syncthreads();
+    if (linha >= b + 1 && linha < SUP_W - b - 1) {
+      const int j0 = max(seg * SUP_SEG, b + 1), j1 = min((seg + 1) * SUP_SEG, SUP_W - b - 1);
+      double a = j0 < j1 ? (double)g[(j0 - 1) * SUP_P + linha] : 0.0, c = j0 < j1 ? (double)g[j0 * SUP_P + linha] : 0.0;
+      for (int j = j0; j < j1; j++) {
+        const double n = (double)g[(j + 1) * SUP_P + linha];
+        const int gy = y0 + j;
+        f[j * SUP_P + linha] = (float)(((gy > 0 ? a : c) + 2 * c + (gy < ny - 1 ? n : c)) * 0.25);
+        a = c;
+        c = n;
+      }
+    }
+    __syncthreads();
+  };
+  estender(0);
+  borrar(3);
+  estender(4);
+  borrar(7);
+  estender(8);
+  // f is done on the tile and 2 cells around it; the normals' components (g and h) on 1 cell around it
+  __shared__ float h[(SUP_T + 2) * (SUP_T + 3)];
+  constexpr int HP = SUP_T + 3;
+  for (int t = threadIdx.x; t < (SUP_T + 2) * (SUP_T + 2); t += SUP_THREADS) {
+    const int i = t % (SUP_T + 2), j = t / (SUP_T + 2), o = (j + 12) * SUP_P + i + 12, gx_ = x0 + i + 12, gy_ = y0 + j + 12;
+    float a = 0.0f, b = 0.0f;
+    if (gx_ >= 1 && gy_ >= 1 && gx_ < nx - 1 && gy_ < ny - 1) {
+      const double gx = ((double)f[o + 1] - (double)f[o - 1]) * 0.5, gy = ((double)f[o + SUP_P] - (double)f[o - SUP_P]) * 0.5;
+      const double n = hypot(gx, gy);
+      a = n > 1e-3 ? (float)(gx / n) : 0.0f;
+      b = n > 1e-3 ? (float)(gy / n) : 0.0f;
+    }
+    g[o] = a;
+    h[j * HP + i] = b;
   }
-  excesso = fmin(EXCESSO_MAX, fmax(EXCESSO_MIN, excesso));
-  double ar = 0;
-  long N = d.N;
-  if (tipoEm(d.tipo, (long)c - 1, N, AR)) ar += (double)d.qAr[c - 1];
-  if (tipoEm(d.tipo, (long)c + 1, N, AR)) ar += (double)d.qAr[c + 1];
-  if (tipoEm(d.tipo, (long)c - nx, N, AR)) ar += (double)d.qAr[c - nx];
-  if (tipoEm(d.tipo, (long)c + nx, N, AR)) ar += (double)d.qAr[c + nx];
-  d.div[c] = (float)(dv - alvo * excesso - ar);
+  __syncthreads();
+  for (int t = threadIdx.x; t < SUP_T * SUP_T; t += SUP_THREADS) {
+    const int i = t % SUP_T, j = t / SUP_T, gx = x0 + SUP_H + i, gy = y0 + SUP_H + j;
+    if (gx >= nx || gy >= ny) continue;
+    const int c = gx + gy * nx, o = (j + SUP_H) * SUP_P + i + SUP_H, oh = (j + 1) * HP + i + 1;
+    d.fase[c] = f[o];
+    if (gx < 1 || gy < 1 || gx >= nx - 1 || gy >= ny - 1) continue;
+    const double a = ((double)g[o + 1] - (double)g[o - 1]) + ((double)h[oh + HP] - (double)h[oh - HP]);
+    d.nX[c] = g[o];
+    d.nY[c] = h[oh];
+    d.kap[c] = (float)(-a / (2 * d.h));
+  }
 }
 
-// #ladoDireitoDasBolhas (js/fisica-cpu.js:429-454): per bubble, the water flowing into it
-// now minus the surface-tension term of each water face, its cell count, then the volume
-// recovery term and the initial pressure guess.  The per-bubble sums are 64-bit fixed point
-// (2^-32) so their value does not depend on the order cells arrive in.
-__global__ void k_bolhas_somar(Dev d) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
+// #pressaoDoAr (js/fisica-cpu.js:381-403): the surface-tension jump of cell c, interior air (0 elsewhere),
+// in units of q = p*dt/(rho*h).
+__device__ inline float pressaoDoAr(const Dev& d, int c, int i, int j, double dt, double tensao) {
   const int nx = d.nx;
-  int i = c % nx, j = c / nx;
-  if (i < 1 || j < 1 || i >= nx - 1 || j >= d.ny - 1) return;
-  uint32_t r = d.rotulo[c];
-  if (d.tipo[c] != AR || r < 2 || r >= (uint32_t)MAX_BOLHAS) return;
-  atomicAdd(&d.volB[r], 1u);
-  double t = d.qAr[c];
-  double s = 0;
-  if (d.tipo[c - 1] == AGUA) s += (double)d.u[i + j * (nx + 1)] - t;
-  if (d.tipo[c + 1] == AGUA) s += -(double)d.u[i + 1 + j * (nx + 1)] - t;
-  if (d.tipo[c - nx] == AGUA) s += (double)d.v[i + j * nx] - t;
-  if (d.tipo[c + nx] == AGUA) s += -(double)d.v[i + (j + 1) * nx] - t;
-  somaFixa(&d.accB[r], s, ESCALA_BOLHA);
-}
-
-__global__ void k_bolhas_fechar(Dev d, double dt) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= MAX_BOLHAS) return;
-  uint32_t vol = r >= 2 ? d.volB[r] : 0u;
-  double soma = (double)d.accB[r] / ESCALA_BOLHA;
-  float rhs = (float)soma;
-  d.volumeBolhaF[r] = (float)vol;
-  if (vol) {
-    rhs = (float)((double)rhs + VOLTA_VOLUME_BOLHA * ((double)d.volumeAlvo[r] - (double)vol) * d.h / dt);
-    float y = (float)((double)d.pressaoBolha[r] * (dt / (DENSIDADE_AGUA * d.h)));
-    d.yBolhaF[r] = y;
+  if (!(i >= 1 && j >= 1 && i < nx - 1 && j < d.ny - 1) || d.tipo[c] != AR) return 0.0f;
+  double pp = 0;
+  if (tensao > 0) {
+    const float* kap = d.kap;
+    double s = kap[c];
+    int k = 1;
+    if (d.tipo[c - 1] == AGUA) { s += (double)kap[c - 1]; k++; }
+    if (d.tipo[c + 1] == AGUA) { s += (double)kap[c + 1]; k++; }
+    if (d.tipo[c - nx] == AGUA) { s += (double)kap[c - nx]; k++; }
+    if (d.tipo[c + nx] == AGUA) { s += (double)kap[c + nx]; k++; }
+    double kMax = 1 / d.h;
+    if (k > 1) pp += tensao * fmax(-kMax, fmin(kMax, s / k));
   }
-  d.rhsBolhaF[r] = rhs;
-  d.rhsB[r] = rhs;
-  d.yB[r] = d.yBolhaF[r];
+  return (float)(pp * (dt / (DENSIDADE_AGUA * d.h)));
 }
 
-// #pressao after resolverPCG (js/fisica-cpu.js:503-514): air cells get the surface-tension
-// pressure plus their bubble's pressure; bubbles keep their pressure in Pa (clamped).
-__global__ void k_pos_pressao(Dev d, int ar) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.N) return;
-  if (d.tipo[c] != AR) return;
-  uint32_t r = d.rotulo[c];
-  bool bolha = ar && r >= 2 && r < (uint32_t)MAX_BOLHAS && d.volumeBolhaF[r] != 0.0f;
-  d.q[c] = (float)((double)d.qAr[c] + (bolha ? (double)d.yBolhaF[r] : 0.0));
-}
-__global__ void k_pos_pressao_bolhas(Dev d, double dt) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < 2 || r >= MAX_BOLHAS) return;
-  if (d.volumeBolhaF[r] == 0.0f) return;
-  double paraPa = (DENSIDADE_AGUA * d.h) / dt;
-  d.pressaoBolha[r] = (float)fmax(-PRESSAO_BOLHA_MAX, fmin(PRESSAO_BOLHA_MAX, (double)d.yBolhaF[r] * paraPa));
+// #pressaoDoAr, #classificar + #miolo (js/fisica-cpu.js:456-494) and the cells' part of
+// #ladoDireitoDasBolhas (:429-454) in one pass over the grid: the air's pressure; the right-hand side of
+// the projection, divergence minus the density correction minus the known air pressure of the
+// neighbours (each neighbour's made again here, few cells have one); per bubble the water flowing
+// into it now minus the surface-tension term of each water face, and its cells.  The per-bubble sums
+// are 64-bit fixed point (2^-32) so their value does not depend on the order cells arrive in.  The last
+// block closes the bubbles' right-hand sides: the volume recovery term and the initial pressure.
+__global__ void __launch_bounds__(256) k_lado_direito(Dev d, double dt, double tensao, double tau, int bolhas) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nx = d.nx, ny = d.ny;
+  uint32_t b = 0;
+  if (c < d.N) {
+    const int i = c % nx, j = c / nx, t0 = d.tipo[c];
+    const float qa = pressaoDoAr(d, c, i, j, dt, tensao);
+    d.qAr[c] = qa;
+    if (t0 != AGUA) {
+      d.div[c] = 0.0f;
+      d.q[c] = 0.0f;
+    } else {
+      double alvo = d.h / fmax(tau, dt);
+      double dv = (double)d.u[i + 1 + j * (nx + 1)] - (double)d.u[i + j * (nx + 1)] +
+                  (double)d.v[i + (j + 1) * nx] - (double)d.v[i + j * nx];
+      double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
+      double excesso = dens / PARTICULAS_POR_CELULA - 1;
+      if (excesso < 0) {
+        bool miolo = i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1;
+        for (int b2 = -1; b2 <= 1 && miolo; b2++)
+          for (int a = -1; a <= 1; a++) {
+            int n = i + a + (j + b2) * nx;
+            if (d.solido[n] || d.accCel[n].y == 0) { miolo = false; break; }
+          }
+        if (!miolo) excesso = 0;
+      }
+      excesso = fmin(EXCESSO_MAX, fmax(EXCESSO_MIN, excesso));
+      double ar = 0;
+      long N = d.N;
+      const int nb[4] = {c - 1, c + 1, c - nx, c + nx};  // flat neighbours, as the reference reads them
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (tipoEm(d.tipo, (long)nb[k], N, AR)) ar += (double)pressaoDoAr(d, nb[k], nb[k] % nx, nb[k] / nx, dt, tensao);
+      d.div[c] = (float)(dv - alvo * excesso - ar);
+    }
+    if (bolhas && t0 == AR && i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1) {
+      const uint32_t r = d.rotulo[c];
+      if (r >= 2 && r < (uint32_t)MAX_BOLHAS) {
+        b = r;
+        double t = qa;
+        double s = 0;
+        if (d.tipo[c - 1] == AGUA) s += (double)d.u[i + j * (nx + 1)] - t;
+        if (d.tipo[c + 1] == AGUA) s += -(double)d.u[i + 1 + j * (nx + 1)] - t;
+        if (d.tipo[c - nx] == AGUA) s += (double)d.v[i + j * nx] - t;
+        if (d.tipo[c + nx] == AGUA) s += -(double)d.v[i + (j + 1) * nx] - t;
+        somaFixa(&d.accB[r], s, ESCALA_BOLHA);
+      }
+    }
+  }
+  if (!bolhas) return;  // uniform over the grid
+  if (__any_sync(0xffffffffu, b != 0)) {  // the cells of a bubble lie together: an atomic a warp and bubble
+    const unsigned g = __match_any_sync(0xffffffffu, b);
+    if (b && (int)(threadIdx.x & 31) == __ffs(g) - 1) atomicAdd(&d.volB[b], (unsigned)__popc(g));
+  }
+  __shared__ bool ultimo;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    ultimo = atomicAdd(&d.esc->tickets[1], 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!ultimo) return;
+  __threadfence();
+  if (threadIdx.x == 0) d.esc->tickets[1] = 0;
+  for (int r = threadIdx.x; r < MAX_BOLHAS; r += blockDim.x) {
+    uint32_t vol = r >= 2 ? __ldcg(&d.volB[r]) : 0u;
+    double soma = (double)__ldcg(&d.accB[r]) / ESCALA_BOLHA;
+    float rhs = (float)soma;
+    d.volumeBolhaF[r] = (float)vol;
+    float y = d.yBolhaF[r];
+    if (vol) {
+      rhs = (float)((double)rhs + VOLTA_VOLUME_BOLHA * ((double)d.volumeAlvo[r] - (double)vol) * d.h / dt);
+      y = (float)((double)d.pressaoBolha[r] * (dt / (DENSIDADE_AGUA * d.h)));
+      d.yBolhaF[r] = y;
+    }
+    d.rhsBolhaF[r] = rhs;
+    d.rhsB[r] = rhs;
+    d.yB[r] = y;
+  }
 }
 
-// #gradiente (js/fisica-cpu.js:519-545)
-__global__ void k_gradiente(Dev d) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+// #pressao after resolverPCG (js/fisica-cpu.js:503-514) and #gradiente (:519-545) in one pass: air cells get
+// the surface-tension pressure plus their bubble's pressure; bubbles keep their pressure in Pa
+// (clamped); the faces beside water take the gradient, into uTmp / vTmp.  A face reads an air cell's
+// pressure from its parts, so no thread waits for the q another writes.
+__global__ void __launch_bounds__(256) k_gradiente(Dev d, double dt, int ar) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = d.nx, ny = d.ny;
   const uint8_t* tipo = d.tipo;
-  const float* q = d.q;
+  auto qDoAr = [&](int c) {
+    const uint32_t r = d.rotulo[c];
+    const bool bolha = ar && r >= 2 && r < (uint32_t)MAX_BOLHAS && d.volumeBolhaF[r] != 0.0f;
+    return (float)((double)d.qAr[c] + (bolha ? (double)d.yBolhaF[r] : 0.0));
+  };
+  auto qDe = [&](int c, uint8_t t) { return t == AR ? qDoAr(c) : d.q[c]; };
+  if (k < d.N && tipo[k] == AR) d.q[k] = qDoAr(k);
+  if (ar && k >= 2 && k < MAX_BOLHAS && d.volumeBolhaF[k] != 0.0f) {
+    const double paraPa = (DENSIDADE_AGUA * d.h) / dt;
+    d.pressaoBolha[k] = (float)fmax(-PRESSAO_BOLHA_MAX, fmin(PRESSAO_BOLHA_MAX, (double)d.yBolhaF[k] * paraPa));
+  }
+  if (k == 0) d.esc->vmaxBits = 0;  // k_g2p's largest speed starts from 0
   if (k < d.nu) {
-    int i = k % (nx + 1), j = k / (nx + 1);
-    uint8_t tl = i > 0 ? tipo[i - 1 + j * nx] : SOLIDO;
-    uint8_t tr = i < nx ? tipo[i + j * nx] : SOLIDO;
-    if (tl == SOLIDO || tr == SOLIDO) { d.u[k] = 0.0f; d.uVal[k] = 1; }
-    else if (tl == AGUA || tr == AGUA) {
-      d.u[k] = (float)((double)d.u[k] - ((double)q[i + j * nx] - (double)q[i - 1 + j * nx]));
-      d.uVal[k] = 1;
-    } else d.uVal[k] = 0;
+    const int i = k % (nx + 1), j = k / (nx + 1);
+    const uint8_t tl = i > 0 ? tipo[i - 1 + j * nx] : SOLIDO;
+    const uint8_t tr = i < nx ? tipo[i + j * nx] : SOLIDO;
+    float u = d.u[k];
+    int val = 0;
+    if (tl == SOLIDO || tr == SOLIDO) {
+      u = 0.0f;
+      val = 1;
+    } else if (tl == AGUA || tr == AGUA) {
+      u = (float)((double)u - ((double)qDe(i + j * nx, tr) - (double)qDe(i - 1 + j * nx, tl)));
+      val = 1;
+    }
+    d.uTmp[k] = u;
+    d.uValTmp[k] = (uint8_t)val;
   }
   if (k < d.nv) {
-    int i = k % nx, j = k / nx;
-    uint8_t tb = j > 0 ? tipo[i + (j - 1) * nx] : SOLIDO;
-    uint8_t tt = j < ny ? tipo[i + j * nx] : SOLIDO;
-    if (tb == SOLIDO || tt == SOLIDO) { d.v[k] = 0.0f; d.vVal[k] = 1; }
-    else if (tb == AGUA || tt == AGUA) {
-      d.v[k] = (float)((double)d.v[k] - ((double)q[i + j * nx] - (double)q[i + (j - 1) * nx]));
-      d.vVal[k] = 1;
-    } else d.vVal[k] = 0;
+    const int i = k % nx, j = k / nx;
+    const uint8_t tb = j > 0 ? tipo[i + (j - 1) * nx] : SOLIDO;
+    const uint8_t tt = j < ny ? tipo[i + j * nx] : SOLIDO;
+    float v = d.v[k];
+    int val = 0;
+    if (tb == SOLIDO || tt == SOLIDO) {
+      v = 0.0f;
+      val = 1;
+    } else if (tb == AGUA || tt == AGUA) {
+      v = (float)((double)v - ((double)qDe(i + j * nx, tt) - (double)qDe(i + (j - 1) * nx, tb)));
+      val = 1;
+    }
+    d.vTmp[k] = v;
+    d.vValTmp[k] = (uint8_t)val;
   }
 }
 
-// extrapolarComponente (js/fisica-cpu.js:673-690), one layer for u and v: an invalid face takes
-// the mean of its valid 4-neighbours; reads (a, valid), writes (aOut, validOut).
-__device__ inline void extrapolar1(const float* a, const uint8_t* val, float* ao, uint8_t* vo, int k, int w, int hh) {
-  int i = k % w, j = k / w;
-  if (val[k]) { ao[k] = a[k]; vo[k] = 1; return; }
+// extrapolarComponente (js/fisica-cpu.js:673-690), both layers for u and v: an invalid face takes the mean
+// of its valid 4-neighbours, or, with none, of the neighbours that the first layer made valid (each
+// made again here: few faces need it).  Reads uTmp / vTmp, writes u / v.
+__device__ inline bool camadaExtrapolada(const float* a, const uint8_t* val, int k, int w, int hh, float* out) {
+  const int i = k % w, j = k / w;
   double soma = 0;
   int n = 0;
   if (i > 0 && val[k - 1]) { soma += (double)a[k - 1]; n++; }
   if (i < w - 1 && val[k + 1]) { soma += (double)a[k + 1]; n++; }
   if (j > 0 && val[k - w]) { soma += (double)a[k - w]; n++; }
   if (j < hh - 1 && val[k + w]) { soma += (double)a[k + w]; n++; }
-  if (n > 0) { ao[k] = (float)(soma / n); vo[k] = 1; }
-  else { ao[k] = a[k]; vo[k] = 0; }
+  if (n > 0) *out = (float)(soma / n);
+  return n > 0;
 }
-__global__ void k_extrapolar(Dev d, int volta) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < d.nu) {
-    if (!volta) extrapolar1(d.u, d.uVal, d.uTmp, d.uValTmp, k, d.nx + 1, d.ny);
-    else extrapolar1(d.uTmp, d.uValTmp, d.u, d.uVal, k, d.nx + 1, d.ny);
+__device__ inline void extrapolar2(const float* a, const uint8_t* val, float* ao, uint8_t* vo, int k, int w, int hh) {
+  float x = a[k];
+  bool ok = val[k] != 0;
+  if (!ok) ok = camadaExtrapolada(a, val, k, w, hh, &x);
+  if (!ok) {
+    const int i = k % w, j = k / w;
+    double soma = 0;
+    int n = 0;
+    float y = 0.0f;
+    if (i > 0 && camadaExtrapolada(a, val, k - 1, w, hh, &y)) { soma += (double)y; n++; }
+    if (i < w - 1 && camadaExtrapolada(a, val, k + 1, w, hh, &y)) { soma += (double)y; n++; }
+    if (j > 0 && camadaExtrapolada(a, val, k - w, w, hh, &y)) { soma += (double)y; n++; }
+    if (j < hh - 1 && camadaExtrapolada(a, val, k + w, w, hh, &y)) { soma += (double)y; n++; }
+    if (n > 0) {
+      x = (float)(soma / n);
+      ok = true;
+    }
   }
-  if (k < d.nv) {
-    if (!volta) extrapolar1(d.v, d.vVal, d.vTmp, d.vValTmp, k, d.nx, d.ny + 1);
-    else extrapolar1(d.vTmp, d.vValTmp, d.v, d.vVal, k, d.nx, d.ny + 1);
-  }
+  ao[k] = x;
+  vo[k] = ok ? 1 : 0;
+}
+__global__ void __launch_bounds__(256) k_extrapolar(Dev d) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < d.nu) extrapolar2(d.uTmp, d.uValTmp, d.u, d.uVal, k, d.nx + 1, d.ny);
+  if (k < d.nv) extrapolar2(d.vTmp, d.vValTmp, d.v, d.vVal, k, d.nx, d.ny + 1);
 }
 
 // ---------------------------------------------------------------- host launchers
@@ -394,53 +517,27 @@ void lancarTracar(const Dev& d, double x0m, double y0m, double x1m, double y1m, 
 void lancarZerarMascara(const Dev& d, cudaStream_t s) {
   lanca(k_zerar_mascara, blocos(d.mw * d.mh, 256), 256, 0, s, (float*)d.sdf, d.mw, d.mh);
 }
-void lancarTipos(const Dev& d, bool ar, cudaStream_t s) {
-  lanca(k_tipos, blocos(d.N, 256), 256, 0, s, d, ar ? 1 : 0, 1);
+void lancarTipos(const Dev& d, bool faces, float gdx, float gdy, bool ar, cudaStream_t s) {
+  const int m = !faces ? d.N : d.nu > d.nv ? d.nu : d.nv;
+  lanca(k_tipos, blocos(m, 256), 256, 0, s, d, faces ? 1 : 0, gdx, gdy, ar ? 1 : 0);
 }
-void lancarPropagarRotulos(const Dev& d, cudaStream_t s) {
-  for (int passada = 0; passada < 2; passada++) {
-    lanca(k_rotulos_pendentes, blocos(d.N, 256), 256, 0, s, d, passada);
-    lanca(k_rotulos_resolver, 1, 1024, 0, s, d);
-  }
-}
+void lancarPropagarRotulos(const Dev& d, cudaStream_t s) { lanca(k_rotulos_resolver, 1, 1024, 0, s, d); }
 void lancarSuperficie(const Dev& d, cudaStream_t s) {
-  int nb = blocos(d.N, 256);
-  for (int passada = 0; passada <= 2; passada++) {
-    for (int camada = 1; camada <= 3; camada++) {
-      lanca(k_estender, nb, 256, 0, s, d, camada);
-      lanca(k_estender_gravar, nb, 256, 0, s, d, camada);
-    }
-    if (passada == 2) break;
-    lanca(k_borrar_x, nb, 256, 0, s, d);
-    lanca(k_borrar_y, nb, 256, 0, s, d);
-  }
-  lanca(k_normais, nb, 256, 0, s, d);
-  lanca(k_curvatura, nb, 256, 0, s, d);
+  lanca(k_superficie, dim3(blocos(d.nx, SUP_T), blocos(d.ny, SUP_T)), SUP_THREADS, 0, s, d);
 }
-void lancarPressaoDoAr(const Dev& d, double dt, double tensao, cudaStream_t s) {
-  lanca(k_pressao_ar, blocos(d.N, 256), 256, 0, s, d, dt, tensao);
+void lancarLadoDireito(const Dev& d, double dt, double tensao, double tau, bool bolhas, cudaStream_t s) {
+  // accB, facesB, celsB and volB are one block of memory
+  if (bolhas) cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * (sizeof(long long) + 3 * sizeof(uint32_t)), s);
+  lanca(k_lado_direito, blocos(d.N, 256), 256, 0, s, d, dt, tensao, tau, bolhas ? 1 : 0);
 }
-void lancarClassificar(const Dev& d, double dt, double tau, cudaStream_t s) {
-  lanca(k_classificar, blocos(d.N, 256), 256, 0, s, d, dt, tau);
-}
-void lancarLadoDireitoBolhas(const Dev& d, double dt, cudaStream_t s) {
-  cudaMemsetAsync(d.volB, 0, MAX_BOLHAS * sizeof(uint32_t), s);
-  cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * sizeof(long long), s);
-  lanca(k_bolhas_somar, blocos(d.N, 256), 256, 0, s, d);
-  lanca(k_bolhas_fechar, blocos(MAX_BOLHAS, 256), 256, 0, s, d, dt);
-}
-void lancarPosPressao(const Dev& d, double dt, bool ar, cudaStream_t s) {
-  lanca(k_pos_pressao, blocos(d.N, 256), 256, 0, s, d, ar ? 1 : 0);
-  if (ar) lanca(k_pos_pressao_bolhas, blocos(MAX_BOLHAS, 256), 256, 0, s, d, dt);
-}
-void lancarGradiente(const Dev& d, cudaStream_t s) {
+void lancarGradiente(const Dev& d, double dt, bool ar, cudaStream_t s) {
   int m = d.nu > d.nv ? d.nu : d.nv;
-  lanca(k_gradiente, blocos(m, 256), 256, 0, s, d);
+  m = m > MAX_BOLHAS ? m : MAX_BOLHAS;
+  lanca(k_gradiente, blocos(m, 256), 256, 0, s, d, dt, ar ? 1 : 0);
 }
 void lancarExtrapolar(const Dev& d, cudaStream_t s) {
   int m = d.nu > d.nv ? d.nu : d.nv;
-  lanca(k_extrapolar, blocos(m, 256), 256, 0, s, d, 0);
-  lanca(k_extrapolar, blocos(m, 256), 256, 0, s, d, 1);
+  lanca(k_extrapolar, blocos(m, 256), 256, 0, s, d);
 }
 
 }  // namespace tq

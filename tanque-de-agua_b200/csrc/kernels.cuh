@@ -6,7 +6,6 @@ namespace tq {
 
 // particulas.cu
 void lancarP2G(const Dev& d, int nHint, cudaStream_t s);
-void lancarFaces(const Dev& d, float gdx, float gdy, cudaStream_t s);
 void lancarG2P(const Dev& d, int nHint, double dt, cudaStream_t s);
 void lancarCompactar(const Dev& d, int nHint, int* cont, int* offs, int* estado, cudaStream_t s);
 void lancarAdicionar(const Dev& d, const float* lista, int total, int checar, int* cont, int* offs,
@@ -23,14 +22,12 @@ void lancarSolidos(const Dev& d, cudaStream_t s);
 void lancarTracar(const Dev& d, double x0, double y0, double x1, double y1, double raio, bool apagar, cudaStream_t s);
 void lancarZerarMascara(const Dev& d, cudaStream_t s);
 void lancarMancha(const Dev& d, int n, int w, int hp, unsigned long long* acc, float* out, cudaStream_t s);
-void lancarTipos(const Dev& d, bool ar, cudaStream_t s);
+// cell flags and (faces) the face velocities from the sums; ar: the first step of the labels' propagation
+void lancarTipos(const Dev& d, bool faces, float gdx, float gdy, bool ar, cudaStream_t s);
 void lancarPropagarRotulos(const Dev& d, cudaStream_t s);
 void lancarSuperficie(const Dev& d, cudaStream_t s);
-void lancarPressaoDoAr(const Dev& d, double dt, double tensao, cudaStream_t s);
-void lancarClassificar(const Dev& d, double dt, double tau, cudaStream_t s);
-void lancarLadoDireitoBolhas(const Dev& d, double dt, cudaStream_t s);
-void lancarPosPressao(const Dev& d, double dt, bool ar, cudaStream_t s);
-void lancarGradiente(const Dev& d, cudaStream_t s);
+void lancarLadoDireito(const Dev& d, double dt, double tensao, double tau, bool bolhas, cudaStream_t s);
+void lancarGradiente(const Dev& d, double dt, bool ar, cudaStream_t s);
 void lancarExtrapolar(const Dev& d, cudaStream_t s);
 
 // regioes.cu — the closed regions of a solve (water sealed from every Dirichlet cell): their

@@ -1,6 +1,5 @@
 // particulas.cu — particle kernels of the substep: particle-to-grid transfer (fixed point),
-// face normalisation + gravity + wall faces, grid-to-particle transfer with APIC, micro-step
-// advection and wall collision, and the particle bookkeeping (insert, tools, compaction).
+// grid-to-particle transfer with APIC, micro-step advection and wall collision, and the particle bookkeeping (insert, tools, compaction).
 //
 // Built with -fmad=false: the f32 operations of the fixed-point transfer must be exactly the
 // sequence the oracle restates (no contraction into fused multiply-adds), and the double
@@ -183,29 +182,6 @@ __global__ void __launch_bounds__(P2G_T) k_p2g(Dev d) {
 #pragma unroll
     for (int q = 0; q < 3; q++)
       if (sD[3 * t + q]) atomicAdd(&d.accCor[3 * (i + j * nx) + q], sD[3 * t + q]);
-  }
-}
-
-// Face velocity from the sums, gravity impulse where a particle contributed, zero on wall
-// faces: js/fisica-cpu.js:265-266 + :271-291 in the integer form of js/gpu/fisica.js:135-160.
-__global__ void k_faces(Dev d, float gdx, float gdy) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nx = d.nx, ny = d.ny;
-  if (k < d.nu) {
-    int i = k % (nx + 1), j = k / (nx + 1);
-    int2 a = d.accU[k];
-    float val = 0.0f;
-    if (a.y > 0) val = __fadd_rn(__fdiv_rn((float)a.x, (float)a.y), gdx);
-    bool s = i == 0 || i == nx || d.solido[i - 1 + j * nx] || d.solido[i + j * nx];
-    d.u[k] = s ? 0.0f : val;
-  }
-  if (k < d.nv) {
-    int i = k % nx, j = k / nx;
-    int2 a = d.accV[k];
-    float val = 0.0f;
-    if (a.y > 0) val = __fadd_rn(__fdiv_rn((float)a.x, (float)a.y), gdy);
-    bool s = j == 0 || j == ny || d.solido[i + (j - 1) * nx] || d.solido[i + j * nx];
-    d.v[k] = s ? 0.0f : val;
   }
 }
 
@@ -668,10 +644,6 @@ void lancarMancha(const Dev& d, int n, int w, int hp, unsigned long long* acc, f
 
 void lancarP2G(const Dev& d, int nHint, cudaStream_t s) {
   if (nHint > 0) lanca(k_p2g, blocos(nHint, P2G_T), P2G_T, 0, s, d);
-}
-void lancarFaces(const Dev& d, float gdx, float gdy, cudaStream_t s) {
-  int m = d.nu > d.nv ? d.nu : d.nv;
-  lanca(k_faces, blocos(m, 256), 256, 0, s, d, gdx, gdy);
 }
 void lancarG2P(const Dev& d, int nHint, double dt, cudaStream_t s) {
   if (nHint > 0) lanca(k_g2p, blocos(nHint, 128), 128, 0, s, d, dt);

@@ -149,15 +149,17 @@ void marca(tq_sim* s, int i) {
   if (s->atual) (*s->atual)[i] = evento(s);
 }
 
+// The particle-to-grid sums to 0: one block of memory (Dev::accU, accV, accCel, accCor).
+void zerarSomas(const Dev& d, cudaStream_t st) {
+  cudaMemsetAsync(d.accU, 0, sizeof(int2) * ((size_t)d.nu + d.nv + d.N) + sizeof(int) * 3 * d.N, st);
+}
+
 // P2G + flags only (the first half of atualizarAr when the flags are stale, js/fisica-cpu.js:164).
 void paraGradeETipos(tq_sim* s) {
   const Dev& d = s->d;
-  cudaMemsetAsync(d.accU, 0, sizeof(int2) * d.nu, s->s);
-  cudaMemsetAsync(d.accV, 0, sizeof(int2) * d.nv, s->s);
-  cudaMemsetAsync(d.accCel, 0, sizeof(int2) * d.N, s->s);
-  cudaMemsetAsync(d.accCor, 0, sizeof(int) * 3 * d.N, s->s);
+  zerarSomas(d, s->s);
   lancarP2G(d, s->nHint, s->s);
-  lancarTipos(d, false, s->s);
+  lancarTipos(d, false, 0.0f, 0.0f, false, s->s);
   s->tiposProntos = true;
 }
 
@@ -166,31 +168,23 @@ int subpasso(tq_sim* s, double dt) {
   const bool ar = s->o.air != 0;
   cudaStream_t st = s->s;
   marca(s, 0);
-  cudaMemsetAsync(d.accU, 0, sizeof(int2) * d.nu, st);
-  cudaMemsetAsync(d.accV, 0, sizeof(int2) * d.nv, st);
-  cudaMemsetAsync(d.accCel, 0, sizeof(int2) * d.N, st);
-  cudaMemsetAsync(d.accCor, 0, sizeof(int) * 3 * d.N, st);
+  zerarSomas(d, st);
   lancarP2G(d, s->nHint, st);                                              // #paraGrade
-  lancarFaces(d, (float)(s->o.gravity[0] * dt), (float)(s->o.gravity[1] * dt), st);  // #gravidadeEFronteira
   marca(s, 1);
-  lancarTipos(d, ar, st);                                                  // #tipos
+  lancarTipos(d, true, (float)(s->o.gravity[0] * dt), (float)(s->o.gravity[1] * dt), ar, st);  // #gravidadeEFronteira, #tipos
   s->tiposProntos = true;
   if (ar) lancarPropagarRotulos(d, st);                                    // #propagarRotulos
   marca(s, 2);
   lancarSuperficie(d, st);                                                 // #superficie
   marca(s, 3);
-  lancarPressaoDoAr(d, dt, s->o.surface_tension, st);                      // #pressaoDoAr
-  lancarClassificar(d, dt, s->o.tau_density, st);                          // #classificar
-  if (ar) lancarLadoDireitoBolhas(d, dt, st);                              // #ladoDireitoDasBolhas
+  lancarLadoDireito(d, dt, s->o.surface_tension, s->o.tau_density, ar, st);  // #pressaoDoAr, #classificar, #ladoDireitoDasBolhas
   marca(s, 4);
   int r = resolverPressao(s->pcg, d, s->o.iterations, s->o.tolerance, ar, s->o.preconditioner, st);  // #pressao
   if (r) return r == TQ_E_CUDA ? falha(r, "pressure solve failed") : r;
-  lancarPosPressao(d, dt, ar, st);
   marca(s, 5);
-  lancarGradiente(d, st);                                                  // #gradiente
+  lancarGradiente(d, dt, ar, st);                                          // #pressao's end, #gradiente
   lancarExtrapolar(d, st);                                                 // #extrapolar
   marca(s, 6);
-  cudaMemsetAsync(&d.esc->vmaxBits, 0, sizeof(unsigned long long), st);
   lancarG2P(d, s->nHint, dt, st);                                          // #paraParticulas
   marca(s, 7);
   cudaError_t e = cudaGetLastError();
@@ -330,23 +324,27 @@ int tq_create(const tq_options* o, tq_sim** out) {
   d.sdf = sdf;
   ok = ok && aloca(s, &d.solido, N) && aloca(s, &d.p0, cap) && aloca(s, &d.p1, cap) && aloca(s, &d.p2, cap) &&
        aloca(s, &d.pid, cap) && aloca(s, &d.q0, cap) && aloca(s, &d.q1, cap) && aloca(s, &d.q2, cap) &&
-       aloca(s, &d.qid, cap) && aloca(s, &d.accU, nu) && aloca(s, &d.accV, nv) && aloca(s, &d.accCel, N) &&
-       aloca(s, &d.accCor, 3 * N) && aloca(s, &d.u, nu) && aloca(s, &d.v, nv) && aloca(s, &d.uTmp, nu) &&
+       aloca(s, &d.qid, cap) && aloca(s, &d.accU, nu + nv + N + (3 * N + 1) / 2) &&  // with accV, accCel, accCor behind it (zerarSomas)
+       aloca(s, &d.u, nu) && aloca(s, &d.v, nv) && aloca(s, &d.uTmp, nu) &&
        aloca(s, &d.vTmp, nv) && aloca(s, &d.uVal, nu) && aloca(s, &d.vVal, nv) && aloca(s, &d.uValTmp, nu) &&
        aloca(s, &d.vValTmp, nv) && aloca(s, &d.tipo, N) && aloca(s, &d.rotulo, N) && aloca(s, &d.pend, N) &&
        aloca(s, &d.lista, N) && aloca(s, &d.div, N) && aloca(s, &d.q, N) && aloca(s, &d.qAr, N) &&
-       aloca(s, &d.fase, N) && aloca(s, &d.faseTmp, N) && aloca(s, &d.nX, N) && aloca(s, &d.nY, N) &&
-       aloca(s, &d.kap, N) && aloca(s, &d.cheio, N) && aloca(s, &d.cheioTmp, N) &&
+       aloca(s, &d.fase, N) && aloca(s, &d.nX, N) && aloca(s, &d.nY, N) &&
+       aloca(s, &d.kap, N) &&
        aloca(s, &d.pressaoBolha, MAX_BOLHAS) && aloca(s, &d.volumeAlvo, MAX_BOLHAS) &&
        aloca(s, &d.volumeBolhaF, MAX_BOLHAS) && aloca(s, &d.rhsBolhaF, MAX_BOLHAS) &&
-       aloca(s, &d.yBolhaF, MAX_BOLHAS) && aloca(s, &d.vivo, MAX_BOLHAS) && aloca(s, &d.volB, MAX_BOLHAS) &&
-       aloca(s, &d.accB, 2 * MAX_BOLHAS) &&  // with facesB and celsB behind it (zerarBolhas)
+       aloca(s, &d.yBolhaF, MAX_BOLHAS) && aloca(s, &d.vivo, MAX_BOLHAS) &&
+       aloca(s, &d.accB, 5 * MAX_BOLHAS / 2) &&  // with facesB, celsB and volB behind it (zerarBolhas)
        aloca(s, &d.rhsB, MAX_BOLHAS) && aloca(s, &d.yB, MAX_BOLHAS) && aloca(s, &d.rb, MAX_BOLHAS) &&
        aloca(s, &d.zb, MAX_BOLHAS) && aloca(s, &d.pb, MAX_BOLHAS) && aloca(s, &d.apb, MAX_BOLHAS) &&
        aloca(s, &d.r, N) && aloca(s, &d.z, N) && aloca(s, &d.zOld, N) && aloca(s, &d.p, N) &&
        aloca(s, &d.ap, N) && aloca(s, &d.parciais, 4096) && aloca(s, &d.esc, 1);
   d.facesB = (uint32_t*)(d.accB + MAX_BOLHAS);
   d.celsB = d.facesB + MAX_BOLHAS;
+  d.volB = d.celsB + MAX_BOLHAS;
+  d.accV = d.accU + nu;
+  d.accCel = d.accV + nv;
+  d.accCor = (int*)(d.accCel + N);
   int nbMax = blocos(cap > (int)N ? cap : (int)N, 1024) + 1;
   ok = ok && aloca(s, &s->cont, nbMax) && aloca(s, &s->offs, nbMax) && aloca(s, &s->estado, 4);
   if (ok) s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, o->fused_ctas);
