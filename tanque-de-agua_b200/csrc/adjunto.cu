@@ -840,7 +840,7 @@ struct tq_adj {
   int passos, K, n0, nf, cap, N, nu, nv;
   cudaStream_t s = nullptr;
   Pcg* pcg = nullptr;
-  std::vector<void*> mem;
+  Arena arena;
   // scene
   float* sdf;
   uint8_t* solido;
@@ -885,10 +885,7 @@ thread_local char g_erroAdj[256] = "";
 
 template <class T>
 bool alocar(tq_adj* a, T** p, size_t n) {
-  void* q = nullptr;
-  if (cudaMalloc(&q, (n ? n : 1) * sizeof(T)) != cudaSuccess) return false;
-  a->mem.push_back(q);
-  *p = (T*)q;
+  a->arena.pedir(p, n ? n : 1);
   return true;
 }
 
@@ -1146,8 +1143,8 @@ int tq_adj_create(const tq_adj_scene* d, int32_t device, tq_adj** out) {
        alocar(a, &a->r, N) && alocar(a, &a->z, N) && alocar(a, &a->zv, N) && alocar(a, &a->p, N) &&
        alocar(a, &a->ap, N) && alocar(a, &a->parc, SOMA_CTAS) && alocar(a, &a->esc, E_N) && alocar(a, &a->bf, N) &&
        alocar(a, &a->xf, N) && alocar(a, &a->tipoCG, N) && alocar(a, &a->xCG, N);
-  if (ok) a->pcg = criarPcg(d->nx, d->ny, TQ_PREC_FP32, TQ_ENGINE_PLAIN);
-  if (!ok || !a->pcg) {
+  if (ok) a->pcg = criarPcg(d->nx, d->ny, TQ_PREC_FP32, TQ_ENGINE_PLAIN, a->arena);
+  if (!ok || !a->arena.reservar(a->s) || !iniciarPcg(a->pcg, a->s) || cudaStreamSynchronize(a->s) != cudaSuccess) {
     tq_adj_destroy(a);
     return TQ_E_NOMEM;
   }
@@ -1228,7 +1225,6 @@ int tq_adj_destroy(tq_adj* a) {
   if (a->s) cudaStreamSynchronize(a->s);
   if (a->grafoCG) cudaGraphExecDestroy(a->grafoCG);
   destruirPcg(a->pcg);
-  for (void* p : a->mem) cudaFree(p);
   if (a->s) cudaStreamDestroy(a->s);
   delete a;
   return TQ_OK;

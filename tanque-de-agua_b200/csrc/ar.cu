@@ -428,7 +428,7 @@ __global__ void k_ar_rotular(Rastreador r, uint32_t* rotulo) {
 }
 
 // ---------------------------------------------------------------- host side
-Rastreador* criarRastreador(int nx, int ny) {
+Rastreador* criarRastreador(int nx, int ny, Arena& A) {
   Rastreador* r = new Rastreador();
   r->nx = nx;
   r->ny = ny;
@@ -440,51 +440,38 @@ Rastreador* criarRastreador(int nx, int ny) {
   int cap = 1;
   while (cap < N) cap <<= 1;  // power of two for the global sort
   r->nBlocos = blocos(N, 1024);
-  bool ok = true;
-  ok &= cudaMalloc(&r->pai, N * sizeof(int)) == cudaSuccess;
-  ok &= cudaMalloc(&r->cnt, N * sizeof(uint32_t)) == cudaSuccess;
-  ok &= cudaMalloc(&r->atm, N * sizeof(uint32_t)) == cudaSuccess;
-  ok &= cudaMalloc(&r->topo, N) == cudaSuccess;
-  ok &= cudaMalloc(&r->compIdx, N * sizeof(int)) == cudaSuccess;
-  ok &= cudaMalloc(&r->hk, (size_t)hc * 8) == cudaSuccess;
-  ok &= cudaMalloc(&r->hcnt, (size_t)hc * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->hfirst, (size_t)hc * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->celK, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->atmK, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->rotK, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->topoK, N) == cudaSuccess;
-  ok &= cudaMalloc(&r->novoAlvo, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->dono, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->gasCount, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->gasOff, N * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->parKey, (size_t)cap * 8) == cudaSuccess;
-  ok &= cudaMalloc(&r->parVal, (size_t)cap * 8) == cudaSuccess;
-  ok &= cudaMalloc(&r->ordKey, (size_t)cap * 8) == cudaSuccess;
-  ok &= cudaMalloc(&r->ganhador, MAX_BOLHAS * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->vivoNovo, MAX_BOLHAS) == cudaSuccess;
-  ok &= cudaMalloc(&r->livres, MAX_BOLHAS * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->pNova, MAX_BOLHAS * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->sob, MAX_BOLHAS * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->nasceu, MAX_BOLHAS * 4) == cudaSuccess;
-  ok &= cudaMalloc(&r->cont, 8 * sizeof(int)) == cudaSuccess;
-  ok &= cudaMalloc(&r->blocoCont, (r->nBlocos + 1) * sizeof(int)) == cudaSuccess;
-  ok &= cudaMalloc(&r->blocoOff, (r->nBlocos + 1) * sizeof(int)) == cudaSuccess;
-  if (!ok) {
-    destruirRastreador(r);
-    return nullptr;
-  }
+  A.pedir(&r->pai, N);
+  A.pedir(&r->cnt, N);
+  A.pedir(&r->atm, N);
+  A.pedir(&r->topo, N);
+  A.pedir(&r->compIdx, N);
+  A.pedir(&r->hk, hc);
+  A.pedir(&r->hcnt, hc);
+  A.pedir(&r->hfirst, hc);
+  A.pedir(&r->celK, N);
+  A.pedir(&r->atmK, N);
+  A.pedir(&r->rotK, N);
+  A.pedir(&r->topoK, N);
+  A.pedir(&r->novoAlvo, N);
+  A.pedir(&r->dono, N);
+  A.pedir(&r->gasCount, N);
+  A.pedir(&r->gasOff, N);
+  A.pedir(&r->parKey, cap);
+  A.pedir(&r->parVal, cap);
+  A.pedir(&r->ordKey, cap);
+  A.pedir(&r->ganhador, MAX_BOLHAS);
+  A.pedir(&r->vivoNovo, MAX_BOLHAS);
+  A.pedir(&r->livres, MAX_BOLHAS);
+  A.pedir(&r->pNova, MAX_BOLHAS);
+  A.pedir(&r->sob, MAX_BOLHAS);
+  A.pedir(&r->nasceu, MAX_BOLHAS);
+  A.pedir(&r->cont, 8);
+  A.pedir(&r->blocoCont, r->nBlocos + 1);
+  A.pedir(&r->blocoOff, r->nBlocos + 1);
   return r;
 }
 
-void destruirRastreador(Rastreador* r) {
-  if (!r) return;
-  void* ps[] = {r->pai, r->cnt, r->atm, r->topo, r->compIdx, r->hk, r->hcnt, r->hfirst, r->celK, r->atmK,
-                r->rotK, r->topoK, r->novoAlvo, r->dono, r->gasCount, r->gasOff, r->parKey, r->parVal,
-                r->ordKey, r->ganhador, r->vivoNovo, r->livres, r->pNova, r->sob, r->nasceu, r->cont,
-                r->blocoCont, r->blocoOff};
-  for (void* p : ps) cudaFree(p);
-  delete r;
-}
+void destruirRastreador(Rastreador* r) { delete r; }
 
 // reiniciar (js/ar.js:37-42)
 void reiniciarRastreador(Rastreador* r, const Dev& d, cudaStream_t s) {

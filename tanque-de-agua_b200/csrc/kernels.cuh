@@ -1,5 +1,6 @@
 // kernels.cuh — host launchers of the substep kernels (one translation unit each).
 #pragma once
+#include "arena.cuh"
 #include "common.cuh"
 
 namespace tq {
@@ -33,7 +34,7 @@ void lancarExtrapolar(const Dev& d, cudaStream_t s);
 // regioes.cu — the closed regions of a solve (water sealed from every Dirichlet cell): their
 // right-hand side projected onto A's range and one cell of each pinned at 0 (tolerance mode).
 struct Regioes;
-Regioes* criarRegioes(int N);
+Regioes* criarRegioes(int N, cudaStream_t s);
 void destruirRegioes(Regioes* R);
 // Queues the labelling and projection; *out = d with div / rhsBolhaF / tipo at the solve's copies.
 void projetarFechadas(Regioes* R, const Dev& d, bool bolhas, cudaStream_t s, Dev* out);
@@ -41,8 +42,10 @@ int erroRegioes(Regioes* R, cudaStream_t s);
 
 // pcg.cu — the pressure solve on the handle's grid.
 struct Pcg;
-// ctasFundido: the fused engine's CTA count (0: one per SM).
-Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido = 0);
+// ctasFundido: the fused engine's CTA count (0: one per SM).  Its arrays come from A: call iniciarPcg once A
+// is reserved, and destroy it before A.
+Pcg* criarPcg(int nx, int ny, int precisao, int motor, Arena& A, int ctasFundido = 0);
+bool iniciarPcg(Pcg* p, cudaStream_t s);
 void destruirPcg(Pcg* p);
 // Solves for d.q on the cells d.tipo marks as water; bubbles from d.rotulo / d.rhsB / d.yB when
 // `bolhas`; precond is TQ_PRECOND_*.  The FUSED engine queues the solve without waiting; the
@@ -50,8 +53,8 @@ void destruirPcg(Pcg* p);
 // residual history and convergence record stay in d.esc.  Returns TQ_OK or an error status.
 // In tolerance mode the right-hand side of each closed region first loses its mean (regioes.cu).
 int resolverPressao(Pcg* p, const Dev& d, int iteracoes, double tol, bool bolhas, int precond, cudaStream_t s);
-// Allocates what a tolerance-mode solve allocates on first use (before a stream capture).
-int reservarTolerancia(Pcg* p);
+// Allocates what a tolerance-mode solve allocates on first use (before a stream capture on s).
+int reservarTolerancia(Pcg* p, cudaStream_t s);
 // The last solve's residual history from the device (waits for the stream); its length, or -1.
 int normasPcg(Pcg* p, const Dev& d, double* out, int cap, cudaStream_t s);
 // TQ_E_TIMEOUT if a fused solve since the last call gave up on a bounded wait (waits for the stream).
@@ -76,7 +79,7 @@ int cicloVSemAlocar(void* scratch, int nx, int ny, const uint8_t* tipo, const fl
 
 // ar.cu — RastreadorDeAr.atualizar on the device.
 struct Rastreador;
-Rastreador* criarRastreador(int nx, int ny);
+Rastreador* criarRastreador(int nx, int ny, Arena& A);
 void destruirRastreador(Rastreador* r);
 void reiniciarRastreador(Rastreador* r, const Dev& d, cudaStream_t s);
 int atualizarRastreador(Rastreador* r, const Dev& d, cudaStream_t s);

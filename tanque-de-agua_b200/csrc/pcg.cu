@@ -951,7 +951,7 @@ static int escolherLadrilho(int nx, int ny, bool subir, bool uma) {
 
 
 
-Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
+Pcg* criarPcg(int nx, int ny, int precisao, int motor, Arena& A, int ctasFundido) {
   Pcg* p = new Pcg();
   p->ctasFundido = ctasFundido;
   p->nx = nx;
@@ -973,18 +973,17 @@ Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
     L++;
   }
   p->L = L;
-  bool ok = true;
   for (int l = 0; l < L; l++) {
     size_t n = (size_t)p->nxL[l] * p->nyL[l];
     p->meia[l] = precisao != TQ_PREC_FP32 && n >= (size_t)MEIA_MIN_CELULAS;
-    const size_t e = 4;  // room for FP32 whatever the engine stores
-    ok &= cudaMalloc(&p->tipoL[l], n) == cudaSuccess;
-    ok &= cudaMalloc(&p->vizL[l], n) == cudaSuccess;
-    ok &= cudaMalloc(&p->bL[l], n * e) == cudaSuccess;
-    ok &= cudaMalloc(&p->xL[l], n * e) == cudaSuccess;
-    ok &= cudaMalloc(&p->tmpL[l], n * e) == cudaSuccess;
+    A.pedir(&p->tipoL[l], n);
+    A.pedir(&p->vizL[l], n);
+    // room for FP32 whatever the engine stores
+    A.pedir((float**)&p->bL[l], n);
+    A.pedir((float**)&p->xL[l], n);
+    A.pedir((float**)&p->tmpL[l], n);
   }
-  ok &= cudaMalloc(&p->vizOp, p->N) == cudaSuccess;
+  A.pedir(&p->vizOp, p->N);
   size_t nc = (size_t)p->nxL[L - 1] * p->nyL[L - 1];
   p->smemGrosso = nc * 9 <= 200 * 1024 ? nc * 9 : 0;
   if (p->smemGrosso) {
@@ -996,46 +995,32 @@ Pcg* criarPcg(int nx, int ny, int precisao, int motor, int ctasFundido) {
     };
     if (!subir(k_grosso<float>) || !subir(k_grosso<__half>) || !subir(k_grosso<__nv_bfloat16>)) p->smemGrosso = 0;
   }
-  if (ok && motor == TQ_ENGINE_FUSED) {
+  if (motor == TQ_ENGINE_FUSED) {
     // Grids with a single level (min(nx, ny) <= 12) have nothing to hand to the coarse
     // section: they run on the plain engine.
-    p->fundido = criarFundido(p);
+    p->fundido = criarFundido(p, A);
     if (!p->fundido) {
       cudaGetLastError();
       p->motor = TQ_ENGINE_PLAIN;
     }
   }
-  if (ok && p->motor == TQ_ENGINE_PLAIN) {
+  if (p->motor == TQ_ENGINE_PLAIN) {
     // the partial sums of k_plano_da / k_plano_b's blocks, or of the gather's tiles if more
     const int k = escolherLadrilho(nx, ny, true, false);
     const size_t lad = (size_t)blocos(nx, 16 * k) * blocos(ny, 16 * k);
-    const size_t np = 2 * (lad > (size_t)BLOCOS_PCG ? lad : (size_t)BLOCOS_PCG);
-    ok = cudaMalloc(&p->op, (size_t)p->N * 2) == cudaSuccess && cudaMalloc(&p->p2, (size_t)p->N * 4) == cudaSuccess &&
-         cudaMalloc(&p->parc, np * sizeof(double)) == cudaSuccess &&
-         cudaMalloc(&p->ativos, (MAX_BOLHAS + 1) * sizeof(int)) == cudaSuccess;
-  }
-  if (!ok) {
-    destruirPcg(p);
-    return nullptr;
+    A.pedir(&p->op, p->N);
+    A.pedir(&p->p2, p->N);
+    A.pedir(&p->parc, 2 * (lad > (size_t)BLOCOS_PCG ? lad : (size_t)BLOCOS_PCG));
+    A.pedir(&p->ativos, MAX_BOLHAS + 1);
   }
   return p;
 }
 
+bool iniciarPcg(Pcg* p, cudaStream_t s) { return !p->fundido || iniciarFundido(p->fundido, p, s); }
+
 void destruirPcg(Pcg* p) {
   if (!p) return;
   destruirFundido(p->fundido);
-  for (int l = 0; l < p->L; l++) {
-    cudaFree(p->tipoL[l]);
-    cudaFree(p->vizL[l]);
-    cudaFree(p->bL[l]);
-    cudaFree(p->xL[l]);
-    cudaFree(p->tmpL[l]);
-  }
-  cudaFree(p->vizOp);
-  cudaFree(p->op);
-  cudaFree(p->p2);
-  cudaFree(p->parc);
-  cudaFree(p->ativos);
   if (p->q64) cudaFree(p->q64);
   destruirRegioes(p->regioes);
   delete p;
@@ -1201,8 +1186,8 @@ static void precondicionar(Pcg* p, const Juncao& J, bool bloco, bool umaPassada,
 // exact iteration, with one host round trip per LOTE_VERIFICACAO iterations instead of one each.
 constexpr int LOTE_VERIFICACAO = 8;
 
-int reservarTolerancia(Pcg* p) {
-  if (!p->regioes && !(p->regioes = criarRegioes(p->N))) return TQ_E_NOMEM;
+int reservarTolerancia(Pcg* p, cudaStream_t s) {
+  if (!p->regioes && !(p->regioes = criarRegioes(p->N, s))) return TQ_E_NOMEM;
   if (p->motor != TQ_ENGINE_FUSED && !p->q64 && cudaMalloc(&p->q64, (size_t)p->N * sizeof(double)) != cudaSuccess)
     return TQ_E_NOMEM;
   return TQ_OK;
@@ -1212,7 +1197,7 @@ int resolverPressao(Pcg* p, const Dev& d0, int iteracoes, double tol, bool bolha
   Dev d = d0;
   double* q64 = nullptr;
   if (tol > 0) {
-    if (reservarTolerancia(p)) return TQ_E_NOMEM;
+    if (reservarTolerancia(p, s)) return TQ_E_NOMEM;
     projetarFechadas(p->regioes, d0, bolhas, s, &d);  // d reads the projected right-hand sides
     q64 = p->q64;
   }

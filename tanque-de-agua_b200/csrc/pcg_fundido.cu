@@ -2208,7 +2208,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
 template <class T>
 static void* kernelDe() { return (void*)k_mgpcg<T>; }
 
-Fundido* criarFundido(Pcg* p) {
+Fundido* criarFundido(Pcg* p, Arena& A) {
   if (p->L < 2) return nullptr;  // no coarse level to hand to the coarse section
   Fundido* f = new Fundido();
   // coarse section: the longest suffix of levels (not level 0) fitting the shared budget
@@ -2264,88 +2264,89 @@ Fundido* criarFundido(Pcg* p) {
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaFuncSetAttribute(f->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemMax) == cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&porSM, f->kern, TF, f->smem) == cudaSuccess && porSM >= 1;
-  if (ok) {
-    // one CTA per SM (co-resident, as the grid barrier needs), or the requested fewer
-    f->G = p->ctasFundido > 0 && p->ctasFundido < sms ? p->ctasFundido : sms;
-    const size_t N = p->N;
-    const size_t nLc = (size_t)p->nxL[Lc] * p->nyL[Lc];
-    ok = cudaMalloc(&f->niveis, MAX_NIVEIS * sizeof(NivelF)) == cudaSuccess &&
-         cudaMalloc(&f->parc, (size_t)f->G * NPARC * sizeof(double)) == cudaSuccess &&
-         cudaMalloc(&f->bar, 2 * sizeof(unsigned)) == cudaSuccess && cudaMalloc(&f->erro, sizeof(int)) == cudaSuccess &&
-         cudaMalloc(&f->accZ, MAX_BOLHAS * sizeof(long long)) == cudaSuccess &&
-         cudaMalloc(&f->zb2, MAX_BOLHAS * sizeof(double)) == cudaSuccess &&
-         cudaMalloc(&f->pb2, MAX_BOLHAS * sizeof(double)) == cudaSuccess &&
-         cudaMalloc(&f->ativos, MAX_BOLHAS * sizeof(int)) == cudaSuccess &&
-         cudaMalloc(&f->nAtivos, sizeof(int)) == cudaSuccess && cudaMalloc(&f->p2, N * 4) == cudaSuccess &&
-         cudaMalloc(&f->z2, N * 4) == cudaSuccess && cudaMalloc(&f->xc, nLc * 4) == cudaSuccess &&
-         cudaMalloc(&f->bc, nLc * 4) == cudaSuccess && cudaMalloc(&f->op, N * sizeof(uint16_t)) == cudaSuccess &&
-         cudaMalloc(&f->rotB, N * sizeof(unsigned long long)) == cudaSuccess &&
-         cudaMalloc(&f->q64, N * sizeof(double)) == cudaSuccess &&
-         cudaMalloc(&f->accV, MAX_BOLHAS * sizeof(long long)) == cudaSuccess;
-    // Wall blocks are skipped on levels of at least two full rounds of the grid's warps (a
-    // tank atlas's finest levels): there the flags' one extra load per warp and pass is paid
-    // back; a level of one round (the 450k-cell scene's) keeps no flags.
-    // TQ_WALL_SKIP_MIN_BLOCKS in the environment (read when the handle is created) sets the
-    // threshold in blocks; the tests use 1 to skip on every grid level and 0x7fffffff for none.
-    long long limiar = 2LL * WARPS * f->G;
-    if (const char* e = getenv("TQ_WALL_SKIP_MIN_BLOCKS")) limiar = atoll(e);
-    if (const char* e = getenv("TQ_BARRIER_WAIT_CYCLES")) {
-      const long long v = atoll(e);
-      if (v > 0 && v <= LIMITE_CICLOS) f->limite = v;
-    }
-    if (const char* e = getenv("TQ_BARRIER_HOLD_CTA")) f->segurarCta = atoi(e);
-    if (const char* e = getenv("TQ_BARRIER_HOLD_CYCLES")) {
-      const long long v = atoll(e);
-      f->segurarCiclos = v > 0 && v <= 4 * LIMITE_CICLOS ? v : 0;
-    }
-    size_t nFlags = 0;
-    for (int l = 0; l < Lc; l++) {
-      f->comParedes[l] = blocosNivel(p->nxL[l], p->nyL[l], 0) >= limiar;
-      if (f->comParedes[l]) nFlags += blocosNivel(p->nxL[l], p->nyL[l], 0) + blocosNivel(p->nxL[l], p->nyL[l], 8);
-    }
-    ok = ok && (nFlags == 0 || cudaMalloc(&f->solidos, nFlags) == cudaSuccess);
-    if (ok && f->secaoDensa)
-      ok = cudaMalloc(&f->mSecao, nLc * nLc * 4) == cudaSuccess && cudaMalloc(&f->wSecao, nLc * 4) == cudaSuccess &&
-           cudaMalloc(&f->wInv, nLc * 4) == cudaSuccess && cudaMalloc(&f->nW, 4) == cudaSuccess;
-    if (ok && f->offDenso >= 0) ok = cudaMalloc(&f->densoG, DENSO_BYTES) == cudaSuccess;
-  }
-  if (ok) {
-    NivelF tab[MAX_NIVEIS] = {};
-    for (int l = 0; l < p->L; l++) {
-      NivelF& n = tab[l];
-      n.nx = p->nxL[l];
-      n.ny = p->nyL[l];
-      n.meia = (l < Lc && p->meia[l]) ? (p->precisao == TQ_PREC_FP16 ? 1 : 2) : 0;
-      n.viz = p->vizL[l];
-      n.tipo = p->tipoL[l];
-      n.b = p->bL[l];
-      n.x = p->xL[l];
-      n.tmp = p->tmpL[l];
-    }
-    size_t off = 0;
-    for (int l = 0; l < Lc; l++) {
-      if (!f->comParedes[l]) continue;
-      f->sol[l] = f->solidos + off;
-      off += blocosNivel(p->nxL[l], p->nyL[l], 0) + blocosNivel(p->nxL[l], p->nyL[l], 8);
-    }
-    ok = cudaMemcpy(f->niveis, tab, sizeof tab, cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemset(f->bar, 0, 2 * sizeof(unsigned)) == cudaSuccess && cudaMemset(f->erro, 0, sizeof(int)) == cudaSuccess;
-  }
   if (!ok) {
     cudaGetLastError();
-    destruirFundido(f);
+    delete f;
     return nullptr;
   }
+  // one CTA per SM (co-resident, as the grid barrier needs), or the requested fewer
+  f->G = p->ctasFundido > 0 && p->ctasFundido < sms ? p->ctasFundido : sms;
+  // Wall blocks are skipped on levels of at least two full rounds of the grid's warps (a
+  // tank atlas's finest levels): there the flags' one extra load per warp and pass is paid
+  // back; a level of one round (the 450k-cell scene's) keeps no flags.
+  // TQ_WALL_SKIP_MIN_BLOCKS in the environment (read when the handle is created) sets the
+  // threshold in blocks; the tests use 1 to skip on every grid level and 0x7fffffff for none.
+  long long limiar = 2LL * WARPS * f->G;
+  if (const char* e = getenv("TQ_WALL_SKIP_MIN_BLOCKS")) limiar = atoll(e);
+  if (const char* e = getenv("TQ_BARRIER_WAIT_CYCLES")) {
+    const long long v = atoll(e);
+    if (v > 0 && v <= LIMITE_CICLOS) f->limite = v;
+  }
+  if (const char* e = getenv("TQ_BARRIER_HOLD_CTA")) f->segurarCta = atoi(e);
+  if (const char* e = getenv("TQ_BARRIER_HOLD_CYCLES")) {
+    const long long v = atoll(e);
+    f->segurarCiclos = v > 0 && v <= 4 * LIMITE_CICLOS ? v : 0;
+  }
+  size_t nFlags = 0;
+  for (int l = 0; l < Lc; l++) {
+    f->comParedes[l] = blocosNivel(p->nxL[l], p->nyL[l], 0) >= limiar;
+    if (f->comParedes[l]) nFlags += blocosNivel(p->nxL[l], p->nyL[l], 0) + blocosNivel(p->nxL[l], p->nyL[l], 8);
+  }
+  const size_t N = p->N, nLc = (size_t)p->nxL[Lc] * p->nyL[Lc];
+  A.pedir(&f->niveis, MAX_NIVEIS);
+  A.pedir(&f->parc, (size_t)f->G * NPARC);
+  A.pedir(&f->bar, 2);
+  A.pedir(&f->erro, 1);
+  A.pedir(&f->accZ, MAX_BOLHAS);
+  A.pedir(&f->zb2, MAX_BOLHAS);
+  A.pedir(&f->pb2, MAX_BOLHAS);
+  A.pedir(&f->ativos, MAX_BOLHAS);
+  A.pedir(&f->nAtivos, 1);
+  A.pedir(&f->p2, N);
+  A.pedir(&f->z2, N);
+  A.pedir(&f->xc, nLc);
+  A.pedir(&f->bc, nLc);
+  A.pedir(&f->op, N);
+  A.pedir(&f->rotB, N);
+  A.pedir(&f->q64, N);
+  A.pedir(&f->accV, MAX_BOLHAS);
+  if (nFlags) A.pedir(&f->solidos, nFlags);
+  if (f->secaoDensa) {
+    A.pedir(&f->mSecao, nLc * nLc);
+    A.pedir(&f->wSecao, nLc);
+    A.pedir(&f->wInv, nLc);
+    A.pedir(&f->nW, 1);
+  }
+  if (f->offDenso >= 0) A.pedir(&f->densoG, DENSO_BYTES / 4);
   return f;
+}
+
+// The level table on the device and the wall flags' places, once the arena is reserved.
+bool iniciarFundido(Fundido* f, const Pcg* p, cudaStream_t s) {
+  NivelF tab[MAX_NIVEIS] = {};
+  for (int l = 0; l < p->L; l++) {
+    NivelF& n = tab[l];
+    n.nx = p->nxL[l];
+    n.ny = p->nyL[l];
+    n.meia = (l < f->Lc && p->meia[l]) ? (p->precisao == TQ_PREC_FP16 ? 1 : 2) : 0;
+    n.viz = p->vizL[l];
+    n.tipo = p->tipoL[l];
+    n.b = p->bL[l];
+    n.x = p->xL[l];
+    n.tmp = p->tmpL[l];
+  }
+  size_t off = 0;
+  for (int l = 0; l < f->Lc; l++) {
+    if (!f->comParedes[l]) continue;
+    f->sol[l] = f->solidos + off;
+    off += blocosNivel(p->nxL[l], p->nyL[l], 0) + blocosNivel(p->nxL[l], p->nyL[l], 8);
+  }
+  return cudaMemcpyAsync(f->niveis, tab, sizeof tab, cudaMemcpyHostToDevice, s) == cudaSuccess;
 }
 
 void destruirFundido(Fundido* f) {
   if (!f) return;
-  void* ps[] = {f->niveis, f->parc, f->bar, f->erro, f->accZ, f->zb2, f->pb2, f->ativos,
-                f->nAtivos, f->p2, f->z2, f->xc, f->bc, f->perfil, f->op, f->rotB, f->mSecao, f->wSecao, f->wInv, f->nW,
-                f->densoG, f->solidos, f->q64, f->accV};
-  for (void* q : ps)
-    if (q) cudaFree(q);
+  if (f->perfil) cudaFree(f->perfil);
   delete f;
 }
 

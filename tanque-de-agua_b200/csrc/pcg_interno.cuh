@@ -3,6 +3,7 @@
 #pragma once
 #include <vector>
 
+#include "arena.cuh"
 #include "common.cuh"
 
 namespace tq {
@@ -41,7 +42,8 @@ inline void zerarBolhas(const Dev& d, cudaStream_t s) {
 }
 
 // pcg_fundido.cu
-Fundido* criarFundido(Pcg* p);
+Fundido* criarFundido(Pcg* p, Arena& A);
+bool iniciarFundido(Fundido* f, const Pcg* p, cudaStream_t s);
 void destruirFundido(Fundido* f);
 int resolverPressaoFundido(Pcg* p, const Dev& d, int iteracoes, double tol, bool bolhas, int precond,
                            cudaStream_t s);

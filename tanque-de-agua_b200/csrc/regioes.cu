@@ -34,7 +34,7 @@ namespace tq {
 
 constexpr int MAX_REGIOES = 4096;  // closed regions projected per solve (more: the rest as they are)
 
-struct Regioes {
+struct RegioesDev {
   int N = 0;
   int* pai = nullptr;        // N + MAX_BOLHAS
   int* idR = nullptr;        // N: per root, its closed-region index or -1
@@ -47,10 +47,13 @@ struct Regioes {
   float* rhs = nullptr;      // MAX_BOLHAS: the projected bubble right-hand sides
   uint8_t* tipo = nullptr;   // N: the solve's cell types, closed regions' roots pinned as air
 };
+struct Regioes : RegioesDev {  // the kernels take the pointers alone
+  Arena A;
+};
 
 namespace {
 
-__global__ void k_reg_iniciar(Regioes R, const uint8_t* tipo) {
+__global__ void k_reg_iniciar(RegioesDev R, const uint8_t* tipo) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < R.N) {
     R.pai[c] = tipo[c] == AGUA ? c : -1;
@@ -70,7 +73,7 @@ __global__ void k_reg_iniciar(Regioes R, const uint8_t* tipo) {
 
 // Active bubbles as k_bolhas_faces counts them: an interior air cell of the label with a water
 // neighbour.
-__global__ void k_reg_bolhas(Regioes R, Dev d) {
+__global__ void k_reg_bolhas(RegioesDev R, Dev d) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N) return;
   const int nx = d.nx, i = c % nx, j = c / nx;
@@ -83,7 +86,7 @@ __global__ void k_reg_bolhas(Regioes R, Dev d) {
 
 // Water joins its water neighbours (left and down; the others join it) and the bubble node of
 // each active bubble it faces; any other air neighbour is Dirichlet (valorViz's 0).
-__global__ void k_reg_unir(Regioes R, Dev d, int bolhas) {
+__global__ void k_reg_unir(RegioesDev R, Dev d, int bolhas) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N || d.tipo[c] != AGUA) return;
   const int nx = d.nx, i = c % nx, j = c / nx;
@@ -106,19 +109,19 @@ __global__ void k_reg_unir(Regioes R, Dev d, int bolhas) {
   if (!ok) R.cont[MAX_REGIOES + 1] = 1;
 }
 
-__global__ void k_reg_achatar(Regioes R) {
+__global__ void k_reg_achatar(RegioesDev R) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N + MAX_BOLHAS || R.pai[c] < 0) return;
   R.pai[c] = raizLeitura(R.pai, c);
 }
 
-__global__ void k_reg_abrir(Regioes R) {
+__global__ void k_reg_abrir(RegioesDev R) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N || !R.toca[c]) return;
   R.aberto[R.pai[c]] = 1;
 }
 
-__global__ void k_reg_ids(Regioes R) {
+__global__ void k_reg_ids(RegioesDev R) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N || R.pai[c] != c) return;  // roots only (water cells)
   int id = -1;
@@ -131,12 +134,12 @@ __global__ void k_reg_ids(Regioes R) {
 
 // The closed-region index of a node (water cell or bubble node), -1 when open or uncounted; a
 // bubble node left alone (no water joined it) has no region.
-__device__ inline int regiaoDe(const Regioes& R, int no) {
+__device__ inline int regiaoDe(const RegioesDev& R, int no) {
   const int r = R.pai[no];
   return r >= 0 && r < R.N ? R.idR[r] : -1;
 }
 
-__global__ void k_reg_somar(Regioes R, Dev d, int bolhas) {
+__global__ void k_reg_somar(RegioesDev R, Dev d, int bolhas) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < R.N && d.tipo[c] == AGUA) {
     const int id = regiaoDe(R, c);
@@ -154,7 +157,7 @@ __global__ void k_reg_somar(Regioes R, Dev d, int bolhas) {
   }
 }
 
-__global__ void k_reg_projetar(Regioes R, Dev d, int bolhas) {
+__global__ void k_reg_projetar(RegioesDev R, Dev d, int bolhas) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   auto media = [&](int id) { return R.soma[id] / (double)R.cont[id]; };
   if (c < R.N) {
@@ -187,20 +190,21 @@ __global__ void k_reg_projetar(Regioes R, Dev d, int bolhas) {
 
 }  // namespace
 
-Regioes* criarRegioes(int N) {
+Regioes* criarRegioes(int N, cudaStream_t s) {
   Regioes* R = new Regioes();
   R->N = N;
   const size_t n = (size_t)N;
-  bool ok = cudaMalloc(&R->pai, (n + MAX_BOLHAS) * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&R->idR, n * sizeof(int)) == cudaSuccess && cudaMalloc(&R->toca, n) == cudaSuccess &&
-            cudaMalloc(&R->aberto, n) == cudaSuccess && cudaMalloc(&R->ativa, MAX_BOLHAS) == cudaSuccess &&
-            cudaMalloc(&R->soma, MAX_REGIOES * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&R->cont, (MAX_REGIOES + 3) * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&R->div, n * sizeof(float)) == cudaSuccess &&
-            cudaMalloc(&R->rhs, MAX_BOLHAS * sizeof(float)) == cudaSuccess &&
-            cudaMalloc(&R->tipo, n) == cudaSuccess;
-  if (ok) ok = cudaMemset(R->cont + MAX_REGIOES + 2, 0, sizeof(int)) == cudaSuccess;
-  if (!ok) {
+  R->A.pedir(&R->pai, n + MAX_BOLHAS);
+  R->A.pedir(&R->idR, n);
+  R->A.pedir(&R->toca, n);
+  R->A.pedir(&R->aberto, n);
+  R->A.pedir(&R->ativa, MAX_BOLHAS);
+  R->A.pedir(&R->soma, MAX_REGIOES);
+  R->A.pedir(&R->cont, MAX_REGIOES + 3);
+  R->A.pedir(&R->div, n);
+  R->A.pedir(&R->rhs, MAX_BOLHAS);
+  R->A.pedir(&R->tipo, n);
+  if (!R->A.reservar(s)) {
     destruirRegioes(R);
     return nullptr;
   }
@@ -222,34 +226,21 @@ int erroRegioes(Regioes* R, cudaStream_t s) {
   return TQ_E_TIMEOUT;
 }
 
-void destruirRegioes(Regioes* R) {
-  if (!R) return;
-  cudaFree(R->pai);
-  cudaFree(R->idR);
-  cudaFree(R->toca);
-  cudaFree(R->aberto);
-  cudaFree(R->ativa);
-  cudaFree(R->soma);
-  cudaFree(R->cont);
-  cudaFree(R->div);
-  cudaFree(R->rhs);
-  cudaFree(R->tipo);
-  delete R;
-}
+void destruirRegioes(Regioes* R) { delete R; }
 
 // Queues the labelling and the projection on s; *out gets d with div, rhsBolhaF and tipo
 // pointing at the projected and pinned copies.  Nothing waits for the device.
 void projetarFechadas(Regioes* R, const Dev& d, bool bolhas, cudaStream_t s, Dev* out) {
   const int N = d.N;
   const int nb = blocos(N, 256), nbMax = blocos(N > MAX_BOLHAS ? N : MAX_BOLHAS, 256);
-  lanca(k_reg_iniciar, nbMax, 256, 0, s, *R, (const uint8_t*)d.tipo);
-  if (bolhas) lanca(k_reg_bolhas, nb, 256, 0, s, *R, d);
-  lanca(k_reg_unir, nb, 256, 0, s, *R, d, bolhas ? 1 : 0);
-  lanca(k_reg_achatar, blocos((long)N + MAX_BOLHAS, 256), 256, 0, s, *R);
-  lanca(k_reg_abrir, nb, 256, 0, s, *R);
-  lanca(k_reg_ids, nb, 256, 0, s, *R);
-  lanca(k_reg_somar, nbMax, 256, 0, s, *R, d, bolhas ? 1 : 0);
-  lanca(k_reg_projetar, nbMax, 256, 0, s, *R, d, bolhas ? 1 : 0);
+  lanca(k_reg_iniciar, nbMax, 256, 0, s, (const RegioesDev&)*R, (const uint8_t*)d.tipo);
+  if (bolhas) lanca(k_reg_bolhas, nb, 256, 0, s, (const RegioesDev&)*R, d);
+  lanca(k_reg_unir, nb, 256, 0, s, (const RegioesDev&)*R, d, bolhas ? 1 : 0);
+  lanca(k_reg_achatar, blocos((long)N + MAX_BOLHAS, 256), 256, 0, s, (const RegioesDev&)*R);
+  lanca(k_reg_abrir, nb, 256, 0, s, (const RegioesDev&)*R);
+  lanca(k_reg_ids, nb, 256, 0, s, (const RegioesDev&)*R);
+  lanca(k_reg_somar, nbMax, 256, 0, s, (const RegioesDev&)*R, d, bolhas ? 1 : 0);
+  lanca(k_reg_projetar, nbMax, 256, 0, s, (const RegioesDev&)*R, d, bolhas ? 1 : 0);
   *out = d;
   out->div = R->div;
   out->rhsBolhaF = R->rhs;

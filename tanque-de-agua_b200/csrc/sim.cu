@@ -39,19 +39,6 @@ int falhaCuda(cudaError_t e, const char* onde) {
     if (e_ != cudaSuccess) return falhaCuda(e_, #expr); \
   } while (0)
 
-// Cena#moldura (js/cena.js:132-137): the empty tank's SDF.
-void molduraSdf(std::vector<float>& sdf, int nx, int ny) {
-  const int r = RES_MASCARA, mw = nx * r, mh = ny * r;
-  sdf.resize((size_t)mw * mh);
-  double m = MOLDURA * r - 0.5;
-  for (int y = 0; y < mh; y++)
-    for (int x = 0; x < mw; x++) {
-      double d = std::fmin(std::fmin(x - m, (double)(mw - 1) - m - x), std::fmin(y - m, (double)(mh - 1) - m - y)) / r;
-      d = d > SDF_MAX ? SDF_MAX : d < -SDF_MAX ? -SDF_MAX : d;
-      sdf[(size_t)y * mw + x] = (float)d;
-    }
-}
-
 }  // namespace
 
 struct tq_sim {
@@ -69,7 +56,8 @@ struct tq_sim {
   size_t stagingCap = 0;
   unsigned long long* mancha = nullptr;  // tq_splat's fixed-point sums (5 planes), grown on demand
   size_t manchaCap = 0;
-  std::vector<void*> alocados;
+  Arena arena;       // the handle's device arrays
+  Arena tanques;     // those of tq_set_tanks
   // Stage timing (tq_set_timing): a pool of events recorded at the stage boundaries of every
   // substep and relabel, read back once by tq_get_timing.
   bool timing = false;
@@ -91,16 +79,6 @@ struct tq_sim {
 };
 
 namespace {
-
-template <class T>
-bool aloca(tq_sim* s, T** p, size_t n) {
-  void* q = nullptr;
-  if (cudaMalloc(&q, n * sizeof(T) + 16) != cudaSuccess) return false;
-  cudaMemset(q, 0, n * sizeof(T) + 16);
-  s->alocados.push_back(q);
-  *p = (T*)q;
-  return true;
-}
 
 int garantirStaging(tq_sim* s, size_t floats) {
   if (floats <= s->stagingCap) return TQ_OK;
@@ -278,7 +256,13 @@ const char* tq_status_string(int st) {
 }
 const char* tq_last_error(void) { return g_erro; }
 
-int tq_create(const tq_options* o, tq_sim** out) {
+// tq_create; with soSolver, a handle that holds only what a pressure solve reads and writes
+// (tq_solve_pressure).
+static int criarSim(const tq_options* o, bool soSolver, tq_sim** out);
+
+int tq_create(const tq_options* o, tq_sim** out) { return criarSim(o, false, out); }
+
+static int criarSim(const tq_options* o, bool soSolver, tq_sim** out) {
   if (!o || !out) return falha(TQ_E_ARG, "null argument");
   *out = nullptr;
   if (o->nx < 3 || o->ny < 3 || !(o->h > 0)) return falha(TQ_E_ARG, "grid must be at least 3x3 with h > 0");
@@ -319,47 +303,54 @@ int tq_create(const tq_options* o, tq_sim** out) {
   d.hf = (float)o->h;
   d.cap = cap;
   const size_t N = s->N, nu = s->nu, nv = s->nv;
+  Arena& A = s->arena;
   float* sdf = nullptr;
-  bool ok = aloca(s, &sdf, (size_t)s->mw * s->mh);
-  d.sdf = sdf;
-  ok = ok && aloca(s, &d.solido, N) && aloca(s, &d.p0, cap) && aloca(s, &d.p1, cap) && aloca(s, &d.p2, cap) &&
-       aloca(s, &d.pid, cap) && aloca(s, &d.q0, cap) && aloca(s, &d.q1, cap) && aloca(s, &d.q2, cap) &&
-       aloca(s, &d.qid, cap) && aloca(s, &d.accU, nu + nv + N + (3 * N + 1) / 2) &&  // with accV, accCel, accCor behind it (zerarSomas)
-       aloca(s, &d.u, nu) && aloca(s, &d.v, nv) && aloca(s, &d.uTmp, nu) &&
-       aloca(s, &d.vTmp, nv) && aloca(s, &d.uVal, nu) && aloca(s, &d.vVal, nv) && aloca(s, &d.uValTmp, nu) &&
-       aloca(s, &d.vValTmp, nv) && aloca(s, &d.tipo, N) && aloca(s, &d.rotulo, N) && aloca(s, &d.pend, N) &&
-       aloca(s, &d.lista, N) && aloca(s, &d.div, N) && aloca(s, &d.q, N) && aloca(s, &d.qAr, N) &&
-       aloca(s, &d.fase, N) && aloca(s, &d.nX, N) && aloca(s, &d.nY, N) &&
-       aloca(s, &d.kap, N) &&
-       aloca(s, &d.pressaoBolha, MAX_BOLHAS) && aloca(s, &d.volumeAlvo, MAX_BOLHAS) &&
-       aloca(s, &d.volumeBolhaF, MAX_BOLHAS) && aloca(s, &d.rhsBolhaF, MAX_BOLHAS) &&
-       aloca(s, &d.yBolhaF, MAX_BOLHAS) && aloca(s, &d.vivo, MAX_BOLHAS) &&
-       aloca(s, &d.accB, 5 * MAX_BOLHAS / 2) &&  // with facesB, celsB and volB behind it (zerarBolhas)
-       aloca(s, &d.rhsB, MAX_BOLHAS) && aloca(s, &d.yB, MAX_BOLHAS) && aloca(s, &d.rb, MAX_BOLHAS) &&
-       aloca(s, &d.zb, MAX_BOLHAS) && aloca(s, &d.pb, MAX_BOLHAS) && aloca(s, &d.apb, MAX_BOLHAS) &&
-       aloca(s, &d.r, N) && aloca(s, &d.z, N) && aloca(s, &d.zOld, N) && aloca(s, &d.p, N) &&
-       aloca(s, &d.ap, N) && aloca(s, &d.parciais, 4096) && aloca(s, &d.esc, 1);
-  d.facesB = (uint32_t*)(d.accB + MAX_BOLHAS);
-  d.celsB = d.facesB + MAX_BOLHAS;
-  d.volB = d.celsB + MAX_BOLHAS;
-  d.accV = d.accU + nu;
-  d.accCel = d.accV + nv;
-  d.accCor = (int*)(d.accCel + N);
-  int nbMax = blocos(cap > (int)N ? cap : (int)N, 1024) + 1;
-  ok = ok && aloca(s, &s->cont, nbMax) && aloca(s, &s->offs, nbMax) && aloca(s, &s->estado, 4);
-  if (ok) s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, o->fused_ctas);
-  if (ok && s->pcg) s->ar = criarRastreador(s->nx, s->ny);
-  if (!ok || !s->pcg || !s->ar) {
+  if (!soSolver) {
+    A.pedir(&sdf, (size_t)s->mw * s->mh);
+    A.pedir(&d.solido, N);
+    for (float4** p : {&d.p0, &d.p1, &d.p2, &d.q0, &d.q1, &d.q2}) A.pedir(p, cap);
+    A.pedir(&d.pid, cap);
+    A.pedir(&d.qid, cap);
+    A.pedir(&d.accU, nu + nv + N + (3 * N + 1) / 2);  // with accV, accCel, accCor behind it (zerarSomas)
+    for (float** p : {&d.u, &d.uTmp}) A.pedir(p, nu);
+    for (float** p : {&d.v, &d.vTmp}) A.pedir(p, nv);
+    for (uint8_t** p : {&d.uVal, &d.uValTmp}) A.pedir(p, nu);
+    for (uint8_t** p : {&d.vVal, &d.vValTmp}) A.pedir(p, nv);
+    A.pedir(&d.pend, N);
+    A.pedir(&d.lista, N);
+    for (float** p : {&d.qAr, &d.fase, &d.nX, &d.nY, &d.kap}) A.pedir(p, N);
+    for (float** p : {&d.pressaoBolha, &d.volumeAlvo, &d.volumeBolhaF}) A.pedir(p, MAX_BOLHAS);
+    A.pedir(&d.vivo, MAX_BOLHAS);
+    const int nbMax = blocos(cap > (int)N ? cap : (int)N, 1024) + 1;
+    A.pedir(&s->cont, nbMax);
+    A.pedir(&s->offs, nbMax);
+    A.pedir(&s->estado, 4);
+  }
+  A.pedir(&d.tipo, N);
+  A.pedir(&d.rotulo, N);
+  for (float** p : {&d.div, &d.q, &d.r, &d.z, &d.zOld, &d.p, &d.ap}) A.pedir(p, N);
+  for (float** p : {&d.rhsBolhaF, &d.yBolhaF}) A.pedir(p, MAX_BOLHAS);
+  A.pedir(&d.accB, 5 * MAX_BOLHAS / 2);  // with facesB, celsB and volB behind it (zerarBolhas)
+  for (double** p : {&d.rhsB, &d.yB, &d.rb, &d.zb, &d.pb, &d.apb}) A.pedir(p, MAX_BOLHAS);
+  A.pedir(&d.parciais, 4096);
+  A.pedir(&d.esc, 1);
+  s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, A, o->fused_ctas);
+  if (!soSolver) s->ar = criarRastreador(s->nx, s->ny, A);
+  if (!A.reservar(s->s) || !iniciarPcg(s->pcg, s->s)) {
     tq_destroy(s);
     return falha(TQ_E_NOMEM, "device allocation failed");
   }
-  std::vector<float> m;
-  molduraSdf(m, s->nx, s->ny);
-  if (cudaMemcpy(sdf, m.data(), m.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
-    tq_destroy(s);
-    return falha(TQ_E_CUDA, "upload failed");
+  d.sdf = sdf;
+  d.facesB = (uint32_t*)(d.accB + MAX_BOLHAS);
+  d.celsB = d.facesB + MAX_BOLHAS;
+  d.volB = d.celsB + MAX_BOLHAS;
+  if (!soSolver) {
+    d.accV = d.accU + nu;
+    d.accCel = d.accV + nv;
+    d.accCor = (int*)(d.accCel + N);
+    lancarZerarMascara(d, s->s);  // the walls of an empty tank
+    lancarSolidos(d, s->s);
   }
-  lancarSolidos(d, s->s);
   if (cudaStreamSynchronize(s->s) != cudaSuccess) {
     tq_destroy(s);
     return falha(TQ_E_CUDA, "initialisation failed");
@@ -377,7 +368,6 @@ int tq_destroy(tq_sim* s) {
     if (e) cudaEventDestroy(e);
   destruirPcg(s->pcg);
   destruirRastreador(s->ar);
-  for (void* p : s->alocados) cudaFree(p);
   if (s->staging) cudaFree(s->staging);
   if (s->mancha) cudaFree(s->mancha);
   for (auto& e : s->pool) cudaEventDestroy(e);
@@ -472,9 +462,11 @@ int tq_set_tanks(tq_sim* s, int32_t n, const int32_t* rects) {
   }
   Dev& d = s->d;
   if (!d.colTanque) {
-    if (!aloca(s, &d.colTanque, s->nx) || !aloca(s, &d.y0T, MAX_TANQUES) || !aloca(s, &d.y1T, MAX_TANQUES) ||
-        !aloca(s, &d.r0T, MAX_TANQUES) || !aloca(s, &d.rvT, MAX_TANQUES) || !aloca(s, &d.tanqueBolha, MAX_BOLHAS))
-      return falha(TQ_E_NOMEM, "device allocation failed");
+    s->tanques.pedir(&d.colTanque, s->nx);
+    for (int** p : {&d.y0T, &d.y1T}) s->tanques.pedir(p, MAX_TANQUES);
+    for (double** p : {&d.r0T, &d.rvT}) s->tanques.pedir(p, MAX_TANQUES);
+    s->tanques.pedir(&d.tanqueBolha, MAX_BOLHAS);
+    if (!s->tanques.reservar(s->s)) return falha(TQ_E_NOMEM, "device allocation failed");
   }
   CK(cudaMemcpyAsync(d.colTanque, col.data(), sizeof(int) * s->nx, cudaMemcpyHostToDevice, s->s));
   if (n > 0) {
@@ -643,7 +635,7 @@ static int lancarGrafo(tq_sim* s, double dt, int32_t sub) {
     s->grafoExec = nullptr;
     s->grafo = nullptr;
     s->timing = false;  // stage events are not recorded into the graph
-    if (s->o.tolerance > 0 && reservarTolerancia(s->pcg)) {  // no allocation inside the capture
+    if (s->o.tolerance > 0 && reservarTolerancia(s->pcg, s->s)) {  // no allocation inside the capture
       s->timing = timing;
       return falha(TQ_E_NOMEM, "tolerance-mode buffers");
     }
@@ -1025,7 +1017,7 @@ int tq_solve_pressure(int32_t nx, int32_t ny, const uint8_t* tipo, const float* 
   o.tolerance = tolerance;
   o.preconditioner = precond;
   tq_sim* s = nullptr;
-  int st = tq_create(&o, &s);
+  int st = criarSim(&o, true, &s);
   if (st) return st;
   const size_t N = (size_t)nx * ny;
   const Dev& d = s->d;
@@ -1078,15 +1070,17 @@ int tq_vcycle(int32_t nx, int32_t ny, const uint8_t* tipo, const float* b, float
   int st = iniciarCuda(0);
   if (st) return st;
   if (precision < TQ_PREC_FP32 || precision > TQ_PREC_BF16) return falha(TQ_E_ARG, "bad precision");
-  Pcg* p = criarPcg(nx, ny, precision, TQ_ENGINE_PLAIN);
-  if (!p) return falha(TQ_E_NOMEM, "device allocation failed");
   const size_t N = (size_t)nx * ny;
   uint8_t* dt = nullptr;
   float *db = nullptr, *dx = nullptr;
   cudaStream_t s = nullptr;
+  Arena A;
+  A.pedir(&dt, N);
+  A.pedir(&db, N);
+  A.pedir(&dx, N);
+  Pcg* p = criarPcg(nx, ny, precision, TQ_ENGINE_PLAIN, A);
   int r = TQ_OK;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess || cudaMalloc(&dt, N) != cudaSuccess ||
-      cudaMalloc(&db, N * 4) != cudaSuccess || cudaMalloc(&dx, N * 4) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess || !A.reservar(s) || !iniciarPcg(p, s))
     r = falha(TQ_E_NOMEM, "device allocation failed");
   if (!r && (cudaMemcpyAsync(dt, tipo, N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
              cudaMemcpyAsync(db, b, N * 4, cudaMemcpyHostToDevice, s) != cudaSuccess))
@@ -1095,10 +1089,10 @@ int tq_vcycle(int32_t nx, int32_t ny, const uint8_t* tipo, const float* b, float
   if (!r && (cudaMemcpyAsync(x, dx, N * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
              cudaStreamSynchronize(s) != cudaSuccess))
     r = falha(TQ_E_CUDA, "V-cycle failed");
-  cudaFree(dt);
-  cudaFree(db);
-  cudaFree(dx);
-  if (s) cudaStreamDestroy(s);
+  if (s) {
+    cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+  }
   destruirPcg(p);
   return r;
 }
