@@ -4,15 +4,14 @@
 // One CTA of 384 threads per SM (12 warps: room for ~170 registers a thread); phases are separated by a grid barrier (monotonic arrival
 // counter, release-add / acquire-poll) whose waits are bounded: a wait that exceeds ~1 s sets
 // an error flag, every CTA returns, and the host reports TQ_E_TIMEOUT.
-// Per PCG iteration: [DA] p = z + beta p fused with A p and p.Ap, [B] the q/r/bubble updates
-// with r.r, [C] the convergence test fused with spreading the residual into the V-cycle's
+// Per PCG iteration: [DA] beta and p = z + beta p fused with A p and p.Ap, [B] alpha and the q/r/bubble
+// updates with r.r, [C] the convergence test fused with spreading the residual into the V-cycle's
 // right-hand side, the V-cycle, and the gather of z with r.z and r.zOld.
 // The V-cycle is the reference's preconditioner (cicloV, js/pressao-cpu.js:241-255):
 //   - grid levels: the snapshot block smoother with one WARP per 16x16 block (8 cells per
-//     lane, warp-synchronous red-black sweeps in a per-warp shared tile); the prolongation of
-//     the coarse correction is folded into the tile load of the first smoother pass on the way
-//     up; the restriction is a per-warp tile (a 32-cell coarse row segment and its fine
-//     footprint staged in shared memory);
+//     lane, warp-synchronous red-black sweeps in registers); the prolongation of the coarse
+//     correction is folded into the loads of the first smoother pass on the way up; the
+//     restriction marches up the fine rows in registers;
 //   - the coarse levels (the largest suffix of levels fitting in ~200 KB) run inside CTA 0's
 //     shared memory, warps mapped to rows, while the other CTAs wait at the barrier.
 // Scalars (alpha, beta, norms) are FP64 sums of per-CTA partials in a fixed order, computed
@@ -60,7 +59,10 @@ constexpr int SECAO_EQUIPES = 3;
 constexpr int SECAO_NIVEIS = 6;
 // The coarsest level's sweeps hold their cells in registers, up to GROSSO_REG a colour and thread.
 constexpr int GROSSO_REG = 4;
-constexpr int NPARC = 4;                           // partial slots per CTA
+// Partial sums a CTA leaves for the next phase: channels 0 and 1 of the gather, the true residual and the
+// start, 2 of [DA], 3 of [B].  A phase that reads a channel writes another: a fast CTA may end it before a
+// slow one has read.
+constexpr int NPARC = 4;
 // Tolerance mode replaces the recursive FP32 residual by the true one (FP64) each time the
 // recursive one has fallen by this factor since the last replacement: the rounding it gathers,
 // about 1e-7 of the residual it started from per iteration, then stays far below the tolerance.
@@ -75,8 +77,10 @@ constexpr int PERFIL_SECAO = 1 << 14;              // coarse-section stamps (aft
 // per-warp shared-memory areas (floats)
 constexpr int CT = 121;                            // 11x11 coarse tile for the folded prolongation
 constexpr int SUAV_W = CT + 7;                     // the coarse tile of a PROL pass
-// restriction staging of up to two coarse rows: x (8 x 68), b / residual (floats) + viz (bytes) (6 x 66)
-constexpr int REST_W = 8 * 68 + 3 * 6 * 66;
+// per-bubble tables a CTA keeps in its areas between two grid barriers ([DA]: two doubles a label)
+constexpr size_t AREA_BOLHAS = (size_t)MAX_BOLHAS * 16;
+constexpr size_t AREA_TERMOS = (size_t)(TF - 32) * 16;  // after them, terms of a sum over the bubbles
+constexpr size_t AREA_PRODUTOS = (size_t)4 * (TF + 4) * 8;  // and a batch's products
 
 struct NivelF {
   int nx, ny, meia, pad;
@@ -112,7 +116,7 @@ struct Fundido {
   float* mSecao = nullptr;   // nW x nW, row i = water cell i of level Lc
   int *wSecao = nullptr, *wInv = nullptr, *nW = nullptr;  // water cells of level Lc, cell -> row, count
   unsigned* densoG = nullptr;  // the coarsest level's matrix, list and header, copied to the CTAs that use it
-  uint16_t* op = nullptr;
+  uint16_t *op = nullptr, *rotP = nullptr;
   unsigned long long* rotB = nullptr;
   void* kern = nullptr;
   unsigned long long* perfil = nullptr;
@@ -159,6 +163,7 @@ struct Args {
   // per-cell bubble labels of level 0, 12 bits each: bits 0-11 the cell's own (air of an active
   // bubble), 12-23 / 24-35 / 36-47 / 48-59 its left / right / down / up neighbour's (0: none)
   unsigned long long* rotB;
+  uint16_t* rotP;  // the cell's own label where the V-cycle spreads to and gathers from it, else 0
   unsigned long long* perfil;  // [0] count, [1..] %globaltimer at each barrier (null: off)
   // per level: 1 per 16x16 block whose cells are all wall (out-of-grid cells count as wall), the
   // blocks of shift 0 then those of shift 8; null where the level does not skip wall blocks
@@ -297,78 +302,108 @@ __device__ bool barreira(const Args& a, unsigned& epoca) {
   return falhou == 0;
 }
 
-// Block sum of a double (valid in thread 0).
-__device__ double somaBloco(double v, double* sh) {
+// What bounds the short phases is latency and code: an iteration runs through more of it than the SM's
+// instruction cache holds (about 128 KB; code outside it is fetched at 6 to 15 cycles an instruction, 2
+// inside).  So chains of dependent steps stay rolled loops, and rare work takes little code.
+
+// Block sums of two doubles (valid in thread 0).
+__device__ __forceinline__ double2 somaBloco2(double u, double v, double* sh) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0;
-  if (w == 0) {
-    t = lane < WARPS ? sh[lane] : 0.0;  // only WARPS slots were written
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1) {
+    u += __shfl_down_sync(0xffffffffu, u, o);
+    v += __shfl_down_sync(0xffffffffu, v, o);
   }
-  return t;
+  __syncthreads();
+  if (lane == 0) {
+    sh[w] = u;
+    sh[16 + w] = v;
+  }
+  __syncthreads();
+  if (w == 0) {
+    u = lane < WARPS ? sh[lane] : 0.0;
+    v = lane < WARPS ? sh[16 + lane] : 0.0;
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+      u += __shfl_down_sync(0xffffffffu, u, o);
+      v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+  }
+  return make_double2(u, v);
+}
+__device__ __forceinline__ double somaBloco(double v, double* sh) { return somaBloco2(v, 0.0, sh).x; }
+
+// Warp 0's sums of the per-CTA partials of two channels, in CTA order (valid in lane 0).  Loads go out
+// in batches before the sums (a rolled load-add loop waits one L2 round trip per step); each lane
+// still adds its terms in ascending order.
+__device__ __forceinline__ double2 somaParciais(const double* parc) {
+  const int t = threadIdx.x, G = gridDim.x;
+  double v0 = 0, v1 = 0;
+  constexpr int UC = 5;  // 5 x 32 slots cover one CTA per SM
+#pragma unroll 1
+  for (int k0 = t; k0 < G; k0 += 32 * UC) {
+    double2 p[UC];
+#pragma unroll
+    for (int u = 0; u < UC; u++)
+      p[u] = k0 + 32 * u < G ? __ldcg((const double2*)(parc + (k0 + 32 * u) * NPARC)) : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < UC; u++) {
+      v0 += p[u].x;
+      v1 += p[u].y;
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1) {
+    v0 += __shfl_down_sync(0xffffffffu, v0, o);
+    v1 += __shfl_down_sync(0xffffffffu, v1, o);
+  }
+  return make_double2(v0, v1);
 }
 
-// Sums, in CTA order, of the per-CTA partials of channels 0 and 1, plus up to two sums over
-// the active bubbles (ascending labels).  Warp 0 of every CTA does the same work on the same
-// data, so every CTA obtains the same bits.
-template <class F0, class F1>
-__device__ void somasGlobais(const Args& a, int nAt, F0 f0, F1 f1, double* sh, double out[4]) {
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // Loads go out in batches before the sums (a rolled load-add loop waits one L2 round trip
-    // per step); each lane still adds its terms in ascending order.
-    double v0 = 0, v1 = 0, b0 = 0, b1 = 0;
-    constexpr int UC = 5;  // 5 x 32 slots cover one CTA per SM
-    for (int k0 = 0; k0 < (int)gridDim.x; k0 += 32 * UC) {
-      double p0[UC], p1[UC];
-#pragma unroll
-      for (int u = 0; u < UC; u++) {
-        const int k = k0 + threadIdx.x + 32 * u;
-        p0[u] = k < (int)gridDim.x ? __ldcg(&a.parc[k * NPARC + 0]) : 0.0;
-        p1[u] = k < (int)gridDim.x ? __ldcg(&a.parc[k * NPARC + 1]) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < UC; u++) {
-        v0 += p0[u];
-        v1 += p1[u];
-      }
+// Sums, in CTA order, of the per-CTA partials of channel CANAL (DOIS: and the next), plus up to two sums over
+// the active bubbles (ascending labels): termos(b, t0, t1) makes bubble b's terms.  Warp 0 of every CTA
+// sums the same data in the same order, so every CTA obtains the same bits; the other warps make the
+// terms meanwhile (and what else termos stores in shared memory, visible after the call), a bubble a
+// thread: code for one bubble, not for a batch of them.  Called only after a grid barrier, whose last step
+// is a __syncthreads(): sh is free, and the next writer of sh (a block sum) synchronises first.
+constexpr int LOTE_TERMOS = TF - 32;  // a multiple of 32: lane l of warp 0 adds terms l, l + 32, ...
+template <bool DOIS, int CANAL, class F>
+__device__ __forceinline__ void somasGlobais(const Args& a, int nAt, F termos, double* sh, double out[4], float* areas) {
+  double* T = (double*)(areas + AREA_BOLHAS / 4);
+  const int t = threadIdx.x;
+  double2 v = make_double2(0.0, 0.0);
+  double b0 = 0, b1 = 0;
+  if (t < 32) v = somaParciais(a.parc + (CANAL & 2));
+  if (CANAL & 1) v.x = v.y;
+#pragma unroll 1
+  for (int k0 = 0; k0 < nAt; k0 += LOTE_TERMOS) {
+    const int n = min(LOTE_TERMOS, nAt - k0);
+    if (t >= 32 && t - 32 < n) {
+      double t0 = 0, t1 = 0;
+      termos(__ldcg(&a.ativos[k0 + t - 32]), t0, t1);
+      T[t - 32] = t0;
+      if (DOIS) T[LOTE_TERMOS + t - 32] = t1;
     }
-    constexpr int UB = 4;
-    for (int k0 = 0; k0 < nAt; k0 += 32 * UB) {
-      int bs[UB];
-#pragma unroll
-      for (int u = 0; u < UB; u++) {
-        const int k = k0 + threadIdx.x + 32 * u;
-        bs[u] = k < nAt ? __ldcg(&a.ativos[k]) : -1;
+    __syncthreads();
+    if (t < 32)
+#pragma unroll 1
+      for (int u = t; u < n; u += 32) {
+        b0 += T[u];
+        if (DOIS) b1 += T[LOTE_TERMOS + u];
       }
-      double t0[UB], t1[UB];
-#pragma unroll
-      for (int u = 0; u < UB; u++) {
-        t0[u] = bs[u] >= 0 ? f0(bs[u]) : 0.0;
-        t1[u] = bs[u] >= 0 ? f1(bs[u]) : 0.0;
+    if (k0 + LOTE_TERMOS < nAt) __syncthreads();
+  }
+  if (t < 32) {
+    if (nAt > 0)
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) {
+        b0 += __shfl_down_sync(0xffffffffu, b0, o);
+        if (DOIS) b1 += __shfl_down_sync(0xffffffffu, b1, o);
       }
-#pragma unroll
-      for (int u = 0; u < UB; u++) {
-        b0 += t0[u];
-        b1 += t1[u];
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v0 += __shfl_down_sync(0xffffffffu, v0, o);
-      v1 += __shfl_down_sync(0xffffffffu, v1, o);
-      b0 += __shfl_down_sync(0xffffffffu, b0, o);
-      b1 += __shfl_down_sync(0xffffffffu, b1, o);
-    }
-    if (threadIdx.x == 0) {
-      sh[0] = v0;
-      sh[1] = v1;
+    if (t == 0) {
+      sh[0] = v.x;
+      sh[1] = v.y;
       sh[2] = b0;
       sh[3] = b1;
     }
@@ -378,7 +413,6 @@ __device__ void somasGlobais(const Args& a, int nAt, F0 f0, F1 f1, double* sh, d
   out[1] = sh[1];
   out[2] = sh[2];
   out[3] = sh[3];
-  __syncthreads();
 }
 
 __device__ __forceinline__ bool bolhaAtiva(const Args& a, uint32_t r) {
@@ -426,21 +460,35 @@ constexpr int OP_AGUA = 16, OP_FACE = 32, OP_VIZ_BOLHA = 64, OP_BOLHA = 128;
 // Level 0's neighbour masks also carry, above bits 0-4, the cell's OP_BOLHA and OP_AGUA.
 constexpr int V0_BOLHA = 32, V0_AGUA = 64;
 
+// Adds v to bubble lab's fixed-point sum (lab 0: nothing), by the whole warp: one atomic a label and warp.
+// A large bubble's cells would otherwise queue thousands of atomics on one address, which bounded the
+// phases that make these sums.  Integer sums: any grouping gives the same result.
+__device__ __forceinline__ void somarBolhaWarp(long long* acc, int lab, long long v) {
+  unsigned resto = __ballot_sync(0xffffffffu, lab && v);
+#pragma unroll 1
+  while (resto) {
+    const int l0 = __shfl_sync(0xffffffffu, lab, __ffs(resto) - 1);
+    const bool meu = lab == l0;
+    long long t = meu ? v : 0;
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0 && t) atomicAdd((unsigned long long*)&acc[l0], (unsigned long long)t);
+    resto &= ~__ballot_sync(0xffffffffu, meu);
+  }
+}
+
 // ---------------------------------------------------------------- grid-level smoother
 // Modes of a smoother pass over a grid level:
-//   M_NORMAL   snapshot = src, right side = b (on the way down; M_VOLTA, the same on the way up);
+//   M_NORMAL   snapshot = src, right side = b; with `zero`, snapshot = 0: the first pass on the way
+//              down, whose x the restriction leaves at 0 (js/pressao-cpu.js:186);
 //   M_PROL     snapshot = x + P(x_coarse) (prolongar, js/pressao-cpu.js:191-214), built while
 //              loading: the first pass on the way up;
-//   M_ZERO     snapshot = 0: the first pass on the way down, whose x the restriction (or the
-//              spread) leaves at 0 (js/pressao-cpu.js:186, :354);
-//   M_ESPALHAR level 0, first pass: also spreads the residual into b (precondicionar,
-//              js/pressao-cpu.js:353-355), b = escala * r, bubble cells their bubble's mean;
+//   M_ESPALHAR level 0, first pass: snapshot 0 (:354); also spreads the residual into b
+//              (precondicionar, js/pressao-cpu.js:353-355), b = escala * r, bubble cells their bubble's mean;
 //   M_JUNTAR   level 0, last pass: instead of storing x, gathers z = x / escala (:357-361),
 //              bubble cells' share into the bubble's fixed-point sum, and the partials of r.z
 //              and r.zOld.
-enum { M_NORMAL = 0, M_PROL = 1, M_ZERO = 2, M_ESPALHAR = 3, M_JUNTAR = 4, M_VOLTA = 5 };
-// Red-black on the way down, black-red up: each mode belongs to one leg.
-__host__ __device__ constexpr int ordemDe(int modo) { return modo == M_PROL || modo == M_JUNTAR || modo == M_VOLTA; }
+enum { M_NORMAL = 0, M_PROL = 1, M_ESPALHAR = 2, M_JUNTAR = 3 };
 
 // What the spread and the gather need (level 0).
 struct Reuniao {
@@ -468,11 +516,11 @@ __device__ __forceinline__ float correcaoGrossa(const float* ct, int cx0, int cy
 // meiaReg).  Every global load of the block (cells, frame, flags, right side; with PROL the
 // coarse tile) goes out in one batch.
 template <class T, int MODO>
-__device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, int blk, int nbx, int desl, bool masc,
+__device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, int blk, int nbx, int desl, bool masc, bool zero, int ordem,
                                               const T* src, T* dst, float* area, const NivelF& g,
                                               const float* xcSecao, const Reuniao& ru, double& s0, double& s1) {
   constexpr bool PROL = MODO == M_PROL;
-  constexpr bool ZERO = MODO == M_ZERO || MODO == M_ESPALHAR;
+  const bool ZERO = MODO == M_ESPALHAR || (MODO == M_NORMAL && zero);
   const int lane = threadIdx.x & 31, gl = lane >> 3, k = lane & 7;
   const int bx = blk % nbx, by = blk / nbx;
   const int ox = bx * 16 - desl, oy = by * 16 - desl;
@@ -496,24 +544,27 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
     }
     // the coarse values' storage type is chosen once (warp-uniform), so the four loads are
     // straight-line code in flight together
+    // (a level below the section is stored as T, see criarFundido)
     if (xcSecao) {
 #pragma unroll
       for (int kk = 0; kk < 4; kk++) cv[kk] = ok[kk] ? __ldcg(xcSecao + C[kk]) : 0.0f;
-    } else if (g.meia == 1) {
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) cv[kk] = ok[kk] ? __half2float(ldcg((const __half*)g.x + C[kk])) : 0.0f;
-    } else if (g.meia == 2) {
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++)
-        cv[kk] = ok[kk] ? __bfloat162float(ldcg((const __nv_bfloat16*)g.x + C[kk])) : 0.0f;
     } else {
+      T cR[4];
 #pragma unroll
-      for (int kk = 0; kk < 4; kk++) cv[kk] = ok[kk] ? __ldcg((const float*)g.x + C[kk]) : 0.0f;
+      for (int kk = 0; kk < 4; kk++) {
+        cR[kk] = guardar<T>(0.0f);
+        if (ok[kk]) cR[kk] = ldcg((const T*)g.x + C[kk]);
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++) cv[kk] = carregar(cR[kk]);
     }
   }
   float x[2][4], bq[2][4];  // [colour][m], see meiaReg
+  T bR[2][4], xR[2][4];     // as stored
   int v[2][4], cel[2][4];
-  int om[2][4];  // M_ESPALHAR: the cells' own bubble labels (0: not bubble air)
+  int om[2][4];  // M_ESPALHAR, M_JUNTAR: the cells' own bubble labels (0: not bubble air)
+  float rv[2][4], zv[2][4];  // M_JUNTAR: the residual and the previous z
+  unsigned cels[2][4];       // M_JUNTAR: the cells of the cell's bubble
   Moldura f;
   unsigned aguaF = 0;  // PROL: water flags of the frame cells (bits 0-3 left, 4-7 right, 8-9 below, 10-11 above)
 #pragma unroll
@@ -524,15 +575,50 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
       const bool dentro = gx >= 0 && gy >= 0 && gx < nx && gy < ny;
       const int c = gx + gy * nx;
       cel[cr][m] = dentro ? c : -1;
-      v[cr][m] = dentro ? (ldsv8(n.viz + c) | 128) : 0;
-      x[cr][m] = (!ZERO && dentro) ? carregar(ldsv(src + c)) : 0.0f;
-      if (MODO == M_ESPALHAR) {
-        bq[cr][m] = dentro ? __ldcg(a.d.r + c) : 0.0f;
-        om[cr][m] = (v[cr][m] & V0_BOLHA) ? (int)(__ldcg(a.rotB + c) & 0xfff) : 0;  // own bubble label
-      } else {
-        bq[cr][m] = dentro ? carregar(ldsv(b + c)) : 0.0f;
+      v[cr][m] = 0;
+      bq[cr][m] = 0.0f;
+      bR[cr][m] = xR[cr][m] = guardar<T>(0.0f);
+      // as stored: a load under a branch that also converts waits inside the branch, which cost the
+      // 16-bit kernels 2 to 3 us a phase
+      if (dentro) {
+        v[cr][m] = ldsv8(n.viz + c);
+        if (MODO == M_ESPALHAR) bq[cr][m] = __ldcg(a.d.r + c);
+        else bR[cr][m] = ldsv(b + c);
       }
     }
+  if (!ZERO)
+#pragma unroll
+    for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+      for (int m = 0; m < 4; m++)
+        if (cel[cr][m] >= 0) xR[cr][m] = ldsv(src + cel[cr][m]);
+  // the warp-uniform tests (bubbles the V-cycle sees, a previous z) stay outside the loads, so each
+  // group of loads is straight-line code in flight with the block's
+  if (MODO == M_ESPALHAR || MODO == M_JUNTAR) {
+#pragma unroll
+    for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) om[cr][m] = 0;
+    if (a.bolhas && !a.bloco)
+#pragma unroll
+      for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) om[cr][m] = cel[cr][m] >= 0 ? (int)__ldcg(a.rotP + cel[cr][m]) : 0;
+  }
+  if (MODO == M_JUNTAR) {
+#pragma unroll
+    for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        rv[cr][m] = cel[cr][m] >= 0 ? __ldcg(a.d.r + cel[cr][m]) : 0.0f;
+        zv[cr][m] = 0.0f;
+      }
+    if (ru.zVelho)
+#pragma unroll
+      for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) zv[cr][m] = cel[cr][m] >= 0 ? __ldcg(ru.zVelho + cel[cr][m]) : 0.0f;
+  }
   // The block's frame: lane i loads the left (i < 16) or right column's row i & 15 and the
   // bottom (i < 16) or top row's column i & 15; the lanes next to the frame (k = 0 / 7 for the
   // columns, g = 0 / 3 for the rows) take their values by shuffle.  With PROL the same two cells'
@@ -548,14 +634,25 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
       vzLR = okA ? ldsv8(n.viz + gxA + gyA * nx) : 0;
       vzBT = okB ? ldsv8(n.viz + gxB + gyB * nx) : 0;
     }
+    T fA = guardar<T>(0.0f), fB = guardar<T>(0.0f);
+    if (!ZERO) {
+      if (okA) fA = ldsv(src + gxA + gyA * nx);
+      if (okB) fB = ldsv(src + gxB + gyB * nx);
+    }
+#pragma unroll
+    for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        if (MODO != M_ESPALHAR) bq[cr][m] = carregar(bR[cr][m]);
+        x[cr][m] = ZERO ? 0.0f : carregar(xR[cr][m]);
+      }
     if (ZERO) {
 #pragma unroll
       for (int m = 0; m < 4; m++) f.esq[m] = f.dir[m] = 0.0f;
 #pragma unroll
       for (int j = 0; j < 2; j++) f.bai[j] = f.cim[j] = 0.0f;
     } else {
-      const float xA = okA ? carregar(ldsv(src + gxA + gyA * nx)) : 0.0f;
-      const float xB = okB ? carregar(ldsv(src + gxB + gyB * nx)) : 0.0f;
+      const float xA = carregar(fA), xB = carregar(fB);
 #pragma unroll
       for (int m = 0; m < 4; m++) f.esq[m] = f.dir[m] = __shfl_sync(0xffffffffu, xA, (k == 7 ? 16 : 0) + 4 * gl + m);
 #pragma unroll
@@ -571,7 +668,7 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
       for (int m = 0; m < 4; m++) {
         if (cel[cr][m] < 0) continue;
         float val = bq[cr][m];
-        if (om[cr][m]) val = (float)(__ldcg(a.d.rb + om[cr][m]) / __ldcg(a.d.celsB + om[cr][m]));
+        if (om[cr][m]) val = area[om[cr][m]];
         const T bt = guardar<T>(val * ru.escala);
         ((T*)n.b)[cel[cr][m]] = bt;
         bq[cr][m] = carregar(bt);
@@ -614,6 +711,11 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
     }
     __syncwarp();
   }
+  if (MODO == M_JUNTAR)
+#pragma unroll
+    for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) cels[cr][m] = om[cr][m] ? __ldcg(a.d.celsB + om[cr][m]) : 1u;
   // a block with no cell to update (air, solid, walled-in water) keeps its values: the warp skips
   // the sweeps (fmaf(0, d, q) = q for every cell of the block)
   bool mexe = false;
@@ -623,68 +725,54 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
     for (int m = 0; m < 4; m++) mexe |= (v[cr][m] & 16) && (v[cr][m] & 15);
   // (level 0's masks close no face between water cells: x = 0 off water, so it needs no masking)
   if (__any_sync(0xffffffffu, mexe))
-    varrerReg(x, v, bq, f, ordemDe(MODO), MODO != M_ESPALHAR && MODO != M_JUNTAR && masc, a.varreduras);
+    varrerReg(x, v, bq, f, ordem, MODO != M_ESPALHAR && MODO != M_JUNTAR && masc, a.varreduras);
   if (MODO == M_JUNTAR) {
     const float inv = 1.0f / ru.escala;
-    float rv[2][4], zv[2][4];
-    int lb[2][4];
-    // the warp-uniform tests (bubbles, a previous z) outside the loads, so each group of loads
-    // is straight-line code in flight together
-#pragma unroll
-    for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) rv[cr][m] = __ldcg(a.d.r + (cel[cr][m] < 0 ? 0 : cel[cr][m]));
-    // a cell's own label is set only on bubble air (V0_BOLHA in its mask): loaded there alone
-#pragma unroll
-    for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-        lb[cr][m] = (v[cr][m] & V0_BOLHA) ? (int)(__ldcg(a.rotB + cel[cr][m]) & 0xfff) : 0;
-    if (ru.zVelho) {
-#pragma unroll
-      for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-        for (int m = 0; m < 4; m++) zv[cr][m] = __ldcg(ru.zVelho + (cel[cr][m] < 0 ? 0 : cel[cr][m]));
-    } else {
-#pragma unroll
-      for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-        for (int m = 0; m < 4; m++) zv[cr][m] = 0.0f;
-    }
-    unsigned cels[2][4];
-#pragma unroll
-    for (int cr = 0; cr < 2; cr++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) cels[cr][m] = lb[cr][m] ? __ldcg(a.d.celsB + lb[cr][m]) : 1u;
-    // a bubble cell's share of z goes to its bubble's fixed-point sum; the lane adds its
-    // consecutive cells of one bubble before the atomic (integer sums: same result)
-    int labA = 0;
-    long long acc = 0;
+    bool bolha = false;
 #pragma unroll
     for (int cr = 0; cr < 2; cr++)
 #pragma unroll
       for (int m = 0; m < 4; m++) {
         const int c = cel[cr][m];
-        if (c < 0) continue;
+        bolha |= om[cr][m] != 0;
         const float xz = carregar(guardar<T>((v[cr][m] & 16) ? x[cr][m] : 0.0f)) * inv;
-        if (lb[cr][m]) {
-          const long long q = __double2ll_rn((double)xz / cels[cr][m] * ESC);
-          if (lb[cr][m] != labA) {
-            if (labA && acc) atomicAdd((unsigned long long*)&a.accZ[labA], (unsigned long long)acc);
-            labA = lb[cr][m];
-            acc = 0;
-          }
-          acc += q;
-          ru.zNovo[c] = 0.0f;
-          continue;
-        }
-        ru.zNovo[c] = xz;
-        if (v[cr][m] & V0_AGUA) {
+        x[cr][m] = xz;
+        if (c < 0) continue;
+        ru.zNovo[c] = om[cr][m] ? 0.0f : xz;
+        if ((v[cr][m] & V0_AGUA) && !om[cr][m]) {
           s0 += (double)rv[cr][m] * (double)xz;
           if (ru.zVelho) s1 += (double)rv[cr][m] * (double)zv[cr][m];
         }
       }
-    if (labA && acc) atomicAdd((unsigned long long*)&a.accZ[labA], (unsigned long long)acc);
+    if (__any_sync(0xffffffffu, bolha)) {
+      // a bubble cell's share of z goes to its bubble's fixed-point sum; the lane adds its
+      // consecutive cells of one bubble before the atomic (integer sums: same result).  A rolled loop
+      // over the cells, through shared memory: the FP64 division's code once.
+#pragma unroll
+      for (int cr = 0; cr < 2; cr++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          float* o = area + (4 * cr + m) * 32 + lane;
+          o[0] = x[cr][m];
+          ((int*)o)[256] = om[cr][m];
+          ((unsigned*)o)[512] = cels[cr][m];
+        }
+      int labA = 0;
+      long long acc = 0;
+#pragma unroll 1
+      for (int q = 0; q < 8; q++) {
+        const float* o = area + q * 32 + lane;
+        const int lab = ((const int*)o)[256];
+        if (!lab) continue;
+        if (lab != labA) {
+          if (labA && acc) atomicAdd((unsigned long long*)&a.accZ[labA], (unsigned long long)acc);
+          labA = lab;
+          acc = 0;
+        }
+        acc += __double2ll_rn((double)o[0] / ((const unsigned*)o)[512] * ESC);
+      }
+      somarBolhaWarp(a.accZ, labA, acc);
+    }
   } else {
 #pragma unroll
     for (int cr = 0; cr < 2; cr++)
@@ -695,13 +783,14 @@ __device__ __forceinline__ void suavizarBloco(const Args& a, const NivelF& n, in
 }
 
 template <class T, int MODO>
-__device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, bool paraTmp, float* areas,
-                                           const Reuniao& ru, double* sh) {
+__device__ __forceinline__ void faseSuavizarT(const Args& a, int l, int desl, bool paraTmp, bool zero, int ordem,
+                                           float* areas, const Reuniao& ru, double* sh) {
   const NivelF n = s_niv[l];
   const int nbx = (n.nx + desl + 15) >> 4, nby = (n.ny + desl + 15) >> 4;
   const int nb = nbx * nby;
   const int w = threadIdx.x >> 5;
-  float* area = areas + w * SUAV_W;
+  // the spread reads the CTA's bubble means, the gather takes 3 words a cell of its block
+  float* area = MODO == M_ESPALHAR ? areas : areas + w * (MODO == M_JUNTAR ? 768 : SUAV_W);
   const T* src = (const T*)(paraTmp ? n.x : n.tmp);
   T* dst = (T*)(paraTmp ? n.tmp : n.x);
   NivelF g{};
@@ -725,164 +814,191 @@ __device__ __noinline__ void faseSuavizarT(const Args& a, int l, int desl, bool 
     paredes = __ballot_sync(0xffffffffu, tk < nb && ldcg8(fl + blocoDe(tk)) != 0);
   }
   const bool masc = a.bloco && l >= 1;
-  int k = 0;
+  int k = 0, zr = zero;
+#pragma unroll 1
   for (int t = tw; t < nb; t += tot, k++) {
     const int blk = blocoDe(t);
     if (fl && (k < 32 ? (paredes >> k) & 1u : ldcg8(fl + blk) != 0)) continue;
-    suavizarBloco<T, MODO>(a, n, blk, nbx, desl, masc, src, dst, area, g, xcSecao, ru, s0, s1);
+    if (MODO == M_NORMAL) asm volatile("" : "+r"(zr));  // or the compiler makes a copy of the loop for each leg
+    suavizarBloco<T, MODO>(a, n, blk, nbx, desl, masc, zr != 0, ordem, src, dst, area, g, xcSecao, ru, s0, s1);
   }
   if (MODO == M_JUNTAR) {
-    const double t0 = somaBloco(s0, sh);
-    const double t1 = somaBloco(s1, sh);
+    const double2 t = somaBloco2(s0, s1, sh);
     if (threadIdx.x == 0) {
-      a.parc[blockIdx.x * NPARC + 0] = t0;
-      a.parc[blockIdx.x * NPARC + 1] = t1;
+      a.parc[blockIdx.x * NPARC + 0] = t.x;
+      a.parc[blockIdx.x * NPARC + 1] = t.y;
     }
   }
 }
 
-// Every grid level below the coarse section is stored as T (criarFundido), so a 16-bit kernel
-// carries no FP32 copy of the passes: smaller code, which each phase enters cold.
+// ---------------------------------------------------------------- restriction
+// Two neighbouring cells of a row from an even column on, as stored (nothing is converted before every
+// load is out): one load where the level's rows start on even cells (par); zeros outside the level (d: the
+// first cell is inside, d1: the second).
 template <class T>
-__device__ void faseSuavizar(const Args& a, int l, int desl, bool paraTmp, int modo, float* areas, const Reuniao& ru,
-                             double* sh) {
-  switch (modo) {
-    case M_PROL: faseSuavizarT<T, M_PROL>(a, l, desl, paraTmp, areas, ru, sh); break;
-    case M_ZERO: faseSuavizarT<T, M_ZERO>(a, l, desl, paraTmp, areas, ru, sh); break;
-    case M_ESPALHAR: faseSuavizarT<T, M_ESPALHAR>(a, l, desl, paraTmp, areas, ru, sh); break;
-    case M_JUNTAR: faseSuavizarT<T, M_JUNTAR>(a, l, desl, paraTmp, areas, ru, sh); break;
-    case M_VOLTA: faseSuavizarT<T, M_VOLTA>(a, l, desl, paraTmp, areas, ru, sh); break;
-    default: faseSuavizarT<T, M_NORMAL>(a, l, desl, paraTmp, areas, ru, sh);
+struct Par {
+  unsigned w;
+  T a, b;
+};
+template <>
+struct Par<float> {
+  float2 w;
+  float a, b;
+};
+template <class T>
+__device__ __forceinline__ void lerPar(Par<T>& r, const T* p, int c, bool d, bool d1, bool par) {
+  r.w = {};
+  r.a = r.b = guardar<T>(0.0f);
+  if (par) {
+    if (d) r.w = __ldcg((const decltype(r.w)*)(p + c));
+  } else {
+    if (d) r.a = ldcg(p + c);
+    if (d1) r.b = ldcg(p + c + 1);
+  }
+}
+template <class T>
+__device__ __forceinline__ float2 valores(const Par<T>& r, bool par) {
+  if constexpr (sizeof(T) == 4) {
+    return par ? r.w : make_float2(r.a, r.b);
+  } else {
+    T a, b;
+    if constexpr (std::is_same<T, __half>::value) {
+      a = __ushort_as_half((unsigned short)r.w);
+      b = __ushort_as_half((unsigned short)(r.w >> 16));
+    } else {
+      a = __ushort_as_bfloat16((unsigned short)r.w);
+      b = __ushort_as_bfloat16((unsigned short)(r.w >> 16));
+    }
+    return make_float2(carregar(par ? a : r.a), carregar(par ? b : r.b));
   }
 }
 
-// ---------------------------------------------------------------- restriction
-// restringir (js/pressao-cpu.js:159-188) as a gather, one warp per region of R coarse rows x 32
-// columns: the fine footprint (x on 2R+4 rows x 68 columns; b and flags on 2R+2 x 66) is staged
-// in the warp's shared area, residuals computed once, then each lane sums its 4x4 windows.
-template <class TFino, int R>
-__device__ __forceinline__ void faseRestringirR(const Args& a, int l, float* areas) {
-  constexpr int RXn = (2 * R + 4) * 68, RBn = (2 * R + 2) * 66;
-  constexpr int KX = (RXn + 31) / 32, KB = (RBn + 31) / 32;
-  static_assert(RXn + 3 * RBn <= REST_W, "restriction staging area");
+// restringir (js/pressao-cpu.js:159-188) as a gather in registers: a warp takes 30 coarse columns (a lane
+// each, lanes 0 and 31 the fine columns beside them) and marches up R coarse rows.  A lane holds its two
+// fine columns of the rows in use; the neighbours' come by shuffle, and every value is loaded once a
+// warp, the next row's before this row's sums.  R: one round of the grid's warps, up to 4 rows (a
+// larger grid takes more rounds).  Measured on level 0 of 840x536 cells: 9.0 -> 5.2 us in FP32, 10.9 -> 5.7
+// in FP16, against a footprint staged in shared memory a value a load.
+template <class T>
+__device__ __forceinline__ void faseRestringir(const Args& a, int l) {
   const NivelF f = s_niv[l];
   const NivelF g = s_niv[l + 1];
-  const bool secao = l + 1 == a.Lc;
+  const bool secao = l + 1 == a.Lc, par = !(f.nx & 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float* xs = areas + w * REST_W;
-  float* bs = xs + RXn;
-  float* rs = bs + RBn;
-  uint8_t* vs = (uint8_t*)(rs + RBn);
-  const float pes[4] = {0.25f, 0.75f, 0.75f, 0.25f};
-  const int nseg = (g.nx + 31) >> 5;
-  const int total = nseg * ((g.ny + R - 1) / R);
-  // A region whose coarse cells lie in wall blocks of the coarse level (its shift-0 flags; its
-  // 32 columns span two blocks, its rows one) is skipped: those cells keep b = 0.  The flags of
-  // the warp's first 32 regions come in one load, lane k's for its k-th.
+  const int nseg = (g.nx + 29) / 30, tot = WARPS * gridDim.x;
+  const int R = min(4, (nseg * g.ny + tot - 1) / tot), total = nseg * ((g.ny + R - 1) / R);
+  const T *fx = (const T*)f.x, *fb = (const T*)f.b;
+  // A region whose coarse cells lie in wall blocks of the coarse level (its shift-0 flags) is skipped:
+  // those cells keep b = 0.  The flags of the warp's first 32 regions come in one go, lane k's for its
+  // k-th.
   const uint8_t* flg = a.sol[l + 1];
   const int gbx = (g.nx + 15) >> 4;
-  auto paredeReg = [&](int seg) {
-    const int by = ((seg / nseg) * R) >> 4, bx = ((seg % nseg) * 32) >> 4;
-    return ldcg8(flg + by * gbx + bx) != 0 && (bx + 1 >= gbx || ldcg8(flg + by * gbx + bx + 1) != 0);
+  auto paredeReg = [&](int reg) {
+    const int J = reg / nseg * R, I = reg % nseg * 30, bx1 = min(I + 29, g.nx - 1) >> 4, by1 = min(J + R - 1, g.ny - 1) >> 4;
+    int p = 1;
+#pragma unroll 1
+    for (int by = J >> 4; by <= by1; by++)
+#pragma unroll 1
+      for (int bx = I >> 4; bx <= bx1; bx++) p &= ldcg8(flg + by * gbx + bx);
+    return p != 0;
   };
-  const int t0 = w * gridDim.x + blockIdx.x, tot = WARPS * gridDim.x;
+  const int t0 = w * gridDim.x + blockIdx.x;
   unsigned paredes = 0;
   if (flg) {
     const int tk = t0 + lane * tot;
     paredes = __ballot_sync(0xffffffffu, tk < total && paredeReg(tk));
   }
   int kr = 0;
-  for (int seg = t0; seg < total; seg += tot, kr++) {
-    if (flg && (kr < 32 ? (paredes >> kr) & 1u : paredeReg(seg))) continue;
-    const int J0 = (seg / nseg) * R, I0 = (seg % nseg) * 32;
-    const int fi0 = 2 * I0 - 2, fj0 = 2 * J0 - 2;  // x window origin (fine)
-    const int I = I0 + lane;
-    int gvz[R];
+#pragma unroll 1
+  for (int reg = t0; reg < total; reg += tot, kr++) {
+    if (flg && (kr < 32 ? (paredes >> kr) & 1u : paredeReg(reg))) continue;
+    const int J0 = reg / nseg * R, I = reg % nseg * 30 + lane - 1, i = 2 * I, J1 = min(J0 + R, g.ny);
+    // xr: x of rows 2J .. 2J + 3; bn, vn: right side and masks of rows 2J + 1 and 2J + 2
+    const bool dI = i >= 0 && i < f.nx, dI1 = dI && i + 1 < f.nx;
+    float2 xr[4];
+    Par<T> xn[2], bn[2];
+    int vn[2], vm[2], gv = 0;
+    auto lerX = [&](Par<T>& r, int j) {
+      const bool d = j >= 0 && j < f.ny;
+      lerPar<T>(r, fx, i + j * f.nx, d && dI, d && dI1, par);
+    };
+    auto ler = [&](int J) {
+      gv = I >= 0 && I < g.nx && J >= J0 ? ldcg8(g.viz + I + J * g.nx) : 0;
 #pragma unroll
-    for (int r = 0; r < R; r++) gvz[r] = (I < g.nx && J0 + r < g.ny) ? ldcg8(g.viz + I + (J0 + r) * g.nx) : 0;
-    // staging loads issued as one batch per array (registers, then shared memory)
-    {
-      float xv[KX];
-#pragma unroll
-      for (int k = 0; k < KX; k++) {
-        const int s = lane + 32 * k;
-        const int i = fi0 + s % 68, j = fj0 + s / 68;
-        xv[k] = (s < RXn && i >= 0 && j >= 0 && i < f.nx && j < f.ny) ? carregar(ldcg((const TFino*)f.x + i + j * f.nx)) : 0.0f;
-      }
-      float bv[KB];
-      int vv[KB];
-#pragma unroll
-      for (int k = 0; k < KB; k++) {
-        const int s = lane + 32 * k;
-        const int i = fi0 + 1 + s % 66, j = fj0 + 1 + s / 66;
-        const bool d = s < RBn && i >= 0 && j >= 0 && i < f.nx && j < f.ny;
-        const int c = i + j * f.nx;
-        vv[k] = d ? ldcg8(f.viz + c) : 0;
-        bv[k] = d ? carregar(ldcg((const TFino*)f.b + c)) : 0.0f;
-      }
-#pragma unroll
-      for (int k = 0; k < KX; k++) {
-        const int s = lane + 32 * k;
-        if (s < RXn) xs[s] = xv[k];
-      }
-#pragma unroll
-      for (int k = 0; k < KB; k++) {
-        const int s = lane + 32 * k;
-        if (s < RBn) {
-          vs[s] = (uint8_t)vv[k];
-          bs[s] = bv[k];
+      for (int q = 0; q < 2; q++) {
+        lerX(xn[q], 2 * J + 2 + q);
+        const int j = 2 * J + 1 + q, c = i + j * f.nx;
+        const bool d = j >= 0 && j < f.ny && dI, d1 = d && dI1;
+        lerPar<T>(bn[q], fb, c, d, d1, par);
+        vn[q] = vm[q] = 0;
+        if (par) {
+          if (d) vn[q] = (int)__ldcg((const unsigned short*)(f.viz + c));
+        } else {
+          if (d) vn[q] = ldcg8(f.viz + c);
+          if (d1) vm[q] = ldcg8(f.viz + c + 1);
         }
       }
-    }
-    __syncwarp();
+    };
     {
-      // residuals of the fine cells: every shared load of the lane's cells goes out before the
-      // first store.  x is 0 off water and outside the grid, so the neighbour sum needs no
-      // mask (but TQ_PRECOND_BLOCK's coarse masks can close a face between two water cells);
-      // the residual is 0 off water.
-      const bool masc = a.bloco != 0;
-      float rv[KB];
-#pragma unroll
-      for (int k = 0; k < KB; k++) {
-        const int s = lane + 32 * k < RBn ? lane + 32 * k : 0;
-        const float* xc = xs + (s / 66 + 1) * 68 + s % 66 + 1;
-        const int vz = vs[s];
-        const float t = masc ? ((((vz & 1) ? xc[-1] : 0.0f) + ((vz & 2) ? xc[1] : 0.0f)) + ((vz & 4) ? xc[-68] : 0.0f)) +
-                                   ((vz & 8) ? xc[68] : 0.0f)
-                             : ((xc[-1] + xc[1]) + xc[-68]) + xc[68];
-        rv[k] = (vz & 16) ? bs[s] - ((float)__popc(vz & 15) * xc[0] - t) : 0.0f;
-      }
-#pragma unroll
-      for (int k = 0; k < KB; k++)
-        if (lane + 32 * k < RBn) rs[lane + 32 * k] = rv[k];
+      Par<T> u[2];
+      lerX(u[0], 2 * J0 - 2);
+      lerX(u[1], 2 * J0 - 1);
+      ler(J0 - 1);
+      xr[2] = valores<T>(u[0], par);
+      xr[3] = valores<T>(u[1], par);
     }
-    __syncwarp();
+    float rs[4][4];  // residuals of rows 2J - 1 .. 2J + 2 in columns 2I - 1 .. 2I + 2
 #pragma unroll
-    for (int r = 0; r < R; r++)
-      if (I < g.nx && J0 + r < g.ny) {
-        const int C = I + (J0 + r) * g.nx;
-        float soma = 0.0f;
-        if (gvz[r] & 16) {
+    for (int q = 0; q < 4; q++) rs[2][q] = rs[3][q] = 0.0f;
+#pragma unroll 1
+    for (int J = J0 - 1; J < J1; J++) {
+      xr[0] = xr[2];
+      xr[1] = xr[3];
+      float2 b[2];
+      int v[2];
 #pragma unroll
-          for (int bb = 0; bb < 4; bb++)
-#pragma unroll
-            for (int aa = 0; aa < 4; aa++) soma += rs[(2 * r + bb) * 66 + 2 * lane + aa] * (pes[aa] * pes[bb]);
-        }
-        if (secao) a.bc[C] = soma;
-        else gravarN(g.meia, g.b, C, soma);  // x of the coarse level: its first pass reads 0
+      for (int q = 0; q < 2; q++) {
+        xr[2 + q] = valores<T>(xn[q], par);
+        b[q] = valores<T>(bn[q], par);
+        v[q] = vn[q] | vm[q] << 8;
       }
-    __syncwarp();
+      const int gvz = gv;
+      if (J + 1 < J1) ler(J + 1);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        rs[0][q] = rs[2][q];
+        rs[1][q] = rs[3][q];
+      }
+      // b - A x on water cells, 0 elsewhere (TQ_PRECOND_BLOCK's coarse masks can close a face between
+      // two water cells; elsewhere x is 0 past a closed face)
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const float2 x = xr[1 + q];
+        const float xe = __shfl_up_sync(0xffffffffu, x.y, 1), xd = __shfl_down_sync(0xffffffffu, x.x, 1);
+        auto residuo = [&](int m, float bb, float c, float e, float d, float bai, float cim) {
+          const float t = ((((m & 1) ? e : 0.0f) + ((m & 2) ? d : 0.0f)) + ((m & 4) ? bai : 0.0f)) + ((m & 8) ? cim : 0.0f);
+          return (m & 16) ? bb - fmaf((float)__popc(m & 15), c, -t) : 0.0f;
+        };
+        const float r0 = residuo(v[q] & 255, b[q].x, x.x, xe, x.y, xr[q].x, xr[2 + q].x);
+        const float r1 = residuo(v[q] >> 8, b[q].y, x.y, x.x, xd, xr[q].y, xr[2 + q].y);
+        rs[2 + q][0] = __shfl_up_sync(0xffffffffu, r1, 1);
+        rs[2 + q][1] = r0;
+        rs[2 + q][2] = r1;
+        rs[2 + q][3] = __shfl_down_sync(0xffffffffu, r0, 1);
+      }
+      if (J < J0 || lane < 1 || lane > 30 || I >= g.nx) continue;
+      const float pes[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+      float soma = 0.0f;
+#pragma unroll
+      for (int bb = 0; bb < 4; bb++)
+#pragma unroll
+        for (int aa = 0; aa < 4; aa++) soma = fmaf(rs[bb][aa], pes[aa] * pes[bb], soma);
+      if (!(gvz & 16)) soma = 0.0f;
+      const int C = I + J * g.nx;
+      if (secao) a.bc[C] = soma;
+      else gravarN(g.meia, g.b, C, soma);
+    }
   }
-}
-
-// Two coarse rows per warp where one-row segments would take four or more rounds of the
-// grid's warps (the finest restriction of a large atlas): half the rounds, each with the 6
-// residual rows of 2 coarse rows instead of 2 x 4.
-template <class TFino>
-__device__ void faseRestringir(const Args& a, int l, float* areas) {
-  const NivelF g = s_niv[l + 1];
-  if (((g.nx + 31) >> 5) * g.ny > 4 * WARPS * (int)gridDim.x) faseRestringirR<TFino, 2>(a, l, areas);
-  else faseRestringirR<TFino, 1>(a, l, areas);
 }
 
 // ---------------------------------------------------------------- coarse section (CTA 0)
@@ -1484,38 +1600,47 @@ __device__ __forceinline__ void trocarXTmp(int l) {
 // gather of z (last pass): 5 Lc + 1 phases, each ending at a grid barrier.  With
 // TQ_PRECOND_BLOCK_1 the grid levels above 0 take one smoother pass a leg (shift 8, red-black
 // down and black-red up, so the cycle stays symmetric): 3 Lc + 3 phases.
+// A loop over the phases with one place for each kind of phase and one barrier, everything inlined:
+// across a call, the caller's values go through local memory, which each barrier's acquire drops from
+// L1, and a function reads the kernel's arguments through memory too.  With the loads taken as stored
+// (suavizarBloco, faseRestringir): 112 -> 95 us an iteration on 840x536 cells (BLOCK_1, FP16), 130 -> 115
+// (REFERENCE, FP32), 93 -> 83 on 480x270.
 template <class T>
-__device__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char* smem, NivelS* tabS,
-                       const Reuniao& ru, double* sh, bool secaoDensa) {
-  for (int l = 0; l < a.Lc; l++) {
-    if (a.umaPassada && l >= 1) {
-      faseSuavizar<T>(a, l, 8, true, M_ZERO, areas, ru, sh);
-      trocarXTmp(l);
-      if (!barreira(a, ep)) return false;
+__device__ __forceinline__ bool cicloV(const Args& a, unsigned& ep, float* areas, unsigned char* smem, NivelS* tabS,
+                                       const Reuniao& ru, double* sh, bool secaoDensa) {
+  // a level's phases: 0 and 1 its passes on the way down, 2 its restriction, 4 and 5 its passes on the way
+  // up; 3 the section
+  int l = 0, f = 0;
+#pragma unroll 1
+  for (;;) {
+    const bool uma = a.umaPassada && l >= 1;
+    if (f == 2) {
+      faseRestringir<T>(a, l);
+    } else if (f == 3) {
+      if (secaoDensa) aplicarSecaoDensa(a, smem);
+      else if (blockIdx.x == 0) secaoGrossa(a, smem, smem, tabS, -1, Equipe{(int)threadIdx.x, TF, 0}, true);
+    } else if (f == 4) {
+      faseSuavizarT<T, M_PROL>(a, l, 8, true, false, 1, areas, ru, sh);
+    } else if (f == 0 && l == 0) {
+      faseSuavizarT<T, M_ESPALHAR>(a, 0, 0, true, false, 0, areas, ru, sh);
+    } else if (f == 5 && l == 0) {
+      faseSuavizarT<T, M_JUNTAR>(a, 0, 0, false, false, 1, areas, ru, sh);
     } else {
-      faseSuavizar<T>(a, l, 0, true, l == 0 ? M_ESPALHAR : M_ZERO, areas, ru, sh);
-      if (!barreira(a, ep)) return false;
-      faseSuavizar<T>(a, l, 8, false, M_NORMAL, areas, ru, sh);
-      if (!barreira(a, ep)) return false;
+      faseSuavizarT<T, M_NORMAL>(a, l, f == 1 || uma ? 8 : 0, f == 0, f == 0, f == 5, areas, ru, sh);
     }
-    faseRestringir<T>(a, l, areas);
+    if (uma && (f == 0 || f == 4)) trocarXTmp(l);
     if (!barreira(a, ep)) return false;
-  }
-  if (secaoDensa) aplicarSecaoDensa(a, smem);
-  else if (blockIdx.x == 0) secaoGrossa(a, smem, smem, tabS, -1, Equipe{(int)threadIdx.x, TF, 0}, true);
-  if (!barreira(a, ep)) return false;
-  for (int l = a.Lc - 1; l >= 0; l--) {
-    faseSuavizar<T>(a, l, 8, true, M_PROL, areas, ru, sh);
-    if (a.umaPassada && l >= 1) {
-      trocarXTmp(l);
-      if (!barreira(a, ep)) return false;
-      continue;
+    if (f == 5 && l == 0) return true;
+    if (f == 2) {
+      l++;
+      f = l < a.Lc ? 0 : 3;
+    } else if (f == 3 || f == 5 || (f == 4 && uma)) {
+      l--;
+      f = 4;
+    } else {
+      f = f == 0 && uma ? 2 : f + 1;
     }
-    if (!barreira(a, ep)) return false;
-    faseSuavizar<T>(a, l, 0, false, l == 0 ? M_JUNTAR : M_VOLTA, areas, ru, sh);
-    if (!barreira(a, ep)) return false;
   }
-  return true;
 }
 
 // ---------------------------------------------------------------- PCG pieces
@@ -1540,92 +1665,190 @@ __device__ __forceinline__ float aplicarF(const Args& a, int c, FV val, FB valB)
   return (float)__popc(vz & 15) * val(c) - s;
 }
 
-constexpr int KDA = 4;  // cells per thread per batch in [DA]
+constexpr int KDA = 4;  // cells a thread and batch of the true residual
 
-// [DA] of a PCG iteration over this CTA's cells: p = z + beta p (z alone on the first
+// [DA] of a PCG iteration over this CTA's cells: beta, p = z + beta p (z alone on the first
 // iteration), A p (js/pressao-cpu.js:84-93, bubble neighbours through their p), the partial of
-// p.Ap (channel 0) and, for air of active bubbles, the sums over their water faces.  Cells go in
-// batches of KDA per thread: descriptors first, then every z and p the batch needs.  z and p
-// come through L1 (ld.ca): a warp's five loads of each share lines, which the L1 then serves
-// instead of five L2 requests.  Both were last written before the grid barrier that opens this
-// phase, whose acquire orders these loads after those writes as it does any other load (PTX
-// memory model; the cache operator is a hint).  Measured on the 38,370x316 atlas: 109 against
-// 170 us for the phase, with the bubble labels loaded only where the descriptor needs them and
-// no stores off water.
-__device__ __noinline__ void faseDA(const Args& a, const float* zc, const float* pv, float* pn, bool prim, float betaf,
-                                    double beta, const double* pbVelho, double* sh) {
+// p.Ap (channel 0) and, for air of active bubbles, the sums over their water faces.  Bound by the
+// latency of its loads and by the fetch of its code, which a phase enters cold: cells go in batches of
+// K a thread with every load ahead, left and right neighbours by shuffle (a warp's cells are
+// consecutive), the first batch's loads out before the global sums that make beta; the bubbles' z and
+// previous p wait in shared memory (areas), put there by the warps that do not sum, and the faces of
+// bubble air, the only FP64 sums with atomics, are a rolled loop over the cells that have them.
+// z and p come through L1: they were last written before the grid barrier that opens this phase,
+// whose acquire orders these loads after those writes.
+// Measured: 13.8 -> 10.9 us a phase on 840x536 cells, 8.7 -> 7.3 on 480x270; [B], built alike, keeps its
+// 6.3 to 7.6 us (it now makes the sums behind alpha under its loads).
+// A CTA's cells in [DA] and [B]: TF consecutive ones, then those GT further on, and so on; a batch is 4 such
+// runs, a thread 4 consecutive cells of one of them (a float4 an array).  Each thread then sums the
+// products of cell threadIdx.x of the 4 runs, passed through shared memory.
+constexpr int QUARTO = TF / 4;
+struct Quatro {
+  float v[4];
+};
+// Cells c .. c + 3 of an array (al: c is a multiple of 4 here), 0 outside 0 .. N - 1.
+__device__ __forceinline__ Quatro lerQuatro(const float* p, int c, int N, bool al) {
+  Quatro q;
+  if (al && c >= 0 && c + 3 < N) {
+    const float4 f = __ldca((const float4*)(p + c));
+    q.v[0] = f.x, q.v[1] = f.y, q.v[2] = f.z, q.v[3] = f.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) q.v[k] = c + k >= 0 && c + k < N ? __ldca(p + c + k) : 0.0f;
+  }
+  return q;
+}
+__device__ __forceinline__ void lerOps(const uint16_t* op, int c, int N, int (&m)[4]) {
+  if (c + 3 < N) {
+    const uint2 u = __ldcg((const uint2*)(op + c));
+    m[0] = u.x & 0xffff, m[1] = u.x >> 16, m[2] = u.y & 0xffff, m[3] = u.y >> 16;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) m[k] = c + k < N ? __ldcg(op + c + k) : 0;
+  }
+}
+__device__ __forceinline__ void faseDA(const Args& a, const float* zc, const float* pv, float* pn, bool prim, int nAt,
+                                    const double* pbVelho, double* pbNovo, const double* zbOld, double* zbCur,
+                                    double& rz, double* sh, float* areas) {
   const Dev& d = a.d;
-  const int N = d.N, nx = d.nx;
-  const int gt0 = blockIdx.x * TF + threadIdx.x, GT = gridDim.x * TF, lim = N;
-  auto pbNovoV = [&](int b) {
-    const double zb = zbDe(a, b);
-    return prim ? zb : zb + beta * __ldcg(&pbVelho[b]);
+  const int N = d.N, nx = d.nx, lane = threadIdx.x & 31, GT = gridDim.x * TF;
+  double* zbS = (double*)areas;
+  double* pbS = zbS + MAX_BOLHAS;
+  float2* pares = (float2*)(areas + (AREA_BOLHAS + AREA_TERMOS) / 4);  // p and A p of the batch's cells
+  auto bolha = [&](int b) {
+    zbS[b] = zbDe(a, b);
+    if (!prim) pbS[b] = __ldcg(&pbVelho[b]);
   };
-  double s = 0;
-  for (int c0 = gt0; c0 < lim; c0 += KDA * GT) {
-    int m[KDA];
-#pragma unroll
-    for (int k = 0; k < KDA; k++) {
-      const int c = c0 + k * GT;
-      m[k] = c < lim ? __ldcg(a.op + c) : 0;
-    }
-    float zv[KDA][5], pw[KDA][5];
-    unsigned long long rl[KDA];
-#pragma unroll
-    for (int k = 0; k < KDA; k++) {
-      // neighbour indices from the cell index alone, so these loads go out with the
-      // descriptors' (the descriptor then picks the water neighbours, which are inside the
-      // grid; an index across a row's end reads a value that no flag selects)
-      const int c = c0 + k * GT < lim ? c0 + k * GT : 0;
-      const int nb[5] = {c, c > 0 ? c - 1 : c, c < N - 1 ? c + 1 : c, c >= nx ? c - nx : c, c < N - nx ? c + nx : c};
-#pragma unroll
-      for (int q = 0; q < 5; q++) {
-        zv[k][q] = __ldca(zc + nb[q]);
-        pw[k][q] = prim ? 0.0f : __ldca(pv + nb[q]);
+  double beta = 0.0, s = 0.0;
+  auto pbNovoV = [&](int b) { return prim ? zbS[b] : zbS[b] + beta * pbS[b]; };
+  auto somar = [&] {
+    if (prim) {
+      if (nAt > 0) {
+#pragma unroll 1
+        for (int k = threadIdx.x; k < nAt; k += TF) bolha(__ldcg(&a.ativos[k]));
+        __syncthreads();
       }
+      return;
     }
-    // the packed labels of the bubble neighbours, only where the descriptor says a bubble is
-    // next to the cell (most cells have none: 8 bytes a cell saved)
+    double somas[4];
+    somasGlobais<true, 0>(a, nAt, [&](int b, double& t0, double& t1) {
+      bolha(b);
+      const double r = __ldcg(&d.rb[b]);
+      t0 = r * zbS[b];
+      t1 = r * __ldcg(&zbOld[b]);
+    }, sh, somas, areas);
+    const double rzNovo = somas[0] + somas[2], cruz = somas[1] + somas[3];
+    beta = fabs(rz) < 1e-30 ? 0.0 : fmax(0.0, (rzNovo - cruz) / rz);
+    rz = rzNovo;
+  };
+  const int b0 = blockIdx.x * TF, run = threadIdx.x / QUARTO, pos = threadIdx.x % QUARTO * 4;
+  const bool al = (nx & 3) == 0;
+#pragma unroll 1
+  for (int base = b0; base == b0 || base < N; base += 4 * GT) {
+    // the cells, those below and above (an index across a row's end reads a value that no flag selects),
+    // lane 0's to the left and lane 31's to the right
+    const int c0 = base + run * GT + pos;
+    int m[4];
+    lerOps(a.op, c0, N, m);
+    Quatro z[3], w[3];
+    float zl = 0.0f, wl = 0.0f;
+    const int cl = lane == 0 ? c0 - 1 : c0 + 4;
+    z[0] = lerQuatro(zc, c0, N, true);
+    z[1] = lerQuatro(zc, c0 - nx, N, al);
+    z[2] = lerQuatro(zc, c0 + nx, N, al);
+    if ((lane == 0 || lane == 31) && cl >= 0 && cl < N) zl = __ldca(zc + cl);
+    if (!prim) {
+      w[0] = lerQuatro(pv, c0, N, true);
+      w[1] = lerQuatro(pv, c0 - nx, N, al);
+      w[2] = lerQuatro(pv, c0 + nx, N, al);
+      if ((lane == 0 || lane == 31) && cl >= 0 && cl < N) wl = __ldca(pv + cl);
+    }
+    if (base == b0) {
+      somar();
+      if (blockIdx.x == 0)
+#pragma unroll 1
+        for (int k = threadIdx.x; k < nAt; k += TF) {
+          const int b = __ldcg(&a.ativos[k]);
+          zbCur[b] = zbS[b];
+          pbNovo[b] = pbNovoV(b);
+        }
+    }
+    const float betaf = (float)beta;
+    // the packed labels, only where a bubble's p or row needs them
+    unsigned long long rl[4];
 #pragma unroll
-    for (int k = 0; k < KDA; k++)
-      rl[k] = (a.bolhas && (m[k] & (OP_VIZ_BOLHA | OP_FACE))) ? __ldcg(a.rotB + c0 + k * GT) : 0ull;
+    for (int k = 0; k < 4; k++)
+      rl[k] = (m[k] & OP_VIZ_BOLHA) || ((m[k] & OP_FACE) && (m[k] & 15)) ? __ldcg(a.rotB + c0 + k) : 0ull;
+    if (!prim) {
 #pragma unroll
-    for (int k = 0; k < KDA; k++) {
-      const int c = c0 + k * GT;
-      if (c >= lim) continue;
+      for (int q = 0; q < 3; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) z[q].v[k] = z[q].v[k] + betaf * w[q].v[k];
+      zl = zl + betaf * wl;
+    }
+    const float ze = __shfl_up_sync(0xffffffffu, z[0].v[3], 1), zd = __shfl_down_sync(0xffffffffu, z[0].v[0], 1);
+    const float esq = lane == 0 ? zl : ze, dir = lane == 31 ? zl : zd;
+    int labA = 0;
+    long long acc = 0;
+    float ap[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
       const int mk = m[k];
-      float pq[5];
+      const float p = z[0].v[k];
+      // left, right, down, up: 0 where no water is
+      float pq[4] = {k ? z[0].v[k ? k - 1 : 0] : esq, k < 3 ? z[0].v[k < 3 ? k + 1 : 3] : dir, z[1].v[k], z[2].v[k]};
 #pragma unroll
-      for (int q = 0; q < 5; q++) pq[q] = prim ? zv[k][q] : zv[k][q] + betaf * pw[k][q];
+      for (int q = 0; q < 4; q++) pq[q] = (mk >> q) & 1 ? pq[q] : 0.0f;
+      ap[k] = 0.0f;
       if (mk & OP_AGUA) {
-        // water neighbours in the order left, right, down, up; air of an active bubble
-        // contributes its bubble's p
-        float sv = 0.0f;
+        if (mk & OP_VIZ_BOLHA)  // a neighbour that is air of an active bubble contributes that bubble's p
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          if (mk & (1 << q)) sv += pq[q + 1];
-          else if (mk & OP_VIZ_BOLHA) {  // neighbour q is air of an active bubble: that bubble's p
-            const int r = (int)(rl[k] >> (12 + 12 * q)) & 0xfff;
-            if (r) sv += (float)pbNovoV(r);
+          for (int q = 0; q < 4; q++) {
+            const int b = (int)(rl[k] >> (12 + 12 * q)) & 0xfff;
+            if (b && !((mk >> q) & 1)) pq[q] = (float)pbNovoV(b);
           }
+        ap[k] = (float)(mk >> 8) * p - (((pq[0] + pq[1]) + pq[2]) + pq[3]);
+      } else if ((mk & OP_FACE) && (mk & 15)) {
+        // (p and Ap off water are never read) the bubble's row: the sum of p over its water faces
+        const double f = (((double)pq[0] + (double)pq[1]) + (double)pq[2]) + (double)pq[3];
+        const int lab = (int)(rl[k] & 0xfff);
+        if (lab != labA) {
+          if (acc) atomicAdd((unsigned long long*)&d.accB[labA], (unsigned long long)acc);
+          labA = lab;
+          acc = 0;
         }
-        const float apc = (float)(mk >> 8) * pq[0] - sv;
-        pn[c] = pq[0];
-        d.ap[c] = apc;
-        s += (double)pq[0] * apc;
-      } else {  // p and Ap off water are never read: nothing stored
-        if (mk & OP_FACE) {  // the bubble's row: sum of p over its water faces
-          double t = 0;
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            if (mk & (1 << q)) t += (double)pq[q + 1];
-          if (t != 0) somaFixa(&d.accB[(int)(rl[k] & 0xfff)], t, ESC);
-        }
+        acc += __double2ll_rn(f * ESC);
       }
     }
+    if ((m[0] | m[1] | m[2] | m[3]) & OP_AGUA) {
+      if (c0 + 3 < N) {
+        *(float4*)(pn + c0) = make_float4(z[0].v[0], z[0].v[1], z[0].v[2], z[0].v[3]);
+        *(float4*)(d.ap + c0) = make_float4(ap[0], ap[1], ap[2], ap[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (c0 + k < N) {
+            pn[c0 + k] = z[0].v[k];
+            d.ap[c0 + k] = ap[k];
+          }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {  // (a row of the table has one float2 more: no bank twice)
+      const bool agua = (m[k] & OP_AGUA) != 0;
+      pares[k * (TF + 4) + run * QUARTO + pos / 4] = agua ? make_float2(z[0].v[k], ap[k]) : make_float2(0.0f, 0.0f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {  // cell threadIdx.x of run k
+      const float2 t = pares[(threadIdx.x & 3) * (TF + 4) + k * QUARTO + (threadIdx.x >> 2)];
+      s += (double)t.x * t.y;
+    }
+    if (base + 4 * GT < N) __syncthreads();
+    if (a.bolhas) somarBolhaWarp((long long*)d.accB, labA, acc);
   }
   const double tb = somaBloco(s, sh);
-  if (threadIdx.x == 0) a.parc[blockIdx.x * NPARC + 0] = tb;
+  if (threadIdx.x == 0) a.parc[blockIdx.x * NPARC + 2] = tb;
 }
 
 // Per-tank sums of v^2 over the water cells of each tank of an atlas (tq_set_tanks) into destino:
@@ -1895,6 +2118,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
       }
     }
     a.rotB[c] = rl;
+    a.rotP[c] = a.bloco ? 0 : (uint16_t)(rl & 0xfffu);
   }
   if (a.bolhas) {
     for (int c = gt0; c < N; c += GT) {
@@ -1989,7 +2213,8 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
   auto rbInicial = [&](int b) {
     return (double)d.rhsBolhaF[b] - (__ldcg(&d.facesB[b]) * __ldcg(&d.yB[b]) - (double)__ldcg(&d.accB[b]) / ESC);
   };
-  somasGlobais(a, nAt, [&](int b) { double v = rbInicial(b); return v * v; }, [](int) { return 0.0; }, sh, somas);
+  somasGlobais<false, 0>(a, nAt, [&](int b, double& t, double&) { const double v = rbInicial(b); t = v * v; }, sh, somas,
+                      areas);
   const double norma0 = sqrt(somas[0] + somas[2]);
   if (blockIdx.x == 0) {
     for (int k = threadIdx.x; k < nAt; k += TF) {
@@ -2030,12 +2255,20 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
       a.accZ[b] = 0;
       d.accB[b] = 0;
     }
-  if (!cicloV<T>(a, ep, areas, dyn, tabS[0], Reuniao{escala, d.z, nullptr}, sh, secaoDensa)) return;
+  // the spread reads each active bubble's mean residual from the CTA's areas (the V-cycle sees no
+  // bubbles with BLOCK)
+  auto mediaBolha = [&](int b) { areas[b] = (float)(__ldcg(&d.rb[b]) / __ldcg(&d.celsB[b])); };
+  auto mediasBolhas = [&] {
+    if (a.bloco) return;
+#pragma unroll 1
+    for (int k = threadIdx.x; k < nAt; k += TF) mediaBolha(__ldcg(&a.ativos[k]));
+  };
+  mediasBolhas();
+  __syncthreads();
+  Reuniao ru{escala, d.z, nullptr};
   int cz = 0, cp = 0;  // which of the two z / p buffers holds the latest values
   auto zbAtual = [&](int b) { return zbDe(a, b); };
-  somasGlobais(a, nAt, [&](int b) { return __ldcg(&d.rb[b]) * zbAtual(b); }, [](int) { return 0.0; }, sh, somas);
-  double rz = somas[0] + somas[2];
-  double beta = 0.0;
+  double rz = 0.0;
   bool primeira = true;
   int itersFeitas = 0, trocas = 0;
   bool convergiu = false;
@@ -2046,7 +2279,18 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     return (double)d.rhsBolhaF[b] - (__ldcg(&d.facesB[b]) * __ldcg(&d.yB[b]) - (double)__ldcg(&a.accV[b]) / ESC);
   };
 
-  for (int it = 0; it < a.iteracoes; it++) {
+  for (int it = -1;;) {
+    if (!cicloV<T>(a, ep, areas, dyn, tabS[0], ru, sh, secaoDensa)) return;
+    if (it < 0) {
+      somasGlobais<false, 0>(a, nAt, [&](int b, double& t, double&) { t = __ldcg(&d.rb[b]) * zbAtual(b); }, sh, somas, areas);
+      rz = somas[0] + somas[2];
+      __syncthreads();
+    } else {
+      cz ^= 1;
+      cp ^= 1;
+      primeira = false;
+    }
+    if (++it >= a.iteracoes) break;
     float* zc = cz ? a.z2 : d.z;
     float* zo = cz ? d.z : a.z2;
     const float* pv = cp ? a.p2 : d.p;
@@ -2056,58 +2300,82 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     const double* pbVelho = cp ? a.pb2 : d.pb;
     double* pbNovo = cp ? d.pb : a.pb2;
     // ---- [DA] beta, p = z + beta p, A p, p.Ap, bubble rows
-    if (!primeira) {
-      somasGlobais(a, nAt, [&](int b) { return __ldcg(&d.rb[b]) * zbAtual(b); },
-                   [&](int b) { return __ldcg(&d.rb[b]) * __ldcg(&zbOld[b]); }, sh, somas);
-      const double rzNovo = somas[0] + somas[2], cruz = somas[1] + somas[3];
-      beta = fabs(rz) < 1e-30 ? 0.0 : fmax(0.0, (rzNovo - cruz) / rz);
-      rz = rzNovo;
-    }
-    const float betaf = (float)beta;
-    const bool prim = primeira;
-    auto pbNovoV = [&](int b) { return prim ? zbAtual(b) : zbAtual(b) + beta * __ldcg(&pbVelho[b]); };
-    if (blockIdx.x == 0)
-      for (int k = threadIdx.x; k < nAt; k += TF) {
-        int b = __ldcg(&a.ativos[k]);
-        zbCur[b] = zbAtual(b);
-        pbNovo[b] = pbNovoV(b);
-      }
-    faseDA(a, zc, pv, pn, prim, betaf, beta, pbVelho, sh);
+    faseDA(a, zc, pv, pn, primeira, nAt, pbVelho, pbNovo, zbOld, zbCur, rz, sh, areas);
     if (!barreira(a, ep)) return;
     // ---- [B] alpha; q += alpha p, r -= alpha Ap; bubbles; r.r
     auto apbV = [&](int b) {
       return __ldcg(&d.facesB[b]) * __ldcg(&pbNovo[b]) - (double)__ldcg(&d.accB[b]) / ESC;
     };
-    somasGlobais(a, nAt, [&](int b) { return __ldcg(&pbNovo[b]) * apbV(b); }, [](int) { return 0.0; }, sh, somas);
-    const double pap = somas[0] + somas[2];
-    const double alfa = fabs(pap) < 1e-30 ? 0.0 : rz / pap;
+    double alfa;
     {
-      const float af = (float)alfa;
       double s = 0;
-      for (int c0 = gt0; c0 < N; c0 += 4 * GT) {  // batches of 4 cells: all loads first
+      float af = 0.0f;
+      // the cells as in [DA]; all loads of a batch first
+      const int b0 = blockIdx.x * TF, run = threadIdx.x / QUARTO, pos = threadIdx.x % QUARTO * 4;
+      float* rsS = areas + (AREA_BOLHAS + AREA_TERMOS) / 4;
+#pragma unroll 1
+      for (int base = b0; base == b0 || base < N; base += 4 * GT) {
+        const int c0 = base + run * GT + pos;
+        const bool todo = c0 + 3 < N;
         int m[4];
-        float qv[4], pnv[4], rv[4], apv[4];
+        lerOps(a.op, c0, N, m);
+        Quatro pq = lerQuatro(pn, c0, N, true), rq = lerQuatro(d.r, c0, N, true), aq = lerQuatro(d.ap, c0, N, true), qq;
         double qd[4];
+        if (a.q64) {
+          if (todo) {
+            const double2 u = __ldcg((const double2*)(a.q64 + c0)), v = __ldcg((const double2*)(a.q64 + c0 + 2));
+            qd[0] = u.x, qd[1] = u.y, qd[2] = v.x, qd[3] = v.y;
+          } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const int c = c0 + k * GT < N ? c0 + k * GT : 0;
-          m[k] = c0 + k * GT < N ? __ldcg(a.op + c) : 0;
-          if (a.q64) qd[k] = __ldcg(a.q64 + c);
-          else qv[k] = __ldcg(d.q + c);
-          pnv[k] = __ldcg(pn + c);
-          rv[k] = __ldcg(d.r + c);
-          apv[k] = __ldcg(d.ap + c);
+            for (int k = 0; k < 4; k++) qd[k] = c0 + k < N ? __ldcg(a.q64 + c0 + k) : 0.0;
+          }
+        } else {
+          qq = lerQuatro(d.q, c0, N, true);
         }
+        if (base == b0) {  // the first batch's loads are under way: the sums that make alpha
+          somasGlobais<false, 2>(a, nAt, [&](int b, double& t, double&) { t = __ldcg(&pbNovo[b]) * apbV(b); }, sh, somas,
+                              areas);
+          const double pap = somas[0] + somas[2];
+          alfa = fabs(pap) < 1e-30 ? 0.0 : rz / pap;
+          af = (float)alfa;
+        }
+        const bool alguma = (m[0] | m[1] | m[2] | m[3]) & OP_AGUA;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          if (!(m[k] & OP_AGUA)) continue;
-          const int c = c0 + k * GT;
-          if (a.q64) a.q64[c] = qd[k] + alfa * (double)pnv[k];
-          else d.q[c] = qv[k] + af * pnv[k];
-          const float r = rv[k] - af * apv[k];
-          d.r[c] = r;
+          const bool agua = m[k] & OP_AGUA;
+          if (agua) {
+            if (a.q64) qd[k] = qd[k] + alfa * (double)pq.v[k];
+            else qq.v[k] = qq.v[k] + af * pq.v[k];
+            rq.v[k] = rq.v[k] - af * aq.v[k];
+          }
+          rsS[k * (TF + 4) + run * QUARTO + pos / 4] = agua ? rq.v[k] : 0.0f;
+        }
+        if (alguma) {  // (cells off water get back what they held)
+          if (todo) {
+            *(float4*)(d.r + c0) = make_float4(rq.v[0], rq.v[1], rq.v[2], rq.v[3]);
+            if (a.q64) {
+              *(double2*)(a.q64 + c0) = make_double2(qd[0], qd[1]);
+              *(double2*)(a.q64 + c0 + 2) = make_double2(qd[2], qd[3]);
+            } else {
+              *(float4*)(d.q + c0) = make_float4(qq.v[0], qq.v[1], qq.v[2], qq.v[3]);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              if (c0 + k < N) {
+                d.r[c0 + k] = rq.v[k];
+                if (a.q64) a.q64[c0 + k] = qd[k];
+                else d.q[c0 + k] = qq.v[k];
+              }
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k++) {  // cell threadIdx.x of run k
+          const float r = rsS[(threadIdx.x & 3) * (TF + 4) + k * QUARTO + (threadIdx.x >> 2)];
           s += (double)r * r;
         }
+        if (base + 4 * GT < N) __syncthreads();
       }
       if (blockIdx.x == 0) {
         double sb = 0;
@@ -2127,11 +2395,11 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
           for (int t = threadIdx.x; t < d.nTanques; t += TF) d.rvT[t] = 0.0;
       }
       double tb = somaBloco(s, sh);
-      if (threadIdx.x == 0) a.parc[blockIdx.x * NPARC + 0] = tb;
+      if (threadIdx.x == 0) a.parc[blockIdx.x * NPARC + 3] = tb;
     }
     if (!barreira(a, ep)) return;
     // ---- [C] norm, convergence, spread the residual
-    somasGlobais(a, 0, [](int) { return 0.0; }, [](int) { return 0.0; }, sh, somas);
+    somasGlobais<false, 3>(a, a.bloco ? 0 : nAt, [&](int b, double&, double&) { mediaBolha(b); }, sh, somas, areas);
     double norma = sqrt(somas[0]);
     itersFeitas = it + 1;
     const bool ultima = it == a.iteracoes - 1;
@@ -2143,7 +2411,8 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
       proxVerif = it + VERIF_TANQUES;
       faseVerdade(a, sh);
       if (!barreira(a, ep)) return;
-      somasGlobais(a, nAt, [&](int b) { const double v = rbVerd(b); return v * v; }, [](int) { return 0.0; }, sh, somas);
+      somasGlobais<false, 0>(a, nAt, [&](int b, double& t, double&) { const double v = rbVerd(b); t = v * v; }, sh, somas,
+                          areas);
       normaVerd = sqrt(somas[0] + somas[2]);
       // with tanks, each tank's own residual decides; without, the whole grid's
       convergiu = d.nTanques ? tanquesConvergiram(a, nAt, rbVerd) : normaVerd <= a.tol * norma0;
@@ -2160,6 +2429,8 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
             d.rb[b] = rbVerd(b);
           }
         if (!barreira(a, ep)) return;  // rb visible before the spread
+        mediasBolhas();
+        __syncthreads();
       }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2172,10 +2443,7 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     escala = (a.escalar && norma > 0) ? (float)(1.0 / norma) : 1.0f;
     if (blockIdx.x == 0)
       for (int b = threadIdx.x; b < MAX_BOLHAS; b += TF) d.accB[b] = 0;
-    if (!cicloV<T>(a, ep, areas, dyn, tabS[0], Reuniao{escala, zo, zc}, sh, secaoDensa)) return;
-    cz ^= 1;
-    cp ^= 1;
-    primeira = false;
+    ru = Reuniao{escala, zo, zc};
   }
   // ---- end: q = 0 off water (the FP64 iterate rounded on water); bubbles hand back their
   // pressure; the solve's convergence record
@@ -2231,8 +2499,8 @@ Fundido* criarFundido(Pcg* p, Arena& A) {
   // an element whatever they store
   if (p->precisao != TQ_PREC_FP32)
     for (int l = 0; l < Lc; l++) p->meia[l] = true;
-  size_t porWarp = (size_t)(SUAV_W > REST_W ? SUAV_W : REST_W) * 4;
-  size_t areas = (size_t)WARPS * porWarp;
+  const size_t areas = AREA_BOLHAS + AREA_TERMOS + AREA_PRODUTOS;
+  static_assert(areas >= WARPS * 768 * 4 && areas >= WARPS * SUAV_W * 4, "the warps' areas");
   f->smem = bytes > areas ? bytes : areas;
   f->bytesSecao = (int)bytes;
   // teams that build the section's matrix side by side, where their areas and the coarsest
@@ -2307,6 +2575,7 @@ Fundido* criarFundido(Pcg* p, Arena& A) {
   A.pedir(&f->xc, nLc);
   A.pedir(&f->bc, nLc);
   A.pedir(&f->op, N);
+  A.pedir(&f->rotP, N);
   A.pedir(&f->rotB, N);
   A.pedir(&f->q64, N);
   A.pedir(&f->accV, MAX_BOLHAS);
@@ -2400,6 +2669,7 @@ int resolverPressaoFundido(Pcg* p, const Dev& d, int iteracoes, double tol, bool
   a.densoG = f->densoG;
   a.op = f->op;
   a.rotB = f->rotB;
+  a.rotP = f->rotP;
   a.perfil = f->perfilar ? f->perfil : nullptr;
   if (a.perfil) {
     cudaMemsetAsync(f->perfil, 0, sizeof(unsigned long long), s);
