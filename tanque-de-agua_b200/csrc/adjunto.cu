@@ -202,6 +202,7 @@ __device__ __forceinline__ double* Pc(const Fita& f, int cap, int c) { return f.
 // the faucet's accepted particles of the step, appended after the n current ones
 __global__ void k_adj_torneira(Estado E, int n, const double* fpos, const int* aceitos, int nAceitos, double th0,
                                double th1) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nAceitos) return;
   const int q = aceitos[k];
@@ -215,6 +216,7 @@ __global__ void k_adj_torneira(Estado E, int n, const double* fpos, const int* a
 
 // P2G float sums in double (js/fisica-cpu.js:198-267) and the particle count per cell
 __global__ void k_adj_p2g(Dispositivo D, Estado E, int n, double* U, double* UW, double* V, double* VW, int* cont) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const double x = E.c[0][k], y = E.c[1][k], vx = E.c[2][k], vy = E.c[3][k];
@@ -247,6 +249,7 @@ __global__ void k_adj_p2g(Dispositivo D, Estado E, int n, double* U, double* UW,
 
 // #tipos (:293-299)
 __global__ void k_adj_tipos(Dispositivo D, const int* cont, uint8_t* tipo) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= D.N) return;
   tipo[c] = D.solido[c] ? SOLIDO : cont[c] > 0 ? AGUA : AR;
@@ -255,6 +258,7 @@ __global__ void k_adj_tipos(Dispositivo D, const int* cont, uint8_t* tipo) {
 // u = U / UW where weighted, gravity there, wall faces 0 (:271-291)
 __global__ void k_adj_faces(Dispositivo D, const double* U, const double* UW, const double* V, const double* VW,
                             double* u, double* v) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = D.nx, ny = D.ny;
   if (k < D.nu) {
@@ -273,6 +277,7 @@ __global__ void k_adj_faces(Dispositivo D, const double* U, const double* UW, co
 
 // b = -div on water cells (#classificar without the density and air terms)
 __global__ void k_adj_div(Dispositivo D, const uint8_t* tipo, const double* u, const double* v, double* b) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= D.N) return;
   const int nx = D.nx, i = c % nx, j = c / nx;
@@ -282,6 +287,7 @@ __global__ void k_adj_div(Dispositivo D, const uint8_t* tipo, const double* u, c
 // #gradiente (:519-545) and the valid masks
 __global__ void k_adj_gradiente(Dispositivo D, const uint8_t* tipo, const double* q, double* u, double* v,
                                 uint8_t* vu, uint8_t* vv) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = D.nx, ny = D.ny;
   if (k < D.nu) {
@@ -307,6 +313,7 @@ __global__ void k_adj_gradiente(Dispositivo D, const uint8_t* tipo, const double
 // one extrapolation layer of one component (extrapolarComponente, js/fisica-cpu.js:673-690):
 // reads a and the masks before the layer, writes the new values and masks
 __global__ void k_adj_extrap(const double* a, const uint8_t* val, double* out, uint8_t* valOut, int w, int hh) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= w * hh) return;
   const int i = k % w, j = k / w;
@@ -328,6 +335,7 @@ __global__ void k_adj_extrap(const double* a, const uint8_t* val, double* out, u
 // G2P (#paraParticulas, :556-661, without foam and dye), recording the tape; alive flag per particle
 __global__ void k_adj_g2p(Dispositivo D, Estado E, int n, int cap, const double* ug, const double* vg, Fita f,
                           Estado S, int* vivo) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const double vmax = D.vmax, dt = D.dt, h = D.h;
@@ -404,6 +412,7 @@ __global__ void k_adj_g2p(Dispositivo D, Estado E, int n, int cap, const double*
 // (a few tens of thousands of particles), the alive ones to E in order, their indices to vivos
 __global__ void __launch_bounds__(1024) k_adj_compactar(Estado S, const int* vivo, int n, Estado E, int* vivos,
                                                         int* nVivos) {
+  aposAnterior();
   __shared__ int soma[1024];
   __shared__ int base;
   if (threadIdx.x == 0) base = 0;
@@ -433,6 +442,7 @@ __global__ void __launch_bounds__(1024) k_adj_compactar(Estado S, const int* viv
 
 // density at cell centres (:244-254)
 __global__ void k_adj_densidade(Dispositivo D, Estado E, int n, double* rho) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const Est e = est(D, 2, E.c[0][k], E.c[1][k]);
@@ -445,6 +455,7 @@ __global__ void k_adj_densidade(Dispositivo D, Estado E, int n, double* rho) {
 
 // per-cell loss terms (min(1, rho/4) - target)^2 and their derivative in rho
 __global__ void k_adj_perda(Dispositivo D, const double* rho, const double* alvo, double* termo, double* rhob) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= D.N) return;
   const double r4 = rho[c] / 4, f = fmin(1.0, r4), d = f - alvo[c];
@@ -473,12 +484,14 @@ __device__ double somaCta(double v) {
   return t;
 }
 __global__ void k_adj_produto(const double* a, const double* b, int n, double* parc) {
+  aposAnterior();
   double s = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) s += b ? a[k] * b[k] : a[k];
   const double t = somaCta(s);
   if (threadIdx.x == 0) parc[blockIdx.x] = t;
 }
 __global__ void k_adj_somar(const double* parc, int m, double* out) {
+  aposAnterior();
   double s = 0;
   for (int k = threadIdx.x; k < m; k += blockDim.x) s += parc[k];
   const double t = somaCta(s);
@@ -499,6 +512,7 @@ __device__ inline void pararCG(double* esc, int iteracoes) {
 
 // A v on water cells (js/pressao-cpu.js:84-93, true types; air is 0)
 __global__ void k_adj_aplicar(Dispositivo D, const uint8_t* tipo, const double* v, double* out, const double* esc) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= D.N || (esc && esc[E_PARA] != 0)) return;
   if (tipo[c] != AGUA) { out[c] = 0; return; }
@@ -517,6 +531,7 @@ __global__ void k_adj_aplicar(Dispositivo D, const uint8_t* tipo, const double* 
 }
 __global__ void k_adj_axpy2(int n, const uint8_t* tipo, const double* esc, double* q, const double* p, double* r,
                             const double* ap) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n || tipo[c] != AGUA || esc[E_PARA] != 0) return;
   const double a = esc[E_AL];
@@ -524,30 +539,35 @@ __global__ void k_adj_axpy2(int n, const uint8_t* tipo, const double* esc, doubl
   r[c] -= a * ap[c];
 }
 __global__ void k_adj_direcao(int n, const uint8_t* tipo, const double* esc, const double* z, double* p) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n || esc[E_PARA] != 0) return;
   p[c] = tipo[c] == AGUA ? z[c] + esc[E_BE] * p[c] : 0.0;
 }
 // z from the FP32 V-cycle: r scaled to unit norm (esc[E_D1] = ||r||^2) before, back after
 __global__ void k_adj_para_float(int n, const uint8_t* tipo, const double* r, const double* esc, int qual, float* b) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const double nr = sqrt(esc[qual]);
   b[c] = tipo[c] == AGUA ? (float)(r[c] * (nr > 0 ? 1.0 / nr : 1.0)) : 0.0f;
 }
 __global__ void k_adj_de_float(int n, const uint8_t* tipo, const float* x, const double* esc, int qual, double* z) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n || esc[E_PARA] != 0) return;
   const double nr = sqrt(esc[qual]);
   z[c] = tipo[c] == AGUA ? (double)x[c] * (nr > 0 ? nr : 1.0) : 0.0;
 }
 __global__ void k_adj_mascarar(int n, const uint8_t* tipo, const double* b, double* r, double* q) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   r[c] = tipo[c] == AGUA ? b[c] : 0.0;
   q[c] = 0.0;
 }
 __global__ void k_adj_copiar_se(double* dst, const double* src, size_t n, const double* esc) {
+  aposAnterior();
   if (esc[E_PARA] != 0) return;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
     dst[k] = src[k];
@@ -557,6 +577,7 @@ __global__ void k_adj_copiar_se(double* dst, const double* src, size_t n, const 
 // (E_D1); 2 the stop test on r.r (E_D1); 3 Polak-Ribiere beta from r.z (E_D1) and r.zOld (E_D2),
 // the iteration counted; 4 rz
 __global__ void k_adj_escalares(double* esc, int modo, double tol2) {
+  aposAnterior();
   if (modo == 0) {
     esc[E_B2] = esc[E_D1];
     esc[E_PARA] = 0.0;
@@ -586,6 +607,7 @@ __global__ void k_adj_escalares(double* esc, int modo, double tol2) {
 // ---------------------------------------------------------------- backward kernels
 // final positions' adjoint from the loss (the density stencil's derivatives)
 __global__ void k_adj_perda_T(Dispositivo D, Estado E, int n, const double* rhob, Estado B) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const Est e = est(D, 2, E.c[0][k], E.c[1][k]);
@@ -599,6 +621,7 @@ __global__ void k_adj_perda_T(Dispositivo D, Estado E, int n, const double* rhob
 // G2P reverse of output particle o (input particle vivos[o]): position adjoint into Bin, grid
 // adjoint into ugb / vgb (atomics)
 __global__ void k_adj_g2p_T(Dispositivo D, Fita f, int cap, Estado B, Estado Bin, double* ugb, double* vgb) {
+  aposAnterior();
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= f.nVivos) return;
   const int k = f.vivos[o];
@@ -694,6 +717,7 @@ __global__ void k_adj_g2p_T(Dispositivo D, Fita f, int cap, Estado B, Estado Bin
 // neighbours it averaged; out starts as a copy of xb
 __global__ void k_adj_extrap_T(const double* xb, const uint8_t* val, const uint8_t* valDepois, double* out, int w,
                                int hh) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= w * hh) return;
   if (val[k] || !valDepois[k]) return;
@@ -714,6 +738,7 @@ __global__ void k_adj_extrap_T(const double* xb, const uint8_t* val, const uint8
 // the gradient's reverse as a gather per cell: qb = sum over the cell's faces with a water side
 // and no wall side of -/+ the face adjoint (the cell is the face's right / left side)
 __global__ void k_adj_grad_T(Dispositivo D, const uint8_t* tipo, const double* ugb, const double* vgb, double* qb) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= D.N) return;
   if (tipo[c] != AGUA) { qb[c] = 0; return; }
@@ -733,6 +758,7 @@ __global__ void k_adj_grad_T(Dispositivo D, const uint8_t* tipo, const double* u
 __global__ void k_adj_faces_T(Dispositivo D, const uint8_t* tipo, const double* lam, const double* ugb,
                               const double* vgb, const double* U, const double* UW, const double* V, const double* VW,
                               double* Ub, double* UWb, double* Vb, double* VWb) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = D.nx, ny = D.ny;
   if (k < D.nu) {
@@ -765,6 +791,7 @@ __global__ void k_adj_faces_T(Dispositivo D, const uint8_t* tipo, const double* 
 // position adjoint G2P's reverse left in Bin)
 __global__ void k_adj_p2g_T(Dispositivo D, Fita f, int cap, const double* Ub, const double* UWb, const double* Vb,
                             const double* VWb, Estado Bin) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= f.n) return;
   const double x = Pc(f, cap, 0)[k], y = Pc(f, cap, 1)[k], vx = Pc(f, cap, 2)[k], vy = Pc(f, cap, 3)[k];
@@ -812,15 +839,18 @@ __global__ void k_adj_p2g_T(Dispositivo D, Fita f, int cap, const double* Ub, co
 }
 
 __global__ void k_adj_zerar(double* a, size_t n) {
+  aposAnterior();
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) a[k] = 0;
 }
 __global__ void k_adj_saida_v(Estado B, int n, double escala, float* dv) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   dv[2 * k] = (float)(B.c[2][k] * escala);
   dv[2 * k + 1] = (float)(B.c[3][k] * escala);
 }
 __global__ void k_adj_entrada_v(Estado E, int n, const float* v0, const double* pos0, const double* C0) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   E.c[0][k] = pos0[2 * k];

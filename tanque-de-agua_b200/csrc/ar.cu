@@ -54,6 +54,7 @@ struct Rastreador {
 
 // ---------------------------------------------------------------- union-find (uniao.cuh)
 __global__ void k_ar_iniciar(Rastreador r, const uint8_t* tipo) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= r.N) return;
   r.pai[c] = tipo[c] == AR ? c : -1;
@@ -63,6 +64,7 @@ __global__ void k_ar_iniciar(Rastreador r, const uint8_t* tipo) {
 }
 // js/ar.js:61-69
 __global__ void k_ar_unir(Rastreador r, const uint8_t* tipo) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= r.N || tipo[c] != AR) return;
   int i = c % r.nx, j = c / r.nx;
@@ -75,6 +77,7 @@ __global__ void k_ar_unir(Rastreador r, const uint8_t* tipo) {
 // write here could replace a root some other thread has just stored with a non-root
 // ancestor.  The only writes of this kernel store roots, so concurrent walks stay valid.
 __global__ void k_ar_achatar(Rastreador r) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= r.N || r.pai[c] < 0) return;
   r.pai[c] = raizLeitura(r.pai, c);
@@ -89,6 +92,7 @@ __device__ inline unsigned hashChave(unsigned long long k) {
   return (unsigned)k;
 }
 __global__ void k_ar_estatisticas(Rastreador r, const uint32_t* rotulo) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= r.N) return;
   int rt = r.pai[c];
@@ -163,6 +167,7 @@ __device__ int scanBlocoUnico(const int* cont, int* offs, int n) {
 
 // Component index k = rank of the root among all roots in raster order (js/ar.js:75-85).
 __global__ void k_ar_raizes_contar(Rastreador r) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   bool raizc = c < r.N && r.pai[c] == c;
   int t;
@@ -170,10 +175,12 @@ __global__ void k_ar_raizes_contar(Rastreador r) {
   if (threadIdx.x == 0) r.blocoCont[blockIdx.x] = t;
 }
 __global__ void k_ar_raizes_scan(Rastreador r) {
+  aposAnterior();
   int total = scanBlocoUnico(r.blocoCont, r.blocoOff, r.nBlocos);
   if (threadIdx.x == 0) r.cont[0] = total;
 }
 __global__ void k_ar_raizes_gravar(Rastreador r) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   bool raizc = c < r.N && r.pai[c] == c;
   int t;
@@ -192,6 +199,7 @@ __global__ void k_ar_raizes_gravar(Rastreador r) {
 
 // Occupied hash slots -> pair list keyed (k, first cell); value (label, cells).
 __global__ void k_ar_pares(Rastreador r) {
+  aposAnterior();
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= r.Hc) return;
   unsigned long long chave = r.hk[h];
@@ -209,6 +217,7 @@ __global__ void k_ar_pares(Rastreador r) {
 // Ascending sort of (key, value) pairs: one CTA bitonic network in shared memory up to 2048
 // elements, the same network over global memory beyond that.
 __global__ void k_bitonic_local(unsigned long long* key, unsigned long long* val, int n) {
+  aposAnterior();
   __shared__ unsigned long long sk[2048];
   __shared__ unsigned long long sv[2048];
   int m = 1;
@@ -242,6 +251,7 @@ __global__ void k_bitonic_local(unsigned long long* key, unsigned long long* val
   }
 }
 __global__ void k_bitonic_passo(unsigned long long* key, unsigned long long* val, int m, int kk, int j) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   int l = i ^ j;
@@ -259,6 +269,7 @@ __global__ void k_bitonic_passo(unsigned long long* key, unsigned long long* val
   }
 }
 __global__ void k_preencher(unsigned long long* key, unsigned long long* val, int n, int m) {
+  aposAnterior();
   int i = n + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   key[i] = VAZIO;
@@ -280,6 +291,7 @@ static void ordenar(unsigned long long* key, unsigned long long* val, int n, cud
 
 // ---------------------------------------------------------------- canonicalisation
 __global__ void k_ar_gas_scan(Rastreador r) {
+  aposAnterior();
   int total = scanBlocoUnico(r.gasCount, r.gasOff, r.cont[0]);
   (void)total;
 }
@@ -288,6 +300,7 @@ __device__ inline bool fica(const Rastreador& r, int k) { return r.topoK[k] || r
 
 // sobreposicaoTotal (js/ar.js:102-106): cells of each old label inside components that stay.
 __global__ void k_ar_sobreposicao(Rastreador r) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= r.cont[1]) return;
   int k = (int)(r.parKey[i] >> 32);
@@ -299,6 +312,7 @@ __global__ void k_ar_sobreposicao(Rastreador r) {
 
 // novoAlvo and dono (js/ar.js:108-125), the gas Map walked in insertion order.
 __global__ void k_ar_alvo(Rastreador r, const float* volumeAlvo) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= r.cont[0]) return;
   if (!fica(r, k) || r.topoK[k]) return;
@@ -324,6 +338,7 @@ __global__ void k_ar_alvo(Rastreador r, const float* volumeAlvo) {
 // ordem (js/ar.js:129-130): closed components of >= 4 target cells, by target descending,
 // ties by component index.  Key: (~bits(novoAlvo)) << 32 | k.
 __global__ void k_ar_ordem(Rastreador r) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= r.cont[0]) return;
   if (r.topoK[k] || !(r.novoAlvo[k] >= (float)MIN_BOLHA_CELULAS)) return;
@@ -334,6 +349,7 @@ __global__ void k_ar_ordem(Rastreador r) {
 
 // Owners (js/ar.js:131-134): each old label goes to the earliest component in ordem it owns.
 __global__ void k_ar_donos_marcar(Rastreador r) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= r.cont[2]) return;
   int k = (int)(r.ordKey[i] & 0xffffffffu);
@@ -341,6 +357,7 @@ __global__ void k_ar_donos_marcar(Rastreador r) {
   if (d >= 2 && d < MAX_BOLHAS) atomicMin(&r.ganhador[d], i);
 }
 __global__ void k_ar_donos_gravar(Rastreador r) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= r.cont[2]) return;
   int k = (int)(r.ordKey[i] & 0xffffffffu);
@@ -353,6 +370,7 @@ __global__ void k_ar_donos_gravar(Rastreador r) {
 
 // Free ids (js/ar.js:137-139): labels >= 2 alive neither now nor in the previous frame, in order.
 __global__ void k_ar_livres(Rastreador r, const uint8_t* vivo) {
+  aposAnterior();
   int total = 0;
   // one 1024-thread block; ids 2..4095 in 4 chunks
   for (int base = 0; base < MAX_BOLHAS; base += 1024) {
@@ -371,6 +389,7 @@ __global__ void k_ar_livres(Rastreador r, const uint8_t* vivo) {
 // free id; once the ids run out the rest stay unlabelled (vacuum).  The initial pressure is
 // the owner's previous pressure, written after every read (pNova -> pressaoBolha).
 __global__ void k_ar_nascer_contar(Rastreador r) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool sem = false;
   if (i < r.cont[2]) {
@@ -381,8 +400,10 @@ __global__ void k_ar_nascer_contar(Rastreador r) {
   rankBloco1024(sem, &t);
   if (threadIdx.x == 0) r.blocoCont[blockIdx.x] = t;
 }
-__global__ void k_ar_nascer_scan(Rastreador r, int nb) { scanBlocoUnico(r.blocoCont, r.blocoOff, nb); }
+__global__ void k_ar_nascer_scan(Rastreador r, int nb) {
+  aposAnterior(); scanBlocoUnico(r.blocoCont, r.blocoOff, nb); }
 __global__ void k_ar_nascer(Rastreador r, const float* pressaoBolha) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool sem = false;
   int k = 0;
@@ -403,6 +424,7 @@ __global__ void k_ar_nascer(Rastreador r, const float* pressaoBolha) {
   r.nasceu[id] = 1;
 }
 __global__ void k_ar_aplicar_bolhas(Rastreador r, float* pressaoBolha, float* volumeAlvo, uint8_t* vivo) {
+  aposAnterior();
   int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= MAX_BOLHAS) return;
   if (r.nasceu[id]) pressaoBolha[id] = r.pNova[id];
@@ -411,6 +433,7 @@ __global__ void k_ar_aplicar_bolhas(Rastreador r, float* pressaoBolha, float* vo
 }
 // Atmosphere label, target volumes, final per-cell labels (js/ar.js:145-150).
 __global__ void k_ar_volumes(Rastreador r, float* volumeAlvo) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= r.cont[0]) return;
   if (r.topoK[k]) {
@@ -421,6 +444,7 @@ __global__ void k_ar_volumes(Rastreador r, float* volumeAlvo) {
   if (l >= 2) volumeAlvo[l] = r.novoAlvo[k];
 }
 __global__ void k_ar_rotular(Rastreador r, uint32_t* rotulo) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= r.N) return;
   int rt = r.pai[c];
@@ -484,6 +508,7 @@ int primeiraRastreador(Rastreador* r) { return r->primeira; }
 void definirPrimeiraRastreador(Rastreador* r, int v) { r->primeira = v ? 1 : 0; }
 
 __global__ void k_preencher_int(int* p, int v, int n) {
+  aposAnterior();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }

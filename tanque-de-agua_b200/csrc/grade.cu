@@ -14,6 +14,7 @@ namespace tq {
 
 // Cena.celulaSolida (js/cena.js:119-127) for every cell: SimulacaoCPU.atualizarParedes.
 __global__ void k_solidos(Dev d) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N) return;
   int i = c % d.nx, j = c / d.nx;
@@ -37,6 +38,7 @@ __device__ double molduraMascara(int x, int y, int mw, int mh) {
 // computes it, min into the mask (draw) or max of its negation capped by the frame (erase).
 __global__ void k_tracar(float* sdf, int mw, int mh, int x0, int y0, int nbx, int nby, double ax, double ay, double dx,
                          double dy, double len2, double rp, int apagar) {
+  aposAnterior();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nbx * nby) return;
   const int x = x0 + idx % nbx, y = y0 + idx / nbx;
@@ -54,6 +56,7 @@ __global__ void k_tracar(float* sdf, int mw, int mh, int x0, int y0, int nbx, in
 
 // Cena#zerar (js/cena.js:139-144): the mask of an empty tank, the frame alone.
 __global__ void k_zerar_mascara(float* sdf, int mw, int mh) {
+  aposAnterior();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= mw * mh) return;
   sdf[idx] = (float)molduraMascara(idx % mw, idx / mw, mw, mh);
@@ -74,6 +77,7 @@ __device__ __forceinline__ int reservar(int* cont, bool sim) {
 // js/gpu/fisica.js:135-160).  With `ar`, the first step of #propagarRotulos (:412, non-air cells lose
 // their label) and the list of the cells its first pass may label (see k_rotulos_resolver).
 __global__ void __launch_bounds__(256) k_tipos(Dev d, int faces, float gdx, float gdy, int ar) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = d.nx, ny = d.ny;
   if (faces) {
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(256) k_tipos(Dev d, int faces, float gdx, floa
 // right/upper neighbour the before-the-pass value is 0.  One CTA does both passes: the second's
 // pending cells are those of the first's list that are still unlabelled.
 __global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
+  aposAnterior();
   __shared__ int mudou;
   const int n = d.esc->pendentes;
   const int nx = d.nx;
@@ -180,6 +185,7 @@ constexpr int SUP_THREADS = 256, SUP_SEG = 15;  // 4 segments of 15 cells a line
 constexpr uint8_t SUP_LIVRE = 0, SUP_FUNDO = 200, SUP_FORA = 255;  // marks: no wall; wall beyond layer 3; off the grid
 
 __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
+  aposAnterior();
   __shared__ float f[SUP_W * SUP_P], g[SUP_W * SUP_P];
   __shared__ uint8_t mk[SUP_W * SUP_P];  // SUP_LIVRE, the layer a wall cell is filled in (1-3), SUP_FUNDO, SUP_FORA
   const int nx = d.nx, ny = d.ny, x0 = blockIdx.x * SUP_T - SUP_H, y0 = blockIdx.y * SUP_T - SUP_H;
@@ -322,6 +328,7 @@ __device__ inline float pressaoDoAr(const Dev& d, int c, int i, int j, double dt
 // are 64-bit fixed point (2^-32) so their value does not depend on the order cells arrive in.  The last
 // block closes the bubbles' right-hand sides: the volume recovery term and the initial pressure.
 __global__ void __launch_bounds__(256) k_lado_direito(Dev d, double dt, double tensao, double tau, int bolhas) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = d.nx, ny = d.ny;
   uint32_t b = 0;
@@ -407,6 +414,7 @@ __global__ void __launch_bounds__(256) k_lado_direito(Dev d, double dt, double t
 // (clamped); the faces beside water take the gradient, into uTmp / vTmp.  A face reads an air cell's
 // pressure from its parts, so no thread waits for the q another writes.
 __global__ void __launch_bounds__(256) k_gradiente(Dev d, double dt, int ar) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = d.nx, ny = d.ny;
   const uint8_t* tipo = d.tipo;
@@ -492,6 +500,7 @@ __device__ inline void extrapolar2(const float* a, const uint8_t* val, float* ao
   vo[k] = ok ? 1 : 0;
 }
 __global__ void __launch_bounds__(256) k_extrapolar(Dev d) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < d.nu) extrapolar2(d.uTmp, d.uValTmp, d.u, d.uVal, k, d.nx + 1, d.ny);
   if (k < d.nv) extrapolar2(d.vTmp, d.vValTmp, d.v, d.vVal, k, d.nx, d.ny + 1);

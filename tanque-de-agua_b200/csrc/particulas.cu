@@ -103,6 +103,7 @@ constexpr int P2G_T = 256;
 constexpr int P2G_CAIXA = 1024;
 
 __global__ void __launch_bounds__(P2G_T) k_p2g(Dev d) {
+  aposAnterior();
   __shared__ int2 sU[P2G_CAIXA], sV[P2G_CAIXA], sC[P2G_CAIXA];
   __shared__ int sD[3 * P2G_CAIXA];
   __shared__ int caixa[4];  // min ci, min cj, max ci, max cj of the CTA's live particles
@@ -235,6 +236,7 @@ __device__ __forceinline__ void maxVelocidadeWarp(unsigned ativos, double vel, u
 }
 
 __global__ void k_g2p(Dev d, double dt) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const bool dentro = k < d.esc->n;
   const float4 a = dentro ? d.p0[k] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -382,6 +384,7 @@ __device__ int scanUmBloco(const int* cont, int* offs, int n) {
 // the reference's `remover` keeps the survivors' order (js/fisica-cpu.js:114-126).  All four
 // kernels return at once when nothing died.
 __global__ void k_compactar_contar(Dev d, int* cont) {
+  aposAnterior();
   if (d.esc->mortas == 0) return;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   int n = d.esc->n;
@@ -392,6 +395,7 @@ __global__ void k_compactar_contar(Dev d, int* cont) {
 }
 
 __global__ void k_compactar_scan(Dev d, const int* cont, int* offs, int nb, int* estado) {
+  aposAnterior();
   if (d.esc->mortas == 0) {
     if (threadIdx.x == 0) estado[0] = 0;
     return;
@@ -406,6 +410,7 @@ __global__ void k_compactar_scan(Dev d, const int* cont, int* offs, int nb, int*
 }
 
 __global__ void k_compactar_mover(Dev d, const int* offs, const int* estado) {
+  aposAnterior();
   if (!estado[0]) return;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   int n = estado[1];
@@ -422,6 +427,7 @@ __global__ void k_compactar_mover(Dev d, const int* offs, const int* estado) {
 }
 
 __global__ void k_compactar_copiar(Dev d, const int* estado) {
+  aposAnterior();
   if (!estado[0]) return;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= d.esc->n) return;
@@ -436,6 +442,7 @@ __global__ void k_compactar_copiar(Dev d, const int* estado) {
 // > RAIO_PARTICULA + 0.05 and, with checarCheia, its cell held < PARTICULAS_POR_CELULA - 1
 // particles at the last transfer.  Survivors are appended in list order.
 __global__ void k_adicionar_contar(Dev d, const float* lista, int total, int checar, int* cont) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   bool ok = false;
   if (k < total) {
@@ -457,12 +464,14 @@ __global__ void k_adicionar_contar(Dev d, const float* lista, int total, int che
 }
 
 __global__ void k_adicionar_scan(Dev d, const int* cont, int* offs, int nb) {
+  aposAnterior();
   int total = scanUmBloco(cont, offs, nb);
   if (threadIdx.x == 0) d.esc->aceitas = total;
 }
 
 __global__ void k_adicionar_mover(Dev d, const float* lista, int total, int checar, const int* offs,
                                   unsigned long long idBase) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   bool ok = false;
   const float* o = lista + (size_t)min(k, max(total - 1, 0)) * CAMPOS;
@@ -490,10 +499,12 @@ __global__ void k_adicionar_mover(Dev d, const float* lista, int total, int chec
   }
 }
 
-__global__ void k_adicionar_fim(Dev d) { d.esc->n += d.esc->aceitas; }
+__global__ void k_adicionar_fim(Dev d) {
+  aposAnterior(); d.esc->n += d.esc->aceitas; }
 
 // ---------------------------------------------------------------- state copies
 __global__ void k_empacotar(Dev d, float* out, int n) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   float4 a = d.p0[k], b = d.p1[k], c = d.p2[k];
@@ -504,6 +515,7 @@ __global__ void k_empacotar(Dev d, float* out, int n) {
 }
 
 __global__ void k_desempacotar(Dev d, const float* in, int n, unsigned long long idBase) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float* o = in + (size_t)k * CAMPOS;
@@ -517,6 +529,7 @@ __global__ void k_desempacotar(Dev d, const float* in, int n, unsigned long long
 // SimulacaoCPU.aplicarFerramenta (js/fisica-cpu.js:129-152).  The sponge marks particles dead
 // (removed by the compaction, order kept); the hand pulls velocities; the dye paints.
 __global__ void k_ferramenta(Dev d, tq_tool f) {
+  aposAnterior();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= d.esc->n) return;
   float4 a = d.p0[k];
@@ -569,6 +582,7 @@ __device__ __forceinline__ uint32_t lcgSalto(uint32_t s, uint32_t k) {
 }
 __global__ void k_torneira(float* lista, int n, uint32_t semente, double cx, double cy, double raio, float vx, float vy,
                            float a0, float a1, float a2) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t s1 = lcgSalto(semente, 2u * (uint32_t)k + 1u);
@@ -602,6 +616,7 @@ void lancarTorneira(float* lista, int n, uint32_t semente, double cx, double cy,
 __device__ __forceinline__ long long fixoMancha(float v) { return __double2ll_rn((double)v * 4294967296.0); }
 
 __global__ void k_mancha(Dev d, int n, int w, int hp, float W, float H, float raio, unsigned long long* acc) {
+  aposAnterior();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float4 a = d.p0[k], e = d.p2[k];
@@ -630,6 +645,7 @@ __global__ void k_mancha(Dev d, int n, int w, int hp, float W, float H, float ra
 }
 
 __global__ void k_mancha_float(const long long* acc, float* out, size_t total) {
+  aposAnterior();
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < total) out[k] = (float)((double)acc[k] * (1.0 / 4294967296.0));
 }

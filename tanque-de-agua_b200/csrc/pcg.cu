@@ -29,6 +29,7 @@ constexpr int V0_BOLHA = 32, V0_AGUA = 64;
 // from the true types.  And the bubbles' faces (montarBolhas, js/pressao-cpu.js:271-288): the (interior
 // bubble cell, water neighbour) pairs of each label; a label with any is an active bubble.
 __global__ void k_plano_tipos(Dev d, uint8_t* t0, uint8_t* vizOp, int bolhas, int bloco) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N) return;
   const int nx = d.nx, ny = d.ny, i = c % nx, j = c / nx;
@@ -65,6 +66,7 @@ struct Niveis {
 // launch a level took 2.4-3.6 us each).
 constexpr int NIVEIS_POR_VEZ = 6;
 __global__ void __launch_bounds__(256) k_niveis_tipos(Niveis n, int l0) {
+  aposAnterior();
   __shared__ uint8_t t[2][32 * 32];
   auto mais = [](int a, int b) { return a == AR || b == AR ? (int)AR : a == AGUA || b == AGUA ? (int)AGUA : (int)SOLIDO; };
   const int L = min(n.L - 1, l0 + NIVEIS_POR_VEZ);
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(256) k_niveis_tipos(Niveis n, int l0) {
 // `bloco` (TQ_PRECOND_BLOCK) the coarse levels' bits 0-3 are open where a fine face across the coarse
 // face joins two non-wall fine cells (both coarse cells not wall).
 __global__ void k_niveis_viz(Niveis n, int l0, int bloco) {
+  aposAnterior();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   int l = l0;
   while (l < n.L && g >= n.ini[l + 1]) l++;
@@ -148,6 +151,7 @@ constexpr int T_LADRILHO = 512;
 template <class T, class TG, bool NIVEL0>
 __global__ void __launch_bounds__(T_LADRILHO) k_descer(NivelDev<T> n, NivelDev<TG> g, int kx, int ky, int uma, int masc,
                                                        Fonte F) {
+  aposAnterior();
   extern __shared__ __align__(16) float mem[];
   if (n.parar && *n.parar) return;  // uniform over the CTA
   const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
@@ -171,6 +175,7 @@ __global__ void __launch_bounds__(T_LADRILHO) k_descer(NivelDev<T> n, NivelDev<T
 // Level 0's right side made from F on a grid of one level (k_descer makes it elsewhere).
 template <class T>
 __global__ void k_fonte(NivelDev<T> n0, Fonte F) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n0.nx * n0.ny || (n0.parar && *n0.parar)) return;
   float v = F.v[c];
@@ -202,6 +207,7 @@ __device__ __forceinline__ float dividirViz(float t, float k, float i) {
   return fabsf(q) < INFINITY ? r : q;
 }
 __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
+  aposAnterior();
   // one array, addressed by offsets: x, the snapshots, the right sides, and a 0 for closed neighbours
   constexpr int S = SECAO_PLANA_TOTAL, B = 2 * SECAO_PLANA_TOTAL, ZERO = 3 * SECAO_PLANA_TOTAL;
   __shared__ float X[ZERO + 1];
@@ -363,6 +369,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
 // in shared memory when it fits.  65 half-sweeps as in k_secao.
 template <class T>
 __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
+  aposAnterior();
   extern __shared__ unsigned char dyn[];
   if (n.parar && *n.parar) return;  // uniform over the CTA
   const int N = n.nx * n.ny, nx = n.nx;
@@ -495,6 +502,7 @@ __device__ inline void somasFinais(const Plano& P, int blocosTot, bool dois, dou
 // rb = rhs - (faces y - sum) (:339-341), and the initial norm.
 __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const uint8_t* vizOp, const uint8_t* tipo0,
                                                         uint8_t* viz0, double* q64) {
+  aposAnterior();
   __shared__ double sh[32];
   const int nx = d.nx, N = d.N;
   double s = 0;
@@ -605,6 +613,7 @@ __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const ui
 // active bubble gives a water cell its bubble's p, and takes the sum of p over its water faces.
 // The last block: the bubbles' p and rows, p.Ap and alpha.
 __global__ void __launch_bounds__(T_PCG) k_plano_da(Dev d, Plano P, const float* z, const float* pv, float* pn, int prim) {
+  aposAnterior();
   __shared__ double sh[32];
   if (d.esc->pronto) return;  // uniform over the grid
   const int nx = d.nx, N = d.N;
@@ -665,6 +674,7 @@ __global__ void __launch_bounds__(T_PCG) k_plano_da(Dev d, Plano P, const float*
 // q += alpha p, r -= alpha Ap on water with r.r; the last block the bubbles and the norm
 // (js/pressao-cpu.js:377-386).
 __global__ void __launch_bounds__(T_PCG) k_plano_b(Dev d, Plano P, const float* p, double* q64, int it, double tol, int cap) {
+  aposAnterior();
   __shared__ double sh[32];
   if (d.esc->pronto) return;
   const double alfa = d.esc->alpha;
@@ -753,6 +763,7 @@ __device__ inline void fimJuncao(const Juncao& J, int bloco, int blocosTot, doub
 // The gather on a grid of one level (k_subir's last launch does it elsewhere).
 template <class T>
 __global__ void __launch_bounds__(T_PCG) k_juntar(Juncao J, const uint8_t* viz0, const T* x0) {
+  aposAnterior();
   const Dev& d = J.d;
   if (d.esc->pronto) return;
   const float inv = (float)(1.0 / d.esc->escalaMG);
@@ -768,6 +779,7 @@ template <class T, class TG, bool JUNTA>
 __global__ void __launch_bounds__(T_LADRILHO) k_subir(NivelDev<T> n, NivelDev<TG> g, const TG* xg, int kx, int ky,
                                                       int uma, int masc, float* saida,
                                                       const __grid_constant__ Juncao J) {
+  aposAnterior();
   extern __shared__ __align__(16) float mem[];
   if (n.parar && *n.parar) return;
   const Ladrilho L{(int)blockIdx.x * 16 * kx, (int)blockIdx.y * 16 * ky, kx, ky, n.nx, n.ny, n.viz};
@@ -814,6 +826,7 @@ __global__ void __launch_bounds__(T_LADRILHO) k_subir(NivelDev<T> n, NivelDev<TG
 // before).  k_verdade_fim finishes the norm and decides.
 constexpr int BLOCOS_VERDADE = 296;  // 2 a SM
 __global__ void __launch_bounds__(256) k_verdade(Dev d, const uint8_t* vizOp, const double* q64, int bolhas) {
+  aposAnterior();
   __shared__ double sh[32];
   if (!d.esc->verificar || d.esc->pronto) return;  // uniform over the grid
   double s = 0;
@@ -858,6 +871,7 @@ __global__ void __launch_bounds__(256) k_verdade(Dev d, const uint8_t* vizOp, co
 // residual, reiniciar is set (k_substituir copies the water part into r).
 __global__ void __launch_bounds__(256) k_verdade_fim(Dev d, int blocosVerdade, int cap, double tol, int bolhas,
                                                     int meiaPrecisao) {
+  aposAnterior();
   __shared__ double sh[32];
   __shared__ int substituir;
   Escalares* e = d.esc;
@@ -899,6 +913,7 @@ __global__ void __launch_bounds__(256) k_verdade_fim(Dev d, int blocosVerdade, i
 }
 // After a replacement: r = the true residual on water cells.
 __global__ void k_substituir(Dev d) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N || !d.esc->reiniciar || d.esc->pronto) return;
   if (d.tipo[c] == AGUA) d.r[c] = d.ap[c];
@@ -907,6 +922,7 @@ __global__ void k_substituir(Dev d) {
 // End of the solve: non-water q = 0; bubbles hand back their pressure (js/pressao-cpu.js:399-400).
 // Tolerance mode: q = the FP64 iterate rounded; the solve's convergence record (thread 0).
 __global__ void k_pcg_fim(Dev d, int bolhas, const double* q64, double tol) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (bolhas && c >= 2 && c < MAX_BOLHAS && d.facesB[c] > 0) d.yBolhaF[c] = (float)d.yB[c];
   if (c < d.N) {
@@ -1269,6 +1285,7 @@ int lerPerfilPcg(Pcg* p, unsigned long long* out, int cap) { return lerPerfilFun
 // One V-cycle on caller-provided device buffers (tq_vcycle).
 template <class T>
 __global__ void k_descarregar_x(const T* x0, float* x, int N) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < N) x[c] = carregar(x0[c]);
 }

@@ -54,6 +54,7 @@ struct Regioes : RegioesDev {  // the kernels take the pointers alone
 namespace {
 
 __global__ void k_reg_iniciar(RegioesDev R, const uint8_t* tipo) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < R.N) {
     R.pai[c] = tipo[c] == AGUA ? c : -1;
@@ -74,6 +75,7 @@ __global__ void k_reg_iniciar(RegioesDev R, const uint8_t* tipo) {
 // Active bubbles as k_bolhas_faces counts them: an interior air cell of the label with a water
 // neighbour.
 __global__ void k_reg_bolhas(RegioesDev R, Dev d) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N) return;
   const int nx = d.nx, i = c % nx, j = c / nx;
@@ -87,6 +89,7 @@ __global__ void k_reg_bolhas(RegioesDev R, Dev d) {
 // Water joins its water neighbours (left and down; the others join it) and the bubble node of
 // each active bubble it faces; any other air neighbour is Dirichlet (valorViz's 0).
 __global__ void k_reg_unir(RegioesDev R, Dev d, int bolhas) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.N || d.tipo[c] != AGUA) return;
   const int nx = d.nx, i = c % nx, j = c / nx;
@@ -110,18 +113,21 @@ __global__ void k_reg_unir(RegioesDev R, Dev d, int bolhas) {
 }
 
 __global__ void k_reg_achatar(RegioesDev R) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N + MAX_BOLHAS || R.pai[c] < 0) return;
   R.pai[c] = raizLeitura(R.pai, c);
 }
 
 __global__ void k_reg_abrir(RegioesDev R) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N || !R.toca[c]) return;
   R.aberto[R.pai[c]] = 1;
 }
 
 __global__ void k_reg_ids(RegioesDev R) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R.N || R.pai[c] != c) return;  // roots only (water cells)
   int id = -1;
@@ -140,6 +146,7 @@ __device__ inline int regiaoDe(const RegioesDev& R, int no) {
 }
 
 __global__ void k_reg_somar(RegioesDev R, Dev d, int bolhas) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < R.N && d.tipo[c] == AGUA) {
     const int id = regiaoDe(R, c);
@@ -158,6 +165,7 @@ __global__ void k_reg_somar(RegioesDev R, Dev d, int bolhas) {
 }
 
 __global__ void k_reg_projetar(RegioesDev R, Dev d, int bolhas) {
+  aposAnterior();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   auto media = [&](int id) { return R.soma[id] / (double)R.cont[id]; };
   if (c < R.N) {

@@ -200,10 +200,12 @@ int baixar(tq_sim* s, void* dst, const void* src, size_t bytes) {
 }
 
 __global__ void k_zerar_contagem(int2* acc, int n) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < n) acc[c].y = 0;
 }
 __global__ void k_gravar_contagem(int2* acc, const uint32_t* cnt, int n) {
+  aposAnterior();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < n) acc[c].y = (int)cnt[c];
 }
