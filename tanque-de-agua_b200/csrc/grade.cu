@@ -171,24 +171,37 @@ __global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
 }
 
 // ---------------------------------------------------------------- surface
-// #superficie (js/fisica-cpu.js:306-345) on one 32x32 tile a CTA, in shared memory: the water fraction of
+// #superficie (js/fisica-cpu.js:306-345) on one tile of 16x16 or 32x32 cells a CTA, in shared memory: the water fraction of
 // every cell, three times carried into the walls (#estenderNaParede, :353-374: three layers, each a
 // wall cell taking the mean of its neighbours that are no wall or were filled in an earlier layer) with
 // two separable (1 2 1)/4 blurs in between (:314-328), the normals grad f / |grad f| and the
 // curvature -div n / (2h) on the interior (:330-345; border cells are never written, they stay 0).  A
 // tile also computes the 13 cells around it that its result depends on, each stage needing one or
 // three fewer.  The 24 launches over the grid that this replaces took 105 us a substep on 160x100 cells,
-// where each waited for the one before, and 128 us on 840x536; this one takes 39 and 52 us.
-// The blurs walk a row or column a thread, so each value is converted to double once.
-constexpr int SUP_T = 32, SUP_H = 13, SUP_W = SUP_T + 2 * SUP_H, SUP_P = SUP_W + 1;  // odd pitch: no bank conflicts
-constexpr int SUP_THREADS = 256, SUP_SEG = 15;  // 4 segments of 15 cells a line
+// where each waited for the one before, and 128 us on 840x536.  What bounds it is the chain of its 20-odd
+// stages, each a meeting of the CTA: the wall cells of the three layers are listed once, so an extension
+// takes its own cells and not the whole region; the blurs walk a segment of a row or column a thread, so
+// each value is converted to double once; and a grid whose 16x16 tiles fill the GPU at most once
+// takes those (twice the cells around a tile, half the work of a CTA; with more tiles the larger
+// ones' fewer cells win).  160x100 cells: 35 us with 32x32 tiles of 256 threads that scanned the region
+// for each layer, 13 us now; 840x536: 48 -> 31 us.
+constexpr int SUP_H = 13, SUP_THREADS = 512, SUP_LINHAS = 64, SUP_SEGS = SUP_THREADS / SUP_LINHAS;
+constexpr int SUP_TILES = 592;  // 4 CTAs on each of 148 SMs
 constexpr uint8_t SUP_LIVRE = 0, SUP_FUNDO = 200, SUP_FORA = 255;  // marks: no wall; wall beyond layer 3; off the grid
 
+template <int SUP_T>
 __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
   aposAnterior();
+  constexpr int SUP_W = SUP_T + 2 * SUP_H, SUP_P = SUP_W + 1;  // odd pitch: no bank conflicts
+  constexpr int SUP_SEG = (SUP_W + SUP_SEGS - 1) / SUP_SEGS;   // cells of a line a thread blurs
+  static_assert(SUP_W <= SUP_LINHAS, "a thread a line");
   __shared__ float f[SUP_W * SUP_P], g[SUP_W * SUP_P];
   __shared__ uint8_t mk[SUP_W * SUP_P];  // SUP_LIVRE, the layer a wall cell is filled in (1-3), SUP_FUNDO, SUP_FORA
+  __shared__ uint16_t lista[SUP_W * SUP_W];  // the wall cells of layers 1, 2 and 3
+  __shared__ int nLista;
   const int nx = d.nx, ny = d.ny, x0 = blockIdx.x * SUP_T - SUP_H, y0 = blockIdx.y * SUP_T - SUP_H;
+  if (threadIdx.x == 0) nLista = 0;
+  bool parede = false;
   for (int t = threadIdx.x; t < SUP_W * SUP_W; t += SUP_THREADS) {
     const int i = t % SUP_W, j = t / SUP_W, gx = x0 + i, gy = y0 + j, o = j * SUP_P + i;
     float v = 0.0f;
@@ -199,31 +212,38 @@ __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
       // the initial water fraction (:309)
       const double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
       if (m == SUP_LIVRE) v = (float)fmin(1.0, dens / PARTICULAS_POR_CELULA);
+      else parede = true;
     }
     f[o] = v;
     g[o] = 0.0f;
     mk[o] = m;
   }
-  __syncthreads();
-  // the cells at least `b` inside the tile's region, one after the other over the threads
-  auto cada = [&](int b, auto fn) {
-    const int w = SUP_W - 2 * b;
-    for (int t = threadIdx.x; t < w * w; t += SUP_THREADS) fn((b + t / w) * SUP_P + b + t % w);
-  };
   // the layer each wall cell is filled in follows from the types alone: a wall cell beside a cell of
   // the layer before
-  for (int L = 1; L <= 3; L++) {
-    cada(L, [&](int o) {
-      if (mk[o] == SUP_FUNDO && (mk[o - 1] == L - 1 || mk[o + 1] == L - 1 || mk[o - SUP_P] == L - 1 || mk[o + SUP_P] == L - 1))
-        mk[o] = (uint8_t)L;
-    });
-    __syncthreads();
-  }
-  // one extension from the cells `b` inside on: layer L reads the layers before it
-  auto estender = [&](int b) {
+  int fim[4] = {0, 0, 0, 0};
+  if (__syncthreads_or(parede))
+#pragma unroll
     for (int L = 1; L <= 3; L++) {
-      cada(b + L, [&](int o) {
-        if (mk[o] != L) return;
+      const int w = SUP_W - 2 * L;
+      for (int t = threadIdx.x; t < w * w; t += SUP_THREADS) {
+        const int o = (L + t / w) * SUP_P + L + t % w;
+        if (mk[o] == SUP_FUNDO && (mk[o - 1] == L - 1 || mk[o + 1] == L - 1 || mk[o - SUP_P] == L - 1 || mk[o + SUP_P] == L - 1)) {
+          mk[o] = (uint8_t)L;
+          lista[atomicAdd(&nLista, 1)] = (uint16_t)o;
+        }
+      }
+      __syncthreads();
+      fim[L] = nLista;
+      __syncthreads();
+    }
+  // one extension: layer L reads the layers before it (cells nearer the region's edge than the stage
+  // reaches get values that nothing reads)
+  auto estender = [&] {
+#pragma unroll
+    for (int L = 1; L <= 3; L++) {
+      if (fim[L] == fim[L - 1]) continue;
+      for (int t = fim[L - 1] + threadIdx.x; t < fim[L]; t += SUP_THREADS) {
+        const int o = lista[t];
         double s = 0;
         int k = 0;
         const int nb[4] = {o - 1, o + 1, o - SUP_P, o + SUP_P};
@@ -234,11 +254,11 @@ __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
             k++;
           }
         f[o] = (float)(s / k);
-      });
+      }
       __syncthreads();
     }
   };
-  const int seg = threadIdx.x >> 6, linha = threadIdx.x & 63;
+  const int seg = threadIdx.x / SUP_LINHAS, linha = threadIdx.x % SUP_LINHAS;
   // blur of the cells `b` inside: rows into g, then columns back into f (b + 1 inside)
   auto borrar = [&](int b) {
     if (linha >= b && linha < SUP_W - b) {
@@ -266,11 +286,11 @@ __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
     }
     __syncthreads();
   };
-  estender(0);
+  estender();
   borrar(3);
-  estender(4);
+  estender();
   borrar(7);
-  estender(8);
+  estender();
   // f is done on the tile and 2 cells around it; the normals' components (g and h) on 1 cell around it
   __shared__ float h[(SUP_T + 2) * (SUP_T + 3)];
   constexpr int HP = SUP_T + 3;
@@ -532,7 +552,9 @@ void lancarTipos(const Dev& d, bool faces, float gdx, float gdy, bool ar, cudaSt
 }
 void lancarPropagarRotulos(const Dev& d, cudaStream_t s) { lanca(k_rotulos_resolver, 1, 1024, 0, s, d); }
 void lancarSuperficie(const Dev& d, cudaStream_t s) {
-  lanca(k_superficie, dim3(blocos(d.nx, SUP_T), blocos(d.ny, SUP_T)), SUP_THREADS, 0, s, d);
+  const dim3 pequenos(blocos(d.nx, 16), blocos(d.ny, 16));
+  if (pequenos.x * pequenos.y <= SUP_TILES) lanca(k_superficie<16>, pequenos, SUP_THREADS, 0, s, d);
+  else lanca(k_superficie<32>, dim3(blocos(d.nx, 32), blocos(d.ny, 32)), SUP_THREADS, 0, s, d);
 }
 void lancarLadoDireito(const Dev& d, double dt, double tensao, double tau, bool bolhas, cudaStream_t s) {
   // accB, facesB, celsB and volB are one block of memory

@@ -17,7 +17,7 @@ FLUTUANTES = {"u": 1e-4, "v": 1e-4, "q": 1e-4, "div": 1e-5, "fase": 1e-6, "curva
 
 
 @pytest.mark.parametrize("ar", [True, False], ids=["ar", "sem-ar"])
-@pytest.mark.parametrize("nx,ny", [(11, 9), (31, 33), (32, 32), (45, 64), (65, 31), (97, 66)], ids=str)
+@pytest.mark.parametrize("nx,ny", [(11, 9), (31, 33), (32, 32), (45, 64), (65, 31), (97, 66), (700, 240)], ids=str)
 def test_etapas_da_grade(lib_gpu, nx, ny, ar):
     h = 0.01
     cena_o, cena_g = CenaOraculo(nx, ny, h), Cena(nx, ny, h)
