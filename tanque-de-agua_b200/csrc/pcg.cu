@@ -190,11 +190,17 @@ __global__ void k_fonte(NivelDev<T> n0, Fonte F) {
 // repeat the one before (the last colour of a sweep is the first of the next, and a colour reads
 // only the other) are left out, 65 of 128.  8 us with a coarsest level of
 // 49 cells alone, 17 us for three levels from 943 cells, where six launches a level and the 42-46 us of
-// one CTA's 128 half-sweeps were.
+// one CTA's 128 half-sweeps were.  What a pass needs to know of a cell (where it is, which neighbours are
+// open, which lie in another block) is packed in a word once a launch for all levels together, and a
+// cell that does not change stores to a place of its own kind (FORA) instead of branching: with the
+// words made again in each pass (1,250 cycles of it, its half-sweeps 900 to 1,900) and the branches, three
+// levels from 1,000 cells took 22 us, 20 us now.
 constexpr int SECAO_PLANA = 1024, SECAO_PLANA_NIVEIS = 6, SECAO_PLANA_TOTAL = 1536, T_SECAO = 576;
+constexpr int SECAO_PARES = 1024;  // pairs of cells of all levels, each level's from a multiple of 32 on
 struct SecaoPlana {
   int L, uma;
-  int off[SECAO_PLANA_NIVEIS];
+  int off[SECAO_PLANA_NIVEIS + 1];  // a level's first cell; after the last level, their number
+  int par[SECAO_PLANA_NIVEIS + 1];  // a level's first pair
   NivelDev<float> n[SECAO_PLANA_NIVEIS];
   float* saida;
 };
@@ -209,45 +215,97 @@ __device__ __forceinline__ float dividirViz(float t, float k, float i) {
 __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
   aposAnterior();
   // one array, addressed by offsets: x, the snapshots, the right sides, and a 0 for closed neighbours
-  constexpr int S = SECAO_PLANA_TOTAL, B = 2 * SECAO_PLANA_TOTAL, ZERO = 3 * SECAO_PLANA_TOTAL;
-  __shared__ float X[ZERO + 1];
+  constexpr int S = SECAO_PLANA_TOTAL, B = 2 * SECAO_PLANA_TOTAL, ZERO = 3 * SECAO_PLANA_TOTAL, FORA = ZERO + 1;
+  __shared__ float X[ZERO + 2];
   __shared__ uint8_t V[SECAO_PLANA_TOTAL];
+  // a pair's cells (of colour 0, of colour 1): bits 0-10 the cell, 11-14 open neighbours, 15-18 and 19-22 those
+  // in another block at shift 0 and 8, 23 it changes
+  __shared__ uint2 D[SECAO_PARES];
   if (s.n[0].parar && *s.n[0].parar) return;
-  const int t = threadIdx.x, nt = blockDim.x;
-  for (int l = 0; l < s.L; l++) {
-    const int N = s.n[l].nx * s.n[l].ny, o = s.off[l];
-    for (int c = t; c < N; c += nt) {
-      V[o + c] = s.n[l].viz[c];
-      X[o + c] = X[S + o + c] = 0.0f;  // a pass takes the snapshots of the cells that change alone
-      if (l == 0) X[B + o + c] = s.n[0].b[c];
+  // the levels' sizes, first cells and first pairs: a load from the arguments by a level's number takes several
+  // times one from shared memory
+  __shared__ int NX[SECAO_PLANA_NIVEIS], NY[SECAO_PLANA_NIVEIS], OFF[SECAO_PLANA_NIVEIS + 1], PAR[SECAO_PLANA_NIVEIS + 1];
+  const int t = threadIdx.x, nt = blockDim.x, total = s.off[s.L];
+  if (t <= s.L) {
+    OFF[t] = s.off[t];
+    PAR[t] = s.par[t];
+    if (t < s.L) {
+      NX[t] = s.n[t].nx;
+      NY[t] = s.n[t].ny;
+    }
+  }
+  auto nivelDe = [&](const int* inicio, int k) {
+    int l = 0;
+    while (l + 1 < s.L && k >= inicio[l + 1]) l++;
+    return l;
+  };
+  for (int k0 = t; k0 < total; k0 += 3 * nt) {  // every load of the three out before its store
+    uint8_t v[3];
+    float b[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const int k = k0 + q * nt;
+      v[q] = 0;
+      b[q] = 0.0f;
+      if (k < total) {
+        const int l = nivelDe(s.off, k);
+        v[q] = s.n[l].viz[k - s.off[l]];
+        if (l == 0) b[q] = s.n[0].b[k];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const int k = k0 + q * nt;
+      if (k < total) {
+        V[k] = v[q];
+        X[k] = X[S + k] = 0.0f;  // a pass takes the snapshots of the cells that change alone
+        X[B + k] = b[q];
+      }
     }
   }
   if (t == 0) X[ZERO] = 0.0f;
   __syncthreads();
+  for (int k = t; k < PAR[s.L]; k += nt) {
+    const int l = nivelDe(PAR, k), nx = NX[l], ny = NY[l], hw = (nx + 1) >> 1, r = k - PAR[l], j = r / hw;
+    unsigned w[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int i = 2 * (r - j * hw) + ((e + 1 + j) & 1);
+      w[e] = 0;
+      if (j < ny && i < nx) {
+        const int c = OFF[l] + i + j * nx, vz = V[c];
+        const int i8 = (i + 8) & 15, j8 = (j + 8) & 15, i0 = i & 15, j0 = j & 15;
+        w[e] = c | (vz & 15) << 11 | ((i0 == 0) | (i0 == 15) << 1 | (j0 == 0) << 2 | (j0 == 15) << 3) << 15 |
+               ((i8 == 0) | (i8 == 15) << 1 | (j8 == 0) << 2 | (j8 == 15) << 3) << 19 |
+               ((vz & 16) && (vz & 15) ? 1u << 23 : 0u);
+      }
+    }
+    D[k] = make_uint2(w[0], w[1]);
+  }
+  __syncthreads();
   const float pes[4] = {0.25f, 0.75f, 0.75f, 0.25f};
-  // The thread's two cells of a level (cells 2s and 2s + 1 of a row, colour e ^ ordem at [e]): index
-  // (-1: none that changes), neighbours, free neighbours, right side.
+  // The thread's two cells of a level, colour e ^ ordem at [e]: where it stores (FORA: it does not change),
+  // neighbours, free neighbours, right side.
   struct Par {
     int c[2], v[2][4], k[2];
     float b[2];
   };
-  auto threads = [&](int l) { return (((s.n[l].nx + 1) >> 1) * s.n[l].ny + 31) & ~31; };
+  auto threads = [&](int l) { return PAR[l + 1] - PAR[l]; };
   auto par = [&](int l, int ordem, int desl, bool blocos) {  // desl: the blocks' shift; blocos: snapshots
     Par p;
-    const int nx = s.n[l].nx, ny = s.n[l].ny, hw = (nx + 1) >> 1, o = s.off[l], j = t / hw;
+    const int nx = NX[l];
+    const uint2 d = D[PAR[l] + t];
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-      const int i = 2 * (t % hw) + (((e ^ ordem) + 1 + j) & 1);
-      const bool dentro = j < ny && i < nx;
-      const int c = dentro ? o + i + j * nx : o, vz = dentro ? V[c] : 0, mk = vz & 15;
-      const int bi = (i + desl) & 15, bj = (j + desl) & 15;
+      const unsigned w = e ^ ordem ? d.y : d.x, fora = blocos ? w >> (desl ? 19 : 15) : 0u;
+      const int c = w & 0x7ff;
       // a neighbour of the cell's block is read as swept, one outside it from the snapshot
-      p.c[e] = (vz & 16) && mk ? c : -1;
-      p.v[e][0] = !(mk & 1) ? ZERO : (blocos && bi == 0 ? S : 0) + c - 1;
-      p.v[e][1] = !(mk & 2) ? ZERO : (blocos && bi == 15 ? S : 0) + c + 1;
-      p.v[e][2] = !(mk & 4) ? ZERO : (blocos && bj == 0 ? S : 0) + c - nx;
-      p.v[e][3] = !(mk & 8) ? ZERO : (blocos && bj == 15 ? S : 0) + c + nx;
-      p.k[e] = __popc(mk);
+      p.c[e] = w >> 23 & 1 ? c : FORA;
+      p.v[e][0] = w >> 11 & 1 ? c - 1 + (fora & 1 ? S : 0) : ZERO;
+      p.v[e][1] = w >> 12 & 1 ? c + 1 + (fora & 2 ? S : 0) : ZERO;
+      p.v[e][2] = w >> 13 & 1 ? c - nx + (fora & 4 ? S : 0) : ZERO;
+      p.v[e][3] = w >> 14 & 1 ? c + nx + (fora & 8 ? S : 0) : ZERO;
+      p.k[e] = __popc(w >> 11 & 15);
       p.b[e] = X[B + c];
     }
     return p;
@@ -264,9 +322,9 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
     float q[2], iq[2];
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-      q[e] = p.c[e] >= 0 ? X[p.c[e]] : 0.0f;
+      q[e] = p.c[e] != FORA ? X[p.c[e]] : 0.0f;
       iq[e] = inversoVizinhos(p.k[e]);
-      if (p.c[e] >= 0) X[S + p.c[e]] = q[e];
+      if (p.c[e] != FORA) X[S + p.c[e]] = q[e];
     }
     sinc(n);
 #pragma unroll 1
@@ -275,7 +333,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
       for (int e = 0; e < 2; e++) {
         const float sm = ((X[p.v[e][0]] + X[p.v[e][1]]) + X[p.v[e][2]]) + X[p.v[e][3]];
         q[e] = q[e] + fmaf(sm + p.b[e], iq[e], -q[e]);
-        if (p.c[e] >= 0) X[p.c[e]] = q[e];
+        X[p.c[e]] = q[e];
         sinc(n);
       }
   };
@@ -285,7 +343,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
       __syncthreads();
     }
     passo(l, 8, 0);
-    const int nx = s.n[l].nx, ny = s.n[l].ny, N = nx * ny, o = s.off[l];
+    const int nx = NX[l], ny = NY[l], N = nx * ny, o = OFF[l];
     __syncthreads();
     for (int k = t; k < N; k += nt) {  // residuals into the snapshot array
       const int c = o + k, vz = V[c];
@@ -297,7 +355,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
       X[S + c] = (vz & 16) ? X[B + c] - fmaf((float)__popc(vz & 15), X[c], -sm) : 0.0f;
     }
     __syncthreads();
-    const int gx = s.n[l + 1].nx, G = gx * s.n[l + 1].ny, og = s.off[l + 1];
+    const int gx = NX[l + 1], G = gx * NY[l + 1], og = OFF[l + 1];
     for (int C = t; C < G; C += nt) {
       const int I = C % gx, J = C / gx;
       float sm = 0.0f;
@@ -323,7 +381,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
       auto meia = [&](auto E) {
         constexpr int e = decltype(E)::value;
         const float sm = ((X[p.v[e][0]] + X[p.v[e][1]]) + X[p.v[e][2]]) + X[p.v[e][3]];
-        if (p.c[e] >= 0) X[p.c[e]] = dividirViz(sm + p.b[e], kf[e], iq[e]);
+        X[p.c[e]] = dividirViz(sm + p.b[e], kf[e], iq[e]);
         sinc(n);
       };
 #pragma unroll 1
@@ -336,8 +394,8 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
     __syncthreads();
   }
   for (int l = s.L - 2; l >= 0; l--) {
-    const int nx = s.n[l].nx, N = nx * s.n[l].ny, o = s.off[l];
-    const int gx = s.n[l + 1].nx, gy = s.n[l + 1].ny, og = s.off[l + 1];
+    const int nx = NX[l], N = nx * NY[l], o = OFF[l];
+    const int gx = NX[l + 1], gy = NY[l + 1], og = OFF[l + 1];
     for (int k = t; k < N; k += nt) {
       if (!(V[o + k] & 16)) continue;
       const int i = k % nx, j = k / nx, I0 = grossoBaseF(i), J0 = grossoBaseF(j);
@@ -361,7 +419,7 @@ __global__ void __launch_bounds__(T_SECAO) k_secao(SecaoPlana s) {
       __syncthreads();
     }
   }
-  for (int c = t; c < s.n[0].nx * s.n[0].ny; c += nt) s.saida[c] = X[c];
+  for (int c = t; c < NX[0] * NY[0]; c += nt) s.saida[c] = X[c];
 }
 
 // resolverGrosso (js/pressao-cpu.js:217-238): VARREDURAS_GROSSO alternating red-black sweeps
@@ -1148,11 +1206,12 @@ static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bo
                           const Juncao* J) {
   const int L = p->L;
   // the section: the coarse levels of at most SECAO_PLANA cells (not level 0)
-  int Ls = L, total = 0;
+  int Ls = L, total = 0, pares = 0;
+  auto paresDe = [&](int l) { return (((p->nxL[l] + 1) / 2) * p->nyL[l] + 31) & ~31; };
   while (Ls > 1 && L - Ls < SECAO_PLANA_NIVEIS && p->nxL[Ls - 1] * p->nyL[Ls - 1] <= SECAO_PLANA &&
          ((p->nxL[Ls - 1] + 1) / 2) * p->nyL[Ls - 1] <= T_SECAO &&
-         total + p->nxL[Ls - 1] * p->nyL[Ls - 1] <= SECAO_PLANA_TOTAL)
-    Ls--, total += p->nxL[Ls] * p->nyL[Ls];
+         total + p->nxL[Ls - 1] * p->nyL[Ls - 1] <= SECAO_PLANA_TOTAL && pares + paresDe(Ls - 1) <= SECAO_PARES)
+    Ls--, total += p->nxL[Ls] * p->nyL[Ls], pares += paresDe(Ls);
   const int Lf = Ls < L ? Ls : L - 1;  // the levels with tile legs: 0 .. Lf - 1
   for (int l = 0; l < Lf; l++) descerNivel(p, l, bloco, umaPassada, F, s);
   const void* x;
@@ -1160,15 +1219,14 @@ static const void* cicloV(Pcg* p, const Fonte& F, cudaStream_t s, bool bloco, bo
     SecaoPlana sp{};
     sp.L = L - Ls;
     sp.uma = umaPassada ? 1 : 0;
-    int off = 0;
     for (int l = Ls; l < L; l++) {
       sp.n[l - Ls] = nivel<float>(p, l);
-      sp.off[l - Ls] = off;
-      off += p->nxL[l] * p->nyL[l];
+      sp.off[l - Ls + 1] = sp.off[l - Ls] + p->nxL[l] * p->nyL[l];
+      sp.par[l - Ls + 1] = sp.par[l - Ls] + paresDe(l);
     }
     sp.saida = (float*)p->tmpL[Ls];
     x = sp.saida;
-    lanca(k_secao, 1, (((p->nxL[Ls] + 1) / 2) * p->nyL[Ls] + 31) & ~31, 0, s, sp);
+    lanca(k_secao, 1, paresDe(Ls), 0, s, sp);
   } else {
     comTipo(p, L - 1, [&](auto* t) {
       using T = std::remove_pointer_t<decltype(t)>;
