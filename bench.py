@@ -15,7 +15,7 @@ FP64), with an iteration cap of 1000; each arm reports the fraction of its solve
 and the largest true relative residual.  `value` is the mixed-precision configuration (fused
 engine, FP16 V-cycle storage, block preconditioner, frames replayed from a CUDA graph) timed on
 the device, the faucet's particles made on the device each frame (tq_emit_faucet); `fp32_fused` is the
-same engine with FP32 storage; `fp32_plain` is the one-launch-per-step FP32 engine with the
+same engine with FP32 storage; `fp32_plain` is the FP32 engine of separate launches with the
 reference's preconditioner (the reference's algorithm on the GPU); `e2e` is the mixed
 configuration through the C-ABI with host buffers (faucet particles in, every particle out, each
 frame; the device-timed arms make the same jet on the device, tq_emit_faucet).  --impl reference
@@ -389,7 +389,7 @@ def executar_gpu(args, rank, mundo, dist):
         "fp32_plain": {"value": round(valor_plano, 2), "unit": "steps/s", "solve": plano["solve"],
                        "mgpcg_gbs": round(r_p["gbs"], 1), "pcg_iters": round(r_p["iters"], 2),
                        "ms_solve": round(r_p["ms_solve"], 4),
-                       "engine": "plain (one launch per reference dispatch), reference preconditioner"},
+                       "engine": "plain (a loop of launches, three kernels and a V-cycle an iteration), reference preconditioner"},
         "stages_ms_per_substep": {k: round(misto_etapas["etapas"][k] / max(misto_etapas["etapas"]["subpassos"], 1), 4)
                                   for k in SimulacaoGPU.ETAPAS},
         "particle_stages": particulas_gbs(misto_etapas, misto["particulas"], hbm),

@@ -44,8 +44,8 @@ extern "C" {
 #define TQ_PREC_BF16 2
 
 /* Execution engine of the pressure solve.
- * PLAIN: one kernel launch per reference dispatch (the decomposition of js/gpu/pcg.js and
- *        js/gpu/multigrid.js), host-driven iteration loop.
+ * PLAIN: a loop of launches driven by the host: three kernels and a V-cycle an iteration, the
+ *        V-cycle one launch for each leg of a level and one for the coarse levels.
  * FUSED: the whole MGPCG solve in one persistent cooperative kernel with bounded grid
  *        barriers; the coarse levels run inside one CTA's shared memory. */
 #define TQ_ENGINE_PLAIN 0

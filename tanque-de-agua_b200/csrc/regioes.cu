@@ -72,7 +72,7 @@ __global__ void k_reg_iniciar(RegioesDev R, const uint8_t* tipo) {
   if (c < 2) R.cont[MAX_REGIOES + c] = 0;
 }
 
-// Active bubbles as k_bolhas_faces counts them: an interior air cell of the label with a water
+// Active bubbles as the solvers count them: an interior air cell of the label with a water
 // neighbour.
 __global__ void k_reg_bolhas(RegioesDev R, Dev d) {
   aposAnterior();

@@ -122,7 +122,7 @@ __device__ __forceinline__ void varrerReg(float (&x)[2][4], const int (&v)[2][4]
 // CTAs.  That trades sweeps (on the way down (k+2)^2 + (k+1)^2 blocks instead of 2 k^2, up
 // (k+1)^2 + k^2) for launches: one a leg instead of three, which bound these levels: the plain
 // engine's V-cycle (tq_vcycle_noalloc, FP32) went from 182 to 65 us on 160x100 cells, 282 to
-// 130 us on 840x536, bits unchanged.
+// 130 us on 840x536 (111 since the launches overlap), bits unchanged.
 //
 // Shared arrays hold the cells from (fx0 - 10, fy0 - 10) on, H rows of pitch P = 16 kx + 20 (4 mod
 // 8: a warp's 64-bit accesses of four rows of a block then meet no bank twice).
