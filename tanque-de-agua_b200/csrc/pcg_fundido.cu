@@ -80,7 +80,6 @@ constexpr int SUAV_W = CT + 7;                     // the coarse tile of a PROL 
 // per-bubble tables a CTA keeps in its areas between two grid barriers ([DA]: two doubles a label)
 constexpr size_t AREA_BOLHAS = (size_t)MAX_BOLHAS * 16;
 constexpr size_t AREA_TERMOS = (size_t)(TF - 32) * 16;  // after them, terms of a sum over the bubbles
-constexpr size_t AREA_PRODUTOS = (size_t)4 * (TF + 4) * 8;  // and a batch's products
 
 struct NivelF {
   int nx, ny, meia, pad;
@@ -1665,56 +1664,33 @@ __device__ __forceinline__ float aplicarF(const Args& a, int c, FV val, FB valB)
   return (float)__popc(vz & 15) * val(c) - s;
 }
 
-constexpr int KDA = 4;  // cells a thread and batch of the true residual
+// A hint to bring the line into L1.
+__device__ __forceinline__ void paraL1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+constexpr int KDA = 4;  // cells a thread and batch of [DA], [B] and the true residual
 
 // [DA] of a PCG iteration over this CTA's cells: beta, p = z + beta p (z alone on the first
 // iteration), A p (js/pressao-cpu.js:84-93, bubble neighbours through their p), the partial of
-// p.Ap (channel 0) and, for air of active bubbles, the sums over their water faces.  Bound by the
-// latency of its loads and by the fetch of its code, which a phase enters cold: cells go in batches of
-// K a thread with every load ahead, left and right neighbours by shuffle (a warp's cells are
-// consecutive), the first batch's loads out before the global sums that make beta; the bubbles' z and
-// previous p wait in shared memory (areas), put there by the warps that do not sum, and the faces of
-// bubble air, the only FP64 sums with atomics, are a rolled loop over the cells that have them.
+// p.Ap (channel 2) and, for air of active bubbles, the sums over their water faces.  Bound by the
+// latency of its loads: cells go in batches of KDA a thread, a stride of the grid apart, with every load
+// ahead; the left and right neighbours come by shuffle (a warp's cells are consecutive).  The first
+// batch's lines are on their way to L1 while the global sums behind beta are made (a hint, as values
+// held in registers across the sums cost spills); the bubbles' z and previous p wait in shared memory
+// (areas), put there by the warps that do not sum.
 // z and p come through L1: they were last written before the grid barrier that opens this phase,
 // whose acquire orders these loads after those writes.
-// Measured: 13.8 -> 10.9 us a phase on 840x536 cells, 8.7 -> 7.3 on 480x270; [B], built alike, keeps its
-// 6.3 to 7.6 us (it now makes the sums behind alpha under its loads).
-// A CTA's cells in [DA] and [B]: TF consecutive ones, then those GT further on, and so on; a batch is 4 such
-// runs, a thread 4 consecutive cells of one of them (a float4 an array).  Each thread then sums the
-// products of cell threadIdx.x of the 4 runs, passed through shared memory.
-constexpr int QUARTO = TF / 4;
-struct Quatro {
-  float v[4];
-};
-// Cells c .. c + 3 of an array (al: c is a multiple of 4 here), 0 outside 0 .. N - 1.
-__device__ __forceinline__ Quatro lerQuatro(const float* p, int c, int N, bool al) {
-  Quatro q;
-  if (al && c >= 0 && c + 3 < N) {
-    const float4 f = __ldca((const float4*)(p + c));
-    q.v[0] = f.x, q.v[1] = f.y, q.v[2] = f.z, q.v[3] = f.w;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++) q.v[k] = c + k >= 0 && c + k < N ? __ldca(p + c + k) : 0.0f;
-  }
-  return q;
-}
-__device__ __forceinline__ void lerOps(const uint16_t* op, int c, int N, int (&m)[4]) {
-  if (c + 3 < N) {
-    const uint2 u = __ldcg((const uint2*)(op + c));
-    m[0] = u.x & 0xffff, m[1] = u.x >> 16, m[2] = u.y & 0xffff, m[3] = u.y >> 16;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++) m[k] = c + k < N ? __ldcg(op + c + k) : 0;
-  }
-}
+// Measured, [DA] / [B] a phase, against four consecutive cells a thread whose products the CTA passed on
+// through shared memory: 480x270 cells 6.0 / 4.9 -> 5.9 / 4.1 us, 840x536 9.0 / 6.9 -> 8.2 / 5.0,
+// 7,221x316 40 / 31 -> 28 / 18, 38,370x316 217 / 166 -> 119 / 83 (an iteration 984 -> 807).  Direct loads of the left
+// and right neighbours: 126 us on the last, 8.5 on 840x536; the lines of the next batch ahead as well: 122
+// and 8.7.
 __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const float* pv, float* pn, bool prim, int nAt,
-                                    const double* pbVelho, double* pbNovo, const double* zbOld, double* zbCur,
-                                    double& rz, double* sh, float* areas) {
+                                       const double* pbVelho, double* pbNovo, const double* zbOld, double* zbCur,
+                                       double& rz, double* sh, float* areas) {
   const Dev& d = a.d;
   const int N = d.N, nx = d.nx, lane = threadIdx.x & 31, GT = gridDim.x * TF;
   double* zbS = (double*)areas;
   double* pbS = zbS + MAX_BOLHAS;
-  float2* pares = (float2*)(areas + (AREA_BOLHAS + AREA_TERMOS) / 4);  // p and A p of the batch's cells
   auto bolha = [&](int b) {
     zbS[b] = zbDe(a, b);
     if (!prim) pbS[b] = __ldcg(&pbVelho[b]);
@@ -1741,65 +1717,50 @@ __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const flo
     beta = fabs(rz) < 1e-30 ? 0.0 : fmax(0.0, (rzNovo - cruz) / rz);
     rz = rzNovo;
   };
-  const int b0 = blockIdx.x * TF, run = threadIdx.x / QUARTO, pos = threadIdx.x % QUARTO * 4;
-  const bool al = (nx & 3) == 0;
-#pragma unroll 1
-  for (int base = b0; base == b0 || base < N; base += 4 * GT) {
-    // the cells, those below and above (an index across a row's end reads a value that no flag selects),
-    // lane 0's to the left and lane 31's to the right
-    const int c0 = base + run * GT + pos;
-    int m[4];
-    lerOps(a.op, c0, N, m);
-    Quatro z[3], w[3];
-    float zl = 0.0f, wl = 0.0f;
-    const int cl = lane == 0 ? c0 - 1 : c0 + 4;
-    z[0] = lerQuatro(zc, c0, N, true);
-    z[1] = lerQuatro(zc, c0 - nx, N, al);
-    z[2] = lerQuatro(zc, c0 + nx, N, al);
-    if ((lane == 0 || lane == 31) && cl >= 0 && cl < N) zl = __ldca(zc + cl);
-    if (!prim) {
-      w[0] = lerQuatro(pv, c0, N, true);
-      w[1] = lerQuatro(pv, c0 - nx, N, al);
-      w[2] = lerQuatro(pv, c0 + nx, N, al);
-      if ((lane == 0 || lane == 31) && cl >= 0 && cl < N) wl = __ldca(pv + cl);
-    }
-    if (base == b0) {
-      somar();
-      if (blockIdx.x == 0)
-#pragma unroll 1
-        for (int k = threadIdx.x; k < nAt; k += TF) {
-          const int b = __ldcg(&a.ativos[k]);
-          zbCur[b] = zbS[b];
-          pbNovo[b] = pbNovoV(b);
-        }
-    }
-    const float betaf = (float)beta;
-    // the packed labels, only where a bubble's p or row needs them
-    unsigned long long rl[4];
+  int m[KDA];
+  float z[KDA][3], w[KDA][3], zl[KDA], wl[KDA];
+  // a batch's cells, those below and above (an index across a row's end reads a value that no flag selects),
+  // and one beside the cell: lane 31's to the right, the others' to the left (of which lane 0's counts; a
+  // branch would wait for its load)
+  auto ler = [&](int c0) {
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      rl[k] = (m[k] & OP_VIZ_BOLHA) || ((m[k] & OP_FACE) && (m[k] & 15)) ? __ldcg(a.rotB + c0 + k) : 0ull;
-    if (!prim) {
+    for (int k = 0; k < KDA; k++) m[k] = c0 + k * GT < N ? __ldca(a.op + c0 + k * GT) : 0;
 #pragma unroll
-      for (int q = 0; q < 3; q++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) z[q].v[k] = z[q].v[k] + betaf * w[q].v[k];
-      zl = zl + betaf * wl;
+    for (int k = 0; k < KDA; k++) {
+      const int c = c0 + k * GT < N ? c0 + k * GT : 0;
+      z[k][0] = __ldca(zc + c);
+      z[k][1] = __ldca(zc + (c >= nx ? c - nx : c));
+      z[k][2] = __ldca(zc + (c < N - nx ? c + nx : c));
+      zl[k] = __ldca(zc + (lane == 31 ? min(c + 1, N - 1) : max(c - 1, 0)));
     }
-    const float ze = __shfl_up_sync(0xffffffffu, z[0].v[3], 1), zd = __shfl_down_sync(0xffffffffu, z[0].v[0], 1);
-    const float esq = lane == 0 ? zl : ze, dir = lane == 31 ? zl : zd;
+    if (!prim)
+#pragma unroll
+      for (int k = 0; k < KDA; k++) {
+        const int c = c0 + k * GT < N ? c0 + k * GT : 0;
+        w[k][0] = __ldca(pv + c);
+        w[k][1] = __ldca(pv + (c >= nx ? c - nx : c));
+        w[k][2] = __ldca(pv + (c < N - nx ? c + nx : c));
+        wl[k] = __ldca(pv + (lane == 31 ? min(c + 1, N - 1) : max(c - 1, 0)));
+      }
+  };
+  float betaf = 0.0f;
+  auto fazer = [&](int c0) {
+    unsigned long long rl[KDA];
+#pragma unroll
+    for (int k = 0; k < KDA; k++)
+      rl[k] = (m[k] & OP_VIZ_BOLHA) || ((m[k] & OP_FACE) && (m[k] & 15)) ? __ldcg(a.rotB + c0 + k * GT) : 0ull;
     int labA = 0;
     long long acc = 0;
-    float ap[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int mk = m[k];
-      const float p = z[0].v[k];
-      // left, right, down, up: 0 where no water is
-      float pq[4] = {k ? z[0].v[k ? k - 1 : 0] : esq, k < 3 ? z[0].v[k < 3 ? k + 1 : 3] : dir, z[1].v[k], z[2].v[k]};
+    for (int k = 0; k < KDA; k++) {
+      const int mk = m[k], c = c0 + k * GT;
+      const float p = prim ? z[k][0] : z[k][0] + betaf * w[k][0];
+      const float pl = prim ? zl[k] : zl[k] + betaf * wl[k];
+      const float pe = __shfl_up_sync(0xffffffffu, p, 1), pd = __shfl_down_sync(0xffffffffu, p, 1);
+      float pq[4] = {lane == 0 ? pl : pe, lane == 31 ? pl : pd, prim ? z[k][1] : z[k][1] + betaf * w[k][1],
+                     prim ? z[k][2] : z[k][2] + betaf * w[k][2]};
 #pragma unroll
       for (int q = 0; q < 4; q++) pq[q] = (mk >> q) & 1 ? pq[q] : 0.0f;
-      ap[k] = 0.0f;
       if (mk & OP_AGUA) {
         if (mk & OP_VIZ_BOLHA)  // a neighbour that is air of an active bubble contributes that bubble's p
 #pragma unroll
@@ -1807,7 +1768,10 @@ __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const flo
             const int b = (int)(rl[k] >> (12 + 12 * q)) & 0xfff;
             if (b && !((mk >> q) & 1)) pq[q] = (float)pbNovoV(b);
           }
-        ap[k] = (float)(mk >> 8) * p - (((pq[0] + pq[1]) + pq[2]) + pq[3]);
+        const float ap = (float)(mk >> 8) * p - (((pq[0] + pq[1]) + pq[2]) + pq[3]);
+        pn[c] = p;
+        d.ap[c] = ap;
+        s += (double)p * ap;
       } else if ((mk & OP_FACE) && (mk & 15)) {
         // (p and Ap off water are never read) the bubble's row: the sum of p over its water faces
         const double f = (((double)pq[0] + (double)pq[1]) + (double)pq[2]) + (double)pq[3];
@@ -1820,32 +1784,31 @@ __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const flo
         acc += __double2ll_rn(f * ESC);
       }
     }
-    if ((m[0] | m[1] | m[2] | m[3]) & OP_AGUA) {
-      if (c0 + 3 < N) {
-        *(float4*)(pn + c0) = make_float4(z[0].v[0], z[0].v[1], z[0].v[2], z[0].v[3]);
-        *(float4*)(d.ap + c0) = make_float4(ap[0], ap[1], ap[2], ap[3]);
-      } else {
+    if (__any_sync(0xffffffffu, labA)) somarBolhaWarp((long long*)d.accB, labA, acc);
+  };
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-          if (c0 + k < N) {
-            pn[c0 + k] = z[0].v[k];
-            d.ap[c0 + k] = ap[k];
-          }
-      }
+  for (int k = 0; k < KDA; k++) {
+    const int c = blockIdx.x * TF + threadIdx.x + k * GT;
+    if (c < N) {
+      paraL1(a.op + c);
+      paraL1(zc + c), paraL1(zc + max(c - nx, 0)), paraL1(zc + min(c + nx, N - 1));
+      if (!prim) paraL1(pv + c), paraL1(pv + max(c - nx, 0)), paraL1(pv + min(c + nx, N - 1));
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {  // (a row of the table has one float2 more: no bank twice)
-      const bool agua = (m[k] & OP_AGUA) != 0;
-      pares[k * (TF + 4) + run * QUARTO + pos / 4] = agua ? make_float2(z[0].v[k], ap[k]) : make_float2(0.0f, 0.0f);
+  }
+  somar();
+  betaf = (float)beta;
+  if (blockIdx.x == 0)
+#pragma unroll 1
+    for (int k = threadIdx.x; k < nAt; k += TF) {
+      const int b = __ldcg(&a.ativos[k]);
+      zbCur[b] = zbS[b];
+      pbNovo[b] = pbNovoV(b);
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; k++) {  // cell threadIdx.x of run k
-      const float2 t = pares[(threadIdx.x & 3) * (TF + 4) + k * QUARTO + (threadIdx.x >> 2)];
-      s += (double)t.x * t.y;
-    }
-    if (base + 4 * GT < N) __syncthreads();
-    if (a.bolhas) somarBolhaWarp((long long*)d.accB, labA, acc);
+#pragma unroll 1
+  for (int base = blockIdx.x * TF; base < N; base += KDA * GT) {
+    const int c0 = base + threadIdx.x;
+    ler(c0);
+    fazer(c0);
   }
   const double tb = somaBloco(s, sh);
   if (threadIdx.x == 0) a.parc[blockIdx.x * NPARC + 2] = tb;
@@ -2308,74 +2271,36 @@ __global__ void __launch_bounds__(TF, 1) k_mgpcg(const __grid_constant__ Args a)
     };
     double alfa;
     {
+      somasGlobais<false, 2>(a, nAt, [&](int b, double& t, double&) { t = __ldcg(&pbNovo[b]) * apbV(b); }, sh, somas, areas);
+      const double pap = somas[0] + somas[2];
+      alfa = fabs(pap) < 1e-30 ? 0.0 : rz / pap;
+      const float af = (float)alfa;
       double s = 0;
-      float af = 0.0f;
-      // the cells as in [DA]; all loads of a batch first
-      const int b0 = blockIdx.x * TF, run = threadIdx.x / QUARTO, pos = threadIdx.x % QUARTO * 4;
-      float* rsS = areas + (AREA_BOLHAS + AREA_TERMOS) / 4;
 #pragma unroll 1
-      for (int base = b0; base == b0 || base < N; base += 4 * GT) {
-        const int c0 = base + run * GT + pos;
-        const bool todo = c0 + 3 < N;
-        int m[4];
-        lerOps(a.op, c0, N, m);
-        Quatro pq = lerQuatro(pn, c0, N, true), rq = lerQuatro(d.r, c0, N, true), aq = lerQuatro(d.ap, c0, N, true), qq;
-        double qd[4];
-        if (a.q64) {
-          if (todo) {
-            const double2 u = __ldcg((const double2*)(a.q64 + c0)), v = __ldcg((const double2*)(a.q64 + c0 + 2));
-            qd[0] = u.x, qd[1] = u.y, qd[2] = v.x, qd[3] = v.y;
-          } else {
+      for (int c0 = gt0; c0 < N; c0 += KDA * GT) {  // all loads of a batch first
+        int m[KDA];
+        float qv[KDA], pnv[KDA], rv[KDA], apv[KDA];
+        double qd[KDA];
 #pragma unroll
-            for (int k = 0; k < 4; k++) qd[k] = c0 + k < N ? __ldcg(a.q64 + c0 + k) : 0.0;
-          }
-        } else {
-          qq = lerQuatro(d.q, c0, N, true);
+        for (int k = 0; k < KDA; k++) {
+          const int c = c0 + k * GT < N ? c0 + k * GT : 0;
+          m[k] = c0 + k * GT < N ? __ldcg(a.op + c) : 0;
+          if (a.q64) qd[k] = __ldcg(a.q64 + c);
+          else qv[k] = __ldcg(d.q + c);
+          pnv[k] = __ldcg(pn + c);
+          rv[k] = __ldcg(d.r + c);
+          apv[k] = __ldcg(d.ap + c);
         }
-        if (base == b0) {  // the first batch's loads are under way: the sums that make alpha
-          somasGlobais<false, 2>(a, nAt, [&](int b, double& t, double&) { t = __ldcg(&pbNovo[b]) * apbV(b); }, sh, somas,
-                              areas);
-          const double pap = somas[0] + somas[2];
-          alfa = fabs(pap) < 1e-30 ? 0.0 : rz / pap;
-          af = (float)alfa;
-        }
-        const bool alguma = (m[0] | m[1] | m[2] | m[3]) & OP_AGUA;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const bool agua = m[k] & OP_AGUA;
-          if (agua) {
-            if (a.q64) qd[k] = qd[k] + alfa * (double)pq.v[k];
-            else qq.v[k] = qq.v[k] + af * pq.v[k];
-            rq.v[k] = rq.v[k] - af * aq.v[k];
-          }
-          rsS[k * (TF + 4) + run * QUARTO + pos / 4] = agua ? rq.v[k] : 0.0f;
-        }
-        if (alguma) {  // (cells off water get back what they held)
-          if (todo) {
-            *(float4*)(d.r + c0) = make_float4(rq.v[0], rq.v[1], rq.v[2], rq.v[3]);
-            if (a.q64) {
-              *(double2*)(a.q64 + c0) = make_double2(qd[0], qd[1]);
-              *(double2*)(a.q64 + c0 + 2) = make_double2(qd[2], qd[3]);
-            } else {
-              *(float4*)(d.q + c0) = make_float4(qq.v[0], qq.v[1], qq.v[2], qq.v[3]);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              if (c0 + k < N) {
-                d.r[c0 + k] = rq.v[k];
-                if (a.q64) a.q64[c0 + k] = qd[k];
-                else d.q[c0 + k] = qq.v[k];
-              }
-          }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 4; k++) {  // cell threadIdx.x of run k
-          const float r = rsS[(threadIdx.x & 3) * (TF + 4) + k * QUARTO + (threadIdx.x >> 2)];
+        for (int k = 0; k < KDA; k++) {
+          if (!(m[k] & OP_AGUA)) continue;
+          const int c = c0 + k * GT;
+          if (a.q64) a.q64[c] = qd[k] + alfa * (double)pnv[k];
+          else d.q[c] = qv[k] + af * pnv[k];
+          const float r = rv[k] - af * apv[k];
+          d.r[c] = r;
           s += (double)r * r;
         }
-        if (base + 4 * GT < N) __syncthreads();
       }
       if (blockIdx.x == 0) {
         double sb = 0;
@@ -2499,7 +2424,7 @@ Fundido* criarFundido(Pcg* p, Arena& A) {
   // an element whatever they store
   if (p->precisao != TQ_PREC_FP32)
     for (int l = 0; l < Lc; l++) p->meia[l] = true;
-  const size_t areas = AREA_BOLHAS + AREA_TERMOS + AREA_PRODUTOS;
+  const size_t areas = AREA_BOLHAS + AREA_TERMOS;
   static_assert(areas >= WARPS * 768 * 4 && areas >= WARPS * SUAV_W * 4, "the warps' areas");
   f->smem = bytes > areas ? bytes : areas;
   f->bytesSecao = (int)bytes;
