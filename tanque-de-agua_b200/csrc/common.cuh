@@ -123,7 +123,7 @@ struct Dev {
   uint8_t* vivo;
   uint32_t *volB, *facesB, *celsB;
   long long* accB;  // fixed-point per-bubble sums
-  double *rhsB, *yB, *rb, *zb, *pb, *apb;
+  double *yB, *rb, *zb, *pb, *apb;
   // PCG vectors
   float *r, *z, *zOld, *p, *ap;
   // reductions

@@ -347,62 +347,68 @@ __device__ inline float pressaoDoAr(const Dev& d, int c, int i, int j, double dt
 // into it now minus the surface-tension term of each water face, and its cells.  The per-bubble sums
 // are 64-bit fixed point (2^-32) so their value does not depend on the order cells arrive in.  The last
 // block closes the bubbles' right-hand sides: the volume recovery term and the initial pressure.
-__global__ void __launch_bounds__(256) k_lado_direito(Dev d, double dt, double tensao, double tau, int bolhas) {
+// One round of blocks, 6 an SM at 40 registers: with a block a 256 cells and 79 registers (3 an SM) each
+// block's ticket waited for its writes, which took 15.4 us on 480x270 cells, 32 on 840x536, 150 on 9000x400
+// and 447 on 38,370x316; 13.5, 22, 62 and 142 now (three kernels for the same work: 26, 40, 80 and 207).
+constexpr int BLOCOS_LADO = 888;
+__global__ void __launch_bounds__(256, 6) k_lado_direito(Dev d, double dt, double tensao, double tau, int bolhas) {
   aposAnterior();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = d.nx, ny = d.ny;
-  static_assert(MAX_BOLHAS % (8 * 256) == 0, "the last block's batches");
-  uint32_t b = 0;
-  if (c < d.N) {
-    const int i = c % nx, j = c / nx, t0 = d.tipo[c];
-    const float qa = pressaoDoAr(d, c, i, j, dt, tensao);
-    d.qAr[c] = qa;
-    if (t0 != AGUA) {
-      d.div[c] = 0.0f;
-      d.q[c] = 0.0f;
-    } else {
-      double alvo = d.h / fmax(tau, dt);
-      double dv = (double)d.u[i + 1 + j * (nx + 1)] - (double)d.u[i + j * (nx + 1)] +
-                  (double)d.v[i + (j + 1) * nx] - (double)d.v[i + j * nx];
-      double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
-      double excesso = dens / PARTICULAS_POR_CELULA - 1;
-      if (excesso < 0) {
-        bool miolo = i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1;
-        for (int b2 = -1; b2 <= 1 && miolo; b2++)
-          for (int a = -1; a <= 1; a++) {
-            int n = i + a + (j + b2) * nx;
-            if (d.solido[n] || d.accCel[n].y == 0) { miolo = false; break; }
-          }
-        if (!miolo) excesso = 0;
-      }
-      excesso = fmin(EXCESSO_MAX, fmax(EXCESSO_MIN, excesso));
-      double ar = 0;
-      long N = d.N;
-      const int nb[4] = {c - 1, c + 1, c - nx, c + nx};  // flat neighbours, as the reference reads them
+  static_assert(MAX_BOLHAS % 256 == 0, "the last block's labels");
+  for (int c0 = blockIdx.x * blockDim.x; c0 < d.N; c0 += gridDim.x * blockDim.x) {  // (uniform over the block)
+    const int c = c0 + threadIdx.x;
+    uint32_t b = 0;
+    if (c < d.N) {
+      const int i = c % nx, j = c / nx, t0 = d.tipo[c];
+      const float qa = pressaoDoAr(d, c, i, j, dt, tensao);
+      d.qAr[c] = qa;
+      if (t0 != AGUA) {
+        d.div[c] = 0.0f;
+        d.q[c] = 0.0f;
+      } else {
+        double alvo = d.h / fmax(tau, dt);
+        double dv = (double)d.u[i + 1 + j * (nx + 1)] - (double)d.u[i + j * (nx + 1)] +
+                    (double)d.v[i + (j + 1) * nx] - (double)d.v[i + j * nx];
+        double dens = (float)d.accCel[c].x * (1.0f / 65536.0f);
+        double excesso = dens / PARTICULAS_POR_CELULA - 1;
+        if (excesso < 0) {
+          bool miolo = i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1;
+          for (int b2 = -1; b2 <= 1 && miolo; b2++)
+            for (int a = -1; a <= 1; a++) {
+              int n = i + a + (j + b2) * nx;
+              if (d.solido[n] || d.accCel[n].y == 0) { miolo = false; break; }
+            }
+          if (!miolo) excesso = 0;
+        }
+        excesso = fmin(EXCESSO_MAX, fmax(EXCESSO_MIN, excesso));
+        double ar = 0;
+        long N = d.N;
+        const int nb[4] = {c - 1, c + 1, c - nx, c + nx};  // flat neighbours, as the reference reads them
 #pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (tipoEm(d.tipo, (long)nb[k], N, AR)) ar += (double)pressaoDoAr(d, nb[k], nb[k] % nx, nb[k] / nx, dt, tensao);
-      d.div[c] = (float)(dv - alvo * excesso - ar);
-    }
-    if (bolhas && t0 == AR && i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1) {
-      const uint32_t r = d.rotulo[c];
-      if (r >= 2 && r < (uint32_t)MAX_BOLHAS) {
-        b = r;
-        double t = qa;
-        double s = 0;
-        if (d.tipo[c - 1] == AGUA) s += (double)d.u[i + j * (nx + 1)] - t;
-        if (d.tipo[c + 1] == AGUA) s += -(double)d.u[i + 1 + j * (nx + 1)] - t;
-        if (d.tipo[c - nx] == AGUA) s += (double)d.v[i + j * nx] - t;
-        if (d.tipo[c + nx] == AGUA) s += -(double)d.v[i + (j + 1) * nx] - t;
-        somaFixa(&d.accB[r], s, ESCALA_BOLHA);
+        for (int k = 0; k < 4; k++)
+          if (tipoEm(d.tipo, (long)nb[k], N, AR)) ar += (double)pressaoDoAr(d, nb[k], nb[k] % nx, nb[k] / nx, dt, tensao);
+        d.div[c] = (float)(dv - alvo * excesso - ar);
       }
+      if (bolhas && t0 == AR && i >= 1 && j >= 1 && i < nx - 1 && j < ny - 1) {
+        const uint32_t r = d.rotulo[c];
+        if (r >= 2 && r < (uint32_t)MAX_BOLHAS) {
+          b = r;
+          double t = qa;
+          double s = 0;
+          if (d.tipo[c - 1] == AGUA) s += (double)d.u[i + j * (nx + 1)] - t;
+          if (d.tipo[c + 1] == AGUA) s += -(double)d.u[i + 1 + j * (nx + 1)] - t;
+          if (d.tipo[c - nx] == AGUA) s += (double)d.v[i + j * nx] - t;
+          if (d.tipo[c + nx] == AGUA) s += -(double)d.v[i + (j + 1) * nx] - t;
+          somaFixa(&d.accB[r], s, ESCALA_BOLHA);
+        }
+      }
+    }
+    if (bolhas && __any_sync(0xffffffffu, b != 0)) {  // the cells of a bubble lie together: an atomic a warp and bubble
+      const unsigned g = __match_any_sync(0xffffffffu, b);
+      if (b && (int)(threadIdx.x & 31) == __ffs(g) - 1) atomicAdd(&d.volB[b], (unsigned)__popc(g));
     }
   }
   if (!bolhas) return;  // uniform over the grid
-  if (__any_sync(0xffffffffu, b != 0)) {  // the cells of a bubble lie together: an atomic a warp and bubble
-    const unsigned g = __match_any_sync(0xffffffffu, b);
-    if (b && (int)(threadIdx.x & 31) == __ffs(g) - 1) atomicAdd(&d.volB[b], (unsigned)__popc(g));
-  }
   __shared__ bool ultimo;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -413,36 +419,24 @@ __global__ void __launch_bounds__(256) k_lado_direito(Dev d, double dt, double t
   if (!ultimo) return;
   __threadfence();
   if (threadIdx.x == 0) d.esc->tickets[1] = 0;
-  // eight labels a thread at once, their loads before the first store: a label at a time waited for memory
-  // 16 times over (the kernel on 160x100 cells: 15 -> 11 us)
-  constexpr int K = 8;
-  for (int r0 = threadIdx.x; r0 < MAX_BOLHAS; r0 += K * blockDim.x) {
-    uint32_t vol[K];
-    long long acc[K];
-    float y[K], alvo[K], pb[K];
+  // a thread's labels all at once: a label after the other waited for memory 16 times over (the kernel on
+  // 160x100 cells: 15 -> 11 us).  What only bubbles with cells have is loaded for those alone: batches of it
+  // for every label took the kernel's registers from 40 to 79, which left an SM 3 blocks.
+  constexpr int K = MAX_BOLHAS / 256;
+  uint32_t vol[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const int r = r0 + k * blockDim.x;
-      vol[k] = r >= 2 ? __ldcg(&d.volB[r]) : 0u;
-      acc[k] = __ldcg(&d.accB[r]);
-      y[k] = d.yBolhaF[r];
-      alvo[k] = d.volumeAlvo[r];
-      pb[k] = d.pressaoBolha[r];
-    }
+  for (int k = 0; k < K; k++) vol[k] = __ldcg(&d.volB[threadIdx.x + k * 256]);
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const int r = r0 + k * blockDim.x;
-      float rhs = (float)((double)acc[k] / ESCALA_BOLHA);
-      d.volumeBolhaF[r] = (float)vol[k];
-      if (vol[k]) {
-        rhs = (float)((double)rhs + VOLTA_VOLUME_BOLHA * ((double)alvo[k] - (double)vol[k]) * d.h / dt);
-        y[k] = (float)((double)pb[k] * (dt / (DENSIDADE_AGUA * d.h)));
-        d.yBolhaF[r] = y[k];
-      }
-      d.rhsBolhaF[r] = rhs;
-      d.rhsB[r] = rhs;
-      d.yB[r] = y[k];
+  for (int k = 0; k < K; k++) {
+    const int r = threadIdx.x + k * 256;
+    float rhs = 0.0f;
+    if (vol[k]) {  // (labels 0 and 1 are counted nowhere)
+      rhs = (float)((double)__ldcg(&d.accB[r]) / ESCALA_BOLHA);
+      rhs = (float)((double)rhs + VOLTA_VOLUME_BOLHA * ((double)d.volumeAlvo[r] - (double)vol[k]) * d.h / dt);
+      d.yBolhaF[r] = (float)((double)d.pressaoBolha[r] * (dt / (DENSIDADE_AGUA * d.h)));
     }
+    d.volumeBolhaF[r] = (float)vol[k];
+    d.rhsBolhaF[r] = rhs;
   }
 }
 
@@ -576,7 +570,7 @@ void lancarSuperficie(const Dev& d, cudaStream_t s) {
 void lancarLadoDireito(const Dev& d, double dt, double tensao, double tau, bool bolhas, cudaStream_t s) {
   // accB, facesB, celsB and volB are one block of memory
   if (bolhas) cudaMemsetAsync(d.accB, 0, MAX_BOLHAS * (sizeof(long long) + 3 * sizeof(uint32_t)), s);
-  lanca(k_lado_direito, blocos(d.N, 256), 256, 0, s, d, dt, tensao, tau, bolhas ? 1 : 0);
+  lanca(k_lado_direito, min(blocos(d.N, 256), BLOCOS_LADO), 256, 0, s, d, dt, tensao, tau, bolhas ? 1 : 0);
 }
 void lancarGradiente(const Dev& d, double dt, bool ar, cudaStream_t s) {
   int m = d.nu > d.nv ? d.nu : d.nv;

@@ -47,7 +47,7 @@ struct Pcg;
 Pcg* criarPcg(int nx, int ny, int precisao, int motor, Arena& A, int ctasFundido = 0);
 bool iniciarPcg(Pcg* p, cudaStream_t s);
 void destruirPcg(Pcg* p);
-// Solves for d.q on the cells d.tipo marks as water; bubbles from d.rotulo / d.rhsB / d.yB when
+// Solves for d.q on the cells d.tipo marks as water; bubbles from d.rotulo / d.rhsBolhaF / d.yBolhaF when
 // `bolhas`; precond is TQ_PRECOND_*.  The FUSED engine queues the solve without waiting; the
 // PLAIN engine reads its stop flag every few iterations in tolerance mode.  The iteration count,
 // residual history and convergence record stay in d.esc.  Returns TQ_OK or an error status.

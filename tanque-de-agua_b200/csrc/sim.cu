@@ -333,7 +333,7 @@ static int criarSim(const tq_options* o, bool soSolver, tq_sim** out) {
   for (float** p : {&d.div, &d.q, &d.r, &d.z, &d.zOld, &d.p, &d.ap}) A.pedir(p, N);
   for (float** p : {&d.rhsBolhaF, &d.yBolhaF}) A.pedir(p, MAX_BOLHAS);
   A.pedir(&d.accB, 5 * MAX_BOLHAS / 2);  // with facesB, celsB and volB behind it (zerarBolhas)
-  for (double** p : {&d.rhsB, &d.yB, &d.rb, &d.zb, &d.pb, &d.apb}) A.pedir(p, MAX_BOLHAS);
+  for (double** p : {&d.yB, &d.rb, &d.zb, &d.pb, &d.apb}) A.pedir(p, MAX_BOLHAS);
   A.pedir(&d.parciais, 4096);
   A.pedir(&d.esc, 1);
   s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, A, o->fused_ctas);
