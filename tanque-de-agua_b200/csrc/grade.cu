@@ -128,30 +128,26 @@ __global__ void __launch_bounds__(256) k_tipos(Dev d, int faces, float gdx, floa
 // update until nothing changes reaches it whatever order the cells are visited in.  Only the
 // cells that were unlabelled air at the start of the pass ("pending") change; for a pending
 // right/upper neighbour the before-the-pass value is 0.  One CTA does both passes: the second's
-// pending cells are those of the first's list that are still unlabelled.
+// pending cells are those of the first's list that are still unlabelled.  A step before any label is known
+// has all air pending, a step of a running simulation a few cells.  All pending, no label / one cell in a
+// thousand / in ten labelled, on 480x270 cells: 118 / 4890 / 802 us with the whole list walked in the second
+// pass and each cell asked whether it is pending, 56 / 4100 / 624 now (107 / 3970 / 581 as four launches).
 __global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
   aposAnterior();
-  __shared__ int mudou;
-  const int n = d.esc->pendentes;
+  __shared__ int mudou, ficam;
+  int n = d.esc->pendentes;
   const int nx = d.nx;
   uint32_t* rot = d.rotulo;
   uint8_t* pend = d.pend;
   for (int passada = 0; passada < 2; passada++) {
-    if (passada == 1) {
-      for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int c = d.lista[t];
-        if (pend[c] && rot[c] != 0) pend[c] = 0;
-      }
-      __syncthreads();
-    }
     // Each sweep fixes at least one more cell of the longest dependency chain; n + 2 sweeps
     // always suffice.
+    bool igual = true;
     for (int volta = 0; volta < n + 2; volta++) {
       if (threadIdx.x == 0) mudou = 0;
       __syncthreads();
       for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const int c = d.lista[t];
-        if (!pend[c]) continue;
         uint32_t r = rot[c - 1];
         if (!r) r = pend[c + 1] ? 0u : rot[c + 1];
         if (!r) r = rot[c - nx];
@@ -163,8 +159,22 @@ __global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
       }
       __syncthreads();
       if (!mudou) break;
+      igual = false;
       __syncthreads();
     }
+    if (passada == 1 || igual) break;  // (a pass that changed nothing would be repeated as it was)
+    // the cells still unlabelled to the list's front, a block's worth at a time
+    if (threadIdx.x == 0) ficam = 0;
+    for (int t0 = 0; t0 < n; t0 += blockDim.x) {
+      const int t = t0 + threadIdx.x, c = t < n ? d.lista[t] : 0;
+      const bool fica = t < n && rot[c] == 0;
+      if (t < n && !fica) pend[c] = 0;
+      __syncthreads();
+      const int slot = reservar(&ficam, fica);
+      if (fica) d.lista[slot] = c;
+      __syncthreads();
+    }
+    n = ficam;
     __syncthreads();
   }
   if (threadIdx.x == 0) d.esc->pendentes = 0;
