@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(1024) k_rotulos_resolver(Dev d) {
 // for each layer, 13 us now; 840x536: 48 -> 31 us.
 constexpr int SUP_H = 13, SUP_THREADS = 512, SUP_LINHAS = 64, SUP_SEGS = SUP_THREADS / SUP_LINHAS;
 constexpr int SUP_TILES = 592;  // 4 CTAs on each of 148 SMs
+constexpr int SUP_LINHAS_MAX = 65535;  // rows of tiles in a launch's second dimension; more go to the third
 constexpr uint8_t SUP_LIVRE = 0, SUP_FUNDO = 200, SUP_FORA = 255;  // marks: no wall; wall beyond layer 3; off the grid
 
 template <int SUP_T>
@@ -209,7 +210,9 @@ __global__ void __launch_bounds__(SUP_THREADS) k_superficie(Dev d) {
   __shared__ uint8_t mk[SUP_W * SUP_P];  // SUP_LIVRE, the layer a wall cell is filled in (1-3), SUP_FUNDO, SUP_FORA
   __shared__ uint16_t lista[SUP_W * SUP_W];  // the wall cells of layers 1, 2 and 3
   __shared__ int nLista;
-  const int nx = d.nx, ny = d.ny, x0 = blockIdx.x * SUP_T - SUP_H, y0 = blockIdx.y * SUP_T - SUP_H;
+  const int nx = d.nx, ny = d.ny, x0 = blockIdx.x * SUP_T - SUP_H;
+  const int y0 = (blockIdx.y + blockIdx.z * SUP_LINHAS_MAX) * SUP_T - SUP_H;
+  if (y0 + SUP_H >= ny) return;  // (uniform over the CTA)
   if (threadIdx.x == 0) nLista = 0;
   bool parede = false;
   for (int t = threadIdx.x; t < SUP_W * SUP_W; t += SUP_THREADS) {
@@ -586,9 +589,12 @@ void lancarTipos(const Dev& d, bool faces, float gdx, float gdy, bool ar, cudaSt
 }
 void lancarPropagarRotulos(const Dev& d, cudaStream_t s) { lanca(k_rotulos_resolver, 1, 1024, 0, s, d); }
 void lancarSuperficie(const Dev& d, cudaStream_t s) {
-  const dim3 pequenos(blocos(d.nx, 16), blocos(d.ny, 16));
-  if (pequenos.x * pequenos.y <= SUP_TILES) lanca(k_superficie<16>, pequenos, SUP_THREADS, 0, s, d);
-  else lanca(k_superficie<32>, dim3(blocos(d.nx, 32), blocos(d.ny, 32)), SUP_THREADS, 0, s, d);
+  auto ladrilhos = [&](int t) {
+    const int linhas = blocos(d.ny, t);
+    return dim3(blocos(d.nx, t), min(linhas, SUP_LINHAS_MAX), blocos(linhas, SUP_LINHAS_MAX));
+  };
+  if (blocos(d.nx, 16) * blocos(d.ny, 16) <= SUP_TILES) lanca(k_superficie<16>, ladrilhos(16), SUP_THREADS, 0, s, d);
+  else lanca(k_superficie<32>, ladrilhos(32), SUP_THREADS, 0, s, d);
 }
 void lancarLadoDireito(const Dev& d, double dt, double tensao, double tau, bool bolhas, cudaStream_t s) {
   // accB, facesB, celsB and volB are one block of memory
