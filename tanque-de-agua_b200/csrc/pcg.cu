@@ -57,7 +57,7 @@ __global__ void k_plano_tipos(Dev d, uint8_t* t0, uint8_t* vizOp, int bolhas, in
 struct Niveis {
   int L;
   int nx[MAX_NIVEIS], ny[MAX_NIVEIS];
-  int ini[MAX_NIVEIS + 1];  // k_niveis_viz: first thread of each level
+  long long ini[MAX_NIVEIS + 1];  // k_niveis_viz: first thread of each level (all levels' cells may pass 2^31)
   uint8_t *tipo[MAX_NIVEIS], *viz[MAX_NIVEIS];
 };
 
@@ -101,11 +101,11 @@ __global__ void __launch_bounds__(256) k_niveis_tipos(Niveis n, int l0) {
 // face joins two non-wall fine cells (both coarse cells not wall).
 __global__ void k_niveis_viz(Niveis n, int l0, int bloco) {
   aposAnterior();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int l = l0;
   while (l < n.L && g >= n.ini[l + 1]) l++;
   if (l >= n.L) return;
-  const int c = g - n.ini[l], nx = n.nx[l], ny = n.ny[l], i = c % nx, j = c / nx;
+  const int c = (int)(g - n.ini[l]), nx = n.nx[l], ny = n.ny[l], i = c % nx, j = c / nx;
   const uint8_t* tipo = n.tipo[l];
   int m = 0;
   if (bloco && l >= 1) {
