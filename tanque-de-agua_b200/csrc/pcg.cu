@@ -556,7 +556,7 @@ __device__ inline void somasFinais(const Plano& P, int blocosTot, bool dois, dou
 
 // Level 0's masks and descriptors, the bubbles' cells (every air cell of an active label,
 // js/pressao-cpu.js:345-351), r = -div - A q on water with r.r (:331-338) and the bubbles' sums of q over
-// their water faces; q = 0 off water.  The last block lists the active bubbles and closes their rows,
+// their water faces.  The last block lists the active bubbles and closes their rows,
 // rb = rhs - (faces y - sum) (:339-341), and the initial norm.
 __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const uint8_t* vizOp, const uint8_t* tipo0,
                                                         uint8_t* viz0, double* q64) {
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const ui
   if (P.bolhas)  // (the last block writes the active labels' over these)
     for (int b = blockIdx.x * T_PCG + threadIdx.x; b < MAX_BOLHAS; b += gridDim.x * T_PCG)
       d.pb[b] = d.zb[b] = d.yB[b] = d.rb[b] = 0.0;
-  for (int c = blockIdx.x * T_PCG + threadIdx.x; c < N; c += gridDim.x * T_PCG) {
+  auto celula = [&](int c) {  // the label of the active bubble that the cell is air of, or 0
     const int nb[4] = {c - 1, c + 1, c - nx, c + nx};
     const int t = d.tipo[c], livres = vizOp[c];
     int v0 = tipo0[c] == AGUA ? 16 : 0, op = __popc(livres) << 8;
@@ -616,10 +616,14 @@ __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const ui
     }
     P.op[c] = (uint16_t)op;
     viz0[c] = (uint8_t)v0;
-    const unsigned com = __ballot_sync(__activemask(), b != 0);  // cells of one bubble lie together
-    if (b) {
-      const unsigned g = __match_any_sync(com, b);
-      if ((int)(threadIdx.x & 31) == __ffs(g) - 1) atomicAdd(&d.celsB[b], (unsigned)__popc(g));
+    return b;
+  };
+  const int lane = threadIdx.x & 31;
+  for (int c0 = blockIdx.x * T_PCG + threadIdx.x - lane; c0 < N; c0 += gridDim.x * T_PCG) {  // a warp's trips are the same
+    const uint32_t b = c0 + lane < N ? celula(c0 + lane) : 0u;
+    if (__any_sync(0xffffffffu, b != 0)) {  // cells of one bubble lie together
+      const unsigned g = __match_any_sync(0xffffffffu, b);
+      if (b && lane == __ffs(g) - 1) atomicAdd(&d.celsB[b], (unsigned)__popc(g));
     }
   }
   if (!ultimoBloco(d, P, blockIdx.x, gridDim.x, s, 0, false, sh)) return;
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(T_PCG) k_plano_inicio(Dev d, Plano P, const ui
     constexpr int K = MAX_BOLHAS / T_PCG, W = T_PCG / 32;
     static_assert(K * W <= T_PCG, "a count a thread");
     __shared__ int pref[K * W + 1];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int w = threadIdx.x >> 5;
     unsigned at[K];
 #pragma unroll
     for (int k = 0; k < K; k++) at[k] = __ldcg(&d.facesB[k * T_PCG + threadIdx.x]);
