@@ -435,6 +435,8 @@ __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
   float* bs = xs + N;
   uint8_t* vs = (uint8_t*)(bs + N);
   const uint8_t* viz = n.viz;
+  // in global memory a 16-bit level sweeps in its free array, which has room for FP32
+  float* xg = sizeof(T) == 4 ? (float*)n.x : (float*)n.tmp;
   if (emShared)
     for (int c = threadIdx.x; c < N; c += blockDim.x) {
       xs[c] = 0.0f;
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
       vs[c] = viz[c];
     }
   else
-    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = guardar<T>(0.0f);
+    for (int c = threadIdx.x; c < N; c += blockDim.x) xg[c] = 0.0f;
   __syncthreads();
   for (int h = 0; h <= VARREDURAS_GROSSO; h++) {
     const int cor = h & 1;
@@ -452,7 +454,7 @@ __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
       if (!(vz & 16) || ((i + j + 1) & 1) != cor) continue;
       int q = __popc(vz & 15);
       if (!q) continue;
-      auto x = [&](int k) { return emShared ? xs[k] : carregar(n.x[k]); };
+      auto x = [&](int k) { return emShared ? xs[k] : xg[k]; };
       float s = 0.0f;
       if (vz & 1) s += x(c - 1);
       if (vz & 2) s += x(c + 1);
@@ -460,12 +462,12 @@ __global__ void __launch_bounds__(1024) k_grosso(NivelDev<T> n, int emShared) {
       if (vz & 8) s += x(c + nx);
       const float r = dividirViz(s + (emShared ? bs[c] : carregar(n.b[c])), (float)q, inversoVizinhos(q));
       if (emShared) xs[c] = r;
-      else n.x[c] = guardar<T>(r);
+      else xg[c] = r;
     }
     __syncthreads();
   }
-  if (emShared)
-    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = guardar<T>(xs[c]);
+  if (emShared || sizeof(T) == 2)
+    for (int c = threadIdx.x; c < N; c += blockDim.x) n.x[c] = guardar<T>(emShared ? xs[c] : xg[c]);
 }
 
 // ---------------------------------------------------------------- PCG kernels
