@@ -338,8 +338,15 @@ static int criarSim(const tq_options* o, bool soSolver, tq_sim** out) {
   A.pedir(&d.esc, 1);
   s->pcg = criarPcg(s->nx, s->ny, o->precision, o->engine, A, o->fused_ctas);
   if (!soSolver) s->ar = criarRastreador(s->nx, s->ny, A);
-  if (!A.reservar(s->s) || !iniciarPcg(s->pcg, s->s)) {
+  const bool reservada = A.reservar(s->s);
+  if (!reservada || !iniciarPcg(s->pcg, s->s)) {
+    const bool fundido = motorPcg(s->pcg) == TQ_ENGINE_FUSED;
     tq_destroy(s);
+    if (!reservada && fundido) {  // the plain engine takes less
+      tq_options simples = *o;
+      simples.engine = TQ_ENGINE_PLAIN;
+      return criarSim(&simples, soSolver, out);
+    }
     return falha(TQ_E_NOMEM, "device allocation failed");
   }
   d.sdf = sdf;
