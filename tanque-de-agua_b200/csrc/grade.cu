@@ -54,12 +54,14 @@ __global__ void k_tracar(float* sdf, int mw, int mh, int x0, int y0, int nbx, in
   sdf[k] = (float)v;
 }
 
-// Cena#zerar (js/cena.js:139-144): the mask of an empty tank, the frame alone.
-__global__ void k_zerar_mascara(float* sdf, int mw, int mh) {
+// Cena#zerar (js/cena.js:139-144): the mask of an empty tank, the frame alone.  One round of blocks, several
+// points a thread: a block's wait for the kernel before costs more than its points (a call on 7,221x316 cells took
+// 63 us with a point a thread, 47 now).
+constexpr int BLOCOS_ZERAR = 1184;  // 8 a SM
+__global__ void __launch_bounds__(256) k_zerar_mascara(float* sdf, int mw, int mh) {
   aposAnterior();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= mw * mh) return;
-  sdf[idx] = (float)molduraMascara(idx % mw, idx / mw, mw, mh);
+  for (int idx = blockIdx.x * 256 + threadIdx.x; idx < mw * mh; idx += gridDim.x * 256)
+    sdf[idx] = (float)molduraMascara(idx % mw, idx / mw, mw, mh);
 }
 
 // Adds 1 to *cont for every lane with `sim` and returns the lane's slot: one atomic a warp.
@@ -581,7 +583,7 @@ void lancarTracar(const Dev& d, double x0m, double y0m, double x1m, double y1m, 
         dx * dx + dy * dy, rp, apagar ? 1 : 0);
 }
 void lancarZerarMascara(const Dev& d, cudaStream_t s) {
-  lanca(k_zerar_mascara, blocos(d.mw * d.mh, 256), 256, 0, s, (float*)d.sdf, d.mw, d.mh);
+  lanca(k_zerar_mascara, min(blocos(d.mw * d.mh, 256), BLOCOS_ZERAR), 256, 0, s, (float*)d.sdf, d.mw, d.mh);
 }
 void lancarTipos(const Dev& d, bool faces, float gdx, float gdy, bool ar, cudaStream_t s) {
   const int m = !faces ? d.N : d.nu > d.nv ? d.nu : d.nv;
