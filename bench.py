@@ -343,8 +343,7 @@ def executar_gpu(args, rank, mundo, dist):
 
     def particulas_gbs(res, n, pico):
         """Particle bytes per second of the P2G and G2P stages (BYTES_PARTICULA x particles over
-        the stage's device time per substep); the P2G stage also zeroes the sums and computes
-        the face velocities."""
+        the stage's device time per substep); the P2G stage also zeroes the sums."""
         et = res["etapas"]
         n_sub = max(et["subpassos"], 1)
         out = {"bytes_per_particle": BYTES_PARTICULA, "particles": n}

@@ -321,9 +321,9 @@ int tq_get_stream(tq_sim* s, void** stream);
 
 /* Stage timing with CUDA events on the handle's stream.  tq_set_timing(1) starts (and resets)
  * the accumulation; tq_get_timing returns 11 values accumulated since then:
- * [0..6] ms in p2g+faces, cell flags+labels, surface, divergence+bubbles, pressure solve,
- * gradient+extrapolation, g2p; [7] ms in air relabels; [8] substeps timed; [9] pressure
- * iterations in total; [10] relabels timed. */
+ * [0..6] ms in p2g, cell flags+face velocities+labels, surface, air pressure+divergence+bubbles,
+ * pressure solve, air and bubble pressures after it+gradient+extrapolation, g2p; [7] ms in air
+ * relabels; [8] substeps timed; [9] pressure iterations in total; [10] relabels timed. */
 int tq_set_timing(tq_sim* s, int32_t enabled);
 int tq_get_timing(tq_sim* s, double* ms_out, int32_t cap, int32_t* n);
 

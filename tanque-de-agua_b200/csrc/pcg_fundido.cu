@@ -1560,7 +1560,8 @@ __device__ __noinline__ void secaoGrossa(const Args& a, unsigned char* smem, uns
       const int r = __ldcg(a.wInv + c);
       if (r >= 0) a.mSecao[(size_t)r * nW + coluna] = F[t.xa + c];
     }
-  }  sincEquipe(eq);  // the next column rewrites the table and the arrays
+  }
+  sincEquipe(eq);  // the next column rewrites the table and the arrays
 }
 
 // x of level Lc = M b over its water cells, every CTA staging b in shared memory and each warp
@@ -2420,7 +2421,7 @@ Fundido* criarFundido(Pcg* p, Arena& A) {
   }
   f->Lc = Lc;
   // 16-bit storage on every grid level below the coarse section (the smallest included), so the
-  // kernel's passes exist in one storage type only (faseSuavizar); the level buffers hold 4 bytes
+  // kernel's passes exist in one storage type only (faseSuavizarT); the level buffers hold 4 bytes
   // an element whatever they store
   if (p->precisao != TQ_PREC_FP32)
     for (int l = 0; l < Lc; l++) p->meia[l] = true;

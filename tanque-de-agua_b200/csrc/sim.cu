@@ -966,9 +966,9 @@ int tq_set_timing(tq_sim* s, int32_t on) {
   return TQ_OK;
 }
 
-// Accumulated stage times since tq_set_timing (ms): [0..6] p2g+faces, flags+labels, surface,
-// divergence+bubbles, pressure solve, gradient+extrapolation, g2p; [7] air relabels;
-// [8] substeps timed; [9] pressure iterations in total; [10] relabels timed.
+// Accumulated stage times since tq_set_timing (ms): [0..6] p2g, flags+faces+labels, surface,
+// air pressure+divergence+bubbles, pressure solve, air and bubble pressures+gradient+extrapolation,
+// g2p; [7] air relabels; [8] substeps timed; [9] pressure iterations in total; [10] relabels timed.
 int tq_get_timing(tq_sim* s, double* ms, int32_t cap, int32_t* n) {
   if (!s) return falha(TQ_E_ARG, "null handle");
   double v[11] = {0};
