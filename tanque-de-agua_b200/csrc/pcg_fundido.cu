@@ -1680,11 +1680,10 @@ constexpr int KDA = 4;  // cells a thread and batch of [DA], [B] and the true re
 // (areas), put there by the warps that do not sum.
 // z and p come through L1: they were last written before the grid barrier that opens this phase,
 // whose acquire orders these loads after those writes.
-// Measured, [DA] / [B] a phase, against four consecutive cells a thread whose products the CTA passed on
-// through shared memory: 480x270 cells 6.0 / 4.9 -> 5.9 / 4.1 us, 840x536 9.0 / 6.9 -> 8.2 / 5.0,
-// 7,221x316 40 / 31 -> 28 / 18, 38,370x316 217 / 166 -> 119 / 83 (an iteration 984 -> 807).  Direct loads of the left
-// and right neighbours: 126 us on the last, 8.5 on 840x536; the lines of the next batch ahead as well: 122
-// and 8.7.
+// Measured, [DA] / [B] a phase with its barrier (FP16), against four consecutive cells a thread whose products the CTA
+// passed on through shared memory: 840x536 cells 10.8 / 8.0 -> 9.4 / 6.0 us, 38,370x316 222 / 169 -> 123 / 86 (an
+// iteration 1,005 -> 822).  Direct loads of the left and right neighbours took 7 us more on the last and 0.3 on
+// 840x536; the lines of the next batch ahead as well 3 and 0.5.
 __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const float* pv, float* pn, bool prim, int nAt,
                                        const double* pbVelho, double* pbNovo, const double* zbOld, double* zbCur,
                                        double& rz, double* sh, float* areas) {
