@@ -1681,8 +1681,8 @@ constexpr int KDA = 4;  // cells a thread and batch of [DA], [B] and the true re
 // z and p come through L1: they were last written before the grid barrier that opens this phase,
 // whose acquire orders these loads after those writes.
 // Measured, [DA] / [B] a phase with its barrier (FP16), against four consecutive cells a thread whose products the CTA
-// passed on through shared memory: 840x536 cells 10.8 / 8.0 -> 9.4 / 6.0 us, 38,370x316 222 / 169 -> 123 / 86 (an
-// iteration 1,005 -> 822).  Direct loads of the left and right neighbours took 7 us more on the last and 0.3 on
+// passed on through shared memory: 840x536 cells 10.8 / 8.0 -> 8.4 / 6.0 us, 38,370x316 222 / 169 -> 100 / 84 (an
+// iteration 1,005 -> 784).  Direct loads of the left and right neighbours took 7 us more on the last and 0.3 on
 // 840x536; the lines of the next batch ahead as well 3 and 0.5.
 __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const float* pv, float* pn, bool prim, int nAt,
                                        const double* pbVelho, double* pbNovo, const double* zbOld, double* zbCur,
@@ -1721,7 +1721,8 @@ __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const flo
   float z[KDA][3], w[KDA][3], zl[KDA], wl[KDA];
   // a batch's cells, those below and above (an index across a row's end reads a value that no flag selects),
   // and one beside the cell: lane 31's to the right, the others' to the left (of which lane 0's counts; a
-  // branch would wait for its load)
+  // branch would wait for its load).  The first iteration loads the previous p as well and leaves it out: behind
+  // a branch those loads waited for the ones before it (120 against 100 us on 38,370x316 cells)
   auto ler = [&](int c0) {
 #pragma unroll
     for (int k = 0; k < KDA; k++) m[k] = c0 + k * GT < N ? __ldca(a.op + c0 + k * GT) : 0;
@@ -1733,15 +1734,14 @@ __device__ __forceinline__ void faseDA(const Args& a, const float* zc, const flo
       z[k][2] = __ldca(zc + (c < N - nx ? c + nx : c));
       zl[k] = __ldca(zc + (lane == 31 ? min(c + 1, N - 1) : max(c - 1, 0)));
     }
-    if (!prim)
 #pragma unroll
-      for (int k = 0; k < KDA; k++) {
-        const int c = c0 + k * GT < N ? c0 + k * GT : 0;
-        w[k][0] = __ldca(pv + c);
-        w[k][1] = __ldca(pv + (c >= nx ? c - nx : c));
-        w[k][2] = __ldca(pv + (c < N - nx ? c + nx : c));
-        wl[k] = __ldca(pv + (lane == 31 ? min(c + 1, N - 1) : max(c - 1, 0)));
-      }
+    for (int k = 0; k < KDA; k++) {
+      const int c = c0 + k * GT < N ? c0 + k * GT : 0;
+      w[k][0] = __ldca(pv + c);
+      w[k][1] = __ldca(pv + (c >= nx ? c - nx : c));
+      w[k][2] = __ldca(pv + (c < N - nx ? c + nx : c));
+      wl[k] = __ldca(pv + (lane == 31 ? min(c + 1, N - 1) : max(c - 1, 0)));
+    }
   };
   float betaf = 0.0f;
   auto fazer = [&](int c0) {
