@@ -63,7 +63,7 @@ BYTES_SETUP_BLOCO = {"fp32": 101.3, "fp16": 80.3, "bf16": 80.3}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one fused FP16 solve of this
 # scene with TQ_PRECOND_BLOCK_1, from one ncu capture of the kernel: the solve's working set
 # stays in L2.
-TRAFEGO_SOLVE_BYTES = 30_469_376
+TRAFEGO_SOLVE_BYTES = 19_536_128
 # Particle bytes a substep's particle kernels move per particle: P2G reads its three float4
 # records (position/velocity, affine terms, foam/dye); G2P reads the first and third and
 # writes all three.  The grid reads behind them are cached (L1/L2) and not counted.
